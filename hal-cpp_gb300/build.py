@@ -31,7 +31,7 @@ NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xco
                   "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr", "-I", INCLUDE, "-I", CSRC]
 
 SOURCES = ["core.cu", "diffusion.cu", "adi.cu", "adi_plan.cpp", "agents.cu", "wells.cu", "adjoint.cu", "pde_io.cpp",
-           "tick_blocked.cu", "pdegrid.cu"]
+           "tick_blocked.cu", "tick_patch.cu", "pdegrid.cu"]
 
 
 def _nvcc():

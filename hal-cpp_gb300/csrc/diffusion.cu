@@ -486,6 +486,21 @@ namespace halcuda
         }
     }
 
+    namespace
+    {
+        // A[cell] = value for every point source (no cell twice).
+        __global__ void ScatterPoints(float *__restrict__ A, const int32_t *__restrict__ row,
+                                      const int32_t *__restrict__ col, const float *__restrict__ val, int32_t n,
+                                      int32_t yDim)
+        {
+            const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+            if (k < n)
+            {
+                A[static_cast<int64_t>(row[k]) * yDim + col[k]] = val[k];
+            }
+        }
+    }
+
     int LaunchTickTiles(const TickParams *table, const int4 *tiles, int32_t nTiles, int vec, cudaStream_t s)
     {
         if (nTiles <= 0)
@@ -525,12 +540,19 @@ namespace halcuda
         const hal_cuda_agents *agents = nullptr;
         double uptake = 0.0;
         int32_t nPoints = 0;
-        // Temporal blocking: ticks per launch 1 or 2 (0 = automatic, which
-        // is 1).  The two-tick kernel stages tiles with a tensor map per field
-        // buffer and reads the dense source and the point sources summed into
-        // one array.  Measured on GB300 it is slower at every size (2048^2:
-        // 12.0 vs 7.1 us per tick; 8192^2: 165 vs 94 us, where one tick per
-        // launch already streams at 84% of HBM peak), so it is opt-in.
+        // Several ticks per launch (tick_patch.cu): the point sources as an
+        // array of the grid and the patches that hold one (when no cell is
+        // listed twice; otherwise one tick runs per launch).
+        TickPatchShape patch;
+        DevBuf<float> patchPts;
+        DevBuf<uint8_t> patchFlags;
+        bool patchPtsOk = false;
+        // Temporal blocking through shared memory: ticks per launch 1 or 2 (0
+        // = automatic, which never takes it).  The two-tick kernel stages
+        // tiles with a tensor map per field buffer and reads the dense source
+        // and the point sources summed into one array.  Measured on GB300 it
+        // is slower than one tick per launch at every size (2048^2: 12.0 vs
+        // 7.1 us per tick; 8192^2: 165 vs 94 us), so it is opt-in.
         int32_t blockMode = 0;
         TickBlockTensorMap tmap[2];
         bool tmapOk = false;
@@ -570,6 +592,7 @@ namespace halcuda
             block = dim3(32, kTickWarps);
             grid = dim3((yDim + 32 * vec - 1) / (32 * vec),
                         (xDim + kTickWarps * kTickRowsPerThread - 1) / (kTickWarps * kTickRowsPerThread));
+            patch = TickPatchShapeFor(xDim, yDim);
             tmapOk = vec4 && MakeTickBlockTensorMap(tmap[0], field[0].p, xDim, yDim) &&
                      MakeTickBlockTensorMap(tmap[1], field[1].p, xDim, yDim);
             if (tmapOk)
@@ -586,6 +609,102 @@ namespace halcuda
         bool UseBlocked(int32_t ticks) const
         {
             return tmapOk && ticks >= 2 && blockMode == 2 && agents == nullptr;
+        }
+
+        // Several ticks per launch wherever the patch kernel takes the run: it
+        // has no uptake term, and its point sources no repeated cells.
+        bool UsePatch(int32_t ticks, bool useExtras) const
+        {
+            return patch.windows > 0 && ticks >= 2 && blockMode == 0 && agents == nullptr &&
+                   !(useExtras && hasPoints && !patchPtsOk);
+        }
+
+        // Point sources of the patch kernel: scatters them into an array of
+        // the grid and flags the patches that read each one (the wrapped
+        // columns and rows of the edge patches included).
+        int SetPatchPoints(int32_t n, const int32_t *cells)
+        {
+            patchPtsOk = false;
+            if (patch.windows == 0)
+            {
+                return HAL_CUDA_OK;
+            }
+            std::vector<int32_t> sorted(cells, cells + n);
+            std::sort(sorted.begin(), sorted.end());
+            if (std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end())
+            {
+                return HAL_CUDA_OK;
+            }
+            const auto cover = [](int32_t count, int32_t len, int32_t halo, int32_t dim)
+            {
+                std::vector<std::vector<int32_t>> by(static_cast<size_t>(dim));
+                for (int32_t i = 0; i < count; i++)
+                {
+                    const int32_t at = TickPatchStart(i, count, len, halo, dim) - halo;
+                    for (int32_t c = at; c < at + len + 2 * halo; c++)
+                    {
+                        by[static_cast<size_t>(c < 0 ? c + dim : (c >= dim ? c - dim : c))].push_back(i);
+                    }
+                }
+                return by;
+            };
+            const auto cols = cover(patch.windows, patch.cols, patch.haloCols, yDim);
+            const auto rows = cover(patch.strips, patch.rows, patch.halo, xDim);
+            std::vector<uint8_t> flags(static_cast<size_t>(patch.windows) * patch.strips, 0);
+            for (const int32_t c : sorted)
+            {
+                for (const int32_t st : rows[static_cast<size_t>(c / yDim)])
+                {
+                    for (const int32_t w : cols[static_cast<size_t>(c % yDim)])
+                    {
+                        flags[static_cast<size_t>(st) * patch.windows + w] = 1;
+                    }
+                }
+            }
+            cudaStream_t s = stream.Get();
+            HAL_TRY(CudaStatus(cudaStreamSynchronize(s), "point sources"));
+            if (patchPts.p == nullptr)
+            {
+                HAL_TRY(patchPts.Alloc(Length(), "cudaMalloc(points)"));
+                HAL_TRY(patchFlags.Alloc(flags.size(), "cudaMalloc(points)"));
+            }
+            HAL_TRY(CudaStatus(cudaMemsetAsync(patchPts.p, 0, Length() * sizeof(float), s), "point sources"));
+            ScatterPoints<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(patchPts.p, ptRow.p, ptCol.p, ptVal.p, n,
+                                                                                yDim);
+            CountLaunch();
+            HAL_TRY(LaunchStatus("point sources"));
+            HAL_TRY(CudaStatus(cudaMemcpyAsync(patchFlags.p, flags.data(), flags.size(), cudaMemcpyHostToDevice, s),
+                               "point sources"));
+            // the array is complete before the call returns, whichever stream
+            // the ticks are put on later
+            HAL_TRY(CudaStatus(cudaStreamSynchronize(s), "point sources"));
+            patchPtsOk = true;
+            return HAL_CUDA_OK;
+        }
+
+        TickPatchParams PatchParams(const TickParams &t) const
+        {
+            TickPatchParams q;
+            q.f = t.f;
+            q.out = t.out;
+            q.xDim = t.xDim;
+            q.yDim = t.yDim;
+            q.r = t.r;
+            q.negDecay = t.negDecay;
+            q.wrapX = t.wrapX;
+            q.wrapY = t.wrapY;
+            q.src = t.src;
+            q.pts = t.ptStart != nullptr ? patchPts.p : nullptr;
+            q.flags = t.ptStart != nullptr ? patchFlags.p : nullptr;
+            q.ghost = t.ghost;
+            q.kUp = t.kUp;
+            q.kDn = t.kDn;
+            q.kYm = t.kYm;
+            q.kYp = t.kYp;
+            q.ticks = 1;
+            q.windows = 0;
+            q.strips = 0;
+            return q;
         }
 
         // The dense source plus the point sources as one array (null if
@@ -688,8 +807,8 @@ namespace halcuda
             return u;
         }
 
-        // One tick, launched with programmatic stream serialization (the
-        // kernel's griddepcontrol.wait keeps the ticks ordered): 6.55 against
+        // One tick (runs that the patch kernel does not take), launched with
+        // programmatic stream serialization (the kernel's griddepcontrol.wait keeps the ticks ordered): 6.55 against
         // 6.70 us per 2048^2 tick in a graph, bit-identical fields.
         void LaunchTick(const TickParams &p, const TickUptake &up, cudaStream_t s) const
         {
@@ -756,12 +875,16 @@ namespace halcuda
             {
                 HAL_TRY(CombinedSource(extras, &S, s));
             }
+            const bool patched = !blocked && UsePatch(ticks, extras);
             // launches: two ticks each when blocked (plus one single tick
-            // for an odd count); each launch flips the buffers
-            const int32_t launches = blocked ? ticks / 2 + (ticks & 1) : ticks;
+            // for an odd count), up to the shape's halo when patched; each
+            // launch flips the buffers
+            const int32_t launches = blocked   ? ticks / 2 + (ticks & 1)
+                                     : patched ? ticks / patch.halo + (ticks % patch.halo != 0 ? 1 : 0)
+                                               : ticks;
             char key[256];
             snprintf(key, sizeof(key), "%d|%a|%a|%d|%d|%d|%d|%d|%d|%a|%a|%d|%p|%p|%a|%u|%u", ticks, r, decay, wrapX,
-                     wrapY, extras ? 1 : 0, hasSrc, hasPoints, hasGhost, xVel, yVel, blocked ? 1 : 0,
+                     wrapY, extras ? 1 : 0, hasSrc, hasPoints, hasGhost, xVel, yVel, blocked ? 1 : (patched ? 2 : 0),
                      static_cast<void *>(s), static_cast<const void *>(agents), uptake, testExtraTx, testWaitUs);
             GraphCache &graph = this->graph[cur];
             if (graph.exec == nullptr || graph.key != key)
@@ -781,13 +904,31 @@ namespace halcuda
                         c ^= 1;
                     }
                 }
-                for (; t < ticks; t++)
+                int rc = HAL_CUDA_OK;
+                for (; patched && t < ticks && rc == HAL_CUDA_OK; t += patch.halo)
+                {
+                    const TickParams p = Params(field[c].p, field[c ^ 1].p, r, decay, wrapX, wrapY, extras);
+                    TickPatchParams q = PatchParams(p);
+                    q.ticks = std::min(patch.halo, ticks - t);
+                    const bool adv = p.kUp != p.r || p.kDn != p.r || p.kYm != p.r || p.kYp != p.r;
+                    rc = LaunchTickPatch(patch, q, adv, s);
+                    c ^= 1;
+                }
+                for (; !patched && t < ticks; t++)
                 {
                     TickParams p = Params(field[c].p, field[c ^ 1].p, r, decay, wrapX, wrapY, extras);
                     LaunchTick(p, Uptake(extras), s);
                     c ^= 1;
                 }
                 cudaError_t e = cudaStreamEndCapture(s, &g);
+                if (rc != HAL_CUDA_OK)
+                {
+                    if (g != nullptr)
+                    {
+                        cudaGraphDestroy(g);
+                    }
+                    return rc;
+                }
                 HAL_TRY(CudaStatus(e, "cudaStreamEndCapture"));
                 e = cudaGraphInstantiate(&graph.exec, g, 0);
                 cudaGraphDestroy(g);
@@ -1220,7 +1361,7 @@ extern "C" int hal_cuda_diffusion_set_point_sources(hal_cuda_diffusion *h, int32
                                 "cudaMemcpy(points)"));
     h->hasPoints = true;
     h->nPoints = nPoints;
-    return HAL_CUDA_OK;
+    return h->SetPatchPoints(nPoints, cells);
 }
 
 extern "C" int hal_cuda_diffusion_set_uptake(hal_cuda_diffusion *h, hal_cuda_agents *agents, double uptake)

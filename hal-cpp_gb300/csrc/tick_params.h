@@ -83,4 +83,42 @@ namespace halcuda
     bool MakeTickBlockTensorMap(TickBlockTensorMap &map, const float *field, int32_t xDim, int32_t yDim);
     int PrepareTickBlocked();
     void LaunchTickBlocked2(const TickBlockParams &p, const TickBlockTensorMap &map, cudaStream_t s);
+
+    // ---- several ticks per launch, in registers (tick_patch.cu) -----------
+    struct TickPatchParams
+    {
+        const float *f;
+        float *out;
+        int32_t xDim, yDim;
+        float r, negDecay;
+        int32_t wrapX, wrapY;
+        const float *src;          // dense source or null
+        const float *pts;          // point sources as an array of the grid, or null
+        const uint8_t *flags;      // with pts: windows * strips, 1 where a patch holds one
+        GhostView ghost;           // all null for zero-flux
+        float kUp, kDn, kYm, kYp;  // per-side weights when advecting (see TickParams)
+        int32_t ticks;             // 1 .. the shape's halo
+        int32_t windows, strips;   // set by LaunchTickPatch
+    };
+
+    // A warp's patch of 32 * vec columns x patchRows rows stores cols x rows
+    // cells after at most `halo` ticks.  windows == 0: the grid is too small
+    // for a patch.
+    struct TickPatchShape
+    {
+        int32_t vec = 0, patchRows = 0, halo = 0, haloCols = 0, cols = 0, rows = 0;
+        int32_t windows = 0, strips = 0;
+    };
+
+    // First stored column (row) of window (strip) i of n: the last one ends at
+    // the grid's edge and no other one's halo reaches beyond it.
+    __host__ __device__ inline int32_t TickPatchStart(int32_t i, int32_t n, int32_t len, int32_t halo, int32_t dim)
+    {
+        const int32_t most = dim - len - (i < n - 1 ? halo : 0);
+        const int32_t at = i * len;
+        return at < most ? at : most;
+    }
+
+    TickPatchShape TickPatchShapeFor(int32_t xDim, int32_t yDim);
+    int LaunchTickPatch(const TickPatchShape &shape, TickPatchParams &p, bool adv, cudaStream_t s);
 }

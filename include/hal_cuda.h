@@ -156,15 +156,16 @@ int hal_cuda_diffusion_set_dirichlet(hal_cuda_diffusion *h, const float *ghost);
  * coupling.  Coupled ticks run one per launch. */
 int hal_cuda_diffusion_set_uptake(hal_cuda_diffusion *h, hal_cuda_agents *agents, double uptake);
 
-/* Ticks per launch of the resident explicit tick: 1, 2 (temporal blocking:
- * a CTA stages its tile with a 2-cell halo by TMA and computes two ticks in
- * shared memory, so a pair of ticks reads and writes the field once), or 0
- * (the default: 1, which measures faster on GB300 at every size -- the
- * one-tick kernel streams large fields at over 80% of HBM peak, and the
- * two-tick kernel spends more instructions per cell than it saves in
- * bytes).  Two ticks need yDim % 4 == 0 (ENOTSUP otherwise).  With 2 the
- * dense source and the point sources are added as one pre-summed array, so
- * results match the one-tick launches to FP32 rounding, not bit for bit. */
+/* Ticks per launch of the resident explicit tick: 0 (the default) lets the
+ * library choose: up to 8 ticks of a patch in registers per launch, bit for
+ * bit the one-tick results (measured 7.4x faster at 256^2 and 1.9x to 2.4x at
+ * 2048^2), and one tick per launch where a run has agent uptake, a point
+ * source listed twice in a cell, or a grid smaller than a patch.  1: always
+ * one tick per launch.  2: a CTA stages its tile with a 2-cell halo by TMA
+ * and computes two ticks in shared memory (slower than both; needs yDim % 4
+ * == 0, ENOTSUP otherwise; the dense source and the point sources are added
+ * as one pre-summed array, so results match the others to FP32 rounding, not
+ * bit for bit). */
 int hal_cuda_diffusion_set_blocking(hal_cuda_diffusion *h, int32_t ticksPerLaunch);
 
 /* Uniform advection velocity of every following tick (PDEGrid2D::Advection
