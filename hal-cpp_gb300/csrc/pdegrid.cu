@@ -329,6 +329,13 @@ namespace halcuda
             int32_t L;
             int32_t periodic;
             int32_t fastDiv;     // every bs[i] in [2^-20, 2^20]: DivByPlan is exact
+            // split solve (below): segments per line (1: not split), elements
+            // per segment, the back substitution's multipliers off / bs[i]
+            // negated, and each segment's products of the negated ws and of g
+            int32_t segs, segLen;
+            const double *g;
+            const double *segP;
+            const double *segQ;
         };
 
         // ExplicitDiffusionY2ADI / X2ADI (src/Pde/ADIequations.cpp:19-47 and
@@ -598,6 +605,389 @@ namespace halcuda
             }
         }
 
+        // ---- the same solve, each line split into segments ------------------
+        // One thread per line is one dependent FP64 chain of 2 + 5
+        // instructions per element, 64 cycles each: 580 us for 2048 lines of
+        // 2048 on 64 warps, while the chip could issue from 608.  Split into
+        // segments, the chains of a line run side by side and still give the
+        // serial chain's bits:
+        //   1. AdiSegEnds: every segment's elimination from a zero start (one
+        //      FMA per element).  With the segments' products of -ws, which
+        //      the plan holds, these give every segment's incoming value to
+        //      within a few ulps (a relative error also where the solution
+        //      decays along the line: sums of one sign do not cancel);
+        //   2. AdiSegElim: the elimination in the reference's operations from
+        //      that value.  The recurrence contracts (|ws| < 1), so two
+        //      trajectories a few ulps apart round to the same value after
+        //      some tens of elements and are one from there on;
+        //   3. AdiSegFix: from the end of the segment before, which has met
+        //      the serial trajectory by then, the elements again until one
+        //      comes out bit-equal to what is stored: from there the segment
+        //      is the serial one.  A segment that ends without such a meeting
+        //      marks its line.  Then the back substitution's segments from a
+        //      zero start, as in 1;
+        //   4. AdiSegBack and AdiSegBackFix: the same for the back
+        //      substitution;
+        //   5. AdiSegFinish: solves a marked line again serially.
+        // Every element is thus either checked against the serial recurrence
+        // or follows from one that was: equality is bitwise, so zeros' signs,
+        // infinities and NaN end in a marked line at worst.
+        // 2048 lines of 2048: 122 us in all (19 segments a line; FP64 issue needs
+        // 79 us for the ten operations per element), 580 us as one chain a line.
+
+        // e[i] = d[i] - ws[i] * e[i - 1] over elements [a, b) of a line, from
+        // prev (unused at i = 0), in the reference's operations; returns the
+        // last value.  at(i): the element's offset.
+        template <typename At>
+        __device__ __forceinline__ double ElimRun(const double *__restrict__ d, double *__restrict__ e,
+                                                  const LinePlan64Dev &pl, int32_t a, int32_t b, double prev, At at)
+        {
+            double rc[kChainFwd], wc[kChainFwd];
+#pragma unroll
+            for (int k = 0; k < kChainFwd; k++)
+            {
+                const int32_t i = min(a + k, b - 1);
+                rc[k] = __ldcg(d + at(i));
+                wc[k] = __ldg(pl.ws + i);
+            }
+            for (int32_t i0 = a; i0 < b; i0 += kChainFwd)
+            {
+                double rn[kChainFwd], wn[kChainFwd];
+#pragma unroll
+                for (int k = 0; k < kChainFwd; k++)
+                {
+                    const int32_t i = min(i0 + kChainFwd + k, b - 1);
+                    rn[k] = __ldcg(d + at(i));
+                    wn[k] = __ldg(pl.ws + i);
+                }
+#pragma unroll
+                for (int k = 0; k < kChainFwd; k++)
+                {
+                    const int32_t i = i0 + k;
+                    if (i < b)
+                    {
+                        prev = (i == 0) ? rc[k] : __dsub_rn(rc[k], __dmul_rn(wc[k], prev));
+                        e[at(i)] = prev;
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kChainFwd; k++)
+                {
+                    rc[k] = rn[k];
+                    wc[k] = wn[k];
+                }
+            }
+            return prev;
+        }
+
+        // The exact quotient num / bs[i] for any numerator.
+        __device__ __forceinline__ double DivExact(double num, double2 bh, int2 lo)
+        {
+            return PlanDivisionOutOfRange(num) ? __ddiv_rn(num, bh.x) : DivByPlan(num, bh, lo);
+        }
+
+        // x[i] = (e[i] - off * x[i + 1]) / bs[i] over [a, b) downwards, from x
+        // (unused at i = L - 1), in the reference's operations; returns x[a].
+        // A numerator outside DivByPlan's range has the segment run again.
+        template <typename At>
+        __device__ __forceinline__ double BackRun(const double *__restrict__ e, double *__restrict__ out,
+                                                  const LinePlan64Dev &pl, int32_t a, int32_t b, double x, At at)
+        {
+            const double x0 = x;
+            uint32_t redo = 0;
+            double dc[kChainBwd];
+            double2 bc[kChainBwd];
+            int2 lc[kChainBwd];
+#pragma unroll
+            for (int k = 0; k < kChainBwd; k++)
+            {
+                const int32_t i = max(b - 1 - k, a);
+                dc[k] = __ldcg(e + at(i));
+                bc[k] = __ldg(pl.bh + i);
+                lc[k] = __ldg(pl.lo + i);
+            }
+            for (int32_t i0 = b - 1; i0 >= a; i0 -= kChainBwd)
+            {
+                double dn[kChainBwd];
+                double2 bn[kChainBwd];
+                int2 ln[kChainBwd];
+#pragma unroll
+                for (int k = 0; k < kChainBwd; k++)
+                {
+                    const int32_t i = max(i0 - kChainBwd - k, a);
+                    dn[k] = __ldcg(e + at(i));
+                    bn[k] = __ldg(pl.bh + i);
+                    ln[k] = __ldg(pl.lo + i);
+                }
+#pragma unroll
+                for (int k = 0; k < kChainBwd; k++)
+                {
+                    const int32_t i = i0 - k;
+                    if (i >= a)
+                    {
+                        const double num = (i == pl.L - 1) ? dc[k] : __dsub_rn(dc[k], __dmul_rn(pl.off, x));
+                        x = DivByPlan(num, bc[k], lc[k]);
+                        redo |= PlanDivisionOutOfRange(num);
+                        out[at(i)] = x;
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kChainBwd; k++)
+                {
+                    dc[k] = dn[k];
+                    bc[k] = bn[k];
+                    lc[k] = ln[k];
+                }
+            }
+            if (redo != 0)
+            {
+                x = x0;
+                for (int32_t i = b - 1; i >= a; i--)
+                {
+                    const double v = __ldcg(e + at(i));
+                    x = __ddiv_rn((i == pl.L - 1) ? v : __dsub_rn(v, __dmul_rn(pl.off, x)), pl.bs[i]);
+                    out[at(i)] = x;
+                }
+            }
+            return x;
+        }
+
+        __device__ __forceinline__ bool SameBits(double a, double b)
+        {
+            return __double_as_longlong(a) == __double_as_longlong(b);
+        }
+
+        // Step 1 (segments 0 .. segs - 2): y[seg * lines + line].
+        __global__ void __launch_bounds__(32) AdiSegEnds(const double *__restrict__ d, LinePlan64Dev pl, int32_t lines,
+                                                          double *__restrict__ y)
+        {
+            const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y;
+            if (line >= lines)
+            {
+                return;
+            }
+            const int32_t a = seg * pl.segLen, b = a + pl.segLen;
+            auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
+            double v = 0.0;
+            double rc[kChainFwd], wc[kChainFwd];
+#pragma unroll
+            for (int k = 0; k < kChainFwd; k++)
+            {
+                const int32_t i = min(a + k, b - 1);
+                rc[k] = __ldcg(d + at(i));
+                wc[k] = __ldg(pl.ws + i);
+            }
+            for (int32_t i0 = a; i0 < b; i0 += kChainFwd)
+            {
+                double rn[kChainFwd], wn[kChainFwd];
+#pragma unroll
+                for (int k = 0; k < kChainFwd; k++)
+                {
+                    const int32_t i = min(i0 + kChainFwd + k, b - 1);
+                    rn[k] = __ldcg(d + at(i));
+                    wn[k] = __ldg(pl.ws + i);
+                }
+#pragma unroll
+                for (int k = 0; k < kChainFwd; k++)
+                {
+                    if (i0 + k < b)
+                    {
+                        v = __fma_rn(-wc[k], v, rc[k]);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kChainFwd; k++)
+                {
+                    rc[k] = rn[k];
+                    wc[k] = wn[k];
+                }
+            }
+            y[static_cast<int64_t>(seg) * lines + line] = v;
+        }
+
+        // Step 2: e over every segment; ends[seg * lines + line] = its last.
+        __global__ void __launch_bounds__(32) AdiSegElim(const double *__restrict__ d, double *__restrict__ e,
+                                                          LinePlan64Dev pl, int32_t lines,
+                                                          const double *__restrict__ y, double *__restrict__ ends)
+        {
+            const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y;
+            if (line >= lines)
+            {
+                return;
+            }
+            const int32_t a = seg * pl.segLen, b = min(a + pl.segLen, pl.L);
+            double prev = 0.0;
+            for (int32_t q = 0; q < seg; q++)
+            {
+                prev = __fma_rn(__ldg(pl.segP + q), prev, __ldcg(y + static_cast<int64_t>(q) * lines + line));
+            }
+            prev = ElimRun(d, e, pl, a, b, prev, [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; });
+            ends[static_cast<int64_t>(seg) * lines + line] = prev;
+        }
+
+        // Step 3; z[seg * lines + line]: segments 1 .. segs - 1 of the back
+        // substitution from a zero start.
+        __global__ void __launch_bounds__(32) AdiSegFix(const double *__restrict__ d, double *__restrict__ e,
+                                                         LinePlan64Dev pl, int32_t lines,
+                                                         const double *__restrict__ ends, double *__restrict__ z,
+                                                         int32_t *__restrict__ marks)
+        {
+            constexpr int B = 8;
+            const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y + 1;
+            if (line >= lines)
+            {
+                return;
+            }
+            const int32_t a = seg * pl.segLen, b = min(a + pl.segLen, pl.L);
+            auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
+            double prev = __ldcg(ends + static_cast<int64_t>(seg - 1) * lines + line);
+            bool met = false;
+            for (int32_t i0 = a; i0 < b && !met; i0 += B)
+            {
+                double dv[B], ev[B], wv[B];
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                {
+                    const int32_t i = min(i0 + k, b - 1);
+                    dv[k] = __ldcg(d + at(i));
+                    ev[k] = __ldcg(e + at(i));
+                    wv[k] = __ldg(pl.ws + i);
+                }
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                {
+                    if (i0 + k < b && !met)
+                    {
+                        prev = __dsub_rn(dv[k], __dmul_rn(wv[k], prev));
+                        met = SameBits(prev, ev[k]);
+                        if (!met)
+                        {
+                            e[at(i0 + k)] = prev;
+                        }
+                    }
+                }
+            }
+            if (!met && seg < pl.segs - 1)
+            {
+                marks[line] = 1;
+            }
+            double v = 0.0;
+            for (int32_t i0 = b - 1; i0 >= a; i0 -= kChainBwd)
+            {
+                double ev[kChainBwd], gv[kChainBwd];
+#pragma unroll
+                for (int k = 0; k < kChainBwd; k++)
+                {
+                    const int32_t i = max(i0 - k, a);
+                    ev[k] = __dmul_rn(__ldcg(e + at(i)), __ldg(&pl.bh[i].y));
+                    gv[k] = __ldg(pl.g + i);
+                }
+#pragma unroll
+                for (int k = 0; k < kChainBwd; k++)
+                {
+                    if (i0 - k >= a)
+                    {
+                        v = __fma_rn(gv[k], v, ev[k]);
+                    }
+                }
+            }
+            z[static_cast<int64_t>(seg) * lines + line] = v;
+        }
+
+        // Step 4: the back substitution; starts[seg * lines + line] = its x[a].
+        __global__ void __launch_bounds__(32) AdiSegBack(const double *__restrict__ e, double *__restrict__ out,
+                                                          LinePlan64Dev pl, int32_t lines,
+                                                          const double *__restrict__ z, double *__restrict__ starts)
+        {
+            const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y;
+            if (line >= lines)
+            {
+                return;
+            }
+            const int32_t a = seg * pl.segLen, b = min(a + pl.segLen, pl.L);
+            double x = 0.0;
+            for (int32_t q = pl.segs - 1; q > seg; q--)
+            {
+                x = __fma_rn(__ldg(pl.segQ + q), x, __ldcg(z + static_cast<int64_t>(q) * lines + line));
+            }
+            x = BackRun(e, out, pl, a, b, x, [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; });
+            starts[static_cast<int64_t>(seg) * lines + line] = x;
+        }
+
+        __global__ void __launch_bounds__(32) AdiSegBackFix(const double *__restrict__ e, double *__restrict__ out,
+                                                             LinePlan64Dev pl, int32_t lines,
+                                                             const double *__restrict__ starts,
+                                                             int32_t *__restrict__ marks)
+        {
+            constexpr int B = 8;
+            const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y;
+            if (line >= lines)
+            {
+                return;
+            }
+            const int32_t a = seg * pl.segLen, b = a + pl.segLen;
+            auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
+            double x = __ldcg(starts + static_cast<int64_t>(seg + 1) * lines + line);
+            bool met = false;
+            for (int32_t i0 = b - 1; i0 >= a && !met; i0 -= B)
+            {
+                double ev[B], xv[B];
+                double2 bv[B];
+                int2 lv[B];
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                {
+                    const int32_t i = max(i0 - k, a);
+                    ev[k] = __ldcg(e + at(i));
+                    xv[k] = __ldcg(out + at(i));
+                    bv[k] = __ldg(pl.bh + i);
+                    lv[k] = __ldg(pl.lo + i);
+                }
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                {
+                    if (i0 - k >= a && !met)
+                    {
+                        x = DivExact(__dsub_rn(ev[k], __dmul_rn(pl.off, x)), bv[k], lv[k]);
+                        met = SameBits(x, xv[k]);
+                        if (!met)
+                        {
+                            out[at(i0 - k)] = x;
+                        }
+                    }
+                }
+            }
+            if (!met && seg > 0)
+            {
+                marks[line] = 1;
+            }
+        }
+
+        // Step 5, and a periodic line's factor (see AdiChain64).  Clears the
+        // marks.
+        __global__ void __launch_bounds__(32) AdiSegFinish(const double *__restrict__ d, double *__restrict__ e,
+                                                            double *__restrict__ out, LinePlan64Dev pl, int32_t lines,
+                                                            int32_t *__restrict__ marks, double *__restrict__ factor)
+        {
+            const int32_t line = blockIdx.x * 32 + threadIdx.x;
+            if (line >= lines)
+            {
+                return;
+            }
+            auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
+            if (marks[line] != 0)
+            {
+                marks[line] = 0;
+                ElimRun(d, e, pl, 0, pl.L, 0.0, at);
+                BackRun(e, out, pl, 0, pl.L, 0.0, at);
+            }
+            if (pl.periodic)
+            {
+                const double vy = __dadd_rn(out[at(0)], __dmul_rn(out[at(pl.L - 1)], pl.vEnd));
+                factor[line] = __ddiv_rn(vy, pl.onePlusVz);
+            }
+        }
+
         // The sweeps' division (DivByPlan, or __ddiv_rn where
         // PlanDivisionOutOfRange says so) against __ddiv_rn for every num[i]
         // and divisor j (bh[j], lo[j]: its plan entries); the count of
@@ -696,6 +1086,8 @@ namespace halcuda
             double off = 0, vEnd = 0, onePlusVz = 0;
             bool periodic = false;
             bool fastDiv = false;
+            int32_t segs = 1, segLen = 0;
+            std::vector<double> g, segP, segQ;
         };
 
         // DivByPlan's entries for the divisor b: (b, hi) with hi = RN(1/b),
@@ -860,9 +1252,63 @@ namespace halcuda
             return p;
         }
 
+        constexpr int32_t kSegMaxWarps = 1216;  // 152 SMs x 4 FP64 pipes x 2
+        constexpr int32_t kSegMinLen = 64;
+
+        // Segments of a line's split solve, for `lines` lines.  As many as
+        // give every FP64 pipe two warps, which cover each other's loads (the
+        // kernels of a 2048^2 sweep: 161 us with one warp per pipe, 122 us
+        // with two, 118 us with three, and the whole tick no faster than with
+        // two); segments of at least kSegMinLen elements (shorter ones spend
+        // more on their launches and meetings than the chain saves), and each
+        // long enough that a trajectory's error falls below 2^-64 of itself
+        // over it: otherwise, for large rates, segments would end before they
+        // meet the serial one.  One segment: the serial chain.
+        void AddSegments(LinePlan64Host &p, int32_t lines)
+        {
+            const int32_t L = static_cast<int32_t>(p.bs.size());
+            const int32_t warps = (lines + 31) / 32;
+            p.segs = 1;
+            p.segLen = L;
+            if (!p.fastDiv)
+            {
+                return;
+            }
+            p.g.assign(static_cast<size_t>(L), 0.0);
+            for (int32_t i = 0; i < L; i++)
+            {
+                p.g[static_cast<size_t>(i)] = -p.off * p.bh[static_cast<size_t>(i)].y;
+            }
+            for (int32_t segs = std::min(kSegMaxWarps / warps, L / kSegMinLen); segs >= 2; segs--)
+            {
+                const int32_t len = (L + segs - 1) / segs;
+                const int32_t n = (L + len - 1) / len;
+                std::vector<double> P(static_cast<size_t>(n), 1.0), Q(static_cast<size_t>(n), 1.0);
+                bool ok = true;
+                for (int32_t q = 0; q < n; q++)
+                {
+                    for (int32_t i = q * len; i < std::min(L, (q + 1) * len); i++)
+                    {
+                        P[static_cast<size_t>(q)] *= -p.ws[static_cast<size_t>(i)];
+                        Q[static_cast<size_t>(q)] *= p.g[static_cast<size_t>(i)];
+                    }
+                    ok = ok && (q == n - 1 || (std::fabs(P[static_cast<size_t>(q)]) <= 0x1p-64 &&
+                                               std::fabs(Q[static_cast<size_t>(q)]) <= 0x1p-64));
+                }
+                if (ok && n >= 2)
+                {
+                    p.segs = n;
+                    p.segLen = len;
+                    p.segP = P;
+                    p.segQ = Q;
+                    return;
+                }
+            }
+        }
+
         struct PlanBuf64
         {
-            DevBuf<double> buf;  // ws, bs, zs
+            DevBuf<double> buf;  // the plan's arrays
             LinePlan64Dev dev;
         };
     }
@@ -986,6 +1432,8 @@ namespace halcuda
     {
         DevBuf<double> wA, wB, vB, dS;  // scratch (grown on first use)
         DevBuf<double> fac;             // periodic factors of the current sweep's lines
+        DevBuf<double> segA, segB;      // split solve: values at the segments' ends
+        DevBuf<int32_t> marks;          // split solve: lines to solve again (zero between sweeps)
         std::map<std::string, std::unique_ptr<PlanBuf64>> plans;
 
         int Ensure(DevBuf<double> &b, size_t n, cudaStream_t s, const char *what)
@@ -998,18 +1446,27 @@ namespace halcuda
             return HAL_CUDA_OK;
         }
 
-        int Plan(int32_t L, double r, bool wrap, bool dirichlet, LinePlan64Dev *out)
+        int Plan(int32_t L, int32_t lines, double r, bool wrap, bool dirichlet, LinePlan64Dev *out)
         {
             char key[96];
-            snprintf(key, sizeof(key), "%d|%a|%d|%d", L, r, wrap ? 1 : 0, (dirichlet && !wrap) ? 1 : 0);
+            snprintf(key, sizeof(key), "%d|%d|%a|%d|%d", L, lines, r, wrap ? 1 : 0, (dirichlet && !wrap) ? 1 : 0);
             auto it = plans.find(key);
             if (it == plans.end())
             {
-                const LinePlan64Host h = BuildPlan64(L, r, wrap, dirichlet);
+                LinePlan64Host h = BuildPlan64(L, r, wrap, dirichlet);
+                AddSegments(h, lines);
                 auto pb = std::make_unique<PlanBuf64>();
-                // layout (in doubles): bh [2L], lo [L], ws [L], bs [L], zs [L]
+                // layout (in doubles): bh [2L], lo [L], ws [L], bs [L], zs [L],
+                // and of a split line g [L], segP [segs], segQ [segs]
                 const size_t Ls = static_cast<size_t>(L);
-                std::vector<double> all(6 * Ls, 0.0);
+                const size_t split = h.segs > 1 ? Ls + 2 * static_cast<size_t>(h.segs) : 0;
+                std::vector<double> all(6 * Ls + split, 0.0);
+                if (split > 0)
+                {
+                    std::copy(h.g.begin(), h.g.end(), all.begin() + 6 * Ls);
+                    std::copy(h.segP.begin(), h.segP.end(), all.begin() + 7 * Ls);
+                    std::copy(h.segQ.begin(), h.segQ.end(), all.begin() + 7 * Ls + h.segs);
+                }
                 std::memcpy(all.data(), h.bh.data(), sizeof(double2) * Ls);
                 std::memcpy(all.data() + 2 * Ls, h.lo.data(), sizeof(int2) * Ls);
                 std::copy(h.ws.begin(), h.ws.end(), all.begin() + 3 * Ls);
@@ -1030,6 +1487,11 @@ namespace halcuda
                 pb->dev.onePlusVz = h.onePlusVz;
                 pb->dev.L = L;
                 pb->dev.periodic = h.periodic ? 1 : 0;
+                pb->dev.segs = h.segs;
+                pb->dev.segLen = h.segLen;
+                pb->dev.g = pb->buf.p + 6 * Ls;
+                pb->dev.segP = pb->buf.p + 7 * Ls;
+                pb->dev.segQ = pb->buf.p + 7 * Ls + h.segs;
                 it = plans.emplace(key, std::move(pb)).first;
             }
             *out = it->second->dev;
@@ -1053,8 +1515,8 @@ namespace halcuda
         HAL_TRY(m.Ensure(m.vB, n, s, "cudaMalloc(ADI scratch)"));
         HAL_TRY(m.Ensure(m.dS, n, s, "cudaMalloc(ADI scratch)"));
         LinePlan64Dev px, py;
-        HAL_TRY(m.Plan(xDim, r, wrapX != 0, g != nullptr, &px));
-        HAL_TRY(m.Plan(yDim, r, wrapY != 0, g != nullptr, &py));
+        HAL_TRY(m.Plan(xDim, yDim, r, wrapX != 0, g != nullptr, &px));
+        HAL_TRY(m.Plan(yDim, xDim, r, wrapY != 0, g != nullptr, &py));
         // per sweep: the right-hand sides on every SM, the chains one line
         // per thread and one warp per block (the lines spread over the most
         // SMs), then the transpose that applies the periodic correction
@@ -1065,8 +1527,34 @@ namespace halcuda
         const auto rhsGrid = [](int32_t lines, int32_t L) {
             return dim3(Blocks(lines, 256), static_cast<unsigned>(std::min<int32_t>(std::max<int32_t>(L, 1), 65535)));
         };
-        const auto chain = [&](const LinePlan64Dev &pl, int32_t lines, double *out) {
-            if (pl.fastDiv)
+        const size_t nSeg = static_cast<size_t>(std::max(static_cast<int64_t>(px.segs) * yDim,
+                                                         static_cast<int64_t>(py.segs) * xDim));
+        if (px.segs > 1 || py.segs > 1)
+        {
+            HAL_TRY(m.Ensure(m.segA, nSeg, s, "cudaMalloc(ADI scratch)"));
+            HAL_TRY(m.Ensure(m.segB, nSeg, s, "cudaMalloc(ADI scratch)"));
+            if (m.marks.n < nFac || m.marks.p == nullptr)
+            {
+                HAL_TRY(CudaStatus(cudaStreamSynchronize(s), "cudaMalloc(ADI scratch)"));
+                HAL_TRY(m.marks.Alloc(nFac, "cudaMalloc(ADI scratch)"));
+                HAL_TRY(CudaStatus(cudaMemsetAsync(m.marks.p, 0, nFac * sizeof(int32_t), s), "ADI scratch"));
+            }
+        }
+        // e: a scratch array that the sweep does not use otherwise (the split
+        // solve keeps the right-hand sides)
+        const auto chain = [&](const LinePlan64Dev &pl, int32_t lines, double *out, double *e) {
+            if (pl.segs > 1)
+            {
+                const unsigned b = Blocks(lines, T), segs = static_cast<unsigned>(pl.segs);
+                AdiSegEnds<<<dim3(b, segs - 1), T, 0, s>>>(m.dS.p, pl, lines, m.segA.p);
+                AdiSegElim<<<dim3(b, segs), T, 0, s>>>(m.dS.p, e, pl, lines, m.segA.p, m.segB.p);
+                AdiSegFix<<<dim3(b, segs - 1), T, 0, s>>>(m.dS.p, e, pl, lines, m.segB.p, m.segA.p, m.marks.p);
+                AdiSegBack<<<dim3(b, segs), T, 0, s>>>(e, out, pl, lines, m.segA.p, m.segB.p);
+                AdiSegBackFix<<<dim3(b, segs - 1), T, 0, s>>>(e, out, pl, lines, m.segB.p, m.marks.p);
+                AdiSegFinish<<<b, T, 0, s>>>(m.dS.p, e, out, pl, lines, m.marks.p, m.fac.p);
+                CountLaunch(5);
+            }
+            else if (pl.fastDiv)
             {
                 AdiChain64<true><<<Blocks(lines, T), T, 0, s>>>(m.dS.p, out, pl, lines, m.fac.p);
             }
@@ -1077,12 +1565,12 @@ namespace halcuda
         };
         AdiRhs64<<<rhsGrid(yDim, xDim), 256, 0, s>>>(f, m.dS.p, xDim, yDim, wrapY, wrapX,
                                                         g ? g + 2 * static_cast<size_t>(yDim) : nullptr, g, r);
-        chain(px, yDim, m.wA.p);
+        chain(px, yDim, m.wA.p, m.vB.p);
         Transpose64<false><<<dim3((yDim + 31) / 32, (xDim + 31) / 32), tb, 0, s>>>(
             m.wA.p, m.wB.p, xDim, yDim, nullptr, px.periodic ? m.fac.p : nullptr, px.zs);
         AdiRhs64<<<rhsGrid(xDim, yDim), 256, 0, s>>>(m.wB.p, m.dS.p, yDim, xDim, wrapX, wrapY, g,
                                                         g ? g + 2 * static_cast<size_t>(yDim) : nullptr, r);
-        chain(py, xDim, m.vB.p);
+        chain(py, xDim, m.vB.p, m.wA.p);
         Transpose64<true><<<dim3((xDim + 31) / 32, (yDim + 31) / 32), tb, 0, s>>>(
             m.vB.p, deltas, yDim, xDim, f, py.periodic ? m.fac.p : nullptr, py.zs);
         CountLaunch(6);
