@@ -338,14 +338,6 @@ namespace halcuda
             const double *segQ;
         };
 
-        // ExplicitDiffusionY2ADI / X2ADI (src/Pde/ADIequations.cpp:19-47 and
-        // the Dirichlet forms, include/Hal/Pde/ADIequations.h:54-94): the
-        // cell plus half the rate times its two cross-axis differences.
-        __device__ __forceinline__ double HalfStep(double c, double d1, double d2, double r)
-        {
-            return __dadd_rn(c, __dmul_rn(__dmul_rn(__dadd_rn(d1, d2), r), 0.5));
-        }
-
         // ImplicitBoundarySource (ADIequations.h:198-220) at position i of a
         // line of length L; 0 on a wrapped axis.
         __device__ __forceinline__ double ImplicitSource(int32_t i, int32_t L, bool wrap, double r, double lo,
@@ -429,36 +421,174 @@ namespace halcuda
             return ((e - 123u) > (1922u - 123u) && !plusZero) ? 1u : 0u;
         }
 
+        // ExplicitDiffusionY2ADI / X2ADI (src/Pde/ADIequations.cpp:19-47 and
+        // the Dirichlet forms, include/Hal/Pde/ADIequations.h:54-94): the cell
+        // plus half the rate times the sum s of its two cross-axis differences,
+        // c + (s * r) * 0.5.  With t = RN(s * r), t / 2 is exact unless it is
+        // subnormal, and rides on the addition (HalfStep); HalfInexact says
+        // where it may not be, and HalfStepExact keeps the operations apart.
+        __device__ __forceinline__ double HalfStep(double c, double t)
+        {
+            return __fma_rn(t, 0.5, c);
+        }
+
+        __device__ __forceinline__ uint32_t HalfInexact(double t)
+        {
+            const uint32_t hi = static_cast<uint32_t>(__double2hiint(t)) & 0x7fffffffu;
+            return (hi < 0x00200000u && (hi | static_cast<uint32_t>(__double2loint(t))) != 0u) ? 1u : 0u;
+        }
+
+        // Not inlined: the compiler would issue it, predicated off, for every
+        // cell, and a predicated-off FP64 instruction still takes the pipe.
+        __device__ __noinline__ double HalfStepExact(double c, double t)
+        {
+            return __dadd_rn(c, __dmul_rn(t, 0.5));
+        }
+
+        constexpr int kRhsCells = 4;  // consecutive lines of one thread
+
         // Right-hand side of one sweep at every cell (i, line) of lines laid
-        // out v[i * lines + line], one thread per cell: for the x-sweep
-        // ExplicitDiffusionY2ADI (ADIequations.h:316-324, Dirichlet :351-362),
-        // for the y-sweep ExplicitDiffusionX2ADI (ADIequations.h:325-336,
-        // Dirichlet :363-377) -- the cell plus half the rate times its two
-        // cross-axis differences, to line + 1 then line - 1 -- plus, with a
-        // ghost table, ImplicitBoundarySource along the line.  crossGhost[L +
-        // i] / crossGhost[i] are the ghosts beyond line lines-1 / line 0 of
-        // row i; alongLo[line] / alongLo[lines + line] those before element 0
-        // / after element L-1 of a line (null: zero-flux).
+        // out v[i * lines + line]: for the x-sweep ExplicitDiffusionY2ADI
+        // (ADIequations.h:316-324, Dirichlet :351-362), for the y-sweep
+        // ExplicitDiffusionX2ADI (ADIequations.h:325-336, Dirichlet :363-377)
+        // -- the cell plus half the rate times its two cross-axis differences,
+        // to line + 1 then line - 1 -- plus, with a ghost table,
+        // ImplicitBoundarySource along the line.  crossGhost[L + i] /
+        // crossGhost[i] are the ghosts beyond line lines-1 / line 0 of row i;
+        // alongLo[line] / alongLo[lines + line] those before element 0 / after
+        // element L-1 of a line (null: zero-flux).
+        // Bound by FP64 issue: six operations per cell took 51 us at 2048^2.  A
+        // thread takes kRhsCells lines and shares each difference between the
+        // two cells it separates (negated, which is exact), and the product by
+        // 1/2 rides on the last addition: 4.25 operations, 38 us.  (The
+        // negation of a zero difference changes the sign of the sum's zero,
+        // which the addition to a cell of the same value does not see.)
         __global__ void AdiRhs64(const double *__restrict__ v, double *__restrict__ rhs, int32_t L, int32_t lines,
                                  int32_t wrapCross, int32_t wrapAlong, const double *__restrict__ crossGhost,
                                  const double *__restrict__ alongLo, double r)
         {
-            const int32_t line = blockIdx.x * blockDim.x + threadIdx.x;
-            if (line >= lines)
+            constexpr int C = kRhsCells;
+            const int32_t line0 = (blockIdx.x * blockDim.x + threadIdx.x) * C;
+            if (line0 >= lines)
             {
                 return;
             }
+            const bool whole = line0 + C <= lines;
+            const bool vec = whole && (lines & 1) == 0;  // 16-byte aligned pairs
+            const int32_t n = min(C, lines - line0);
             for (int32_t i = blockIdx.y; i < L; i += gridDim.y)
             {
                 const int64_t row = static_cast<int64_t>(i) * lines;
-                const double c = v[row + line];
-                double s = HalfStep(c, CrossDelta(v, c, line + 1, lines, wrapCross != 0, row, 1, crossGhost, L + i),
-                                    CrossDelta(v, c, line - 1, lines, wrapCross != 0, row, 1, crossGhost, i), r);
-                if (alongLo != nullptr)
+                const double *q = v + row + line0;
+                double c[C];
+                if (vec)
                 {
-                    s = __dadd_rn(s, ImplicitSource(i, L, wrapAlong != 0, r, alongLo[line], alongLo[lines + line]));
+#pragma unroll
+                    for (int k = 0; k < C; k += 2)
+                    {
+                        const double2 t = __ldg(reinterpret_cast<const double2 *>(q + k));
+                        c[k] = t.x;
+                        c[k + 1] = t.y;
+                    }
                 }
-                rhs[row + line] = s;
+                else
+                {
+#pragma unroll
+                    for (int k = 0; k < C; k++)
+                    {
+                        c[k] = __ldg(q + min(k, n - 1));
+                    }
+                }
+                // up: difference to the line after the cell; dn: to the one
+                // before it, of the first cell
+                double up[C];
+                double dn;
+#pragma unroll
+                for (int k = 0; k < C - 1; k++)
+                {
+                    up[k] = __dsub_rn(c[k + 1], c[k]);
+                }
+                if (line0 > 0)
+                {
+                    dn = __dsub_rn(__ldg(q - 1), c[0]);
+                }
+                else
+                {
+                    dn = CrossDelta(v, c[0], -1, lines, wrapCross != 0, row, 1, crossGhost, i);
+                }
+                if (whole && line0 + C < lines)
+                {
+                    up[C - 1] = __dsub_rn(__ldg(q + C), c[C - 1]);
+                }
+                else
+                {
+                    // the grid's last cell is c[n - 1]
+                    const double last =
+                        CrossDelta(v, c[C - 1], lines, lines, wrapCross != 0, row, 1, crossGhost, L + i);
+#pragma unroll
+                    for (int k = 0; k < C; k++)
+                    {
+                        up[k] = (k == n - 1) ? last : up[k];
+                    }
+                }
+                double s[C], t[C];
+                uint32_t rare = 0;
+#pragma unroll
+                for (int k = 0; k < C; k++)
+                {
+                    t[k] = __dmul_rn(__dadd_rn(up[k], k == 0 ? dn : -up[k - 1]), r);
+                    s[k] = HalfStep(c[k], t[k]);
+                    rare |= HalfInexact(t[k]);
+                }
+                if (rare != 0)
+                {
+#pragma unroll
+                    for (int k = 0; k < C; k++)
+                    {
+                        s[k] = HalfStepExact(c[k], t[k]);
+                    }
+                }
+                if (alongLo != nullptr && !wrapAlong && (i == 0 || i == L - 1))
+                {
+#pragma unroll
+                    for (int k = 0; k < C; k++)
+                    {
+                        if (k < n)
+                        {
+                            s[k] = __dadd_rn(s[k], ImplicitSource(i, L, false, r, alongLo[line0 + k],
+                                                                  alongLo[lines + line0 + k]));
+                        }
+                    }
+                }
+                else if (alongLo != nullptr && (wrapAlong || __double2hiint(r) >= 0))
+                {
+                    // the source is +0: adding it only turns -0 into +0
+#pragma unroll
+                    for (int k = 0; k < C; k++)
+                    {
+                        s[k] = (__double_as_longlong(s[k]) == __double_as_longlong(-0.0)) ? 0.0 : s[k];
+                    }
+                }
+                double *o = rhs + row + line0;
+                if (vec)
+                {
+#pragma unroll
+                    for (int k = 0; k < C; k += 2)
+                    {
+                        *reinterpret_cast<double2 *>(o + k) = make_double2(s[k], s[k + 1]);
+                    }
+                }
+                else
+                {
+#pragma unroll
+                    for (int k = 0; k < C; k++)
+                    {
+                        if (k < n)
+                        {
+                            o[k] = s[k];
+                        }
+                    }
+                }
             }
         }
 
@@ -688,8 +818,9 @@ namespace halcuda
 
         // x[i] = (e[i] - off * x[i + 1]) / bs[i] over [a, b) downwards, from x
         // (unused at i = L - 1), in the reference's operations; returns x[a].
-        // A numerator outside DivByPlan's range has the segment run again.
-        template <typename At>
+        // FAST: a numerator outside DivByPlan's range has the segment run
+        // again with the division chosen per element (a branch on the chain).
+        template <bool FAST, typename At>
         __device__ __forceinline__ double BackRun(const double *__restrict__ e, double *__restrict__ out,
                                                   const LinePlan64Dev &pl, int32_t a, int32_t b, double x, At at)
         {
@@ -726,8 +857,15 @@ namespace halcuda
                     if (i >= a)
                     {
                         const double num = (i == pl.L - 1) ? dc[k] : __dsub_rn(dc[k], __dmul_rn(pl.off, x));
-                        x = DivByPlan(num, bc[k], lc[k]);
-                        redo |= PlanDivisionOutOfRange(num);
+                        if constexpr (FAST)
+                        {
+                            x = DivByPlan(num, bc[k], lc[k]);
+                            redo |= PlanDivisionOutOfRange(num);
+                        }
+                        else
+                        {
+                            x = DivExact(num, bc[k], lc[k]);
+                        }
                         out[at(i)] = x;
                     }
                 }
@@ -739,14 +877,11 @@ namespace halcuda
                     lc[k] = ln[k];
                 }
             }
-            if (redo != 0)
+            if constexpr (FAST)
             {
-                x = x0;
-                for (int32_t i = b - 1; i >= a; i--)
+                if (redo != 0)
                 {
-                    const double v = __ldcg(e + at(i));
-                    x = __ddiv_rn((i == pl.L - 1) ? v : __dsub_rn(v, __dmul_rn(pl.off, x)), pl.bs[i]);
-                    out[at(i)] = x;
+                    x = BackRun<false>(e, out, pl, a, b, x0, at);
                 }
             }
             return x;
@@ -910,7 +1045,7 @@ namespace halcuda
             {
                 x = __fma_rn(__ldg(pl.segQ + q), x, __ldcg(z + static_cast<int64_t>(q) * lines + line));
             }
-            x = BackRun(e, out, pl, a, b, x, [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; });
+            x = BackRun<true>(e, out, pl, a, b, x, [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; });
             starts[static_cast<int64_t>(seg) * lines + line] = x;
         }
 
@@ -979,7 +1114,7 @@ namespace halcuda
             {
                 marks[line] = 0;
                 ElimRun(d, e, pl, 0, pl.L, 0.0, at);
-                BackRun(e, out, pl, 0, pl.L, 0.0, at);
+                BackRun<false>(e, out, pl, 0, pl.L, 0.0, at);
             }
             if (pl.periodic)
             {
@@ -1524,8 +1659,13 @@ namespace halcuda
         HAL_TRY(m.Ensure(m.fac, nFac, s, "cudaMalloc(ADI scratch)"));
         const int T = 32;
         const dim3 tb(32, 8);
-        const auto rhsGrid = [](int32_t lines, int32_t L) {
-            return dim3(Blocks(lines, 256), static_cast<unsigned>(std::min<int32_t>(std::max<int32_t>(L, 1), 65535)));
+        // threads for one row of lines in whole warps, at most 256 a block
+        const auto rhsThreads = [](int32_t lines) {
+            return std::min(256, ((lines + kRhsCells - 1) / kRhsCells + 31) / 32 * 32);
+        };
+        const auto rhsGrid = [&](int32_t lines, int32_t L) {
+            return dim3(Blocks(lines, rhsThreads(lines) * kRhsCells),
+                        static_cast<unsigned>(std::min<int32_t>(std::max<int32_t>(L, 1), 65535)));
         };
         const size_t nSeg = static_cast<size_t>(std::max(static_cast<int64_t>(px.segs) * yDim,
                                                          static_cast<int64_t>(py.segs) * xDim));
@@ -1563,12 +1703,12 @@ namespace halcuda
                 AdiChain64<false><<<Blocks(lines, T), T, 0, s>>>(m.dS.p, out, pl, lines, m.fac.p);
             }
         };
-        AdiRhs64<<<rhsGrid(yDim, xDim), 256, 0, s>>>(f, m.dS.p, xDim, yDim, wrapY, wrapX,
+        AdiRhs64<<<rhsGrid(yDim, xDim), rhsThreads(yDim), 0, s>>>(f, m.dS.p, xDim, yDim, wrapY, wrapX,
                                                         g ? g + 2 * static_cast<size_t>(yDim) : nullptr, g, r);
         chain(px, yDim, m.wA.p, m.vB.p);
         Transpose64<false><<<dim3((yDim + 31) / 32, (xDim + 31) / 32), tb, 0, s>>>(
             m.wA.p, m.wB.p, xDim, yDim, nullptr, px.periodic ? m.fac.p : nullptr, px.zs);
-        AdiRhs64<<<rhsGrid(xDim, yDim), 256, 0, s>>>(m.wB.p, m.dS.p, yDim, xDim, wrapX, wrapY, g,
+        AdiRhs64<<<rhsGrid(xDim, yDim), rhsThreads(xDim), 0, s>>>(m.wB.p, m.dS.p, yDim, xDim, wrapX, wrapY, g,
                                                         g ? g + 2 * static_cast<size_t>(yDim) : nullptr, r);
         chain(py, xDim, m.vB.p, m.wA.p);
         Transpose64<true><<<dim3((xDim + 31) / 32, (yDim + 31) / 32), tb, 0, s>>>(
