@@ -6,15 +6,10 @@
 // pDiffRatesX, pDiffRatesY, ...) (src/Pde/PDEequations.cpp:199-230): the
 // face between cells j and j+1 of a line carries cell j's rate, a non-wrapped
 // edge has no face, and L is the face-weighted Laplacian along a line:
-//   w  = (I - Lx/2)^-1 (I + Ly/2) f            x-sweep  (FwdX)
-//   v  = (I - Ly/2)^-1 (I + Lx/2) w            y-sweep  (FwdY)
+//   w  = (I - Lx/2)^-1 (I + Ly/2) f            x-sweep  (FwdLines<M, false>)
+//   v  = (I - Ly/2)^-1 (I + Lx/2) w            y-sweep  (FwdLines<M, true>)
 //   f' = f + (((v - f) + f*(-decay)) + src)    PDEGrid2D tick order
 // For a constant rate this is Internal::Diffusion2DADI plus the tick.
-//
-// Every line has its own tridiagonal matrix, so the line solves are parallel
-// cyclic reduction in shared memory (one CTA per line, one row per thread);
-// a wrapped line of a power-of-two length reduces cyclically, any other
-// wrapped line by a Sherman-Morrison split (PcrSolveSM).
 //
 // Gradient of loss = 1/2 |f_T - target|^2.  I - L/2 and I + L/2 are
 // symmetric, so with gbar the adjoint of a step's output:
@@ -28,17 +23,43 @@
 // States are recomputed segment by segment from checkpoints every k steps,
 // each segment on a second stream while the one after it is differentiated.
 //
-// Layout: every array is row-major x*yDim + y (HAL's layout), except the
-// x-kernels' own copies, which are line by line (y*xDim + x) so that an x-line
-// CTA reads them contiguously: the rates DT (transposed once per call), the
-// kept states w (FwdX writes them so) and the x-faces' part of dL/dD (added
-// into dD once at the end).  Only the arrays passed between the sweeps (f, w
-// for the y-sweep, b2bar, b1bar) keep HAL's layout and are strided for x-lines.
+// What bounds a step.  A field is 1 MB at 512^2: a step's kernels move a few MB
+// through the L2, a microsecond or two, and are bound by latency: the launch,
+// the loads, the solve's dependent chain, the stores.  Parallel cyclic
+// reduction of every line in shared memory took nine stages of two barriers
+// (12 us a forward kernel, 13 to 16 us a backward one).  But the rates do not
+// change between the steps of a call, so each line is factored once per call, in FP64
+// (Factor), and a step only runs the right-hand side through the factors:
+//   - a warp solves one line, a lane M consecutive positions of it in
+//     registers: Thomas with the precomputed multipliers (fw, ib, cb) over the
+//     lane's first M - 1 positions, the last one being a separator;
+//   - the separators' tridiagonal system (one per lane) by cyclic reduction
+//     over shuffles with precomputed multipliers (five stages, no division);
+//   - x = z - s_left p - s_right q with the precomputed coupling vectors;
+//   - a wrapped line is split as T + u v^T (TdmaSolver::TDMAperiodic's form,
+//     include/Hal/Pde/TdmaSolver.h:68-120): x = y - (y_0 + bog y_n-1) zf with
+//     zf precomputed.
+// No barriers but one, for the transposed write-out: a CTA's four lines leave
+// through shared memory as 16-byte pieces, in the layout in which the next
+// kernel's lines are contiguous.  The kernels are chained by programmatic
+// launches; everything that does not come from the kernel just before
+// (factors, rates, kept states, accumulators) is loaded before the wait for it.
+// A run of steps between checkpoints is replayed from a small CUDA graph.
+// Measured at 512^2, 500 steps, zero-flux: forward 3.2 ms (12.3 ms with the
+// reductions), gradient with checkpoints every 22 steps 8.8 ms (28.8 ms); its
+// error against 64 bits is unchanged (1.5e-6 for dL/dD).  What is left per
+// kernel is latency: 1.7 us of it is there on a 64^2 field too.
+//
+// Layout: "by y" arrays are x * ldY + y (HAL's order), "by x" arrays y * ldX +
+// x; ldX and ldY are the sides rounded up to multiples of 4 and the padding
+// holds zeros, so every line is read and written in 16-byte pieces.
 #include "common.cuh"
-#include "adi_sweep.h"
 
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <string>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -47,305 +68,798 @@ namespace halcuda
     namespace
     {
         constexpr int kMaxAdjLine = HAL_CUDA_ADJOINT_MAX_SIDE;
+        constexpr int kAdjLines = 4;  // lines (warps) per CTA: a 16-byte piece of the transposed write-out
+        constexpr unsigned kAll = 0xffffffffu;
 
-        enum LineDir : int
+        // Coefficient vectors of a factored line (kCoefZ on wrapped axes only).
+        enum AdjCoef : int
         {
-            kDirX = 0,  // line = fixed y, positions along x (stride yDim)
-            kDirY = 1   // line = fixed x, positions along y (contiguous)
+            kCoefFw = 0,
+            kCoefIb = 1,
+            kCoefCb = 2,
+            kCoefP = 3,
+            kCoefQ = 4,
+            kCoefZ = 5
         };
 
-        struct Grid
+        // Per-lane values of a factored line: the separator stages' multipliers
+        // (five below, five above), the reciprocal of its reduced diagonal, the
+        // separator row's off-diagonals, and a wrapped line's beta / gamma.
+        enum AdjExt : int
         {
-            int32_t xDim, yDim;
-            int32_t wrapX, wrapY;
+            kExtLo = 0,
+            kExtHi = 5,
+            kExtBinv = 10,
+            kExtA = 11,
+            kExtC = 12,
+            kExtBog = 13,
+            kExtCount = 14
         };
 
-        template <int DIR>
-        __device__ __forceinline__ int64_t Idx(const Grid &g, int32_t line, int32_t pos)
+        // One axis of the grid: lines of n positions, nl of them.
+        struct Axis
         {
-            return (DIR == kDirY) ? static_cast<int64_t>(line) * g.yDim + pos
-                                  : static_cast<int64_t>(pos) * g.yDim + line;
+            int32_t n, nl;
+            int32_t ld;                   // row stride of arrays whose rows are this axis's lines
+            int32_t ldT;                  // row stride of the other layout
+            int32_t wrap, wrapCross;
+            const float *D;               // rates, line by line
+            const float *coef;            // [line][coef][M / 4][32 lanes][4]
+            const float *ext;             // [line][kExtCount][32]
+        };
+
+        __device__ __forceinline__ void WaitForPredecessor()
+        {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            // the next kernel may start loading what this one does not write:
+            // whatever it reads before its own wait was complete before this
+            // kernel's predecessor had finished
+            asm volatile("griddepcontrol.launch_dependents;");
         }
 
-        template <int DIR>
-        __device__ __forceinline__ int32_t LineLen(const Grid &g)
+        // The lane's M positions of a line (0 beyond the row).  Through the
+        // L2: rows written by kernels of the same chain.
+        template <int M>
+        __device__ __forceinline__ void LoadRow(const float *__restrict__ row, int32_t ld, int lane, float (&v)[M])
         {
-            return (DIR == kDirY) ? g.yDim : g.xDim;
-        }
-
-        template <int DIR>
-        __device__ __forceinline__ int32_t Lines(const Grid &g)
-        {
-            return (DIR == kDirY) ? g.xDim : g.yDim;
-        }
-
-        template <int DIR>
-        __device__ __forceinline__ bool Wrap(const Grid &g)
-        {
-            return (DIR == kDirY) ? g.wrapY != 0 : g.wrapX != 0;
-        }
-
-        template <int DIR>
-        __device__ __forceinline__ bool WrapCross(const Grid &g)
-        {
-            return (DIR == kDirY) ? g.wrapX != 0 : g.wrapY != 0;
-        }
-
-        // Face weights below (eL) and above (eR) position j of a line whose
-        // rates sit in sD (one per position).
-        __device__ __forceinline__ void Faces(const float *sD, int32_t j, int32_t n, bool wrap, float &eL, float &eR)
-        {
-            eL = (j > 0) ? sD[j - 1] : (wrap ? sD[n - 1] : 0.0f);
-            eR = (j < n - 1) ? sD[j] : (wrap ? sD[n - 1] : 0.0f);
-        }
-
-        // (L u)_j along the line, with the line's u and rates in shared memory.
-        __device__ __forceinline__ float LapAlong(const float *su, const float *sD, int32_t j, int32_t n, bool wrap)
-        {
-            float eL, eR;
-            Faces(sD, j, n, wrap, eL, eR);
-            const float c = su[j];
-            const float lo = (j > 0) ? su[j - 1] : (wrap ? su[n - 1] : c);
-            const float hi = (j < n - 1) ? su[j + 1] : (wrap ? su[0] : c);
-            return eR * (hi - c) + eL * (lo - c);
-        }
-
-        // (L_cross u) at (line, j): the neighbours are lines line-1 and
-        // line+1; the face (line, line+1) carries D(line, j), the face
-        // (line-1, line) carries D(line-1, j).
-        template <int DIR>
-        __device__ __forceinline__ float LapCross(const Grid &g, const float *__restrict__ u,
-                                                  const float *__restrict__ D, int32_t line, int32_t j, float c)
-        {
-            const int32_t nl = Lines<DIR>(g);
-            const bool wrap = WrapCross<DIR>(g);
-            float acc = 0.0f;
-            if (line + 1 < nl || (wrap && nl > 1))
+#pragma unroll
+            for (int q = 0; q < M / 4; q++)
             {
-                const int32_t up = (line + 1 < nl) ? line + 1 : 0;
-                acc += D[Idx<DIR>(g, line, j)] * (u[Idx<DIR>(g, up, j)] - c);
-            }
-            if (line > 0 || (wrap && nl > 1))
-            {
-                const int32_t dn = (line > 0) ? line - 1 : nl - 1;
-                acc += D[Idx<DIR>(g, dn, j)] * (u[Idx<DIR>(g, dn, j)] - c);
-            }
-            return acc;
-        }
-
-        // LapCross<kDirX> with the rates read from DT, D transposed (DT[y *
-        // xDim + x] = D(x, y)): the two cross faces' rates of an x-line are then
-        // contiguous along the line, like the line's own.
-        __device__ __forceinline__ float LapCrossXT(const Grid &g, const float *__restrict__ u,
-                                                    const float *__restrict__ DT, int32_t line, int32_t j, float c)
-        {
-            const int32_t nl = g.yDim;
-            const bool wrap = g.wrapY != 0;
-            float acc = 0.0f;
-            if (line + 1 < nl || (wrap && nl > 1))
-            {
-                const int32_t up = (line + 1 < nl) ? line + 1 : 0;
-                acc += DT[static_cast<int64_t>(line) * g.xDim + j] * (u[Idx<kDirX>(g, up, j)] - c);
-            }
-            if (line > 0 || (wrap && nl > 1))
-            {
-                const int32_t dn = (line > 0) ? line - 1 : nl - 1;
-                acc += DT[static_cast<int64_t>(dn) * g.xDim + j] * (u[Idx<kDirX>(g, dn, j)] - c);
-            }
-            return acc;
-        }
-
-        // -1/2 (p_j+1 - p_j)(q_j+1 - q_j) for the face above position j (the
-        // face owned by j), 0 if it does not exist.
-        __device__ __forceinline__ float FaceGrad(const float *sp, const float *sq, int32_t j, int32_t n, bool wrap)
-        {
-            if (j < n - 1)
-            {
-                return -0.5f * (sp[j + 1] - sp[j]) * (sq[j + 1] - sq[j]);
-            }
-            if (wrap && n > 1)
-            {
-                return -0.5f * (sp[0] - sp[j]) * (sq[0] - sq[j]);
-            }
-            return 0.0f;
-        }
-
-        // A wrapped line whose length is not a power of two: the cyclic
-        // system A x = d is split as A = T + u v^T (TdmaSolver::TDMAperiodic's
-        // form, include/Hal/Pde/TdmaSolver.h:68-120: gamma = -b_0, T's
-        // diagonal b_0 - gamma and b_{n-1} - a_0 c_{n-1} / gamma, u = (gamma,
-        // 0, .., 0, c_{n-1}), v = (1, 0, .., 0, a_0 / gamma)); T y = d and
-        // T z = u are solved together by non-wrapped parallel cyclic reduction
-        // (the reductions of T are shared), then x = y - (v.y / (1 + v.z)) z.
-        // sm holds 4 * blockDim.x floats, sm2 blockDim.x + 4.
-        __device__ float PcrSolveSM(const float *sD, float d, int32_t j, int32_t n, float *sm, float *sm2)
-        {
-            float *sa = sm, *sb = sm + blockDim.x, *sc = sb + blockDim.x, *sd = sc + blockDim.x;
-            float *sd2 = sm2, *sx = sm2 + blockDim.x;
-            float eL0, eR0, eLn, eRn;
-            Faces(sD, 0, n, true, eL0, eR0);
-            Faces(sD, n - 1, n, true, eLn, eRn);
-            const float a0 = -0.5f * eL0;                 // row 0's coefficient of x_{n-1}
-            const float cn = -0.5f * eRn;                 // row n-1's coefficient of x_0
-            const float gam = -(1.0f + 0.5f * (eL0 + eR0));  // -b_0
-            float a = 0.0f, b = 1.0f, c = 0.0f, d2 = 0.0f;
-            if (j < n)
-            {
-                float eL, eR;
-                Faces(sD, j, n, true, eL, eR);
-                a = (j > 0) ? -0.5f * eL : 0.0f;
-                c = (j < n - 1) ? -0.5f * eR : 0.0f;
-                b = 1.0f + 0.5f * (eL + eR);
-                if (j == 0)
+                const int32_t pos = lane * M + 4 * q;
+                float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (pos < ld)
                 {
-                    b -= gam;
-                    d2 = gam;
+                    t = __ldcg(reinterpret_cast<const float4 *>(row + pos));
                 }
-                if (j == n - 1)
+                v[4 * q] = t.x;
+                v[4 * q + 1] = t.y;
+                v[4 * q + 2] = t.z;
+                v[4 * q + 3] = t.w;
+            }
+        }
+
+        template <int M>
+        __device__ __forceinline__ void StoreRow(float *__restrict__ row, int32_t ld, int lane, const float (&v)[M])
+        {
+#pragma unroll
+            for (int q = 0; q < M / 4; q++)
+            {
+                const int32_t pos = lane * M + 4 * q;
+                if (pos < ld)
                 {
-                    b -= a0 * cn / gam;
-                    d2 = cn;
+                    *reinterpret_cast<float4 *>(row + pos) =
+                        make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                 }
             }
-            for (int32_t delta = 1; delta < n; delta <<= 1)
+        }
+
+        // row += v
+        template <int M>
+        __device__ __forceinline__ void AddRow(float *__restrict__ row, int32_t ld, int lane, const float (&v)[M])
+        {
+            float t[M];
+            LoadRow<M>(row, ld, lane, t);
+#pragma unroll
+            for (int i = 0; i < M; i++)
             {
-                if (j < n)
+                t[i] += v[i];
+            }
+            StoreRow<M>(row, ld, lane, t);
+        }
+
+        // A line's factors in registers.
+        template <int M>
+        struct Factors
+        {
+            float fw[M], ib[M], cb[M], p[M], q[M];
+            float lo[5], hi[5], binv, a, c;
+
+            __device__ __forceinline__ void Load(const Axis &ax, int32_t line, int lane)
+            {
+                const int nc = ax.wrap ? 6 : 5;
+                const float4 *base = reinterpret_cast<const float4 *>(ax.coef) +
+                                     static_cast<int64_t>(line) * nc * (M / 4) * 32 + lane;
+                auto vec = [&](int k, float (&v)[M])
                 {
-                    sa[j] = a;
-                    sb[j] = b;
-                    sc[j] = c;
-                    sd[j] = d;
-                    sd2[j] = d2;
-                }
-                __syncthreads();
-                if (j < n)
-                {
-                    float al = 0.0f, bl = 1.0f, cl = 0.0f, dl = 0.0f, dl2 = 0.0f;
-                    float ar = 0.0f, br = 1.0f, cr = 0.0f, dr = 0.0f, dr2 = 0.0f;
-                    const int32_t il = j - delta, ir = j + delta;
-                    if (il >= 0)
+#pragma unroll
+                    for (int j = 0; j < M / 4; j++)
                     {
-                        al = sa[il];
-                        bl = sb[il];
-                        cl = sc[il];
-                        dl = sd[il];
-                        dl2 = sd2[il];
+                        const float4 t = __ldg(base + (k * (M / 4) + j) * 32);
+                        v[4 * j] = t.x;
+                        v[4 * j + 1] = t.y;
+                        v[4 * j + 2] = t.z;
+                        v[4 * j + 3] = t.w;
                     }
-                    if (ir < n)
-                    {
-                        ar = sa[ir];
-                        br = sb[ir];
-                        cr = sc[ir];
-                        dr = sd[ir];
-                        dr2 = sd2[ir];
-                    }
-                    const float alpha = -__fdividef(a, bl);
-                    const float beta = -__fdividef(c, br);
-                    b = b + alpha * cl + beta * ar;
-                    d = d + alpha * dl + beta * dr;
-                    d2 = d2 + alpha * dl2 + beta * dr2;
-                    a = alpha * al;
-                    c = beta * cr;
+                };
+                vec(kCoefFw, fw);
+                vec(kCoefIb, ib);
+                vec(kCoefCb, cb);
+                vec(kCoefP, p);
+                vec(kCoefQ, q);
+                const float *e = ax.ext + static_cast<int64_t>(line) * kExtCount * 32 + lane;
+#pragma unroll
+                for (int t = 0; t < 5; t++)
+                {
+                    lo[t] = __ldg(e + (kExtLo + t) * 32);
+                    hi[t] = __ldg(e + (kExtHi + t) * 32);
                 }
-                __syncthreads();
+                binv = __ldg(e + kExtBinv * 32);
+                a = __ldg(e + kExtA * 32);
+                c = __ldg(e + kExtC * 32);
             }
-            const float y = d / b, z = d2 / b;
-            if (j == 0)
+        };
+
+        // Position n-1's value of a row (its lane's register li).
+        template <int M>
+        __device__ __forceinline__ float LastOf(const float (&u)[M], int li, int lastLane)
+        {
+            float v = 0.0f;
+#pragma unroll
+            for (int i = 0; i < M; i++)
             {
-                sx[0] = y;
-                sx[2] = z;
+                v = (i == li) ? u[i] : v;
             }
-            if (j == n - 1)
+            return __shfl_sync(kAll, v, lastLane);
+        }
+
+        // (I - L/2)^-1 d in place, from the line's factors.
+        template <int M>
+        __device__ __forceinline__ void Solve(const Axis &ax, const Factors<M> &k, int32_t line, int lane, float (&d)[M])
+        {
+#pragma unroll
+            for (int i = 1; i < M - 1; i++)
             {
-                sx[1] = y;
-                sx[3] = z;
+                d[i] = fmaf(-k.fw[i], d[i - 1], d[i]);
+            }
+            d[M - 2] *= k.ib[M - 2];
+#pragma unroll
+            for (int i = M - 3; i >= 0; i--)
+            {
+                d[i] = fmaf(-k.cb[i], d[i + 1], d[i] * k.ib[i]);
+            }
+            // the separator's equation with the lane's and the next lane's
+            // positions eliminated (a missing neighbour's multiplier is 0)
+            const float next = __shfl_down_sync(kAll, d[0], 1);
+            float r = fmaf(-k.c, next, fmaf(-k.a, d[M - 2], d[M - 1]));
+#pragma unroll
+            for (int t = 0; t < 5; t++)
+            {
+                const float lo = __shfl_up_sync(kAll, r, 1 << t);
+                const float hi = __shfl_down_sync(kAll, r, 1 << t);
+                r = fmaf(k.lo[t], lo, fmaf(k.hi[t], hi, r));
+            }
+            const float s = r * k.binv;
+            const float sl = __shfl_up_sync(kAll, s, 1);
+#pragma unroll
+            for (int i = 0; i < M - 1; i++)
+            {
+                d[i] = fmaf(-sl, k.p[i], fmaf(-s, k.q[i], d[i]));
+            }
+            d[M - 1] = s;
+            if (ax.wrap)
+            {
+                const float bog = __ldg(ax.ext + (static_cast<int64_t>(line) * kExtCount + kExtBog) * 32 + lane);
+                const float y0 = __shfl_sync(kAll, d[0], 0);
+                const float yn = LastOf<M>(d, ax.n - 1 - lane * M, (ax.n - 1) / M);
+                const float f = fmaf(bog, yn, y0);
+                const float4 *z = reinterpret_cast<const float4 *>(ax.coef) +
+                                  (static_cast<int64_t>(line) * 6 + kCoefZ) * (M / 4) * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < M / 4; j++)
+                {
+                    const float4 t = __ldg(z + j * 32);
+                    d[4 * j] = fmaf(-f, t.x, d[4 * j]);
+                    d[4 * j + 1] = fmaf(-f, t.y, d[4 * j + 1]);
+                    d[4 * j + 2] = fmaf(-f, t.z, d[4 * j + 2]);
+                    d[4 * j + 3] = fmaf(-f, t.w, d[4 * j + 3]);
+                }
+            }
+        }
+
+        // The rates of a line as face weights: face (j, j+1) carries e[j], 0
+        // at the last position (a wrapped line's last face is its own, eW).
+        template <int M>
+        __device__ __forceinline__ void MaskLast(float (&e)[M], int li)
+        {
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                e[i] = (i == li) ? 0.0f : e[i];
+            }
+        }
+
+        // out = L u along the line.
+        template <int M>
+        __device__ __forceinline__ void LapAlong(const Axis &ax, const float (&u)[M], const float (&e)[M], float eW,
+                                                 int lane, float (&out)[M])
+        {
+            float dif[M];
+            const float next = __shfl_down_sync(kAll, u[0], 1);
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                dif[i] = (i < M - 1 ? u[i < M - 1 ? i + 1 : i] : next) - u[i];
+            }
+            float below = __shfl_up_sync(kAll, e[M - 1] * dif[M - 1], 1);
+            below = lane == 0 ? 0.0f : below;
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                out[i] = fmaf(e[i], dif[i], i > 0 ? -e[i > 0 ? i - 1 : 0] * dif[i > 0 ? i - 1 : 0] : -below);
+            }
+            if (ax.wrap)
+            {
+                const int li = ax.n - 1 - lane * M;
+                const float u0 = __shfl_sync(kAll, u[0], 0);
+                const float un = LastOf<M>(u, li, (ax.n - 1) / M);
+                const float fw = eW * (u0 - un);
+                out[0] -= lane == 0 ? fw : 0.0f;
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    out[i] += (i == li) ? fw : 0.0f;
+                }
+            }
+        }
+
+        // acc[j] += -1/2 (p_j+1 - p_j)(q_j+1 - q_j), the gradient of the face
+        // above position j.
+        template <int M>
+        __device__ __forceinline__ void AddFaceGrad(const Axis &ax, const float (&p)[M], const float (&q)[M], int lane,
+                                                    float (&acc)[M])
+        {
+            const int li = ax.n - 1 - lane * M;
+            const float pn = __shfl_down_sync(kAll, p[0], 1), qn = __shfl_down_sync(kAll, q[0], 1);
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                const float dp = (i < M - 1 ? p[i < M - 1 ? i + 1 : i] : pn) - p[i];
+                const float dq = (i < M - 1 ? q[i < M - 1 ? i + 1 : i] : qn) - q[i];
+                // li and beyond: no face (or the wrapped one below)
+                acc[i] = (i < li) ? fmaf(-0.5f * dp, dq, acc[i]) : acc[i];
+            }
+            if (ax.wrap && ax.n > 1)
+            {
+                const int last = (ax.n - 1) / M;
+                const float p0 = __shfl_sync(kAll, p[0], 0), q0 = __shfl_sync(kAll, q[0], 0);
+                const float pl = LastOf<M>(p, li, last), ql = LastOf<M>(q, li, last);
+                const float g = -0.5f * (p0 - pl) * (q0 - ql);
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    acc[i] += (i == li) ? g : 0.0f;
+                }
+            }
+        }
+
+        // The CTA's lines, transposed, into out (row stride ax.ldT): four lines
+        // of one position are one 16-byte piece.  Chunks of M positions sit M +
+        // 4 floats apart, so that the lanes' 16-byte writes meet no bank
+        // conflicts.  Lines beyond the last write the zeros of the padding.
+        template <int M>
+        __device__ __forceinline__ void StoreTransposed(const Axis &ax, float (&tile)[kAdjLines][32 * (M + 4)],
+                                                        int32_t line0, bool live, int lane, const float (&v)[M],
+                                                        float *__restrict__ out)
+        {
+            float *mine = tile[threadIdx.x >> 5] + lane * (M + 4);
+#pragma unroll
+            for (int q = 0; q < M / 4; q++)
+            {
+                *reinterpret_cast<float4 *>(mine + 4 * q) =
+                    live ? make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3])
+                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
             __syncthreads();
-            const float bog = a0 / gam;
-            const float fct = (sx[0] + bog * sx[1]) / (1.0f + (sx[2] + bog * sx[3]));
-            return y - fct * z;
+            for (int32_t pos = threadIdx.x; pos < ax.n; pos += 32 * kAdjLines)
+            {
+                const int at = pos / M * (M + 4) + pos % M;
+                *reinterpret_cast<float4 *>(out + static_cast<int64_t>(pos) * ax.ldT + line0) =
+                    make_float4(tile[0][at], tile[1][at], tile[2][at], tile[3][at]);
+            }
         }
 
-        // Solves (I - L/2) x = d along the line by parallel cyclic reduction;
-        // thread j holds row j (j < n); sm holds 4 * blockDim.x floats.  SMW:
-        // the line wraps and its length is not a power of two (PcrSolveSM,
-        // which uses blockDim.x + 4 more floats after the four line arrays);
-        // a separate instantiation, so that the other line kernels keep their
-        // registers (32 against 38 with both forms in one kernel, and four
-        // 512-thread CTAs per SM).
-        template <bool SMW>
-        __device__ __forceinline__ float PcrSolve(const float *sD, float d, int32_t j, int32_t n, bool wrap, float *sm)
+        // One sweep of a forward step over the lines of an axis, in residual
+        // form: u + (I - L/2)^-1 (L + Lcross) u / 2, so that the solve's
+        // rounding scales with the step's change, not the field.
+        // x-sweep (COMMIT false): in = f by x; out = w by y (transposed), keep =
+        // w by x (or null).  y-sweep (COMMIT true): in = w by y, f by y; out =
+        // f' by x (transposed), fOut = f' by y, keep = v by y (or null).
+        template <int M, bool COMMIT>
+        __global__ void __launch_bounds__(32 * kAdjLines)
+            FwdLines(Axis ax, const float *__restrict__ in, const float *__restrict__ f, const float *__restrict__ src,
+                     const float *__restrict__ par, float *__restrict__ out, float *__restrict__ fOut,
+                     float *__restrict__ keep)
         {
-            if constexpr (SMW)
+            __shared__ __align__(16) float tile[kAdjLines][32 * (M + 4)];
+            const int lane = threadIdx.x & 31;
+            const int32_t line0 = blockIdx.x * kAdjLines;
+            const bool live = line0 + static_cast<int32_t>(threadIdx.x >> 5) < ax.nl;
+            const int32_t line = min(line0 + static_cast<int32_t>(threadIdx.x >> 5), ax.nl - 1);
+            const int li = ax.n - 1 - lane * M;
+            const bool hasUp = line + 1 < ax.nl || (ax.wrapCross && ax.nl > 1);
+            const bool hasDn = line > 0 || (ax.wrapCross && ax.nl > 1);
+            const int64_t up = hasUp ? (line + 1 < ax.nl ? line + 1 : 0) : line;
+            const int64_t dn = hasDn ? (line > 0 ? line - 1 : ax.nl - 1) : line;
+            Factors<M> k;
+            k.Load(ax, line, lane);
+            float e[M], eDn[M], f0[COMMIT ? M : 1], sv[COMMIT ? M : 1];
+            LoadRow<M>(ax.D + line * static_cast<int64_t>(ax.ld), ax.ld, lane, e);
+            LoadRow<M>(ax.D + dn * ax.ld, ax.ld, lane, eDn);
+            const float eW = ax.wrap ? __ldcg(ax.D + static_cast<int64_t>(line) * ax.ld + ax.n - 1) : 0.0f;
+            if constexpr (COMMIT)
             {
-                return PcrSolveSM(sD, d, j, n, sm, sm + 8 * blockDim.x);
-            }
-            float *sa = sm, *sb = sm + blockDim.x, *sc = sb + blockDim.x, *sd = sc + blockDim.x;
-            float a = 0.0f, b = 1.0f, c = 0.0f;
-            if (j < n)
-            {
-                float eL, eR;
-                Faces(sD, j, n, wrap, eL, eR);
-                a = -0.5f * eL;
-                c = -0.5f * eR;
-                b = 1.0f + 0.5f * (eL + eR);
-            }
-            for (int32_t delta = 1; delta < n; delta <<= 1)
-            {
-                if (j < n)
+                LoadRow<M>(f + line * static_cast<int64_t>(ax.ld), ax.ld, lane, f0);
+                if (src != nullptr)
                 {
-                    sa[j] = a;
-                    sb[j] = b;
-                    sc[j] = c;
-                    sd[j] = d;
+                    LoadRow<M>(src + line * static_cast<int64_t>(ax.ld), ax.ld, lane, sv);
                 }
-                __syncthreads();
-                if (j < n)
-                {
-                    float al = 0.0f, bl = 1.0f, cl = 0.0f, dl = 0.0f;
-                    float ar = 0.0f, br = 1.0f, cr = 0.0f, dr = 0.0f;
-                    int32_t il = j - delta, ir = j + delta;
-                    if (wrap)
-                    {
-                        il = (il < 0) ? il + n : il;
-                        ir = (ir >= n) ? ir - n : ir;
-                    }
-                    if (il >= 0)
-                    {
-                        al = sa[il];
-                        bl = sb[il];
-                        cl = sc[il];
-                        dl = sd[il];
-                    }
-                    if (ir < n)
-                    {
-                        ar = sa[ir];
-                        br = sb[ir];
-                        cr = sc[ir];
-                        dr = sd[ir];
-                    }
-                    // fast reciprocal division (about 2 ulp): the rows are
-                    // diagonally dominant, so the reduction stays well
-                    // conditioned
-                    const float alpha = -__fdividef(a, bl);
-                    const float gamma = -__fdividef(c, br);
-                    b = b + alpha * cl + gamma * ar;
-                    d = d + alpha * dl + gamma * dr;
-                    a = alpha * al;
-                    c = gamma * cr;
-                }
-                __syncthreads();
             }
-            // non-wrapped: every coupling left the line; wrapped: the last
-            // step coupled each row to itself
-            return wrap ? d / (a + b + c) : d / b;
+            const float negDecay = COMMIT ? __ldg(par + 1) : 0.0f;
+            WaitForPredecessor();
+            float c[M], d[M];
+            {
+                float uu[M], ud[M];
+                LoadRow<M>(in + line * static_cast<int64_t>(ax.ld), ax.ld, lane, c);
+                LoadRow<M>(in + up * ax.ld, ax.ld, lane, uu);
+                LoadRow<M>(in + dn * ax.ld, ax.ld, lane, ud);
+                const float wu = hasUp ? 1.0f : 0.0f, wd = hasDn ? 1.0f : 0.0f;
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    uu[i] = fmaf(wd * eDn[i], ud[i] - c[i], wu * e[i] * (uu[i] - c[i]));
+                }
+                MaskLast<M>(e, li);
+                LapAlong<M>(ax, c, e, eW, lane, d);
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    d[i] = 0.5f * (uu[i] + d[i]);
+                }
+            }
+            Solve<M>(ax, k, line, lane, d);
+            if constexpr (COMMIT)
+            {
+                float fn[M];
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    // v - f = (w - f) + e: both small, so the commit keeps the
+                    // field's precision
+                    float delta = (c[i] - f0[i]) + d[i];
+                    delta = fmaf(f0[i], negDecay, delta);
+                    delta = src != nullptr ? delta + sv[i] : delta;
+                    fn[i] = f0[i] + delta;
+                    d[i] = c[i] + d[i];
+                }
+                if (live)
+                {
+                    StoreRow<M>(fOut + line * static_cast<int64_t>(ax.ld), ax.ld, lane, fn);
+                    if (keep != nullptr)
+                    {
+                        StoreRow<M>(keep + line * static_cast<int64_t>(ax.ld), ax.ld, lane, d);
+                    }
+                }
+                StoreTransposed<M>(ax, tile, line0, live, lane, fn, out);
+            }
+            else
+            {
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    d[i] = c[i] + d[i];
+                }
+                if (live && keep != nullptr)
+                {
+                    StoreRow<M>(keep + line * static_cast<int64_t>(ax.ld), ax.ld, lane, d);
+                }
+                StoreTransposed<M>(ax, tile, line0, live, lane, d, out);
+            }
         }
+
+        // Sums of two floats (or a product) and their rounding errors.
+        __device__ __forceinline__ void AddTwo(float &hi, float &lo, float x)
+        {
+            const float s = __fadd_rn(hi, x);
+            const float b = __fsub_rn(s, hi);
+            lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
+            hi = s;
+        }
+
+        enum BwdYMode : int
+        {
+            kBwdFirst = 0,  // gbar given (the last step's output adjoint)
+            kBwdNext = 1,   // gbar = (I + Ly/2) b1bar - decay gbarPrev
+            kBwdTail = 2    // the y-stencil part of kBwdNext only (after step 0)
+        };
+
+        // Backward along y for step t: [gbar from step t+1] then the y-solve.
+        // All arrays by y, but b2bar, which leaves by x.  ddecay's sum goes to
+        // one float pair (sum, its rounding) per lane and line: FP32 pairs
+        // hold the exact products and the sum to 2^-48, without the FP64
+        // instructions that would stand on the step's critical path.
+        template <int M>
+        __global__ void __launch_bounds__(32 * kAdjLines)
+            BwdY(Axis ax, int mode, const float *__restrict__ par,
+                 const float *__restrict__ b1bar,  // step t+1's x-solve adjoint (kBwdNext/Tail)
+                 const float *__restrict__ gPrev,  // adjoint of f_t+2 (kBwdNext/Tail), or gbar (kBwdFirst)
+                 const float *__restrict__ fNext,  // f_t+1 (kBwdNext/Tail)
+                 const float *__restrict__ fT,     // f_t (input of step t)
+                 const float *__restrict__ vT,     // v_t
+                 float *__restrict__ gOut,         // adjoint of f_t+1 (gbar of step t)
+                 float *__restrict__ b2bar, float *__restrict__ dD, float *__restrict__ dS,
+                 float2 *__restrict__ dDecay)
+        {
+            __shared__ __align__(16) float tile[kAdjLines][32 * (M + 4)];
+            const int lane = threadIdx.x & 31;
+            const int32_t line0 = blockIdx.x * kAdjLines;
+            const bool live = line0 + static_cast<int32_t>(threadIdx.x >> 5) < ax.nl;
+            const int32_t line = min(line0 + static_cast<int32_t>(threadIdx.x >> 5), ax.nl - 1);
+            const int64_t row = line * static_cast<int64_t>(ax.ld);
+            Factors<M> k;
+            k.Load(ax, line, lane);
+            float e[M], g[M], acc[M], q[M], t[M];
+            LoadRow<M>(ax.D + row, ax.ld, lane, e);
+            const float eW = ax.wrap ? __ldcg(ax.D + row + ax.n - 1) : 0.0f;
+            MaskLast<M>(e, ax.n - 1 - lane * M);
+            const float decay = __ldg(par);
+            LoadRow<M>(gPrev + row, ax.ld, lane, g);
+            LoadRow<M>(fNext + row, ax.ld, lane, q);
+            // this step's terms of dD, small beside the sum so far
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                acc[i] = 0.0f;
+            }
+            WaitForPredecessor();
+            if (mode != kBwdFirst)
+            {
+                float b[M];
+                LoadRow<M>(b1bar + row, ax.ld, lane, b);
+                LapAlong<M>(ax, b, e, eW, lane, t);
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    g[i] = fmaf(0.5f, t[i], b[i]) - decay * g[i];
+                }
+                AddFaceGrad<M>(ax, b, q, lane, acc);
+                if (mode == kBwdTail)
+                {
+                    if (live)
+                    {
+                        AddRow<M>(dD + row, ax.ld, lane, acc);
+                    }
+                    return;
+                }
+            }
+            // residual form: b2bar = gbar + (I - Ly/2)^-1 (Ly gbar) / 2
+            float d[M];
+            LapAlong<M>(ax, g, e, eW, lane, d);
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                d[i] *= 0.5f;
+            }
+            Solve<M>(ax, k, line, lane, d);
+            // the accumulators' rows, in flight during the write-out (the
+            // factors' registers are free now)
+            float sD[M], sS[M], ft[M];
+            LoadRow<M>(vT + row, ax.ld, lane, q);
+            LoadRow<M>(dD + row, ax.ld, lane, sD);
+            LoadRow<M>(dS + row, ax.ld, lane, sS);
+            LoadRow<M>(fT + row, ax.ld, lane, ft);
+            float2 sum = __ldcg(dDecay + static_cast<int64_t>(line) * 32 + lane);
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                d[i] += g[i];
+            }
+            StoreTransposed<M>(ax, tile, line0, live, lane, d, b2bar);
+            AddFaceGrad<M>(ax, d, q, lane, acc);
+            if (!live)
+            {
+                return;
+            }
+            StoreRow<M>(gOut + row, ax.ld, lane, g);
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                sD[i] += acc[i];
+                sS[i] += g[i];
+                const float p = __fmul_rn(-g[i], ft[i]);
+                const float pe = __fmaf_rn(-g[i], ft[i], -p);
+                AddTwo(sum.x, sum.y, p);
+                sum.y = __fadd_rn(sum.y, pe);
+            }
+            StoreRow<M>(dD + row, ax.ld, lane, sD);
+            StoreRow<M>(dS + row, ax.ld, lane, sS);
+            const float s = __fadd_rn(sum.x, sum.y);
+            sum.y = __fsub_rn(sum.y, __fsub_rn(s, sum.x));
+            sum.x = s;
+            dDecay[static_cast<int64_t>(line) * 32 + lane] = sum;
+        }
+
+        // Backward along x for step t: wbar = (I + Lx/2) b2bar, b1bar = (I - Lx/2)^-1 wbar.
+        // All arrays by x, but b1bar, which leaves by y.
+        template <int M>
+        __global__ void __launch_bounds__(32 * kAdjLines)
+            BwdX(Axis ax, const float *__restrict__ b2bar, const float *__restrict__ wT, float *__restrict__ b1bar,
+                 float *__restrict__ dD)
+        {
+            __shared__ __align__(16) float tile[kAdjLines][32 * (M + 4)];
+            const int lane = threadIdx.x & 31;
+            const int32_t line0 = blockIdx.x * kAdjLines;
+            const bool live = line0 + static_cast<int32_t>(threadIdx.x >> 5) < ax.nl;
+            const int32_t line = min(line0 + static_cast<int32_t>(threadIdx.x >> 5), ax.nl - 1);
+            const int64_t row = line * static_cast<int64_t>(ax.ld);
+            Factors<M> k;
+            k.Load(ax, line, lane);
+            float e[M], w[M], acc[M], b[M], l[M], d[M];
+            LoadRow<M>(ax.D + row, ax.ld, lane, e);
+            const float eW = ax.wrap ? __ldcg(ax.D + row + ax.n - 1) : 0.0f;
+            MaskLast<M>(e, ax.n - 1 - lane * M);
+            LoadRow<M>(wT + row, ax.ld, lane, w);
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                acc[i] = 0.0f;
+            }
+            WaitForPredecessor();
+            LoadRow<M>(b2bar + row, ax.ld, lane, b);
+            LapAlong<M>(ax, b, e, eW, lane, l);
+            // residual form: b1bar = wbar + (I - Lx/2)^-1 (Lx wbar) / 2, with
+            // Lx wbar = Lx b2bar + Lx (Lx b2bar) / 2
+            LapAlong<M>(ax, l, e, eW, lane, d);
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                d[i] = 0.5f * fmaf(0.5f, d[i], l[i]);
+            }
+            Solve<M>(ax, k, line, lane, d);
+            float sD[M];
+            LoadRow<M>(dD + row, ax.ld, lane, sD);
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                d[i] += fmaf(0.5f, l[i], b[i]);
+            }
+            StoreTransposed<M>(ax, tile, line0, live, lane, d, b1bar);
+            AddFaceGrad<M>(ax, b, w, lane, acc);
+            AddFaceGrad<M>(ax, d, w, lane, acc);
+            if (live)
+            {
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    sD[i] += acc[i];
+                }
+                StoreRow<M>(dD + row, ax.ld, lane, sD);
+            }
+        }
+
+        // ---- the factors -----------------------------------------------------
+
+        // Factors every line of an axis (one warp a line, FP64): see the top of
+        // this file.  Positions beyond the line are rows of the identity.
+        template <int M>
+        __global__ void __launch_bounds__(32 * kAdjLines) Factor(Axis ax, float *__restrict__ coef, float *__restrict__ ext)
+        {
+            const int lane = threadIdx.x & 31;
+            const int32_t line = blockIdx.x * kAdjLines + static_cast<int32_t>(threadIdx.x >> 5);
+            if (line >= ax.nl)
+            {
+                return;
+            }
+            const float *D = ax.D + static_cast<int64_t>(line) * ax.ld;
+            const int32_t n = ax.n;
+            // a wrapped pair has two faces between its cells, a wrapped single
+            // cell couples only to itself (L = 0); longer wrapped lines are
+            // split as T + u v^T
+            const bool split = ax.wrap && n >= 3;
+            const double eW = split ? static_cast<double>(D[n - 1]) : 0.0;
+            auto face = [&](int32_t j)  // face (j, j+1) within the line
+            {
+                if (j < 0 || j >= n - 1)
+                {
+                    return 0.0;
+                }
+                return static_cast<double>(D[j]) + ((ax.wrap && n == 2) ? static_cast<double>(D[1]) : 0.0);
+            };
+            const double a0 = -0.5 * eW;  // row 0's coefficient of x_n-1, and row n-1's of x_0
+            const double gamma = -(1.0 + 0.5 * (eW + face(0)));
+            double a[M], b[M], c[M];
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                const int32_t j = lane * M + i;
+                const double lo = face(j - 1), hi = face(j);
+                a[i] = (j < n) ? -0.5 * lo : 0.0;
+                c[i] = (j < n) ? -0.5 * hi : 0.0;
+                b[i] = 1.0;
+                if (j < n)
+                {
+                    b[i] = 1.0 + 0.5 * (lo + hi + ((j == 0 || j == n - 1) ? eW : 0.0));
+                    if (split && j == 0)
+                    {
+                        b[i] -= gamma;
+                    }
+                    if (split && j == n - 1)
+                    {
+                        b[i] -= a0 * a0 / gamma;
+                    }
+                }
+            }
+            double fw[M], ib[M], cb[M], p[M], q[M];
+            double bp = b[0];
+            fw[0] = 0.0;
+            ib[0] = 1.0 / bp;
+#pragma unroll
+            for (int i = 1; i < M - 1; i++)
+            {
+                fw[i] = a[i] * ib[i - 1];
+                bp = b[i] - fw[i] * c[i - 1];
+                ib[i] = 1.0 / bp;
+            }
+#pragma unroll
+            for (int i = 0; i < M - 1; i++)
+            {
+                cb[i] = (i < M - 2) ? c[i] * ib[i] : 0.0;
+            }
+            fw[M - 1] = ib[M - 1] = cb[M - 1] = 0.0;
+            // p = A^-1 (a_0 e_0), q = A^-1 (c_M-2 e_M-2)
+            p[0] = a[0];
+#pragma unroll
+            for (int i = 1; i < M - 1; i++)
+            {
+                p[i] = -fw[i] * p[i - 1];
+            }
+            q[M - 2] = c[M - 2] * ib[M - 2];
+            p[M - 2] *= ib[M - 2];
+#pragma unroll
+            for (int i = M - 3; i >= 0; i--)
+            {
+                p[i] = p[i] * ib[i] - cb[i] * p[i + 1];
+                q[i] = -cb[i] * q[i + 1];
+            }
+            p[M - 1] = q[M - 1] = 0.0;
+            const double as = a[M - 1], cs = lane < 31 ? c[M - 1] : 0.0;
+            const double pn = __shfl_down_sync(kAll, p[0], 1), qn = __shfl_down_sync(kAll, q[0], 1);
+            double A = -as * p[M - 2], B = b[M - 1] - as * q[M - 2] - cs * pn, C = -cs * qn;
+            double lo[5], hi[5];
+#pragma unroll
+            for (int t = 0; t < 5; t++)
+            {
+                const int s = 1 << t;
+                const double al = __shfl_up_sync(kAll, A, s), bl = __shfl_up_sync(kAll, B, s),
+                             cl = __shfl_up_sync(kAll, C, s);
+                const double ar = __shfl_down_sync(kAll, A, s), br = __shfl_down_sync(kAll, B, s),
+                             cr = __shfl_down_sync(kAll, C, s);
+                lo[t] = lane >= s ? -A / bl : 0.0;
+                hi[t] = lane + s < 32 ? -C / br : 0.0;
+                B += (lane >= s ? lo[t] * cl : 0.0) + (lane + s < 32 ? hi[t] * ar : 0.0);
+                A = lane >= s ? lo[t] * al : 0.0;
+                C = lane + s < 32 ? hi[t] * cr : 0.0;
+            }
+            const double binv = 1.0 / B;
+            const int nc = ax.wrap ? 6 : 5;
+            float *o = coef + static_cast<int64_t>(line) * nc * M * 32 + 4 * lane;
+            auto put = [&](int k, const double (&v)[M])
+            {
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    o[(k * (M / 4) + i / 4) * 128 + (i & 3)] = static_cast<float>(v[i]);
+                }
+            };
+            put(kCoefFw, fw);
+            put(kCoefIb, ib);
+            put(kCoefCb, cb);
+            put(kCoefP, p);
+            put(kCoefQ, q);
+            double bog = 0.0;
+            if (ax.wrap)
+            {
+                double z[M];
+#pragma unroll
+                for (int i = 0; i < M; i++)
+                {
+                    z[i] = 0.0;
+                }
+                if (split)
+                {
+                    // T z = u = (gamma, 0, .., 0, a0)
+                    bog = a0 / gamma;
+#pragma unroll
+                    for (int i = 0; i < M; i++)
+                    {
+                        const int32_t j = lane * M + i;
+                        z[i] = (j == 0) ? gamma : ((j == n - 1) ? a0 : 0.0);
+                    }
+#pragma unroll
+                    for (int i = 1; i < M - 1; i++)
+                    {
+                        z[i] -= fw[i] * z[i - 1];
+                    }
+                    z[M - 2] *= ib[M - 2];
+#pragma unroll
+                    for (int i = M - 3; i >= 0; i--)
+                    {
+                        z[i] = z[i] * ib[i] - cb[i] * z[i + 1];
+                    }
+                    double r = z[M - 1] - as * z[M - 2] - cs * __shfl_down_sync(kAll, z[0], 1);
+#pragma unroll
+                    for (int t = 0; t < 5; t++)
+                    {
+                        const double rl = __shfl_up_sync(kAll, r, 1 << t), rr = __shfl_down_sync(kAll, r, 1 << t);
+                        r += lo[t] * rl + hi[t] * rr;
+                    }
+                    const double s = r * binv;
+                    double sl = __shfl_up_sync(kAll, s, 1);
+                    sl = lane == 0 ? 0.0 : sl;
+#pragma unroll
+                    for (int i = 0; i < M - 1; i++)
+                    {
+                        z[i] -= sl * p[i] + s * q[i];
+                    }
+                    z[M - 1] = s;
+                    double zn = 0.0;
+#pragma unroll
+                    for (int i = 0; i < M; i++)
+                    {
+                        zn = (lane * M + i == n - 1) ? z[i] : zn;
+                    }
+                    zn = __shfl_sync(kAll, zn, (n - 1) / M);
+                    const double den = 1.0 + __shfl_sync(kAll, z[0], 0) + bog * zn;
+#pragma unroll
+                    for (int i = 0; i < M; i++)
+                    {
+                        z[i] /= den;
+                    }
+                }
+                put(kCoefZ, z);
+            }
+            float *x = ext + static_cast<int64_t>(line) * kExtCount * 32 + lane;
+#pragma unroll
+            for (int t = 0; t < 5; t++)
+            {
+                x[(kExtLo + t) * 32] = static_cast<float>(lo[t]);
+                x[(kExtHi + t) * 32] = static_cast<float>(hi[t]);
+            }
+            x[kExtBinv * 32] = static_cast<float>(binv);
+            x[kExtA * 32] = static_cast<float>(as);
+            x[kExtC * 32] = static_cast<float>(cs);
+            x[kExtBog * 32] = static_cast<float>(bog);
+        }
+
+        // ---- the rest of a call --------------------------------------------
+
+        constexpr int kLossThreads = 256;
+        constexpr int kLossBlocks = 1024;
 
         __device__ __forceinline__ double BlockSum(double v, double *sred)
         {
             for (int o = 16; o > 0; o >>= 1)
             {
-                v += __shfl_down_sync(0xffffffffu, v, o);
+                v += __shfl_down_sync(kAll, v, o);
             }
             const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
             __syncthreads();
@@ -365,115 +879,10 @@ namespace halcuda
             return t;
         }
 
-        // A wrapped line of length n that is not a power of two: its solve is
-        // the Sherman-Morrison form (the line kernels' SMW instantiation).
-        __host__ __device__ constexpr bool SmLine(int32_t n, bool wrap)
-        {
-            return wrap && n > 2 && (n & (n - 1)) != 0;
-        }
-
-        // Shared memory of the line kernels: 4 PCR arrays + 4 line arrays,
-        // and for an SmLine the second right-hand side and the broadcast
-        // values of PcrSolveSM.
-        __host__ __device__ constexpr size_t LineSmemFloats(int threads, int32_t n, bool wrap)
-        {
-            return SmLine(n, wrap) ? 9 * static_cast<size_t>(threads) + 4 : 8 * static_cast<size_t>(threads);
-        }
-
-        // x-sweep: w = (I - Lx/2)^-1 (I + Ly/2) f, one CTA per line y, in
-        // residual form: w = f + (I - Lx/2)^-1 (Lx + Ly) f / 2, so that the
-        // solve's rounding scales with the step's change, not the field.  The
-        // rates come from DT (D transposed), contiguous along the line.  w is
-        // written in HAL's layout for the y-sweep, and, when wB is set, also
-        // line by line (wB[y * xDim + x]) as the state the backward x-kernel
-        // reads along the same lines.
-        template <bool SMW>
-        __global__ void FwdX(Grid g, const float *__restrict__ f, const float *__restrict__ DT, float *__restrict__ w,
-                             float *__restrict__ wB)
-        {
-            extern __shared__ float sm[];
-            float *sD = sm + 4 * blockDim.x;
-            float *su = sD + blockDim.x;
-            const int32_t line = blockIdx.x;
-            const int32_t n = g.xDim;
-            const int32_t j = threadIdx.x;
-            float c = 0.0f, lap = 0.0f;
-            if (j < n)
-            {
-                const int64_t i = Idx<kDirX>(g, line, j);
-                sD[j] = DT[static_cast<int64_t>(line) * n + j];
-                c = f[i];
-                su[j] = c;
-                lap = LapCrossXT(g, f, DT, line, j, c);
-            }
-            __syncthreads();
-            if (j < n)
-            {
-                lap += LapAlong(su, sD, j, n, g.wrapX != 0);
-            }
-            const float e = PcrSolve<SMW>(sD, 0.5f * lap, j, n, g.wrapX != 0, sm);
-            if (j < n)
-            {
-                w[Idx<kDirX>(g, line, j)] = c + e;
-                if (wB != nullptr)
-                {
-                    wB[static_cast<int64_t>(line) * n + j] = c + e;
-                }
-            }
-        }
-
-        // y-sweep and commit: v = (I - Ly/2)^-1 (I + Lx/2) w,
-        // f' = f + (((v - f) + f*(-decay)) + src); v is kept when vOut != null.
-        template <bool SMW>
-        __global__ void FwdY(Grid g, const float *__restrict__ w, const float *__restrict__ f,
-                             const float *__restrict__ D, const float *__restrict__ src, float negDecay,
-                             float *__restrict__ fOut, float *__restrict__ vOut)
-        {
-            extern __shared__ float sm[];
-            float *sD = sm + 4 * blockDim.x;
-            float *su = sD + blockDim.x;
-            const int32_t line = blockIdx.x;
-            const int32_t n = g.yDim;
-            const int32_t j = threadIdx.x;
-            float c = 0.0f, lap = 0.0f;
-            if (j < n)
-            {
-                const int64_t i = Idx<kDirY>(g, line, j);
-                sD[j] = D[i];
-                c = w[i];
-                su[j] = c;
-                lap = LapCross<kDirY>(g, w, D, line, j, c);
-            }
-            __syncthreads();
-            if (j < n)
-            {
-                lap += LapAlong(su, sD, j, n, g.wrapY != 0);
-            }
-            // residual form: v = w + (I - Ly/2)^-1 (Lx + Ly) w / 2
-            const float e = PcrSolve<SMW>(sD, 0.5f * lap, j, n, g.wrapY != 0, sm);
-            if (j < n)
-            {
-                const int64_t i = Idx<kDirY>(g, line, j);
-                const float f0 = f[i];
-                // v - f = (w - f) + e: both small, so the commit keeps the
-                // field's precision
-                float delta = (c - f0) + e;
-                delta = delta + f0 * negDecay;
-                if (src != nullptr)
-                {
-                    delta = delta + src[i];
-                }
-                fOut[i] = f0 + delta;
-                if (vOut != nullptr)
-                {
-                    vOut[i] = c + e;
-                }
-            }
-        }
-
-        // loss += 1/2 (f - target)^2; gbar = f - target.
-        __global__ void LossGrad(int64_t n, const float *__restrict__ f, const float *__restrict__ target,
-                                 float *__restrict__ gbar, double *__restrict__ loss)
+        // part[block] = sum of 1/2 (f - target)^2; gbar = f - target.
+        __global__ void __launch_bounds__(kLossThreads)
+            LossGrad(int64_t n, const float *__restrict__ f, const float *__restrict__ target,
+                     float *__restrict__ gbar, double *__restrict__ part)
         {
             __shared__ double sred[32];
             double acc = 0.0;
@@ -490,185 +899,108 @@ namespace halcuda
             const double t = BlockSum(acc, sred);
             if (threadIdx.x == 0)
             {
-                atomicAdd(loss, t);
+                part[blockIdx.x] = t;
             }
         }
 
-        enum BwdYMode : int
+        // acc[0] = sum of part; acc[1] = sum of the pairs (one CTA, a fixed
+        // order).
+        __global__ void __launch_bounds__(1024)
+            Totals(const double *__restrict__ part, int32_t nPart, const float2 *__restrict__ pairs, int64_t nPairs,
+                   double *__restrict__ acc)
         {
-            kBwdFirst = 0,  // gbar given (the last step's output adjoint)
-            kBwdNext = 1,   // gbar = (I + Ly/2) b1bar - decay gbarPrev
-            kBwdTail = 2    // the y-stencil part of kBwdNext only (after step 0)
-        };
-
-        // Backward along y for step t: [gbar from step t+1] then the y-solve.
-        template <bool SMW>
-        __global__ void BwdY(Grid g, int mode, const float *__restrict__ D, float decay,
-                             const float *__restrict__ b1bar,     // step t+1's x-solve adjoint (kBwdNext/Tail)
-                             const float *__restrict__ gPrev,     // adjoint of f_t+2 (kBwdNext/Tail), or gbar (kBwdFirst)
-                             const float *__restrict__ fNext,     // f_t+1 (kBwdNext/Tail)
-                             const float *__restrict__ fT,        // f_t (input of step t)
-                             const float *__restrict__ vT,        // v_t
-                             float *__restrict__ gOut,            // adjoint of f_t+1 (gbar of step t)
-                             float *__restrict__ b2bar, float *__restrict__ dD, float *__restrict__ dS,
-                             double *__restrict__ dDecay)
-        {
-            extern __shared__ float sm[];
-            float *sD = sm + 4 * blockDim.x;
-            float *sp = sD + blockDim.x;
-            float *sq = sp + blockDim.x;
-            float *sr = sq + blockDim.x;
             __shared__ double sred[32];
-            const int32_t line = blockIdx.x;
-            const int32_t n = g.yDim;
-            const bool wrap = g.wrapY != 0;
-            const int32_t j = threadIdx.x;
-            const int64_t i = (j < n) ? Idx<kDirY>(g, line, j) : 0;
-            float gbar = 0.0f, dDacc = 0.0f;
-            if (j < n)
+            double a = 0.0, b = 0.0;
+            for (int32_t i = threadIdx.x; i < nPart; i += blockDim.x)
             {
-                sD[j] = D[i];
-                if (mode == kBwdFirst)
-                {
-                    gbar = gPrev[i];
-                }
-                else
-                {
-                    sp[j] = b1bar[i];
-                    sq[j] = fNext[i];
-                }
+                a += part[i];
             }
-            __syncthreads();
-            if (mode != kBwdFirst)
+            for (int64_t i = threadIdx.x; i < nPairs; i += blockDim.x)
             {
-                if (j < n)
-                {
-                    gbar = (sp[j] + 0.5f * LapAlong(sp, sD, j, n, wrap)) - decay * gPrev[i];
-                    dDacc += FaceGrad(sp, sq, j, n, wrap);
-                }
-                if (mode == kBwdTail)
-                {
-                    if (j < n)
-                    {
-                        dD[i] += dDacc;
-                    }
-                    return;
-                }
+                b += static_cast<double>(pairs[i].x) + static_cast<double>(pairs[i].y);
             }
-            double kacc = 0.0;
-            if (j < n)
-            {
-                dS[i] += gbar;
-                kacc = -static_cast<double>(gbar) * static_cast<double>(fT[i]);
-                gOut[i] = gbar;
-            }
-            const double ksum = BlockSum(kacc, sred);
+            a = BlockSum(a, sred);
+            b = BlockSum(b, sred);
             if (threadIdx.x == 0)
             {
-                atomicAdd(dDecay, ksum);
-            }
-            // residual form: b2bar = gbar + (I - Ly/2)^-1 (Ly gbar) / 2
-            if (j < n)
-            {
-                sq[j] = gbar;
-            }
-            __syncthreads();
-            const float lapg = (j < n) ? LapAlong(sq, sD, j, n, wrap) : 0.0f;
-            const float x = gbar + PcrSolve<SMW>(sD, 0.5f * lapg, j, n, wrap, sm);
-            if (j < n)
-            {
-                sp[j] = x;
-                sr[j] = vT[i];
-            }
-            __syncthreads();
-            if (j < n)
-            {
-                dDacc += FaceGrad(sp, sr, j, n, wrap);
-                b2bar[i] = x;
-                dD[i] += dDacc;
+                acc[0] = a;
+                acc[1] = b;
             }
         }
 
-        // Backward along x for step t: wbar = (I + Lx/2) b2bar, b1bar = (I - Lx/2)^-1 wbar.
-        // The rates DT, the state wB and the x-face gradient dDT are all
-        // line by line (y * xDim + x), contiguous along the CTA's line; only
-        // b2bar and b1bar, which the y-kernels read and write, are strided.
-        template <bool SMW>
-        __global__ void BwdX(Grid g, const float *__restrict__ DT, const float *__restrict__ b2bar,
-                             const float *__restrict__ wB, float *__restrict__ b1bar, float *__restrict__ dDT)
-        {
-            extern __shared__ float sm[];
-            float *sD = sm + 4 * blockDim.x;
-            float *sp = sD + blockDim.x;
-            float *sw = sp + blockDim.x;
-            const int32_t line = blockIdx.x;
-            const int32_t n = g.xDim;
-            const bool wrap = g.wrapX != 0;
-            const int32_t j = threadIdx.x;
-            const int64_t i = (j < n) ? Idx<kDirX>(g, line, j) : 0;
-            const int64_t iB = static_cast<int64_t>(line) * n + j;
-            if (j < n)
-            {
-                sD[j] = DT[iB];
-                sp[j] = b2bar[i];
-                sw[j] = wB[iB];
-            }
-            __syncthreads();
-            float wbar = 0.0f, dDacc = 0.0f, lapb = 0.0f;
-            if (j < n)
-            {
-                lapb = LapAlong(sp, sD, j, n, wrap);
-                wbar = sp[j] + 0.5f * lapb;
-                dDacc = FaceGrad(sp, sw, j, n, wrap);
-            }
-            // residual form: b1bar = wbar + (I - Lx/2)^-1 (Lx wbar) / 2, with
-            // Lx wbar = Lx b2bar + Lx (Lx b2bar) / 2
-            float *sl = sw + blockDim.x;
-            if (j < n)
-            {
-                sl[j] = lapb;
-            }
-            __syncthreads();
-            const float lapw = (j < n) ? lapb + 0.5f * LapAlong(sl, sD, j, n, wrap) : 0.0f;
-            __syncthreads();
-            const float x = wbar + PcrSolve<SMW>(sD, 0.5f * lapw, j, n, wrap, sm);
-            if (j < n)
-            {
-                sp[j] = x;
-            }
-            __syncthreads();
-            if (j < n)
-            {
-                dDacc += FaceGrad(sp, sw, j, n, wrap);
-                b1bar[i] = x;
-                dDT[iB] += dDacc;
-            }
-        }
-
-        // dD(x, y) += dDT[y * xDim + x]: the x-faces' gradient, accumulated
-        // line by line, added into HAL's layout through a 32 x 32 tile.
-        __global__ void AddTransposed(float *__restrict__ dD, const float *__restrict__ dDT, int32_t xDim,
-                                      int32_t yDim)
+        // out[c * ldOut + r] (+)= in[r * ldIn + c], rows x cols.
+        template <bool ADD>
+        __global__ void TransposeRows(const float *__restrict__ in, int32_t ldIn, float *__restrict__ out, int32_t ldOut,
+                                      int32_t rows, int32_t cols)
         {
             __shared__ float tile[32][33];
-            const int32_t x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-            for (int32_t r = threadIdx.y; r < 32; r += blockDim.y)
+            const int32_t r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+            for (int32_t k = threadIdx.y; k < 32; k += blockDim.y)
             {
-                const int32_t y = y0 + r, x = x0 + threadIdx.x;
-                if (y < yDim && x < xDim)
+                const int32_t r = r0 + k, c = c0 + threadIdx.x;
+                if (r < rows && c < cols)
                 {
-                    tile[r][threadIdx.x] = dDT[static_cast<int64_t>(y) * xDim + x];
+                    tile[k][threadIdx.x] = in[static_cast<int64_t>(r) * ldIn + c];
                 }
             }
             __syncthreads();
-            for (int32_t r = threadIdx.y; r < 32; r += blockDim.y)
+            for (int32_t k = threadIdx.y; k < 32; k += blockDim.y)
             {
-                const int32_t x = x0 + r, y = y0 + threadIdx.x;
-                if (x < xDim && y < yDim)
+                const int32_t c = c0 + k, r = r0 + threadIdx.x;
+                if (r < rows && c < cols)
                 {
-                    dD[static_cast<int64_t>(x) * yDim + y] += tile[threadIdx.x][r];
+                    float *o = out + static_cast<int64_t>(c) * ldOut + r;
+                    *o = ADD ? *o + tile[threadIdx.x][k] : tile[threadIdx.x][k];
                 }
             }
+        }
+
+        // Positions per lane of a line: M = 4 * ceil(n / 128).
+        constexpr int32_t LaneLen(int32_t n)
+        {
+            return (n + 127) / 128 * 4;
+        }
+
+        // Calls fn with M as a compile-time constant.
+        template <typename Fn>
+        auto WithLaneLen(int32_t m, Fn fn)
+        {
+            switch (m / 4)
+            {
+            case 1:
+                return fn(std::integral_constant<int, 4>());
+            case 2:
+                return fn(std::integral_constant<int, 8>());
+            case 3:
+                return fn(std::integral_constant<int, 12>());
+            case 4:
+                return fn(std::integral_constant<int, 16>());
+            case 5:
+                return fn(std::integral_constant<int, 20>());
+            case 6:
+                return fn(std::integral_constant<int, 24>());
+            case 7:
+                return fn(std::integral_constant<int, 28>());
+            default:
+                return fn(std::integral_constant<int, 32>());
+            }
+        }
+
+        // Launches `kernel`, as a programmatic dependent of the kernel before
+        // it in the stream if chained.
+        template <typename... P, typename... A>
+        int LaunchChained(void (*kernel)(P...), int32_t nl, bool chained, cudaStream_t s, A... args)
+        {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(static_cast<unsigned>((nl + kAdjLines - 1) / kAdjLines));
+            cfg.blockDim = dim3(32 * kAdjLines);
+            cfg.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = chained ? 1 : 0;
+            return CudaStatus(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), "adjoint launch");
         }
     }
 
@@ -676,31 +1008,48 @@ namespace halcuda
     {
         int device = 0;
         StreamSlot stream;
-        Grid g{};
-        int64_t n = 0;
+        int32_t xDim = 0, yDim = 0, ldX = 0, ldY = 0;
+        Axis axX{}, axY{};                  // x-lines (by x) and y-lines (by y)
+        int64_t n = 0;                      // cells
+        size_t nA = 0, nB = 0;              // padded array sizes, by y and by x
         int32_t steps = 0, every = 1;
         bool keepAll = false;               // checkpoint interval 0: every state kept, nothing recomputed
         bool hasProblem = false;
-        DevBuf<float> f0, target, D, src;
+        // by y: the problem, the fields, the adjoints (but b2), the y-faces'
+        // part of dL/dD
+        DevBuf<float> f0, target, D, src, work[2], wA, gA, gB, b1, dD, dS;
         DevBuf<float> ckpt;                 // checkpoints: one field every `every` steps
-        DevBuf<float> segF[2], segW[2], segV[2];  // states of a segment, double-buffered
+        DevBuf<float> segF[2], segV[2];     // states of a segment, double-buffered
+        // by x: the rates, the current field, b2, the x-faces' part of dL/dD,
+        // and the w of a segment
+        DevBuf<float> DT, fB, b2, dDT;
+        DevBuf<float> segW[2];
         StreamSlot recomputeStream;         // recomputes segment s-1 while segment s is differentiated
-        DevBuf<float> work[2];              // forward ping-pong
-        DevBuf<float> gA, gB, b1, b2, dD, dS;
-        // line-by-line (y * xDim + x) copies for the x-kernels: the rates,
-        // the x-faces' part of dL/dD, and the x-sweep's w in HAL's layout for
-        // the y-sweep (scratch: the forward on the main stream and the
-        // recomputations on the second one never run at the same time)
-        DevBuf<float> DT, dDT, wA;
-        DevBuf<double> acc;                 // [0] loss, [1] d loss / d decay
+        DevBuf<float> coefX, extX, coefY, extY;
+        DevBuf<float> par;                  // decay, -decay
+        DevBuf<float2> dDecay;              // BwdY's sums
+        DevBuf<double> part, acc;           // the loss's partial sums; [0] loss, [1] d loss / d decay
         float msForward = 0.0f, msGradient = 0.0f;
+        // runs of steps as graphs (the pointers are the problem's): see Replay
+        std::map<std::string, std::pair<cudaGraphExec_t, int64_t>> graphs;
+
+        ~Adjoint() { DropGraphs(); }
+
+        void DropGraphs()
+        {
+            for (auto &g : graphs)
+            {
+                cudaGraphExecDestroy(g.second.first);
+            }
+            graphs.clear();
+        }
 
         int32_t Segments() const
         {
             return (steps + every - 1) / every;
         }
 
-        int Init(int32_t xDim, int32_t yDim, int32_t wrapX, int32_t wrapY)
+        int Init(int32_t xd, int32_t yd, int32_t wrapX, int32_t wrapY)
         {
             device = CurrentDevice();
             HAL_TRY(CudaStatus(cudaSetDevice(device), "cudaSetDevice"));
@@ -711,112 +1060,295 @@ namespace halcuda
             HAL_TRY(CudaStatus(cudaDeviceGetStreamPriorityRange(&least, &greatest), "cudaDeviceGetStreamPriorityRange"));
             HAL_TRY(stream.Create("cudaStreamCreate", greatest));
             HAL_TRY(recomputeStream.Create("cudaStreamCreate", least));
-            g.xDim = xDim;
-            g.yDim = yDim;
-            g.wrapX = wrapX != 0;
-            g.wrapY = wrapY != 0;
+            xDim = xd;
+            yDim = yd;
+            ldX = (xDim + 3) & ~3;
+            ldY = (yDim + 3) & ~3;
             n = static_cast<int64_t>(xDim) * yDim;
-            const size_t m = static_cast<size_t>(n);
-            HAL_TRY(f0.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(target.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(D.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(src.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(work[0].Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(work[1].Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(gA.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(gB.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(b1.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(b2.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(dD.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(DT.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(dDT.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(wA.Alloc(m, "cudaMalloc(adjoint)"));
-            HAL_TRY(dS.Alloc(m, "cudaMalloc(adjoint)"));
+            nA = static_cast<size_t>(xDim) * ldY;
+            nB = static_cast<size_t>(yDim) * ldX;
+            for (DevBuf<float> *b : {&f0, &target, &D, &src, &work[0], &work[1], &wA, &gA, &gB, &b1, &dD, &dS})
+            {
+                HAL_TRY(Zeroed(*b, nA));
+            }
+            for (DevBuf<float> *b : {&DT, &fB, &b2, &dDT})
+            {
+                HAL_TRY(Zeroed(*b, nB));
+            }
+            const size_t mx = static_cast<size_t>(LaneLen(xDim)), my = static_cast<size_t>(LaneLen(yDim));
+            HAL_TRY(coefX.Alloc(static_cast<size_t>(yDim) * (wrapX ? 6 : 5) * mx * 32, "cudaMalloc(adjoint)"));
+            HAL_TRY(coefY.Alloc(static_cast<size_t>(xDim) * (wrapY ? 6 : 5) * my * 32, "cudaMalloc(adjoint)"));
+            HAL_TRY(extX.Alloc(static_cast<size_t>(yDim) * kExtCount * 32, "cudaMalloc(adjoint)"));
+            HAL_TRY(extY.Alloc(static_cast<size_t>(xDim) * kExtCount * 32, "cudaMalloc(adjoint)"));
+            HAL_TRY(par.Alloc(2, "cudaMalloc(adjoint)"));
+            HAL_TRY(dDecay.Alloc(static_cast<size_t>(xDim) * 32, "cudaMalloc(adjoint)"));
+            HAL_TRY(part.Alloc(kLossBlocks, "cudaMalloc(adjoint)"));
             HAL_TRY(acc.Alloc(2, "cudaMalloc(adjoint)"));
+            axX = Axis{xDim, yDim, ldX, ldY, wrapX != 0, wrapY != 0, DT.p, coefX.p, extX.p};
+            axY = Axis{yDim, xDim, ldY, ldX, wrapY != 0, wrapX != 0, D.p, coefY.p, extY.p};
             return HAL_CUDA_OK;
         }
 
-        static int Threads(int32_t len)
+        // A zeroed buffer: the padding stays zero from here on.
+        static int Zeroed(DevBuf<float> &b, size_t count)
         {
-            return (len + 31) & ~31;
+            HAL_TRY(b.Alloc(count, "cudaMalloc(adjoint)"));
+            return CudaStatus(cudaMemset(b.p, 0, count * sizeof(float)), "cudaMemset(adjoint)");
         }
 
-        // One forward step fIn -> fOut; the step's w is kept line by line in
-        // wKeep and its v in vOut when they are set.
-        int LaunchFwd(const float *fIn, float *fOut, float *wKeep, float *vOut, const float *srcp, float negDecay,
+        // Host arrays (xDim x yDim) to and from the padded "by y" layout.
+        int ToDevice(float *d, const float *h, cudaStream_t s, const char *what) const
+        {
+            return CudaStatus(cudaMemcpy2DAsync(d, ldY * sizeof(float), h, yDim * sizeof(float), yDim * sizeof(float),
+                                                static_cast<size_t>(xDim), cudaMemcpyHostToDevice, s), what);
+        }
+
+        int ToHost(float *h, const float *d, cudaStream_t s, const char *what) const
+        {
+            return CudaStatus(cudaMemcpy2DAsync(h, yDim * sizeof(float), d, ldY * sizeof(float), yDim * sizeof(float),
+                                                static_cast<size_t>(xDim), cudaMemcpyDeviceToHost, s), what);
+        }
+
+        int CopyField(float *to, const float *from, cudaStream_t s) const
+        {
+            return CudaStatus(cudaMemcpyAsync(to, from, nA * sizeof(float), cudaMemcpyDeviceToDevice, s),
+                              "cudaMemcpy(field)");
+        }
+
+        // out (by x) = in (by y)
+        int ByX(const float *in, float *out, cudaStream_t s) const
+        {
+            TransposeRows<false><<<dim3((xDim + 31) / 32, (yDim + 31) / 32), dim3(32, 8), 0, s>>>(in, ldY, out, ldX,
+                                                                                                  xDim, yDim);
+            CountLaunch();
+            return LaunchStatus("adjoint transpose");
+        }
+
+        // One forward step fIn -> fOut (by y; fB holds fIn by x and then
+        // fOut); the step's w is kept in wKeep and its v in vKeep when they
+        // are set.  chained: the kernel before it on s may be overlapped.
+        int LaunchFwd(const float *fIn, float *fOut, float *wKeep, float *vKeep, const float *srcp, bool chained,
                       cudaStream_t s)
         {
-            const int tx = Threads(g.xDim), ty = Threads(g.yDim);
-            const auto fwdX = SmLine(g.xDim, g.wrapX != 0) ? FwdX<true> : FwdX<false>;
-            const auto fwdY = SmLine(g.yDim, g.wrapY != 0) ? FwdY<true> : FwdY<false>;
-            fwdX<<<g.yDim, tx, LineSmemFloats(tx, g.xDim, g.wrapX != 0) * sizeof(float), s>>>(g, fIn, DT.p, wA.p, wKeep);
-            fwdY<<<g.xDim, ty, LineSmemFloats(ty, g.yDim, g.wrapY != 0) * sizeof(float), s>>>(g, wA.p, fIn, D.p,
-                                                                                               srcp, negDecay, fOut,
-                                                                         vOut);
+            HAL_TRY(WithLaneLen(LaneLen(xDim), [&](auto m) {
+                return LaunchChained(FwdLines<m(), false>, yDim, chained, s, axX, fB.p, nullptr, nullptr, par.p, wA.p,
+                                     nullptr, wKeep);
+            }));
+            HAL_TRY(WithLaneLen(LaneLen(yDim), [&](auto m) {
+                return LaunchChained(FwdLines<m(), true>, xDim, true, s, axY, wA.p, fIn, srcp, par.p, fB.p, fOut, vKeep);
+            }));
             CountLaunch(2);
-            return LaunchStatus("adjoint forward step");
+            return HAL_CUDA_OK;
         }
 
-        int Upload(const float *hD, const float *hSrc, bool &useSrc, cudaStream_t s)
+        int LaunchBwdY(int mode, const float *gPrev, const float *fNext, const float *fT, const float *vT, float *gOut,
+                       bool chained, cudaStream_t s)
         {
-            const size_t bytes = static_cast<size_t>(n) * sizeof(float);
-            HAL_TRY(CudaStatus(cudaMemcpyAsync(D.p, hD, bytes, cudaMemcpyHostToDevice, s), "cudaMemcpy(D)"));
-            HAL_TRY(LaunchTranspose(D.p, DT.p, g.xDim, g.yDim, s));
+            CountLaunch();
+            return WithLaneLen(LaneLen(yDim), [&](auto m) {
+                return LaunchChained(BwdY<m()>, xDim, chained, s, axY, mode, par.p, b1.p, gPrev, fNext, fT, vT, gOut,
+                                     b2.p, dD.p, dS.p, dDecay.p);
+            });
+        }
+
+        int LaunchBwdX(const float *wT, cudaStream_t s)
+        {
+            CountLaunch();
+            return WithLaneLen(LaneLen(xDim), [&](auto m) {
+                return LaunchChained(BwdX<m()>, yDim, true, s, axX, b2.p, wT, b1.p, dDT.p);
+            });
+        }
+
+        // Enqueues on s what `body(s)` enqueues, replayed from a graph of that
+        // key: a launch of a run of steps instead of one per kernel.
+        template <typename Body>
+        int Replay(const std::string &key, cudaStream_t s, Body body)
+        {
+            auto it = graphs.find(key);
+            if (it == graphs.end())
+            {
+                const int64_t before = g_launches.load();
+                HAL_TRY(CudaStatus(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture"));
+                const int rc = body(s);
+                cudaGraph_t g = nullptr;
+                const cudaError_t e = cudaStreamEndCapture(s, &g);
+                // counted again by each replay
+                const int64_t count = g_launches.load() - before;
+                CountLaunch(-count);
+                if (rc != HAL_CUDA_OK || e != cudaSuccess)
+                {
+                    if (g != nullptr)
+                    {
+                        cudaGraphDestroy(g);
+                    }
+                    return rc != HAL_CUDA_OK ? rc : CudaStatus(e, "cudaStreamEndCapture");
+                }
+                cudaGraphExec_t x = nullptr;
+                const cudaError_t ei = cudaGraphInstantiate(&x, g, 0);
+                cudaGraphDestroy(g);
+                HAL_TRY(CudaStatus(ei, "cudaGraphInstantiate"));
+                it = graphs.emplace(key, std::make_pair(x, count)).first;
+            }
+            CountLaunch(it->second.second);
+            return CudaStatus(cudaGraphLaunch(it->second.first, s), "cudaGraphLaunch");
+        }
+
+        // `count` steps between the work fields, from work[c]; returns the
+        // field's index.
+        int RunPlain(int &c, int32_t count, const float *srcp, cudaStream_t s)
+        {
+            const int c0 = c;
+            c ^= count & 1;
+            const auto body = [&](cudaStream_t t)
+            {
+                int k = c0;
+                for (int32_t i = 0; i < count; i++)
+                {
+                    HAL_TRY(LaunchFwd(work[k].p, work[k ^ 1].p, nullptr, nullptr, srcp, i > 0, t));
+                    k ^= 1;
+                }
+                return static_cast<int>(HAL_CUDA_OK);
+            };
+            return Run("F" + std::to_string(c0) + "." + std::to_string(count) + (srcp ? "s" : ""), count, s, body);
+        }
+
+        // The states of `count` steps in buffer b, from its first field (fB
+        // holds it by x).
+        int RunStates(int b, int32_t count, const float *srcp, cudaStream_t s)
+        {
+            const auto body = [&](cudaStream_t t)
+            {
+                for (int32_t i = 0; i < count; i++)
+                {
+                    const size_t k = static_cast<size_t>(i);
+                    HAL_TRY(LaunchFwd(segF[b].p + k * nA, segF[b].p + (k + 1) * nA, segW[b].p + k * nB,
+                                      segV[b].p + k * nA, srcp, i > 0, t));
+                }
+                return static_cast<int>(HAL_CUDA_OK);
+            };
+            return Run("S" + std::to_string(b) + "." + std::to_string(count) + (srcp ? "s" : ""), count, s, body);
+        }
+
+        // Reverse steps over the `count` states in buffer b; g: the index of
+        // the latest adjoint (0: gA, 1: gB).
+        int RunBackward(int b, int32_t count, int &g, bool first, cudaStream_t s)
+        {
+            const int g0 = g;
+            g ^= count & 1;
+            const auto body = [&](cudaStream_t t)
+            {
+                int cur = g0;
+                for (int32_t i = count - 1; i >= 0; i--)
+                {
+                    const size_t k = static_cast<size_t>(i);
+                    const float *gc = cur == 0 ? gA.p : gB.p;
+                    float *gn = cur == 0 ? gB.p : gA.p;
+                    const bool lead = i == count - 1;
+                    HAL_TRY(LaunchBwdY(first && lead ? kBwdFirst : kBwdNext, gc, segF[b].p + (k + 1) * nA,
+                                       segF[b].p + k * nA, segV[b].p + k * nA, gn, !lead, t));
+                    HAL_TRY(LaunchBwdX(segW[b].p + k * nB, t));
+                    cur ^= 1;
+                }
+                return static_cast<int>(HAL_CUDA_OK);
+            };
+            return Run("B" + std::to_string(b) + "." + std::to_string(g0) + "." + std::to_string(count) +
+                           (first ? "f" : ""),
+                       first ? steps : count, s, body);
+        }
+
+        // A run of steps: whole segments from a graph; runs that occur once in
+        // a call (every state kept, the last segment) launch by launch, which
+        // takes the host less than capturing them.
+        template <typename Body>
+        int Run(const std::string &key, int32_t count, cudaStream_t s, Body body)
+        {
+            if (count != Chunk())
+            {
+                return body(s);
+            }
+            return Replay(key, s, body);
+        }
+
+        // Steps of a run that a call repeats.
+        int32_t Chunk() const
+        {
+            return keepAll || Segments() <= 2 ? kPlainChunk : every;
+        }
+        static constexpr int32_t kPlainChunk = 16;  // a forward pass without checkpoints
+
+        // Uploads a call's inputs and factors its lines (timed from begin).
+        int Prepare(const float *hD, double decay, const float *hSrc, bool &useSrc, cudaEvent_t begin, cudaStream_t s)
+        {
+            HAL_TRY(ToDevice(D.p, hD, s, "cudaMemcpy(D)"));
+            HAL_TRY(ByX(D.p, DT.p, s));
             useSrc = (hSrc != nullptr);
             if (useSrc)
             {
-                HAL_TRY(CudaStatus(cudaMemcpyAsync(src.p, hSrc, bytes, cudaMemcpyHostToDevice, s), "cudaMemcpy(src)"));
+                HAL_TRY(ToDevice(src.p, hSrc, s, "cudaMemcpy(src)"));
             }
+            const float hp[2] = {static_cast<float>(decay), static_cast<float>(-decay)};
+            HAL_TRY(CudaStatus(cudaMemcpyAsync(par.p, hp, sizeof(hp), cudaMemcpyHostToDevice, s), "cudaMemcpy(decay)"));
+            HAL_TRY(CudaStatus(cudaEventRecord(begin, s), "cudaEventRecord"));
+            HAL_TRY(WithLaneLen(LaneLen(xDim), [&](auto m) {
+                return LaunchChained(Factor<m()>, yDim, false, s, axX, coefX.p, extX.p);
+            }));
+            HAL_TRY(WithLaneLen(LaneLen(yDim), [&](auto m) {
+                return LaunchChained(Factor<m()>, xDim, false, s, axY, coefY.p, extY.p);
+            }));
+            CountLaunch(2);
             return HAL_CUDA_OK;
-        }
-
-        // `steps` forward steps from f0; checkpoints stored when ck != null.
-        // Returns the buffer holding f_T.
-        const float *Forward(const float *srcp, float negDecay, float *ck, cudaStream_t s, int &rc)
-        {
-            const size_t bytes = static_cast<size_t>(n) * sizeof(float);
-            rc = CudaStatus(cudaMemcpyAsync(work[0].p, f0.p, bytes, cudaMemcpyDeviceToDevice, s), "cudaMemcpy(f0)");
-            int c = 0;
-            for (int32_t t = 0; t < steps && rc == HAL_CUDA_OK; t++)
-            {
-                if (ck != nullptr && t % every == 0)
-                {
-                    rc = CudaStatus(cudaMemcpyAsync(ck + static_cast<size_t>(t / every) * n, work[c].p, bytes,
-                                                    cudaMemcpyDeviceToDevice, s), "cudaMemcpy(checkpoint)");
-                }
-                if (rc == HAL_CUDA_OK)
-                {
-                    rc = LaunchFwd(work[c].p, work[c ^ 1].p, nullptr, nullptr, srcp, negDecay, s);
-                }
-                c ^= 1;
-            }
-            return work[c].p;
         }
 
         int LaunchLoss(const float *fT, float *gbar, cudaStream_t s)
         {
-            const int T = 256;
-            const int blocks = static_cast<int>(std::min<int64_t>((n + T - 1) / T, 1024));
-            LossGrad<<<blocks, T, 0, s>>>(n, fT, target.p, gbar, acc.p);
+            const int64_t cells = static_cast<int64_t>(nA);
+            LossGrad<<<LossParts(), kLossThreads, 0, s>>>(cells, fT, target.p, gbar, part.p);
             CountLaunch();
             return LaunchStatus("adjoint loss");
+        }
+
+        int LossParts() const
+        {
+            return static_cast<int>(
+                std::min<int64_t>((static_cast<int64_t>(nA) + kLossThreads - 1) / kLossThreads, kLossBlocks));
+        }
+
+        int LaunchTotals(bool decayToo, cudaStream_t s)
+        {
+            Totals<<<1, 1024, 0, s>>>(part.p, LossParts(), dDecay.p, decayToo ? static_cast<int64_t>(xDim) * 32 : 0,
+                                      acc.p);
+            CountLaunch();
+            return LaunchStatus("adjoint totals");
+        }
+
+        int EnqueueForward(bool useSrc, const float *&fT, cudaStream_t s)
+        {
+            HAL_TRY(CopyField(work[0].p, f0.p, s));
+            HAL_TRY(ByX(f0.p, fB.p, s));
+            int c = 0;
+            for (int32_t t = 0; t < steps;)
+            {
+                const int32_t k = std::min(Chunk(), steps - t);
+                HAL_TRY(RunPlain(c, k, useSrc ? src.p : nullptr, s));
+                t += k;
+            }
+            fT = work[c].p;
+            HAL_TRY(LaunchLoss(fT, nullptr, s));
+            return LaunchTotals(false, s);
         }
 
         int RunForward(const float *hD, double decay, const float *hSrc, double *loss, float *hFT)
         {
             cudaStream_t s = stream.Get();
             bool useSrc = false;
-            HAL_TRY(Upload(hD, hSrc, useSrc, s));
-            HAL_TRY(CudaStatus(cudaMemsetAsync(acc.p, 0, 2 * sizeof(double), s), "cudaMemset(acc)"));
             cudaEvent_t e0, e1;
             HAL_TRY(CudaStatus(cudaEventCreate(&e0), "cudaEventCreate"));
             HAL_TRY(CudaStatus(cudaEventCreate(&e1), "cudaEventCreate"));
-            cudaEventRecord(e0, s);
-            int rc = HAL_CUDA_OK;
-            const float *fT = Forward(useSrc ? src.p : nullptr, static_cast<float>(-decay), nullptr, s, rc);
+            int rc = Prepare(hD, decay, hSrc, useSrc, e0, s);
+            const float *fT = nullptr;
             if (rc == HAL_CUDA_OK)
             {
-                rc = LaunchLoss(fT, nullptr, s);
+                rc = EnqueueForward(useSrc, fT, s);
             }
             cudaEventRecord(e1, s);
             double h[2] = {0, 0};
@@ -827,8 +1359,7 @@ namespace halcuda
             }
             if (rc == HAL_CUDA_OK && hFT != nullptr)
             {
-                rc = CudaStatus(cudaMemcpyAsync(hFT, fT, static_cast<size_t>(n) * sizeof(float), cudaMemcpyDeviceToHost,
-                                                s), "cudaMemcpy(f_T)");
+                rc = ToHost(hFT, fT, s, "cudaMemcpy(f_T)");
             }
             if (rc == HAL_CUDA_OK)
             {
@@ -844,200 +1375,22 @@ namespace halcuda
             return rc;
         }
 
-        int RunGradient(const float *hD, double decay, const float *hSrc, double *loss, float *hgD, double *hgK,
-                        float *hgS)
+        // Events of a checkpointed gradient.
+        struct Events
         {
-            cudaStream_t s = stream.Get();
-            bool useSrc = false;
-            HAL_TRY(Upload(hD, hSrc, useSrc, s));
-            const size_t bytes = static_cast<size_t>(n) * sizeof(float);
-            const float *srcp = useSrc ? src.p : nullptr;
-            const float negDecay = static_cast<float>(-decay);
-            HAL_TRY(CudaStatus(cudaMemsetAsync(acc.p, 0, 2 * sizeof(double), s), "cudaMemset(acc)"));
-            HAL_TRY(CudaStatus(cudaMemsetAsync(dD.p, 0, bytes, s), "cudaMemset(dD)"));
-            HAL_TRY(CudaStatus(cudaMemsetAsync(dDT.p, 0, bytes, s), "cudaMemset(dD)"));
-            HAL_TRY(CudaStatus(cudaMemsetAsync(dS.p, 0, bytes, s), "cudaMemset(dS)"));
-            cudaEvent_t e0, e1;
-            HAL_TRY(CudaStatus(cudaEventCreate(&e0), "cudaEventCreate"));
-            HAL_TRY(CudaStatus(cudaEventCreate(&e1), "cudaEventCreate"));
-            cudaEventRecord(e0, s);
-            int rc = HAL_CUDA_OK;
-            float *gCur = gA.p, *gNext = gB.p;  // gCur: adjoint of the latest output handled
-            const int tx = Threads(g.xDim), ty = Threads(g.yDim);
-            const size_t smx = LineSmemFloats(tx, g.xDim, g.wrapX != 0) * sizeof(float);
-            const size_t smy = LineSmemFloats(ty, g.yDim, g.wrapY != 0) * sizeof(float);
-            const auto bwdX = SmLine(g.xDim, g.wrapX != 0) ? BwdX<true> : BwdX<false>;
-            const auto bwdY = SmLine(g.yDim, g.wrapY != 0) ? BwdY<true> : BwdY<false>;
-            bool first = true;
-            // states f_t0..f_t1, w and v of one segment into buffer b, from
-            // the field at t0, on stream rs
-            auto recompute = [&](int b, const float *from, int32_t t0, int32_t t1, cudaStream_t rs) {
-                int r = CudaStatus(cudaMemcpyAsync(segF[b].p, from, bytes, cudaMemcpyDeviceToDevice, rs),
-                                   "cudaMemcpy(segment)");
-                for (int32_t t = t0; t < t1 && r == HAL_CUDA_OK; t++)
-                {
-                    const size_t k = static_cast<size_t>(t - t0);
-                    r = LaunchFwd(segF[b].p + k * n, segF[b].p + (k + 1) * n, segW[b].p + k * n, segV[b].p + k * n,
-                                  srcp, negDecay, rs);
-                }
-                return r;
-            };
-            // reverse steps t1-1 .. t0 over the states in buffer b
-            auto backward = [&](int b, int32_t t0, int32_t t1) {
-                int r = HAL_CUDA_OK;
-                for (int32_t t = t1 - 1; t >= t0 && r == HAL_CUDA_OK; t--)
-                {
-                    const size_t k = static_cast<size_t>(t - t0);
-                    const float *fNext = segF[b].p + (k + 1) * n;
-                    bwdY<<<g.xDim, ty, smy, s>>>(g, first ? kBwdFirst : kBwdNext, D.p, static_cast<float>(decay),
-                                                 b1.p, gCur, fNext, segF[b].p + k * n, segV[b].p + k * n, gNext,
-                                                 b2.p, dD.p, dS.p, acc.p + 1);
-                    bwdX<<<g.yDim, tx, smx, s>>>(g, DT.p, b2.p, segW[b].p + k * n, b1.p, dDT.p);
-                    CountLaunch(2);
-                    r = LaunchStatus("adjoint backward step");
-                    std::swap(gCur, gNext);
-                    first = false;
-                }
-                return r;
-            };
-            int lastBuf = 0;  // buffer of segment 0, read by the tail step
-            if (keepAll)
+            cudaEvent_t ready = nullptr, recDone[2] = {nullptr, nullptr}, bwdDone[2] = {nullptr, nullptr};
+
+            int Create()
             {
-                // every state of the run is kept: one forward pass, no recomputation
-                rc = recompute(0, f0.p, 0, steps, s);
-                if (rc == HAL_CUDA_OK)
-                {
-                    rc = LaunchLoss(segF[0].p + static_cast<size_t>(steps) * n, gCur, s);
-                }
-                if (rc == HAL_CUDA_OK)
-                {
-                    rc = backward(0, 0, steps);
-                }
-            }
-            else
-            {
-                // Segments are differentiated last to first.  Segment s-1 is
-                // recomputed from its checkpoint on a second stream into the
-                // other buffer while segment s is differentiated; events order
-                // each buffer's writer (recompute) and reader (backward).
-                cudaStream_t rs = recomputeStream.Get();
-                cudaEvent_t ready = nullptr, recDone[2] = {nullptr, nullptr}, bwdDone[2] = {nullptr, nullptr};
                 for (cudaEvent_t *e : {&ready, &recDone[0], &recDone[1], &bwdDone[0], &bwdDone[1]})
                 {
-                    if (rc == HAL_CUDA_OK)
-                    {
-                        rc = CudaStatus(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
-                    }
+                    HAL_TRY(CudaStatus(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate"));
                 }
-                // The forward pass keeps checkpoints, and writes the states of
-                // the last two segments (one per buffer) as it goes, so the
-                // backward starts without waiting for a recomputation.
-                const int32_t S = Segments();
-                const int32_t firstKept = std::max(S - 2, 0);
-                const float *fT = nullptr;
-                if (rc == HAL_CUDA_OK)
-                {
-                    rc = CudaStatus(cudaMemcpyAsync(work[0].p, f0.p, bytes, cudaMemcpyDeviceToDevice, s),
-                                    "cudaMemcpy(f0)");
-                }
-                const float *fCur = work[0].p;
-                int c = 0;
-                for (int32_t t = 0; t < steps && rc == HAL_CUDA_OK; t++)
-                {
-                    const int32_t seg = t / every;
-                    if (t % every == 0)
-                    {
-                        rc = CudaStatus(cudaMemcpyAsync(ckpt.p + static_cast<size_t>(seg) * n, fCur, bytes,
-                                                        cudaMemcpyDeviceToDevice, s), "cudaMemcpy(checkpoint)");
-                        if (rc == HAL_CUDA_OK && seg >= firstKept)
-                        {
-                            rc = CudaStatus(cudaMemcpyAsync(segF[seg & 1].p, fCur, bytes, cudaMemcpyDeviceToDevice, s),
-                                            "cudaMemcpy(segment)");
-                        }
-                    }
-                    if (rc != HAL_CUDA_OK)
-                    {
-                        break;
-                    }
-                    if (seg >= firstKept)
-                    {
-                        const int b = seg & 1;
-                        const size_t k = static_cast<size_t>(t - seg * every);
-                        float *fOut = segF[b].p + (k + 1) * n;
-                        rc = LaunchFwd(fCur, fOut, segW[b].p + k * n, segV[b].p + k * n, srcp, negDecay, s);
-                        fCur = fOut;
-                    }
-                    else
-                    {
-                        rc = LaunchFwd(fCur, work[c ^ 1].p, nullptr, nullptr, srcp, negDecay, s);
-                        c ^= 1;
-                        fCur = work[c].p;
-                    }
-                }
-                fT = fCur;
-                if (rc == HAL_CUDA_OK)
-                {
-                    rc = LaunchLoss(fT, gCur, s);
-                }
-                auto enqueueRecompute = [&](int32_t seg) {
-                    if (seg >= firstKept)
-                    {
-                        return static_cast<int>(HAL_CUDA_OK);  // written by the forward pass
-                    }
-                    const int b = seg & 1;
-                    const int32_t t0 = seg * every;
-                    // the buffer's previous reader is the backward of segment seg+2
-                    int r = CudaStatus(cudaStreamWaitEvent(rs, bwdDone[b], 0), "cudaStreamWaitEvent");
-                    if (r == HAL_CUDA_OK)
-                    {
-                        r = recompute(b, ckpt.p + static_cast<size_t>(seg) * n, t0, std::min(steps, t0 + every), rs);
-                    }
-                    if (r == HAL_CUDA_OK)
-                    {
-                        r = CudaStatus(cudaEventRecord(recDone[b], rs), "cudaEventRecord");
-                    }
-                    return r;
-                };
-                if (rc == HAL_CUDA_OK)
-                {
-                    // the checkpoints are written by the forward pass on s
-                    rc = CudaStatus(cudaEventRecord(ready, s), "cudaEventRecord");
-                }
-                if (rc == HAL_CUDA_OK)
-                {
-                    rc = CudaStatus(cudaStreamWaitEvent(rs, ready, 0), "cudaStreamWaitEvent");
-                }
-                if (rc == HAL_CUDA_OK && S > 0)
-                {
-                    rc = enqueueRecompute(S - 1);
-                }
-                for (int32_t seg = S - 1; seg >= 0 && rc == HAL_CUDA_OK; seg--)
-                {
-                    if (seg > 0)
-                    {
-                        rc = enqueueRecompute(seg - 1);
-                    }
-                    const int b = seg & 1;
-                    const int32_t t0 = seg * every;
-                    if (rc == HAL_CUDA_OK)
-                    {
-                        rc = CudaStatus(cudaStreamWaitEvent(s, recDone[b], 0), "cudaStreamWaitEvent");
-                    }
-                    if (rc == HAL_CUDA_OK)
-                    {
-                        rc = backward(b, t0, std::min(steps, t0 + every));
-                    }
-                    if (rc == HAL_CUDA_OK)
-                    {
-                        rc = CudaStatus(cudaEventRecord(bwdDone[b], s), "cudaEventRecord");
-                    }
-                }
-                // s now follows every recompute (each backward waited on its
-                // own); an early failure still leaves rs to be drained
-                if (rc != HAL_CUDA_OK)
-                {
-                    cudaStreamSynchronize(rs);
-                }
+                return HAL_CUDA_OK;
+            }
+
+            ~Events()
+            {
                 for (cudaEvent_t e : {ready, recDone[0], recDone[1], bwdDone[0], bwdDone[1]})
                 {
                     if (e != nullptr)
@@ -1046,22 +1399,131 @@ namespace halcuda
                     }
                 }
             }
-            if (rc == HAL_CUDA_OK && steps > 0)
+        };
+
+        // Every state of the run kept: one forward pass, no recomputation.
+        int EnqueueKept(const float *srcp, int &g, cudaStream_t s)
+        {
+            HAL_TRY(CopyField(segF[0].p, f0.p, s));
+            HAL_TRY(ByX(f0.p, fB.p, s));
+            HAL_TRY(RunStates(0, steps, srcp, s));
+            HAL_TRY(LaunchLoss(segF[0].p + static_cast<size_t>(steps) * nA, gA.p, s));
+            return steps > 0 ? RunBackward(0, steps, g, true, s) : static_cast<int>(HAL_CUDA_OK);
+        }
+
+        // Segments are differentiated last to first.  Segment s-1 is
+        // recomputed from its checkpoint on a second stream into the other
+        // buffer while segment s is differentiated; events order each
+        // buffer's writer (recompute) and reader (backward).  The forward pass
+        // keeps checkpoints, and writes the states of the last two segments
+        // (one per buffer) as it goes, so the backward starts without waiting
+        // for a recomputation.
+        int EnqueueCheckpointed(const float *srcp, int &g, Events &ev, cudaStream_t s, cudaStream_t rs)
+        {
+            const int32_t S = Segments();
+            const int32_t firstKept = std::max(S - 2, 0);
+            const auto length = [&](int32_t seg) { return std::min(steps - seg * every, every); };
+            HAL_TRY(CopyField(work[0].p, f0.p, s));
+            HAL_TRY(ByX(f0.p, fB.p, s));
+            const float *fCur = work[0].p;
+            int c = 0;
+            for (int32_t seg = 0; seg < S; seg++)
+            {
+                HAL_TRY(CopyField(ckpt.p + static_cast<size_t>(seg) * nA, fCur, s));
+                if (seg >= firstKept)
+                {
+                    HAL_TRY(CopyField(segF[seg & 1].p, fCur, s));
+                    HAL_TRY(RunStates(seg & 1, length(seg), srcp, s));
+                    fCur = segF[seg & 1].p + static_cast<size_t>(length(seg)) * nA;
+                }
+                else
+                {
+                    HAL_TRY(RunPlain(c, every, srcp, s));
+                    fCur = work[c].p;
+                }
+            }
+            HAL_TRY(LaunchLoss(fCur, gA.p, s));
+            // the checkpoints are written by the forward pass on s
+            HAL_TRY(CudaStatus(cudaEventRecord(ev.ready, s), "cudaEventRecord"));
+            HAL_TRY(CudaStatus(cudaStreamWaitEvent(rs, ev.ready, 0), "cudaStreamWaitEvent"));
+            for (int32_t seg = S - 1; seg >= 0; seg--)
+            {
+                const int32_t next = seg - 1;
+                if (next >= 0 && next < firstKept)
+                {
+                    // the buffer's previous reader is the backward of segment next+2
+                    const int b = next & 1;
+                    HAL_TRY(CudaStatus(cudaStreamWaitEvent(rs, ev.bwdDone[b], 0), "cudaStreamWaitEvent"));
+                    HAL_TRY(CopyField(segF[b].p, ckpt.p + static_cast<size_t>(next) * nA, rs));
+                    HAL_TRY(ByX(segF[b].p, fB.p, rs));
+                    HAL_TRY(RunStates(b, every, srcp, rs));
+                    HAL_TRY(CudaStatus(cudaEventRecord(ev.recDone[b], rs), "cudaEventRecord"));
+                }
+                const int b = seg & 1;
+                if (seg < firstKept)
+                {
+                    HAL_TRY(CudaStatus(cudaStreamWaitEvent(s, ev.recDone[b], 0), "cudaStreamWaitEvent"));
+                }
+                HAL_TRY(RunBackward(b, length(seg), g, seg == S - 1, s));
+                HAL_TRY(CudaStatus(cudaEventRecord(ev.bwdDone[b], s), "cudaEventRecord"));
+            }
+            return HAL_CUDA_OK;
+        }
+
+        int EnqueueGradient(bool useSrc, Events &ev, cudaStream_t s)
+        {
+            HAL_TRY(CudaStatus(cudaMemsetAsync(dD.p, 0, nA * sizeof(float), s), "cudaMemset(dD)"));
+            HAL_TRY(CudaStatus(cudaMemsetAsync(dDT.p, 0, nB * sizeof(float), s), "cudaMemset(dD)"));
+            HAL_TRY(CudaStatus(cudaMemsetAsync(dS.p, 0, nA * sizeof(float), s), "cudaMemset(dS)"));
+            HAL_TRY(CudaStatus(cudaMemsetAsync(dDecay.p, 0, static_cast<size_t>(xDim) * 32 * sizeof(float2), s),
+                               "cudaMemset(dDecay)"));
+            const float *srcp = useSrc ? src.p : nullptr;
+            int g = 0;
+            if (keepAll)
+            {
+                HAL_TRY(EnqueueKept(srcp, g, s));
+            }
+            else
+            {
+                HAL_TRY(EnqueueCheckpointed(srcp, g, ev, s, recomputeStream.Get()));
+            }
+            if (steps > 0)
             {
                 // the y-stencil part of step 0's (I + Ly/2) b1bar: its D terms
-                bwdY<<<g.xDim, ty, smy, s>>>(g, kBwdTail, D.p, static_cast<float>(decay), b1.p, gCur,
-                                             segF[lastBuf].p, segF[lastBuf].p, segV[lastBuf].p, gNext, b2.p, dD.p,
-                                             dS.p, acc.p + 1);
-                CountLaunch();
-                rc = LaunchStatus("adjoint backward tail");
+                // (buffer 0 holds segment 0's states)
+                HAL_TRY(LaunchBwdY(kBwdTail, g == 0 ? gA.p : gB.p, segF[0].p, segF[0].p, segV[0].p,
+                                   g == 0 ? gB.p : gA.p, false, s));
+            }
+            // the x-faces' part of dL/dD
+            TransposeRows<true><<<dim3((yDim + 31) / 32, (xDim + 31) / 32), dim3(32, 8), 0, s>>>(dDT.p, ldX, dD.p, ldY,
+                                                                                                 yDim, xDim);
+            CountLaunch();
+            HAL_TRY(LaunchStatus("adjoint dD"));
+            return LaunchTotals(true, s);
+        }
+
+        int RunGradient(const float *hD, double decay, const float *hSrc, double *loss, float *hgD, double *hgK,
+                        float *hgS)
+        {
+            cudaStream_t s = stream.Get();
+            bool useSrc = false;
+            cudaEvent_t e0, e1;
+            HAL_TRY(CudaStatus(cudaEventCreate(&e0), "cudaEventCreate"));
+            HAL_TRY(CudaStatus(cudaEventCreate(&e1), "cudaEventCreate"));
+            Events ev;
+            int rc = ev.Create();
+            if (rc == HAL_CUDA_OK)
+            {
+                rc = Prepare(hD, decay, hSrc, useSrc, e0, s);
             }
             if (rc == HAL_CUDA_OK)
             {
-                // the x-faces' part of dL/dD, accumulated line by line
-                AddTransposed<<<dim3((g.xDim + 31) / 32, (g.yDim + 31) / 32), dim3(32, 8), 0, s>>>(dD.p, dDT.p,
-                                                                                               g.xDim, g.yDim);
-                CountLaunch();
-                rc = LaunchStatus("adjoint dD");
+                rc = EnqueueGradient(useSrc, ev, s);
+            }
+            if (rc != HAL_CUDA_OK)
+            {
+                // s follows every recomputation only when all of it was enqueued
+                cudaStreamSynchronize(recomputeStream.Get());
             }
             cudaEventRecord(e1, s);
             double h[2] = {0, 0};
@@ -1072,11 +1534,11 @@ namespace halcuda
             }
             if (rc == HAL_CUDA_OK && hgD != nullptr)
             {
-                rc = CudaStatus(cudaMemcpyAsync(hgD, dD.p, bytes, cudaMemcpyDeviceToHost, s), "cudaMemcpy(dD)");
+                rc = ToHost(hgD, dD.p, s, "cudaMemcpy(dD)");
             }
             if (rc == HAL_CUDA_OK && hgS != nullptr)
             {
-                rc = CudaStatus(cudaMemcpyAsync(hgS, dS.p, bytes, cudaMemcpyDeviceToHost, s), "cudaMemcpy(dS)");
+                rc = ToHost(hgS, dS.p, s, "cudaMemcpy(dS)");
             }
             if (rc == HAL_CUDA_OK)
             {
@@ -1149,11 +1611,14 @@ extern "C" int hal_cuda_adjoint_set_problem(hal_cuda_adjoint *h, const float *f0
     HAL_REQUIRE(checkpointEvery >= 0, "hal_cuda_adjoint_set_problem: negative checkpoint interval");
     using namespace halcuda;
     HAL_TRY(CudaStatus(cudaSetDevice(h->device), "cudaSetDevice"));
-    const size_t m = static_cast<size_t>(h->n);
+    // (a call that failed may have left work in flight)
+    HAL_TRY(CudaStatus(cudaStreamSynchronize(h->stream.Get()), "hal_cuda_adjoint_set_problem"));
+    h->DropGraphs();
+    h->hasProblem = false;
     h->steps = steps;
     h->keepAll = (checkpointEvery == 0);
     h->every = h->keepAll ? std::max(steps, 1) : std::min(checkpointEvery, std::max(steps, 1));
-    HAL_TRY(h->ckpt.Alloc(m * static_cast<size_t>(std::max(h->Segments(), 1)), "cudaMalloc(checkpoints)"));
+    HAL_TRY(h->ckpt.Alloc(h->nA * static_cast<size_t>(std::max(h->Segments(), 1)), "cudaMalloc(checkpoints)"));
     // one segment buffer when every state is kept or there is one segment,
     // two (recompute of one overlapping the backward of the other) otherwise
     const int nBuf = (h->keepAll || h->Segments() <= 1) ? 1 : 2;
@@ -1161,9 +1626,10 @@ extern "C" int hal_cuda_adjoint_set_problem(hal_cuda_adjoint *h, const float *f0
     {
         if (b < nBuf)
         {
-            HAL_TRY(h->segF[b].Alloc(m * static_cast<size_t>(h->every + 1), "cudaMalloc(segment)"));
-            HAL_TRY(h->segW[b].Alloc(m * static_cast<size_t>(h->every), "cudaMalloc(segment)"));
-            HAL_TRY(h->segV[b].Alloc(m * static_cast<size_t>(h->every), "cudaMalloc(segment)"));
+            // (whole arrays are written before they are read, padding included)
+            HAL_TRY(h->segF[b].Alloc(h->nA * static_cast<size_t>(h->every + 1), "cudaMalloc(segment)"));
+            HAL_TRY(h->segW[b].Alloc(h->nB * static_cast<size_t>(h->every), "cudaMalloc(segment)"));
+            HAL_TRY(h->segV[b].Alloc(h->nA * static_cast<size_t>(h->every), "cudaMalloc(segment)"));
         }
         else
         {
@@ -1173,9 +1639,8 @@ extern "C" int hal_cuda_adjoint_set_problem(hal_cuda_adjoint *h, const float *f0
         }
     }
     cudaStream_t s = h->stream.Get();
-    HAL_TRY(CudaStatus(cudaMemcpyAsync(h->f0.p, f0, m * sizeof(float), cudaMemcpyHostToDevice, s), "cudaMemcpy(f0)"));
-    HAL_TRY(CudaStatus(cudaMemcpyAsync(h->target.p, target, m * sizeof(float), cudaMemcpyHostToDevice, s),
-                       "cudaMemcpy(target)"));
+    HAL_TRY(h->ToDevice(h->f0.p, f0, s, "cudaMemcpy(f0)"));
+    HAL_TRY(h->ToDevice(h->target.p, target, s, "cudaMemcpy(target)"));
     HAL_TRY(CudaStatus(cudaStreamSynchronize(s), "hal_cuda_adjoint_set_problem"));
     h->hasProblem = true;
     return HAL_CUDA_OK;
