@@ -1289,6 +1289,477 @@ namespace halcuda
             }
         }
 
+
+        // ---- short lines: a warp solves whole lines in registers -------------
+        // SweepTile's CTAs stage their lines in shared memory and meet at four
+        // barriers; on lines of up to 1024 positions a sweep has too few CTAs
+        // and too little work in each to hide that: 8 to 12 us a sweep whatever
+        // the grid's size (20 us per 300 x 517 tick, as much as a 2048^2 one).
+        // Here a CTA has a few lines, a warp one or more whole lines and a lane
+        // one chunk; the lines are staged by coalesced 16-byte copies, the
+        // separators exchanged by shuffles.  Every value is computed by the
+        // same operations in the same order as in SweepTile, bit for bit.  The
+        // launches are chained: the plan, the field and the source of the
+        // commit are loaded before the wait for the sweep before.  What bounds
+        // a small sweep now is latency (launch, loads, the chunk's chain,
+        // stores), a 1024^2 one the transposed write-out.
+        // Measured on GB300, us per tick (zero-flux, with source), SweepTile /
+        // here: 64^2 13.2 / 4.5, 256^2 11.0 / 5.5, 300 x 517 19.0 / 7.5, 512^2
+        // 11.5 / 6.9, 777 x 1000 19.2 / 11.1, 1024^2 12.9 / 12.3.
+        // Lanes that read their chunks straight from global memory, 128 bytes
+        // apart, were slower (1024^2 17.1): a request per lane.
+        constexpr int kLineMaxP = 32;     // chunks: lines up to 1024
+        constexpr int kLinePre = 4;       // commit units loaded ahead per thread
+        constexpr int kLineFewLines = 608;  // 152 SMs x 4 lines
+
+        constexpr int LineStride(int P) { return P * kChunkStride + 4; }
+
+        // CTA: W warps of lpw lines each (lpw a power of two, lpw * P <= 32
+        // lanes).
+        template <int MODE, bool UPT, int W>
+        __global__ void __launch_bounds__(32 * W) AdiLines(SweepParams p, int32_t lpw)
+        {
+            // the CTA's lines and one on either side, LineStride(P) floats each
+            extern __shared__ __align__(16) float rows[];
+            __shared__ __align__(16) float sCoef[kCoefSmemFloats];
+            __shared__ float sG[kGbandSmem];
+            __shared__ float sZ[kLineMaxP * M];
+            const int P = p.plan.P;
+            const int32_t L = p.L;
+            const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+            constexpr int T = 32 * W;
+            const int lines = W * lpw;               // lines of the CTA, a multiple of 4
+            const int32_t x0 = static_cast<int32_t>(blockIdx.x) * lines;
+            const int sub = lane / P;                // line of the lane within the warp
+            const int k = lane - sub * P;            // chunk
+            const int b0 = sub * P;                  // first lane of the line
+            const int ll = warp * lpw + sub;         // line within the CTA
+            const bool mine = sub < lpw;             // (idle lanes past the warp's lines)
+            const int32_t line = x0 + ll;
+            const bool act = mine && line < p.Nlines;
+            const int lineStride = LineStride(P);
+
+            // what does not come from the kernel before
+            for (int q = tid; q < kCoefFloats / 4; q += T)
+            {
+                const int t = q / (kCoefCount * M / 4);
+                St4(sCoef + t * kCoefTypeStride + 4 * (q - t * (kCoefCount * M / 4)),
+                    __ldg(reinterpret_cast<const float4 *>(p.plan.coef) + q));
+            }
+            const int gCount = (P > 1) ? (P - 1) * (2 * p.plan.B + 1) : 0;
+            for (int q = tid; q < gCount; q += T)
+            {
+                sG[q] = __ldg(p.plan.gband + q);
+            }
+            if (p.plan.periodic)
+            {
+                for (int q = tid; q < P * M; q += T)
+                {
+                    sZ[q] = (q < L) ? __ldg(p.plan.zsm + q) : 0.0f;
+                }
+            }
+            // write-out units: (position, quad of lines), quads fastest
+            const int Q = lines >> 2;  // a power of two
+            const int qShift = 31 - __clz(Q);
+            const int nUnits = L * Q;
+            const int64_t nl = p.outStride;
+            float4 fv[kLinePre], sv[kLinePre];
+            if constexpr (MODE == kSweepTick)
+            {
+#pragma unroll
+                for (int b = 0; b < kLinePre; b++)
+                {
+                    const int u = tid + b * T;
+                    const int32_t line0 = x0 + 4 * (u & (Q - 1));
+                    const bool ok = u < nUnits && line0 < p.Nlines;
+                    const int64_t gi = static_cast<int64_t>(u >> qShift) * nl + line0;
+                    fv[b] = sv[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (ok)
+                    {
+                        fv[b] = __ldcg(reinterpret_cast<const float4 *>(p.f + gi));
+                        if (p.src != nullptr)
+                        {
+                            sv[b] = __ldcg(reinterpret_cast<const float4 *>(p.src + gi));
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            // (after the wait: the next sweep's early loads are of arrays that
+            // were complete before this kernel's predecessor finished)
+            asm volatile("griddepcontrol.launch_dependents;");
+
+            // ---- stage lines x0-1 .. x0+lines ----------------------------------
+            // a warp copies whole lines, 16 bytes a lane, into 36-float chunks
+            for (int r = warp; r < lines + 2; r += W)
+            {
+                const int32_t at = x0 - 1 + r;
+                const float *src = nullptr;
+                bool vec = true;
+                if (at >= 0 && at < p.Nlines)
+                {
+                    src = p.in + static_cast<int64_t>(at) * p.inStride;
+                }
+                else if (at == -1 || at == p.Nlines)
+                {
+                    if (p.wrapLines)
+                    {
+                        src = p.in + static_cast<int64_t>(at < 0 ? p.Nlines - 1 : 0) * p.inStride;
+                    }
+                    else
+                    {
+                        src = at < 0 ? p.ghostLo : p.ghostHi;
+                        vec = false;  // a ghost table's row: any alignment, no padding
+                    }
+                }
+                for (int f = lane; f < P * (M / 4); f += 32)
+                {
+                    float *dst = rows + r * lineStride + (f >> 3) * kChunkStride + 4 * (f & 7);
+                    const int32_t pos = 4 * f;
+                    if (src != nullptr && vec && pos < L)
+                    {
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(SmemAddr(dst)), "l"(src + pos)
+                                     : "memory");
+                    }
+                    else if (src != nullptr && pos < L)
+                    {
+                        St4(dst, make_float4(src[pos], pos + 1 < L ? src[pos + 1] : 0.0f,
+                                             pos + 2 < L ? src[pos + 2] : 0.0f, pos + 3 < L ? src[pos + 3] : 0.0f));
+                    }
+                    else
+                    {
+                        St4(dst, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+                    }
+                }
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+
+            // ---- right-hand sides ---------------------------------------------
+            const bool hasGhost = (p.ghostLo != nullptr);
+            const float wUp = (line >= 1 || p.wrapLines) ? 1.0f : (hasGhost ? 2.0f : 0.0f);
+            const float wDn = (line + 1 < p.Nlines || p.wrapLines) ? 1.0f : (hasGhost ? 2.0f : 0.0f);
+            float *own = rows + ((mine ? ll : 0) + 1) * lineStride + min(k, P - 1) * kChunkStride;
+            float z[M];
+            {
+                float4 up[M / 4], c[M / 4], dn[M / 4];
+#pragma unroll
+                for (int q = 0; q < M / 4; q++)
+                {
+                    up[q] = Ld4(own - lineStride + 4 * q);
+                    c[q] = Ld4(own + 4 * q);
+                    dn[q] = Ld4(own + lineStride + 4 * q);
+                }
+                if (wUp == 1.0f && wDn == 1.0f)
+                {
+#pragma unroll
+                    for (int q = 0; q < M / 4; q++)
+                    {
+                        z[4 * q + 0] = fmaf((dn[q].x - c[q].x) + (up[q].x - c[q].x), p.halfR, c[q].x);
+                        z[4 * q + 1] = fmaf((dn[q].y - c[q].y) + (up[q].y - c[q].y), p.halfR, c[q].y);
+                        z[4 * q + 2] = fmaf((dn[q].z - c[q].z) + (up[q].z - c[q].z), p.halfR, c[q].z);
+                        z[4 * q + 3] = fmaf((dn[q].w - c[q].w) + (up[q].w - c[q].w), p.halfR, c[q].w);
+                    }
+                }
+                else
+                {
+#pragma unroll
+                    for (int q = 0; q < M / 4; q++)
+                    {
+                        z[4 * q + 0] = fmaf((dn[q].x - c[q].x) * wDn + (up[q].x - c[q].x) * wUp, p.halfR, c[q].x);
+                        z[4 * q + 1] = fmaf((dn[q].y - c[q].y) * wDn + (up[q].y - c[q].y) * wUp, p.halfR, c[q].y);
+                        z[4 * q + 2] = fmaf((dn[q].z - c[q].z) * wDn + (up[q].z - c[q].z) * wUp, p.halfR, c[q].z);
+                        z[4 * q + 3] = fmaf((dn[q].w - c[q].w) * wDn + (up[q].w - c[q].w) * wUp, p.halfR, c[q].w);
+                    }
+                }
+            }
+            if (p.implLo != nullptr && act)
+            {
+                if (k == 0)
+                {
+                    z[0] = fmaf(p.r, __ldg(p.implLo + line), z[0]);
+                }
+                const int lastIdx = (L - 1) - k * M;
+                if (lastIdx >= 0 && lastIdx < M)
+                {
+                    const float add = p.r * __ldg(p.implHi + line);
+#pragma unroll
+                    for (int e = 0; e < M; e++)
+                    {
+                        z[e] += (e == lastIdx) ? add : 0.0f;
+                    }
+                }
+            }
+
+            // ---- Thomas on the chunk (BlockSolveN's operations) -----------------
+            const float *cf = sCoef + AdiBlockType(min(k, P - 1), P) * kCoefTypeStride;
+            {
+                const float4 *fw = reinterpret_cast<const float4 *>(cf + kCoefFw * M);
+                const float4 *ib = reinterpret_cast<const float4 *>(cf + kCoefIb * M);
+                const float4 *cb = reinterpret_cast<const float4 *>(cf + kCoefCb * M);
+#pragma unroll
+                for (int j = 0; j < M / 4; j++)
+                {
+                    const float4 w4 = fw[j];
+                    if (j > 0)
+                    {
+                        z[4 * j] = fmaf(-w4.x, z[4 * j - 1], z[4 * j]);
+                    }
+                    z[4 * j + 1] = fmaf(-w4.y, z[4 * j], z[4 * j + 1]);
+                    z[4 * j + 2] = fmaf(-w4.z, z[4 * j + 1], z[4 * j + 2]);
+                    z[4 * j + 3] = fmaf(-w4.w, z[4 * j + 2], z[4 * j + 3]);
+                }
+#pragma unroll
+                for (int j = M / 4 - 1; j >= 0; j--)
+                {
+                    const float4 i4 = ib[j];
+                    const float4 c4 = cb[j];
+                    if (j == M / 4 - 1)
+                    {
+                        z[4 * j + 3] *= i4.w;
+                    }
+                    else
+                    {
+                        z[4 * j + 3] = fmaf(-c4.w, z[4 * j + 4], z[4 * j + 3] * i4.w);
+                    }
+                    z[4 * j + 2] = fmaf(-c4.z, z[4 * j + 3], z[4 * j + 2] * i4.z);
+                    z[4 * j + 1] = fmaf(-c4.y, z[4 * j + 2], z[4 * j + 1] * i4.y);
+                    z[4 * j + 0] = fmaf(-c4.x, z[4 * j + 1], z[4 * j + 0] * i4.x);
+                }
+            }
+
+            // ---- separators: row k of the banded inverse (BandDot2's order; the
+            // separator below a chunk is the one above the next) -----------------
+            const float a = p.plan.a;
+            const float fromNext = __shfl_down_sync(0xffffffffu, -a * z[0], 1);
+            const float sm = fmaf(-a, z[M - 2], z[M - 1]) + fromNext;  // k < P - 1
+            float sR = 0.0f;
+            {
+                const int S = P - 1, B = p.plan.B, W = 2 * B + 1;
+                for (int t = -B; t <= B; t++)
+                {
+                    const int m = k + t;
+                    const float v = __shfl_sync(0xffffffffu, sm, b0 + min(max(m, 0), P - 1));
+                    if (k < S && m >= 0 && m < S)
+                    {
+                        sR = fmaf(sG[k * W + (t + B)], v, sR);
+                    }
+                }
+            }
+            float sL = __shfl_up_sync(0xffffffffu, sR, 1);
+            sL = (k == 0) ? 0.0f : sL;
+            {
+                const float4 *pv = reinterpret_cast<const float4 *>(cf + kCoefP * M);
+                const float4 *qv = reinterpret_cast<const float4 *>(cf + kCoefQ * M);
+#pragma unroll
+                for (int j = 0; j < M / 4; j++)
+                {
+                    const float4 p4 = pv[j];
+                    const float4 q4 = qv[j];
+                    z[4 * j + 0] = fmaf(-sL, p4.x, fmaf(-sR, q4.x, z[4 * j + 0]));
+                    z[4 * j + 1] = fmaf(-sL, p4.y, fmaf(-sR, q4.y, z[4 * j + 1]));
+                    z[4 * j + 2] = fmaf(-sL, p4.z, fmaf(-sR, q4.z, z[4 * j + 2]));
+                    z[4 * j + 3] = fmaf(-sL, p4.w, fmaf(-sR, q4.w, z[4 * j + 3]));
+                }
+                if (k < P - 1)
+                {
+                    z[M - 1] = sR;
+                }
+            }
+            if (p.plan.periodic)
+            {
+                // Sherman-Morrison, as in SweepTile
+                float yl = 0.0f;
+                const int lastIdx = (L - 1) - (P - 1) * M;
+#pragma unroll
+                for (int e = 0; e < M; e++)
+                {
+                    yl = (e == lastIdx) ? z[e] : yl;
+                }
+                const int hi = min(b0 + P - 1, 31);
+                const float y0 = __shfl_sync(0xffffffffu, z[0], min(b0, 31));
+                yl = __shfl_sync(0xffffffffu, yl, hi);
+                const float fct = fmaf(yl, p.plan.bog, y0) * p.plan.invDenom;
+#pragma unroll
+                for (int e = 0; e < M; e++)
+                {
+                    z[e] = fmaf(-fct, sZ[min(k, P - 1) * M + e], z[e]);
+                }
+            }
+
+            // ---- write out ------------------------------------------------------
+            // over the staged lines: every read of them is behind the barrier
+            __syncthreads();
+            if (mine)
+            {
+#pragma unroll
+                for (int q = 0; q < M / 4; q++)
+                {
+                    St4(own + 4 * q, act ? make_float4(z[4 * q], z[4 * q + 1], z[4 * q + 2], z[4 * q + 3])
+                                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+                }
+            }
+            __syncthreads();
+            const float *tile = rows + lineStride;
+            if constexpr (MODE == kSweepDeltas)
+            {
+                for (int l = 0; l < lines && x0 + l < p.Nlines; l++)
+                {
+                    const int64_t base = static_cast<int64_t>(x0 + l) * L;
+                    for (int32_t pos = tid; pos < L; pos += T)
+                    {
+                        const double v =
+                            static_cast<double>(tile[l * lineStride + (pos >> 5) * kChunkStride + (pos & 31)]);
+                        p.deltas[base + pos] = p.deltas[base + pos] + (v - p.f64[base + pos]);
+                    }
+                }
+                return;
+            }
+            auto unit = [&](int u, float4 f4, float4 s4)
+            {
+                const int32_t pos = u >> qShift;
+                const int qd = u & (Q - 1);
+                const int32_t line0 = x0 + 4 * qd;
+                if (line0 >= p.Nlines)
+                {
+                    return;
+                }
+                const float *t = tile + 4 * qd * lineStride + (pos >> 5) * kChunkStride + (pos & 31);
+                float4 v = make_float4(t[0], t[lineStride], t[2 * lineStride], t[3 * lineStride]);
+                if constexpr (MODE == kSweepTick)
+                {
+                    int32_t nc[4] = {0, 0, 0, 0};
+                    if constexpr (UPT)
+                    {
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                        {
+                            if (line0 + e < p.Nlines)
+                            {
+                                const int32_t *oc = p.cellOffsets + static_cast<int64_t>(line0 + e) * L + pos;
+                                nc[e] = __ldcg(oc + 1) - __ldcg(oc);
+                            }
+                        }
+                    }
+                    auto commit = [&](float vv, float f0, float s0, int32_t nv) {
+                        float d = vv - f0;
+                        d = fmaf(f0, p.negDecay, d);
+                        d += s0;
+                        if constexpr (UPT)
+                        {
+                            d = fmaf(f0, p.negUptake * static_cast<float>(nv), d);
+                        }
+                        return f0 + d;
+                    };
+                    v.x = commit(v.x, f4.x, s4.x, nc[0]);
+                    v.y = commit(v.y, f4.y, s4.y, nc[1]);
+                    v.z = commit(v.z, f4.z, s4.z, nc[2]);
+                    v.w = commit(v.w, f4.w, s4.w, nc[3]);
+                }
+                const int32_t left = p.Nlines - line0;  // past them: the row's padding, zeros
+                v.y = (left > 1) ? v.y : 0.0f;
+                v.z = (left > 2) ? v.z : 0.0f;
+                v.w = (left > 3) ? v.w : 0.0f;
+                St4(p.out + static_cast<int64_t>(pos) * nl + line0, v);
+            };
+            const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            int u = tid;
+            if constexpr (MODE == kSweepTick)
+            {
+#pragma unroll
+                for (int b = 0; b < kLinePre; b++)
+                {
+                    if (u < nUnits)
+                    {
+                        unit(u, fv[b], sv[b]);
+                    }
+                    u += T;
+                }
+            }
+            for (; u < nUnits; u += T)
+            {
+                float4 f4 = zero4, s4 = zero4;
+                if constexpr (MODE == kSweepTick)
+                {
+                    const int32_t line0 = x0 + 4 * (u & (Q - 1));
+                    if (line0 < p.Nlines)
+                    {
+                        const int64_t gi = static_cast<int64_t>(u >> qShift) * nl + line0;
+                        f4 = __ldcg(reinterpret_cast<const float4 *>(p.f + gi));
+                        if (p.src != nullptr)
+                        {
+                            s4 = __ldcg(reinterpret_cast<const float4 *>(p.src + gi));
+                        }
+                    }
+                }
+                unit(u, f4, s4);
+            }
+        }
+
+        // Lines up to kLineMaxP chunks go to AdiLines.
+        bool UseLines(const SweepParams &p)
+        {
+            return p.plan.P <= kLineMaxP;
+        }
+
+        template <int MODE, bool UPT, int W>
+        int LaunchLinesOf(SweepParams &p, cudaStream_t s)
+        {
+            static SmemLimit s_limit;
+            const int32_t P = p.plan.P;
+            // one line per warp until every SM has a CTA; then as many as the
+            // warp's lanes hold
+            int32_t lpw = 1;
+            while (2 * lpw * P <= 32 && p.Nlines >= 2 * lpw * W * 152)
+            {
+                lpw *= 2;
+            }
+            const int32_t lines = W * lpw;
+            const size_t smem = sizeof(float) * static_cast<size_t>(lines + 2) * LineStride(P);
+            HAL_TRY(s_limit.Ensure(AdiLines<MODE, UPT, W>, smem, "cudaFuncSetAttribute(AdiLines)"));
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(static_cast<unsigned>((p.Nlines + lines - 1) / lines));
+            cfg.blockDim = dim3(32 * W);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            CountLaunch();
+            return CudaStatus(cudaLaunchKernelEx(&cfg, AdiLines<MODE, UPT, W>, p, lpw), "AdiLines launch");
+        }
+
+        template <int MODE, bool UPT>
+        int LaunchLinesW(SweepParams &p, cudaStream_t s)
+        {
+            // A CTA of four warps, or, where a warp holds one line only and
+            // four lines would leave as 16-byte pieces, of eight (32-byte
+            // pieces): once there are enough lines for it, and where the
+            // output's rows are a multiple of 1 KB apart, on which 16-byte
+            // pieces are slowest (us per tick with four / eight warps: 1024^2
+            // 17.7 / 12.3, 600 x 3000 26.0 / 24.9, 777 x 1000 11.1 / 12.1,
+            // 512^2 6.9 / 7.2, 64^2 4.5 / 5.4).
+            const bool wide = p.plan.P > 16 && p.Nlines > kLineFewLines &&
+                              (p.outStride % 256 == 0 || p.Nlines >= 2 * kLineFewLines);
+            return wide ? LaunchLinesOf<MODE, UPT, 8>(p, s) : LaunchLinesOf<MODE, UPT, 4>(p, s);
+        }
+
+        template <int MODE>
+        int LaunchLines(SweepParams &p, cudaStream_t s)
+        {
+            if constexpr (MODE == kSweepTick)
+            {
+                if (p.cellOffsets != nullptr)
+                {
+                    return LaunchLinesW<MODE, true>(p, s);
+                }
+            }
+            return LaunchLinesW<MODE, false>(p, s);
+        }
+
         // Device copy of one line plan.
         struct LinePlanBuf
         {
@@ -1583,9 +2054,14 @@ namespace halcuda
         int32_t xDim = 0, yDim = 0;
         int device = 0;
         StreamSlot stream;
-        DevBuf<float> field[2];  // layout B (y*xDim + x)
+        // Rows are padded to a multiple of 4 floats (ldX in layout B, ldY in
+        // layout A), so that every line is read and written in 16-byte units
+        // whatever its length.  The padding of field and src holds zeros; w's
+        // is rewritten with zeros by every x-sweep.
+        int32_t ldX = 0, ldY = 0;
+        DevBuf<float> field[2];  // layout B (y*ldX + x)
         int cur = 0;
-        DevBuf<float> w;         // x-sweep output, layout A; also staging for uploads
+        DevBuf<float> w;         // x-sweep output, layout A (x*ldY + y); also dense staging of host arrays
         DevBuf<float> src;       // layout B
         bool hasSrc = false;
         DevBuf<float> ghost;     // ghost table (hal_cuda.h layout)
@@ -1628,26 +2104,37 @@ namespace halcuda
             device = CurrentDevice();
             HAL_TRY(CudaStatus(cudaSetDevice(device), "cudaSetDevice"));
             HAL_TRY(stream.Create("cudaStreamCreate"));
-            size_t n = Length();
+            ldX = (xDim + 3) & ~3;
+            ldY = (yDim + 3) & ~3;
+            const size_t n = LengthB();
             HAL_TRY(field[0].Alloc(n, "cudaMalloc(field)"));
             HAL_TRY(field[1].Alloc(n, "cudaMalloc(field)"));
-            HAL_TRY(w.Alloc(n, "cudaMalloc(scratch)"));
+            HAL_TRY(w.Alloc(static_cast<size_t>(xDim) * static_cast<size_t>(ldY), "cudaMalloc(scratch)"));
             HAL_TRY(err.Alloc(1, "cudaMalloc(err)"));
             HAL_TRY(CudaStatus(cudaMemset(field[0].p, 0, n * sizeof(float)), "cudaMemset"));
+            HAL_TRY(CudaStatus(cudaMemset(field[1].p, 0, n * sizeof(float)), "cudaMemset"));
             HAL_TRY(CudaStatus(cudaMemset(err.p, 0, sizeof(int32_t)), "cudaMemset"));
             std::memset(tmapX, 0, sizeof(tmapX));
             std::memset(&tmapY, 0, sizeof(tmapY));
             const int32_t Px = (xDim + M - 1) / M, Py = (yDim + M - 1) / M;
             const int32_t Rx = ShapeFor(Px, yDim, true).R, Ry = ShapeFor(Py, xDim, true).R;
-            swzX = MakeLineTensorMap(tmapX[0], field[0].p, xDim, yDim, Rx) &&
+            // (the tensor-staged sweep writes dense rows: the number of its
+            // lines a multiple of 4)
+            swzX = ldY == yDim && MakeLineTensorMap(tmapX[0], field[0].p, xDim, yDim, Rx) &&
                    MakeLineTensorMap(tmapX[1], field[1].p, xDim, yDim, Rx);
-            swzY = MakeLineTensorMap(tmapY, w.p, yDim, xDim, Ry);
+            swzY = ldX == xDim && MakeLineTensorMap(tmapY, w.p, yDim, xDim, Ry);
             return HAL_CUDA_OK;
         }
 
         size_t Length() const
         {
             return static_cast<size_t>(xDim) * static_cast<size_t>(yDim);
+        }
+
+        // Floats of a padded layout-B array.
+        size_t LengthB() const
+        {
+            return static_cast<size_t>(yDim) * static_cast<size_t>(ldX);
         }
 
         int Plan(int32_t L, double r, int ends, const LinePlanDev **out)
@@ -1705,23 +2192,33 @@ namespace halcuda
             return HAL_CUDA_OK;
         }
 
+        // A dense HAL-layout array into a padded layout-B one.
         template <typename TIn>
-        int TransposeTo(const TIn *in, float *out, int32_t rows, int32_t cols, cudaStream_t s)
+        int ToLayoutB(const TIn *in, float *out, cudaStream_t s)
         {
             dim3 block(32, 8);
-            dim3 grid((cols + 31) / 32, (rows + 31) / 32);
-            Transpose<TIn><<<grid, block, 0, s>>>(in, out, rows, cols, cols, rows);
+            dim3 grid((yDim + 31) / 32, (xDim + 31) / 32);
+            Transpose<TIn><<<grid, block, 0, s>>>(in, out, xDim, yDim, yDim, ldX);
             CountLaunch();
             return LaunchStatus("Transpose launch");
+        }
+
+        // ... and back.
+        int FromLayoutB(const float *in, float *out, cudaStream_t s)
+        {
+            return LaunchTransposeStrided(in, ldX, out, yDim, yDim, xDim, s);
         }
 
         template <int MODE>
         int LaunchSweep(SweepParams &p, cudaStream_t s, const CUtensorMap *tmap)
         {
             const bool swz = (tmap != nullptr);
-            // the single grid's lines and output rows are dense
-            p.inStride = p.L;
-            p.outStride = p.Nlines;
+            p.inStride = (p.L + 3) & ~3;
+            p.outStride = (p.Nlines + 3) & ~3;
+            if (UseLines(p))
+            {
+                return LaunchLines<MODE>(p, s);
+            }
             SweepShape sh = ShapeFor(p.plan.P, p.Nlines, swz);
             p.R = sh.R;
             p.LS = sh.LS;
@@ -1999,11 +2496,11 @@ namespace halcuda
         {
             if (const void *d = MappedHost(host))
             {
-                return TransposeTo<float>(static_cast<const float *>(d), field[cur].p, xDim, yDim, s);
+                return ToLayoutB(static_cast<const float *>(d), field[cur].p, s);
             }
             HAL_TRY(CudaStatus(cudaMemcpyAsync(w.p, host, Length() * sizeof(float), cudaMemcpyHostToDevice, s),
                                "cudaMemcpy(field)"));
-            return TransposeTo<float>(w.p, field[cur].p, xDim, yDim, s);
+            return ToLayoutB(w.p, field[cur].p, s);
         }
 
         // field[cur] (layout B) -> host (layout A).
@@ -2011,9 +2508,9 @@ namespace halcuda
         {
             if (void *d = MappedHost(host))
             {
-                return TransposeTo<float>(field[cur].p, static_cast<float *>(d), yDim, xDim, s);
+                return FromLayoutB(field[cur].p, static_cast<float *>(d), s);
             }
-            HAL_TRY(TransposeTo<float>(field[cur].p, w.p, yDim, xDim, s));
+            HAL_TRY(FromLayoutB(field[cur].p, w.p, s));
             return CudaStatus(cudaMemcpyAsync(host, w.p, Length() * sizeof(float), cudaMemcpyDeviceToHost, s),
                               "cudaMemcpy(field)");
         }
@@ -2022,17 +2519,18 @@ namespace halcuda
         {
             if (src.p == nullptr)
             {
-                HAL_TRY(src.Alloc(Length(), "cudaMalloc(src)"));
+                HAL_TRY(src.Alloc(LengthB(), "cudaMalloc(src)"));
+                HAL_TRY(CudaStatus(cudaMemsetAsync(src.p, 0, LengthB() * sizeof(float), s), "cudaMemset(src)"));
             }
             if (const void *d = MappedHost(host))
             {
-                HAL_TRY(TransposeTo<float>(static_cast<const float *>(d), src.p, xDim, yDim, s));
+                HAL_TRY(ToLayoutB(static_cast<const float *>(d), src.p, s));
             }
             else
             {
                 HAL_TRY(CudaStatus(cudaMemcpyAsync(w.p, host, Length() * sizeof(float), cudaMemcpyHostToDevice, s),
                                    "cudaMemcpy(src)"));
-                HAL_TRY(TransposeTo<float>(w.p, src.p, xDim, yDim, s));
+                HAL_TRY(ToLayoutB(w.p, src.p, s));
             }
             hasSrc = true;
             return HAL_CUDA_OK;
@@ -2156,7 +2654,7 @@ namespace
                            "cudaMemcpy(deltas)"));
         // the field in layout B, in float, in the spare buffer of the pair
         float *fB = h->field[h->cur ^ 1].p;
-        HAL_TRY(h->TransposeTo<double>(h->f64.p, fB, h->xDim, h->yDim, s));
+        HAL_TRY(h->ToLayoutB(h->f64.p, fB, s));
         HAL_TRY(h->LaunchX(fB, r, wrapX != 0, wrapY != 0, g, s));
         HAL_TRY(h->LaunchY<kSweepDeltas>(nullptr, nullptr, h->f64.p, h->d64.p, r, 0.0, wrapX != 0, wrapY != 0, g,
                                           false, s));
