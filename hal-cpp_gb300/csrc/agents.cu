@@ -542,6 +542,46 @@ namespace halcuda
             }
         }
 
+        // The FP32 force of a pair at displacement (xComp, yComp): whether it
+        // is within 0 < d < R, the force and its product with 1/d.  1/d comes
+        // from rsqrt (d^2 = 0 gives NaN, which fails both tests like the CPU's
+        // d > 0).
+        template <int LAW>
+        __device__ __forceinline__ bool PairScale32(float xComp, float yComp, float radSum, float R,
+                                                    const LawParams<float> &lp, float &force, float &scale)
+        {
+            const float d2 = fmaf(xComp, xComp, __fmul_rn(yComp, yComp));
+            const float inv = rsqrtf(d2);
+            const float dist = __fmul_rn(d2, inv);
+            force = 0.0f;
+            scale = 0.0f;
+            if (!((dist < R) && (dist > 0.0f)))
+            {
+                return false;
+            }
+            force = OverlapForce<LAW>(__fsub_rn(radSum, dist), lp);
+            scale = __fmul_rn(inv, force);
+            return true;
+        }
+
+        // The linear law's term without a branch, so that several candidates'
+        // chains interleave: (x, y, scale) with v - (x, y) * scale the pair's
+        // contribution, all 0 where the pair has none.  Subtracting such a
+        // term adds -0, which leaves every v as it is.
+        __device__ __forceinline__ bool PairTerm32(bool valid, float dx, float dy, float radSum, float R, float k,
+                                                   float &x, float &y, float &scale)
+        {
+            const float d2 = fmaf(dx, dx, __fmul_rn(dy, dy));
+            const float inv = rsqrtf(d2);
+            const float dist = __fmul_rn(d2, inv);
+            const float sc = __fmul_rn(inv, __fmul_rn(k, __fsub_rn(radSum, dist)));
+            const bool near = valid && dist < R && dist > 0.0f;
+            x = near ? dx : 0.0f;
+            y = near ? dy : 0.0f;
+            scale = near ? sc : 0.0f;
+            return near;
+        }
+
         // One neighbour's contribution (CpuAgentForceBackend2D.cpp:153-169,
         // SphericalAgent2D.h:83-98): the displacement to pj, and for
         // 0 < d < R the force law's force along it, subtracted from (vx, vy);
@@ -583,17 +623,11 @@ namespace halcuda
             }
             else
             {
-                // FP32 path: 1/d from rsqrt (d^2 = 0 gives NaN, which fails
-                // both tests like the CPU's d > 0)
-                const T d2 = fmaf(xComp, xComp, yComp * yComp);
-                const T inv = rsqrtf(d2);
-                const T dist = d2 * inv;
-                if ((dist < R) && (dist > T(0)))
+                T force, scale;
+                if (PairScale32<LAW>(xComp, yComp, rad + radj, R, lp, force, scale))
                 {
-                    const T force = OverlapForce<LAW>((rad + radj) - dist, lp);
-                    const T scale = inv * force;
-                    vx -= xComp * scale;
-                    vy -= yComp * scale;
+                    vx = fmaf(-xComp, scale, vx);
+                    vy = fmaf(-yComp, scale, vy);
                     if constexpr (SUM)
                     {
                         if (force > T(0))
@@ -745,6 +779,8 @@ namespace halcuda
 #pragma unroll
                     for (int u = 0; u < kGroup; u++)
                     {
+                        pj[u] = pf;
+                        rj[u] = rad;
                         const int32_t k = k0 + u;
                         qs[u] = (k >= total) ? -1
                                 : (k < c1)   ? rs[0] + k
@@ -756,6 +792,25 @@ namespace halcuda
                             pj[u] = sPos[qs[u]];
                             rj[u] = sRad[qs[u]];
                         }
+                    }
+                    if constexpr (std::is_same<T, float>::value && LAW == kLawLinear && !SUM)
+                    {
+                        // the terms side by side, then their sum in order
+                        float x[kGroup], y[kGroup], sc[kGroup];
+#pragma unroll
+                        for (int u = 0; u < kGroup; u++)
+                        {
+                            PairTerm32(qs[u] >= 0 && qs[u] != slot, Disp(px, pj[u].x, xDimF, wrapX != 0),
+                                       Disp(py, pj[u].y, yDimF, wrapY != 0), __fadd_rn(rad, rj[u]), R, lp.scale, x[u],
+                                       y[u], sc[u]);
+                        }
+#pragma unroll
+                        for (int u = 0; u < kGroup; u++)
+                        {
+                            vx = fmaf(-x[u], sc[u], vx);
+                            vy = fmaf(-y[u], sc[u], vy);
+                        }
+                        continue;
                     }
 #pragma unroll
                     for (int u = 0; u < kGroup; u++)
@@ -976,6 +1031,241 @@ namespace halcuda
                 cellOf[i] = c;
                 arrival[i] = atomicAdd(counts + c, 1);
             }
+        }
+
+
+        // ---- few agents: eight lanes per agent ------------------------------
+        // With one thread per agent, 20000 agents are a warp per scheduler, and
+        // the tick waits for the longest chain: the agents of a dense cluster
+        // walk their window's candidates (60 and more) one after another, 13 of
+        // the step's 24 us.  Here a group of kGroupLanes lanes takes an agent:
+        // each lane finds one run of the window's cells, the lanes evaluate
+        // that many candidates at a time, and the terms are then added in the
+        // candidates' order by every lane (a candidate out of range adds -0),
+        // so the sum is ForceSlotLaw's, bit for bit.  It issues more
+        // instructions per pair than one thread per agent does, so the latter
+        // stays beyond kGroupAgents agents.  Measured, us per resident step
+        // (benchmark distribution, thread / group per agent): 20k agents in
+        // 256^2 24.1 / 17.6, 50k in 512^2 133 / 62, 100k in 1024^2 36.6 / 36.0,
+        // 200k in 1024^2 36.5 / 52.4, 1M in 2048^2 90 / 214.  Leaving only the
+        // agents of long windows to groups, in a second launch, cost 3 us per
+        // 1M-agent step and lost up to 2x where many agents had long windows.
+        constexpr int kGroupLanes = 8;
+        constexpr int32_t kGroupAgents = 100000;
+
+        // floor(v - r) and ceil(v + r) as the CPU takes them, in FP64.  For an
+        // integer r the FP32 floor and ceiling give the same (v is exact, and
+        // the FP64 sum exact, for the magnitudes below; nearer zero the sum can
+        // round onto an integer) without FP64 instructions on the chain.
+        __device__ __forceinline__ void WindowOf(float v, double r, bool intR, int32_t &lo, int32_t &hi)
+        {
+            const float a = fabsf(v);
+            if (intR && (a == 0.0f || (a >= 0x1p-28f && a < 0x1p24f)))
+            {
+                const int32_t ri = static_cast<int32_t>(static_cast<float>(r));
+                lo = static_cast<int32_t>(floorf(v)) - ri;
+                hi = static_cast<int32_t>(ceilf(v)) + ri;
+            }
+            else
+            {
+                lo = static_cast<int32_t>(floor(static_cast<double>(v) - r));
+                hi = static_cast<int32_t>(ceil(static_cast<double>(v) + r));
+            }
+        }
+
+        // The force sum (linear law, from zero) of the agent in slot `slot`
+        // (live: there is one), on every lane of its group.  All lanes of the
+        // warp call it.
+        __device__ __forceinline__ float2 ForceSlotGroup(const int32_t slot, const bool live,
+                                                         const int32_t *__restrict__ offsets,
+                                                         const float2 *__restrict__ sPos,
+                                                         const float *__restrict__ sRad, double interactionRad,
+                                                         bool intR, float R, const LawParams<float> lp, int32_t xDim,
+                                                         int32_t yDim, int32_t wrapX, int32_t wrapY)
+        {
+            constexpr int G = kGroupLanes;
+            const int j = threadIdx.x & (G - 1);
+            const float2 pf = sPos[slot];
+            const float rad = sRad[slot];
+            int32_t xStart, xEnd, yStart, yEnd;
+            WindowOf(pf.x, interactionRad, intR, xStart, xEnd);
+            WindowOf(pf.y, interactionRad, intR, yStart, yEnd);
+            if (!wrapX)
+            {
+                xStart = max(xStart, 0);
+                xEnd = min(xEnd, xDim);
+            }
+            if (!wrapY)
+            {
+                yStart = max(yStart, 0);
+                yEnd = min(yEnd, yDim);
+            }
+            // the window as runs of cells, in the visiting order: one per row,
+            // or two where a wrapped y-range crosses the edge
+            const int32_t nRows = max(xEnd - xStart, 0);
+            const bool below = yStart < 0, above = yEnd > yDim;
+            const int32_t perRow = (below || above) ? 2 : 1;
+            const bool empty = nRows == 0 || yEnd <= yStart;
+            const bool fits = empty || (nRows <= G / perRow && yEnd - yStart <= yDim && !(below && above));
+            int32_t s0 = 0, len = 0;
+            if (live && fits && !empty && j < nRows * perRow)
+            {
+                int32_t row = xStart + ((perRow == 2) ? (j >> 1) : j);
+                if (row < 0 || row >= xDim)
+                {
+                    row %= xDim;  // only reached on a wrapped axis (clamped otherwise)
+                    row = (row < 0) ? row + xDim : row;
+                }
+                int32_t y0 = yStart, y1 = yEnd;
+                if (perRow == 2)
+                {
+                    const bool first = (j & 1) == 0;
+                    y0 = first ? (below ? yStart + yDim : yStart) : 0;
+                    y1 = first ? yDim : (below ? yEnd : yEnd - yDim);
+                }
+                s0 = __ldg(offsets + row * yDim + y0);
+                len = __ldg(offsets + row * yDim + y1) - s0;
+            }
+            // candidate k is slot k + shift[r] of the first run r with k < end[r]
+            int32_t end[G], shift[G];
+            int32_t total = 0;
+#pragma unroll
+            for (int r = 0; r < G; r++)
+            {
+                shift[r] = __shfl_sync(0xffffffffu, s0, r, G) - total;
+                total += __shfl_sync(0xffffffffu, len, r, G);
+                end[r] = total;
+            }
+            const float xDimF = static_cast<float>(xDim), yDimF = static_cast<float>(yDim);
+            float vx = 0.0f, vy = 0.0f;
+            const int32_t most = __reduce_max_sync(0xffffffffu, total);
+            auto candidate = [&](int32_t k, int32_t &q, float2 &pj, float &rj)
+            {
+                q = -1;
+                if (k < total)
+                {
+                    int32_t sh = shift[G - 1];
+#pragma unroll
+                    for (int r = G - 2; r >= 0; r--)
+                    {
+                        sh = (k < end[r]) ? shift[r] : sh;
+                    }
+                    q = k + sh;
+                    pj = sPos[q];
+                    rj = sRad[q];
+                }
+            };
+            int32_t q;
+            float2 pj = make_float2(0.0f, 0.0f);
+            float rj = 0.0f;
+            candidate(j, q, pj, rj);
+            for (int32_t k0 = 0; k0 < most; k0 += G)
+            {
+                // the next round's loads, in flight during this one's sums
+                int32_t qn;
+                float2 pn = make_float2(0.0f, 0.0f);
+                float rn = 0.0f;
+                candidate(k0 + G + j, qn, pn, rn);
+                float x, y, scale;
+                const bool near = PairTerm32(
+                           q >= 0 && q != slot, Disp(pf.x, pj.x, xDimF, wrapX != 0), Disp(pf.y, pj.y, yDimF, wrapY != 0),
+                           __fadd_rn(rad, rj), R, lp.scale, x, y, scale);
+                // the terms, in the candidates' order, on every lane (walking
+                // only the ones in range took more instructions than it saved)
+                if (__any_sync(0xffffffffu, near))
+                {
+#pragma unroll
+                    for (int t = 0; t < G; t++)
+                    {
+                        const float sc = __shfl_sync(0xffffffffu, scale, t, G);
+                        vx = fmaf(-__shfl_sync(0xffffffffu, x, t, G), sc, vx);
+                        vy = fmaf(-__shfl_sync(0xffffffffu, y, t, G), sc, vy);
+                    }
+                }
+                q = qn;
+                pj = pn;
+                rj = rn;
+            }
+            if (!fits && live)
+            {
+                // a window of more runs than lanes: one lane's walk for all
+                const ForceAcc<float> acc = ForceSlotLaw<float, kLawLinear, false, false>(
+                    slot, offsets, sPos, sRad, interactionRad, R, lp, xDim, yDim, wrapX, wrapY,
+                    make_float2(0.0f, 0.0f));
+                vx = acc.v.x;
+                vy = acc.v.y;
+            }
+            return make_float2(vx, vy);
+        }
+
+        // Forces and ForcesMove (linear law, no sums) with a group per agent.
+        template <bool WALLS>
+        __global__ void ForcesGroup(const int32_t *__restrict__ bucket, const int32_t *__restrict__ offsets,
+                                    const float2 *__restrict__ sPos, const float *__restrict__ sRad, int32_t n,
+                                    double interactionRad, bool intR, float R, LawParams<float> lp, int32_t xDim,
+                                    int32_t yDim, int32_t wrapX, int32_t wrapY, float *__restrict__ vel)
+        {
+            ChainEntry();
+            const int32_t at = (blockIdx.x * blockDim.x + threadIdx.x) / kGroupLanes;
+            const bool live = at < n;
+            const int32_t slot = live ? at : n - 1;
+            const float2 d = ForceSlotGroup(slot, live, offsets, sPos, sRad, interactionRad, intR, R, lp, xDim, yDim,
+                                            WALLS ? 0 : wrapX, WALLS ? 0 : wrapY);
+            if (live && (threadIdx.x & (kGroupLanes - 1)) == 0)
+            {
+                StoreDelta(vel, bucket[slot], d);
+            }
+        }
+
+        // One agent's forces and move, by its group.
+        template <bool WALLS>
+        __device__ __forceinline__ void MoveSlotGroup(const int32_t slot, const bool live,
+                                                      const int32_t *__restrict__ bucket,
+                                                      const int32_t *__restrict__ offsets,
+                                                      const float2 *__restrict__ sPos, const float *__restrict__ sRad,
+                                                      double interactionRad, bool intR, float R, LawParams<float> lp,
+                                                      int32_t xDim, int32_t yDim, const MoveParams &mp,
+                                                      float *__restrict__ deltas, float2 *__restrict__ pos,
+                                                      float2 *__restrict__ velocity, int32_t *__restrict__ cellOf,
+                                                      int32_t *__restrict__ arrival, int32_t *__restrict__ counts)
+        {
+            const bool lead = live && (threadIdx.x & (kGroupLanes - 1)) == 0;
+            // the move's inputs, in flight during the sums
+            const int32_t i = bucket[slot];
+            float2 v = lead ? velocity[i] : make_float2(0.0f, 0.0f);
+            const float2 d = ForceSlotGroup(slot, live, offsets, sPos, sRad, interactionRad, intR, R, lp, xDim, yDim,
+                                            WALLS ? 0 : mp.wrapX, WALLS ? 0 : mp.wrapY);
+            if (!lead)
+            {
+                return;
+            }
+            StoreDelta(deltas, i, d);
+            float2 p = sPos[slot];
+            v.x = __fadd_rn(v.x, d.x);
+            v.y = __fadd_rn(v.y, d.y);
+            MoveAgent(mp, p, v);
+            pos[i] = p;
+            velocity[i] = v;
+            const int32_t c = CellCoord(p.x, xDim) * yDim + CellCoord(p.y, yDim);
+            cellOf[i] = c;
+            arrival[i] = atomicAdd(counts + c, 1);
+        }
+
+        template <bool WALLS>
+        __global__ void ForcesMoveGroup(const int32_t *__restrict__ bucket, const int32_t *__restrict__ offsets,
+                                        const float2 *__restrict__ sPos, const float *__restrict__ sRad, int32_t n,
+                                        double interactionRad, bool intR, float R, LawParams<float> lp, int32_t xDim,
+                                        int32_t yDim, MoveParams mp, float *__restrict__ deltas,
+                                        float2 *__restrict__ pos, float2 *__restrict__ velocity,
+                                        int32_t *__restrict__ cellOf, int32_t *__restrict__ arrival,
+                                        int32_t *__restrict__ counts)
+        {
+            ChainEntry();
+            const int32_t at = (blockIdx.x * blockDim.x + threadIdx.x) / kGroupLanes;
+            const bool live = at < n;
+            const int32_t slot = live ? at : n - 1;
+            MoveSlotGroup<WALLS>(slot, live, bucket, offsets, sPos, sRad, interactionRad, intR, R, lp, xDim, yDim, mp,
+                                 deltas, pos, velocity, cellOf, arrival, counts);
         }
 
         // ---- many independent wells in one pass ------------------------------
@@ -1242,6 +1532,12 @@ namespace halcuda
         }
     }
 
+    // Whether WindowOf may take the FP32 form for this radius.
+    inline bool IntegerRadius(double r)
+    {
+        return r >= 0.0 && r <= 0x1p20 && r == std::floor(r);
+    }
+
     struct ForceLawSpec
     {
         int kind = kLawLinear;
@@ -1431,6 +1727,15 @@ namespace halcuda
                 // the interface's law on a grid with walls: the wrap tests compiled out
                 if constexpr (std::is_same<T, float>::value)
                 {
+                    if (n <= kGroupAgents && velIn == nullptr)
+                    {
+                        const unsigned groups =
+                            static_cast<unsigned>((static_cast<int64_t>(n) * kGroupLanes + T_ - 1) / T_);
+                        LaunchChained(!wrapX && !wrapY ? ForcesGroup<true> : ForcesGroup<false>, groups, T_, s, bucket.p,
+                                      offsets.p, SortedPosBuf(T()), sRad, n, R, IntegerRadius(R), static_cast<T>(R), lp,
+                                      xDim, yDim, static_cast<int32_t>(wrapX), static_cast<int32_t>(wrapY), vel);
+                        break;
+                    }
                     if (!wrapX && !wrapY)
                     {
                         go(Forces<T, TV, kLawLinear, false, false, true>);
@@ -1508,10 +1813,20 @@ namespace
                           reinterpret_cast<float2 *>(a.pos32.p), a.velState.p, sums, a.cellOf.p, a.arrival.p,
                           a.counts.p);
         };
+        const bool walls = !mp.wrapX && !mp.wrapY;
+        if (law.kind == kLawLinear && !law.sums && a.n <= kGroupAgents)
+        {
+            const unsigned groups = static_cast<unsigned>((static_cast<int64_t>(a.n) * kGroupLanes + T - 1) / T);
+            LaunchChained(walls ? ForcesMoveGroup<true> : ForcesMoveGroup<false>, groups, T, s, a.bucket.p, a.offsets.p,
+                          a.sPos.p, a.sRad32.p, a.n, R, IntegerRadius(R), static_cast<float>(R), lp, a.xDim, a.yDim, mp,
+                          a.vel32.p, reinterpret_cast<float2 *>(a.pos32.p), a.velState.p, a.cellOf.p, a.arrival.p,
+                          a.counts.p);
+        }
+        else
         switch (law.kind * 2 + (law.sums ? 1 : 0))
         {
         case 0:
-            if (!mp.wrapX && !mp.wrapY)
+            if (walls)
             {
                 go(ForcesMove<kLawLinear, false, true>);  // walls: the wrap tests compiled out
             }
