@@ -582,6 +582,9 @@ namespace halcuda
             return near;
         }
 
+        // Windows of this many candidates are walked run by run (WalkRuns32).
+        constexpr int32_t kLongWindow = 64;
+
         // One neighbour's contribution (CpuAgentForceBackend2D.cpp:153-169,
         // SphericalAgent2D.h:83-98): the displacement to pj, and for
         // 0 < d < R the force law's force along it, subtracted from (vx, vy);
@@ -647,6 +650,94 @@ namespace halcuda
             V2<T> v;
             T sum;
         };
+
+        // The FP32 linear law over the slots of up to four runs [rs, re), one
+        // after another in order, added to (vx, vy).  The terms of a group of
+        // candidates are formed side by side, without branches, after the
+        // loads of the whole group.  A long walk (a dense cluster, a pile at an
+        // edge) is bound by its one thread's instructions and goes run by run,
+        // without the choice of the run per candidate; a short one keeps the
+        // runs joined, where groups cut short at each run's end would cost more.
+        // Measured on GB300, 1M agents in 2048^2, 30% in a cluster, forces and
+        // move, branches per pair / here: cluster inside 38 / 37 us, half
+        // clipped at an edge 93 / 74 us, at a corner 387 / 285 us (groups of
+        // eight in the long walk: 298 us).
+        __device__ __forceinline__ void WalkRuns32(const int32_t (&rs)[4], const int32_t (&re)[4], int32_t slot,
+                                                   float2 pf, float rad, const float2 *__restrict__ sPos,
+                                                   const float *__restrict__ sRad, float R, float k, float xDimF,
+                                                   float yDimF, int32_t wrapX, int32_t wrapY, float &vx, float &vy)
+        {
+            const int32_t c1 = re[0] - rs[0];
+            const int32_t c2 = c1 + (re[1] - rs[1]);
+            const int32_t c3 = c2 + (re[2] - rs[2]);
+            const int32_t total = c3 + (re[3] - rs[3]);
+            constexpr int G = 4;
+            auto add = [&](const int32_t(&q)[G], const float2(&pj)[G], const float(&rj)[G])
+            {
+                float x[G], y[G], sc[G];
+#pragma unroll
+                for (int u = 0; u < G; u++)
+                {
+                    PairTerm32(q[u] >= 0 && q[u] != slot, Disp(pf.x, pj[u].x, xDimF, wrapX != 0),
+                               Disp(pf.y, pj[u].y, yDimF, wrapY != 0), __fadd_rn(rad, rj[u]), R, k, x[u], y[u], sc[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < G; u++)
+                {
+                    vx = fmaf(-x[u], sc[u], vx);
+                    vy = fmaf(-y[u], sc[u], vy);
+                }
+            };
+            if (total >= kLongWindow)
+            {
+#pragma unroll 1
+                for (int r = 0; r < 4; r++)
+                {
+                    const int32_t q0 = r == 0 ? rs[0] : (r == 1 ? rs[1] : (r == 2 ? rs[2] : rs[3]));
+                    const int32_t q1 = r == 0 ? re[0] : (r == 1 ? re[1] : (r == 2 ? re[2] : re[3]));
+                    for (int32_t qb = q0; qb < q1; qb += G)
+                    {
+                        int32_t q[G];
+                        float2 pj[G];
+                        float rj[G];
+#pragma unroll
+                        for (int u = 0; u < G; u++)
+                        {
+                            const int32_t at = min(qb + u, q1 - 1);
+                            q[u] = (qb + u < q1) ? at : -1;
+                            pj[u] = sPos[at];
+                            rj[u] = sRad[at];
+                        }
+                        add(q, pj, rj);
+                    }
+                }
+                return;
+            }
+            for (int32_t k0 = 0; k0 < total; k0 += G)
+            {
+                int32_t q[G];
+                float2 pj[G];
+                float rj[G];
+#pragma unroll
+                for (int u = 0; u < G; u++)
+                {
+                    const int32_t at = k0 + u;
+                    q[u] = (at >= total) ? -1
+                           : (at < c1)   ? rs[0] + at
+                           : (at < c2)   ? rs[1] + (at - c1)
+                           : (at < c3)   ? rs[2] + (at - c2)
+                                         : rs[3] + (at - c3);
+                    pj[u] = pf;
+                    rj[u] = rad;
+                    if (q[u] >= 0)
+                    {
+                        pj[u] = sPos[q[u]];
+                        rj[u] = sRad[q[u]];
+                    }
+                }
+                add(q, pj, rj);
+            }
+        }
 
         // Pass 4 (CpuAgentForceBackend2D.cpp:112-175) for the agent in sorted
         // slot `slot`; offsets are the cell offsets of its grid.  Starting
@@ -761,6 +852,11 @@ namespace halcuda
                         re[j] = __ldg(offsets + cell + (yEnd - yStart));
                     }
                 }
+                if constexpr (std::is_same<T, float>::value && LAW == kLawLinear && !SUM)
+                {
+                    WalkRuns32(rs, re, slot, pf, rad, sPos, sRad, R, lp.scale, xDimF, yDimF, wrapX, wrapY, vx, vy);
+                    return result();
+                }
                 // The rows' runs, one after another, form one sequence of
                 // candidates in the visiting order; it is walked in groups of
                 // kGroup whose loads are issued before any of them is used, so
@@ -779,8 +875,6 @@ namespace halcuda
 #pragma unroll
                     for (int u = 0; u < kGroup; u++)
                     {
-                        pj[u] = pf;
-                        rj[u] = rad;
                         const int32_t k = k0 + u;
                         qs[u] = (k >= total) ? -1
                                 : (k < c1)   ? rs[0] + k
@@ -792,25 +886,6 @@ namespace halcuda
                             pj[u] = sPos[qs[u]];
                             rj[u] = sRad[qs[u]];
                         }
-                    }
-                    if constexpr (std::is_same<T, float>::value && LAW == kLawLinear && !SUM)
-                    {
-                        // the terms side by side, then their sum in order
-                        float x[kGroup], y[kGroup], sc[kGroup];
-#pragma unroll
-                        for (int u = 0; u < kGroup; u++)
-                        {
-                            PairTerm32(qs[u] >= 0 && qs[u] != slot, Disp(px, pj[u].x, xDimF, wrapX != 0),
-                                       Disp(py, pj[u].y, yDimF, wrapY != 0), __fadd_rn(rad, rj[u]), R, lp.scale, x[u],
-                                       y[u], sc[u]);
-                        }
-#pragma unroll
-                        for (int u = 0; u < kGroup; u++)
-                        {
-                            vx = fmaf(-x[u], sc[u], vx);
-                            vy = fmaf(-y[u], sc[u], vy);
-                        }
-                        continue;
                     }
 #pragma unroll
                     for (int u = 0; u < kGroup; u++)
@@ -1312,7 +1387,7 @@ namespace halcuda
                 return;
             }
             const int32_t i = bucketTmp[q];
-            const AgentWellDev wd = wells[wellOf[i]];
+            const AgentWellDev wd = wells[wellOf[q]];
             const float2 p = posF[i];
             const int32_t c = CellCoord(p.x, wd.xDim) * wd.yDim + CellCoord(p.y, wd.yDim);
             const int32_t b = binOf[i];
@@ -1341,15 +1416,14 @@ namespace halcuda
                                                            const float2 *__restrict__ sPos,
                                                            const float *__restrict__ sRad,
                                                            const int32_t *__restrict__ sCell, double interactionRad,
-                                                           float R, float k, const AgentWellDev &wd)
+                                                           bool intR, float R, float k, const AgentWellDev &wd)
         {
             const float2 pf = sPos[slot];
             const float rad = sRad[slot];
             const int32_t xDim = wd.xDim, yDim = wd.yDim;
-            int32_t xStart = static_cast<int32_t>(floor(static_cast<double>(pf.x) - interactionRad));
-            int32_t xEnd = static_cast<int32_t>(ceil(static_cast<double>(pf.x) + interactionRad));
-            int32_t yStart = static_cast<int32_t>(floor(static_cast<double>(pf.y) - interactionRad));
-            int32_t yEnd = static_cast<int32_t>(ceil(static_cast<double>(pf.y) + interactionRad));
+            int32_t xStart, xEnd, yStart, yEnd;
+            WindowOf(pf.x, interactionRad, intR, xStart, xEnd);
+            WindowOf(pf.y, interactionRad, intR, yStart, yEnd);
             if (!wd.wrapX)
             {
                 xStart = max(xStart, 0);
@@ -1373,9 +1447,10 @@ namespace halcuda
                 // One cell per bin and a window whose y-range does not wrap:
                 // each window row is one run of consecutive bins, so one
                 // stretch of slots.  All rows' bounds are loaded before the
-                // first candidate; the rows' stretches, one after another,
-                // are walked in groups of four whose loads are issued before
-                // any of them is used.  The visiting order is unchanged.
+                // first candidate (WalkRuns32).  The visiting order is unchanged.
+                // (Walking the coarser bins' stretches the same way, with a
+                // filter for the other cells' agents, took as long as the walk
+                // below: fewer chained loads, more candidates.)
                 int32_t rs[4], re[4];
 #pragma unroll
                 for (int j = 0; j < 4; j++)
@@ -1395,41 +1470,7 @@ namespace halcuda
                         re[j] = __ldg(offsets + bin + (yEnd - yStart));
                     }
                 }
-                constexpr int kGroup = 4;
-                const int32_t c1 = re[0] - rs[0];
-                const int32_t c2 = c1 + (re[1] - rs[1]);
-                const int32_t c3 = c2 + (re[2] - rs[2]);
-                const int32_t total = c3 + (re[3] - rs[3]);
-                for (int32_t k0 = 0; k0 < total; k0 += kGroup)
-                {
-                    int32_t qs[kGroup];
-                    float2 pj[kGroup];
-                    float rj[kGroup];
-#pragma unroll
-                    for (int u = 0; u < kGroup; u++)
-                    {
-                        const int32_t kk = k0 + u;
-                        qs[u] = (kk >= total) ? -1
-                                : (kk < c1)   ? rs[0] + kk
-                                : (kk < c2)   ? rs[1] + (kk - c1)
-                                : (kk < c3)   ? rs[2] + (kk - c2)
-                                              : rs[3] + (kk - c3);
-                        if (qs[u] >= 0)
-                        {
-                            pj[u] = sPos[qs[u]];
-                            rj[u] = sRad[qs[u]];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < kGroup; u++)
-                    {
-                        if (qs[u] >= 0 && qs[u] != slot)
-                        {
-                            PairStep<float, kLawLinear, false, false>(pf.x, pf.y, rad, pj[u], rj[u], R, lp, xDimF,
-                                                                      yDimF, wd.wrapX, wd.wrapY, vx, vy, sum);
-                        }
-                    }
-                }
+                WalkRuns32(rs, re, slot, pf, rad, sPos, sRad, R, lp.scale, xDimF, yDimF, wd.wrapX, wd.wrapY, vx, vy);
                 return make_float2(vx, vy);
             }
             const int32_t bs = 1 << sh;
@@ -1482,8 +1523,8 @@ namespace halcuda
         __global__ void ForcesWells(const int32_t *__restrict__ bucket, const int32_t *__restrict__ offsets,
                                     const float2 *__restrict__ sPos, const float *__restrict__ sRad,
                                     const int32_t *__restrict__ sCell, const int32_t *__restrict__ wellOf,
-                                    const AgentWellDev *__restrict__ wells, int32_t n, double interactionRad, float R,
-                                    float k, float *__restrict__ vel)
+                                    const AgentWellDev *__restrict__ wells, int32_t n, double interactionRad,
+                                    bool intR, float R, float k, float *__restrict__ vel)
         {
             ChainEntry();
             const int32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1492,8 +1533,8 @@ namespace halcuda
                 return;
             }
             const int32_t i = bucket[slot];
-            const AgentWellDev wd = wells[wellOf[i]];
-            StoreDelta(vel, i, ForceSlotWell(slot, offsets, sPos, sRad, sCell, interactionRad, R, k, wd));
+            const AgentWellDev wd = wells[wellOf[slot]];  // the slots go well by well, as the agents do
+            StoreDelta(vel, i, ForceSlotWell(slot, offsets, sPos, sRad, sCell, interactionRad, intR, R, k, wd));
         }
 
         // ForcesWells with each agent's SphericalAgent2D update fused, moved
@@ -1502,7 +1543,7 @@ namespace halcuda
                                         const float2 *__restrict__ sPos, const float *__restrict__ sRad,
                                         const int32_t *__restrict__ sCell, const int32_t *__restrict__ wellOf,
                                         const AgentWellDev *__restrict__ wells, int32_t n, double interactionRad,
-                                        float R, float k, float friction, float maxVel, float *__restrict__ vel,
+                                        bool intR, float R, float k, float friction, float maxVel, float *__restrict__ vel,
                                         float2 *__restrict__ pos, float2 *__restrict__ velocity)
         {
             ChainEntry();
@@ -1512,8 +1553,8 @@ namespace halcuda
                 return;
             }
             const int32_t i = bucket[slot];
-            const AgentWellDev wd = wells[wellOf[i]];
-            const V2<float> d = ForceSlotWell(slot, offsets, sPos, sRad, sCell, interactionRad, R, k, wd);
+            const AgentWellDev wd = wells[wellOf[slot]];  // the slots go well by well, as the agents do
+            const V2<float> d = ForceSlotWell(slot, offsets, sPos, sRad, sCell, interactionRad, intR, R, k, wd);
             StoreDelta(vel, i, d);
             MoveParams mp;
             mp.friction = friction;
@@ -2679,13 +2720,13 @@ namespace halcuda
         if (a.velState != nullptr)
         {
             LaunchChained(ForcesWellsMove, fblocks, TF, s, a.bucket, a.offsets, a.sPos, a.sRad, a.sCell, a.wellOf,
-                          a.wells, a.n, a.interactionRad, a.R, a.k, a.friction, a.maxVel, a.vel, a.posOut,
+                          a.wells, a.n, a.interactionRad, IntegerRadius(a.interactionRad), a.R, a.k, a.friction, a.maxVel, a.vel, a.posOut,
                           a.velState);
         }
         else
         {
             LaunchChained(ForcesWells, fblocks, TF, s, a.bucket, a.offsets, a.sPos, a.sRad, a.sCell, a.wellOf,
-                          a.wells, a.n, a.interactionRad, a.R, a.k, a.vel);
+                          a.wells, a.n, a.interactionRad, IntegerRadius(a.interactionRad), a.R, a.k, a.vel);
         }
         CountLaunch(7);
         return LaunchStatus("agent wells");

@@ -49,3 +49,25 @@ def test_group_equals_thread(hal, n, dim, radius, wrap):
     # (a pair at the very edge of the radius may be in for one precision only)
     bad = np.abs(small - exact) > 1e-4 * max(np.abs(exact).max(), 1e-6)
     assert bad.mean() <= 2e-3
+
+
+@pytest.mark.parametrize("n", [450, 470, 1300])
+def test_long_windows_equal_group(hal, n):
+    """Windows around the length (64) from which a thread walks its runs one
+    by one, and far past it, against the group's sums; some runs empty."""
+    dim = 8
+    rng = np.random.default_rng(n)
+    pos = (rng.random((n, 2)) * dim).astype(np.float32)
+    pos[: n // 8] = [2.5, 2.5]                       # a pile in one cell
+    pos[(np.floor(pos[:, 0]) == 5)] = [0.25, 7.5]    # an empty column, a full corner
+    rad = (0.3 + 0.4 * rng.random(n)).astype(np.float32)
+    far = LIMIT + 1
+    fpos = np.stack([dim + 16.0 + 32.0 * rng.random(far), dim * rng.random(far)], 1).astype(np.float32)
+    with hal.Agents(dim + 64, dim, n + far) as a:
+        a.upload(np.concatenate([pos, fpos]).ravel(), np.concatenate([rad, np.full(far, 0.5, np.float32)]))
+        a.dispatch(1.0, 0.1, False, False)
+        want = a.download()[: 2 * n]
+    with hal.Agents(dim + 64, dim, n) as a:
+        a.upload(pos.ravel(), rad)
+        a.dispatch(1.0, 0.1, False, False)
+        assert np.array_equal(a.download(), want)
