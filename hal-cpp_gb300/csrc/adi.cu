@@ -13,16 +13,22 @@
 // index y*xDim + x) so that the x-sweep's lines are contiguous.  Each sweep
 // reads contiguous lines and writes its result transposed: the x-sweep reads
 // f (B) and writes w in HAL's layout ("layout A", x*yDim + y), whose y-lines
-// the y-sweep reads, writing f' back in layout B.  Both sweeps therefore run
-// the same kernel, AdiSweep:
+// the y-sweep reads, writing f' back in layout B.  The rows of both layouts
+// are padded to whole 16-byte units (zeros), so that lines of any length are
+// copied and written 16 bytes at a time.  Both sweeps therefore run the same
+// kernel: lines of up to 1024 positions AdiLines (a warp per line, below),
+// longer ones AdiSweep:
 //   1. stage the CTA's R lines plus the line on either side (the explicit
-//      cross-axis term) into shared memory with TMA, completion on an
-//      mbarrier whose wait is bounded.  When L is a multiple of 256 one 3-D
-//      tensor copy (cp.async.bulk.tensor, box 32 x P x (R+2), 128-byte
-//      swizzle, zero fill outside the field) stages the whole tile and the
-//      kernel indexes shared memory through the same swizzle; otherwise each
-//      32-element chunk is a 1-D cp.async.bulk (or plain loads for ragged
-//      lines) into a 36-float slot.  Either way every later access is a
+//      cross-axis term) into shared memory.  When L is a multiple of 256 one
+//      3-D tensor copy (cp.async.bulk.tensor, box 32 x P x (R+2), 128-byte
+//      swizzle, zero fill outside the field), complete on an mbarrier whose
+//      wait is bounded, stages the whole tile and the kernel indexes shared
+//      memory through the same swizzle; otherwise a warp copies whole lines by
+//      16-byte asynchronous copies, each 32-element chunk into a 36-float
+//      slot.  (A bulk copy per chunk took longer: 128 bytes each, thousands a
+//      CTA; us per tick bulk / here: 2047 x 2049 40.7 / 37.0, 3179 x 2193
+//      80.4 / 71.6, 4000^2 192 / 141, 2040^2 29.0 / 26.4 against 20.7 for
+//      2048^2 through the tensor copy.)  Either way every later access is a
 //      conflict-free 128-bit LDS/STS;
 //   2. each thread solves one 32-row chunk of two lines (two interleaved
 //      Thomas chains in registers), exchanges the separator right-hand sides
@@ -378,7 +384,6 @@ namespace halcuda
             extern __shared__ __align__(1024) float smem[];
             __shared__ __align__(8) unsigned long long mbar;
             __shared__ int s_fail;
-            __shared__ uint32_t s_tmaBytes;
             const int P = p.plan.P;
             const int R = p.R;
             // staged lines first, on a 1024-byte boundary (128-byte swizzle)
@@ -433,8 +438,6 @@ namespace halcuda
             const bool inPadded = p.inStride >= L4 && (p.inStride & 3) == 0;
 
             // ---- 1. stage lines x0-1 .. x0+R --------------------------------
-            __shared__ const float *sSrc[kMaxR + 2];
-            __shared__ int sTma[kMaxR + 2];
             const uint32_t bar = SmemAddr(&mbar);
             const int nStaged = R + 2;
             uint32_t tmaBytes = 0;
@@ -476,36 +479,60 @@ namespace halcuda
                 if (tid == 0)
                 {
                     s_fail = 0;
-                    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
-                    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
                 }
-                for (int rs = tid; rs < nStaged; rs += nthreads)
+                // a warp copies whole lines, 16 bytes a lane, into the padded
+                // chunks; a line that its stride does not pad to 16-byte units
+                // (a ghost line) goes through registers
+                const int warps = nthreads >> 5, lane = tid & 31;
+                for (int rr = tid >> 5; rr < nStaged; rr += warps)
                 {
-                    // source of staged line rs: a grid line, the neighbour line
+                    // source of staged line rr: a grid line, the neighbour line
                     // beyond an edge (wrapped, a Dirichlet ghost line, or zeros);
                     // lines further out (a CTA past the last line) are never read
-                    const int32_t line = x0 - 1 + rs;
+                    const int32_t line = x0 - 1 + rr;
                     const float *src = nullptr;
-                    bool padded = false;  // the line's stride pads it to a multiple of 4 floats
+                    bool vec = inPadded;  // the line's stride pads it to a multiple of 4 floats
                     if (line >= 0 && line < p.Nlines)
                     {
                         src = p.in + static_cast<int64_t>(line) * p.inStride;
-                        padded = inPadded;
                     }
                     else if (line == -1 || line == p.Nlines)
                     {
                         if (p.wrapLines)
                         {
                             src = p.in + static_cast<int64_t>((line < 0) ? p.Nlines - 1 : 0) * p.inStride;
-                            padded = inPadded;
                         }
                         else
                         {
                             src = (line < 0) ? p.ghostLo : p.ghostHi;
+                            vec = vecL;
                         }
                     }
-                    sSrc[rs] = src;
-                    sTma[rs] = (src != nullptr) && (vecL || padded) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
+                    vec = vec && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+                    for (int u = lane; u < P * (M / 4); u += 32)
+                    {
+                        float *dst = sLines + SOff4<SWZ>(rr, u >> 3, u & 7, P, p.LS);
+                        const int32_t pos = 4 * u;
+                        if (src != nullptr && pos < L)
+                        {
+                            if (vec)
+                            {
+                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(SmemAddr(dst)),
+                                             "l"(src + pos)
+                                             : "memory");
+                            }
+                            else
+                            {
+                                St4(dst, make_float4(src[pos], pos + 1 < L ? src[pos + 1] : 0.0f,
+                                                     pos + 2 < L ? src[pos + 2] : 0.0f,
+                                                     pos + 3 < L ? src[pos + 3] : 0.0f));
+                            }
+                        }
+                        else
+                        {
+                            St4(dst, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+                        }
+                    }
                 }
                 for (int q = tid; q < kCoefFloats / 4; q += nthreads)
                 {
@@ -520,71 +547,7 @@ namespace halcuda
                         sG[q] = __ldg(p.plan.gband + q);
                     }
                 }
-                __syncthreads();  // mbarrier initialised, line sources known
-                if (tid == 0)
-                {
-                    for (int rr = 0; rr < nStaged; rr++)
-                    {
-                        tmaBytes += sTma[rr] ? static_cast<uint32_t>(L4) * 4u : 0u;
-                    }
-                    if (tmaBytes > 0)
-                    {
-                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tmaBytes)
-                                     : "memory");
-                    }
-                    s_tmaBytes = tmaBytes;
-                }
-                __syncthreads();  // the expected byte count is in place before any copy lands
-                tmaBytes = s_tmaBytes;
-                {
-                    // thread -> chunk kc of lines rr0, rr0 + rstride, ...
-                    const int kc = tid % P;
-                    const int rstride = nthreads / P;
-                    const int32_t n = min(M, L - kc * M);  // elements of this chunk inside the line
-                    const int32_t n4 = (n + 3) & ~3;          // the same in whole 16-byte units
-                    for (int rr = tid / P; rr < nStaged && tid < rstride * P; rr += rstride)
-                    {
-                        const float *src = sSrc[rr];
-                        float *dst = sLines + rr * p.LS + kc * kChunkStride;
-                        int32_t filled = n;  // elements the copies write
-                        if (sTma[rr])
-                        {
-                            // a padded line's last chunk takes its padding
-                            // (zeros) along, to a whole 16-byte unit
-                            filled = n4;
-                            asm volatile(
-                                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                    SmemAddr(dst)),
-                                "l"(src + kc * M), "r"(static_cast<uint32_t>(n4) * 4u), "r"(bar)
-                                : "memory");
-                        }
-                        else if (src != nullptr)
-                        {
-                            // a line the bulk copy cannot take (unaligned or
-                            // ragged): 4-byte asynchronous copies, all of the
-                            // chunk in flight at once; the thread waits for
-                            // its own copies below
-                            for (int i = 0; i < n; i++)
-                            {
-                                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(SmemAddr(dst + i)),
-                                             "l"(src + kc * M + i)
-                                             : "memory");
-                            }
-                        }
-                        else
-                        {
-                            for (int i = 0; i < n; i++)
-                            {
-                                dst[i] = 0.0f;
-                            }
-                        }
-                        for (int i = filled; i < M; i++)
-                        {
-                            dst[i] = 0.0f;  // padding past the line end (disjoint from the copy)
-                        }
-                    }
-                    asm volatile("cp.async.wait_all;" ::: "memory");
-                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
             }
             if (tmaBytes > 0)
             {
@@ -1304,8 +1267,11 @@ namespace halcuda
         // a small sweep now is latency (launch, loads, the chunk's chain,
         // stores), a 1024^2 one the transposed write-out.
         // Measured on GB300, us per tick (zero-flux, with source), SweepTile /
-        // here: 64^2 13.2 / 4.5, 256^2 11.0 / 5.5, 300 x 517 19.0 / 7.5, 512^2
-        // 11.5 / 6.9, 777 x 1000 19.2 / 11.1, 1024^2 12.9 / 12.3.
+        // here: 64^2 13.8 / 4.5, 256^2 11.4 / 5.5, 300 x 517 16.1 / 7.7, 512^2
+        // 11.6 / 6.9, 777 x 1000 15.7 / 11.2, 1024^2 12.9 / 12.3.  (A batch of
+        // many grids keeps every SM busy without it: 24 grids of 64 to 1024
+        // squared, 5.1M cells, x- and y-sweep 25 + 27 us by SweepTile, 30 + 44
+        // in this form.)
         // Lanes that read their chunks straight from global memory, 128 bytes
         // apart, were slower (1024^2 17.1): a request per lane.
         constexpr int kLineMaxP = 32;     // chunks: lines up to 1024
