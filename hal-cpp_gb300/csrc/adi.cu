@@ -2477,6 +2477,7 @@ namespace halcuda
                 return FromLayoutB(field[cur].p, static_cast<float *>(d), s);
             }
             HAL_TRY(FromLayoutB(field[cur].p, w.p, s));
+            PopulateOutput(host, Length() * sizeof(float));
             return CudaStatus(cudaMemcpyAsync(host, w.p, Length() * sizeof(float), cudaMemcpyDeviceToHost, s),
                               "cudaMemcpy(field)");
         }

@@ -2154,6 +2154,8 @@ extern "C" int hal_cuda_agents_get_state(hal_cuda_agents *h, float *positions, f
     HAL_TRY(CudaStatus(cudaSetDevice(h->device), "cudaSetDevice"));
     cudaStream_t s = h->stream.Get();
     const size_t bytes = static_cast<size_t>(n) * sizeof(float2);
+    PopulateOutput(positions, bytes);
+    PopulateOutput(velocities, bytes);
     if (n > 0 && positions != nullptr)
     {
         HAL_TRY(CudaStatus(cudaMemcpyAsync(positions, h->pos32.p, bytes, cudaMemcpyDeviceToHost, s),

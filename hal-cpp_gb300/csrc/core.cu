@@ -1,6 +1,9 @@
 // core.cu -- library-wide entry points: version, errors, device selection.
 #include "common.cuh"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <cstring>
 
 namespace halcuda
@@ -29,6 +32,35 @@ namespace halcuda
     int CurrentDevice()
     {
         return t_device;
+    }
+
+    void PopulateOutput(void *p, size_t bytes)
+    {
+#ifndef MADV_POPULATE_WRITE
+        constexpr int MADV_POPULATE_WRITE = 23;
+#endif
+        // (the fields of 24 wells of up to 3.7 MB each: from 4 MB on 4.8 ms,
+        // from 1 MB 3.4, from 512 KB 3.1, from 256 KB 3.1)
+        constexpr size_t kMinBytes = size_t(512) << 10;
+        if (p == nullptr || bytes < kMinBytes)
+        {
+            return;
+        }
+        cudaPointerAttributes attr;
+        if (cudaPointerGetAttributes(&attr, p) != cudaSuccess)
+        {
+            cudaGetLastError();  // not CUDA's memory: an older runtime's answer
+        }
+        else if (attr.type != cudaMemoryTypeUnregistered)
+        {
+            return;
+        }
+        const uintptr_t page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
+        const uintptr_t lo = reinterpret_cast<uintptr_t>(p) / page * page;
+        const uintptr_t hi = (reinterpret_cast<uintptr_t>(p) + bytes + page - 1) / page * page;
+        // a hint: where the kernel does not know it, or the pages cannot be
+        // written, the copy itself faults or fails as before
+        (void)madvise(reinterpret_cast<void *>(lo), hi - lo, MADV_POPULATE_WRITE);
     }
 
     namespace

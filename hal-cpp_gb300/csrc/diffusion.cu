@@ -1256,6 +1256,7 @@ extern "C" int hal_cuda_diffusion_get_field(hal_cuda_diffusion *h, float *field,
                 "hal_cuda_diffusion_get_field: field must hold xDim*yDim values");
     HAL_TRY(halcuda::CudaStatus(cudaSetDevice(h->device), "cudaSetDevice"));
     cudaStream_t s = h->stream.Get();
+    halcuda::PopulateOutput(field, h->Length() * sizeof(float));
     HAL_TRY(halcuda::CudaStatus(cudaMemcpyAsync(field, h->field[h->cur].p, h->Length() * sizeof(float),
                                                 cudaMemcpyDeviceToHost, s),
                                 "cudaMemcpy(field)"));

@@ -1802,6 +1802,8 @@ extern "C" int hal_cuda_pdegrid_get_state(hal_cuda_pdegrid *h, double *field, do
     HAL_TRY(Prepare(h, "hal_cuda_pdegrid_get_state"));
     cudaStream_t s = h->stream.Get();
     const size_t bytes = static_cast<size_t>(h->Length()) * sizeof(double);
+    halcuda::PopulateOutput(field, bytes);
+    halcuda::PopulateOutput(deltas, bytes);
     if (field != nullptr)
     {
         HAL_TRY(CudaStatus(cudaMemcpyAsync(field, h->f.p, bytes, cudaMemcpyDeviceToHost, s), "cudaMemcpy(field)"));

@@ -889,6 +889,7 @@ extern "C" int hal_cuda_wells_get_field(hal_cuda_wells *h, int32_t well, float *
         HAL_TRY(LaunchTransposeStrided(from, h->strideF[well], h->W(well), d.yDim, d.yDim, d.xDim, s));
         from = h->W(well);
     }
+    PopulateOutput(field, bytes);
     HAL_TRY(CudaStatus(cudaMemcpyAsync(field, from, bytes, cudaMemcpyDeviceToHost, s), "cudaMemcpy(field)"));
     return CudaStatus(cudaStreamSynchronize(s), "hal_cuda_wells_get_field");
 }
@@ -1009,6 +1010,8 @@ extern "C" int hal_cuda_wells_get_agents(hal_cuda_wells *h, float *positions, fl
     HAL_TRY(CudaStatus(cudaSetDevice(h->device), "cudaSetDevice"));
     cudaStream_t s = h->stream.Get();
     const size_t bytes = static_cast<size_t>(len) * sizeof(float);
+    PopulateOutput(positions, bytes);
+    PopulateOutput(velocities, bytes);
     if (len > 0 && positions != nullptr)
     {
         HAL_TRY(CudaStatus(cudaMemcpyAsync(positions, h->apos.p, bytes, cudaMemcpyDeviceToHost, s),
