@@ -26,7 +26,7 @@
 //      memory through the same swizzle; otherwise a warp copies whole lines by
 //      16-byte asynchronous copies, each 32-element chunk into a 36-float
 //      slot.  (A bulk copy per chunk took longer: 128 bytes each, thousands a
-//      CTA; us per tick bulk / here: 2047 x 2049 40.7 / 37.0, 3179 x 2193
+//      CTA; us per tick bulk / here: 2047 x 2049 40.8 / 37.0, 3179 x 2193
 //      80.4 / 71.6, 4000^2 192 / 141, 2040^2 29.0 / 26.4 against 20.7 for
 //      2048^2 through the tensor copy.)  Either way every later access is a
 //      conflict-free 128-bit LDS/STS;
@@ -338,6 +338,23 @@ namespace halcuda
             return true;
         }
 
+        // What an earlier kernel wrote.  The chunked form is launched chained
+        // (ChainWait), so its loads must not move ahead of its wait and are
+        // coherent; the tensor-staged form starts after the kernel before and
+        // takes the read-only path (20.8 against 21.1 us per 2048^2 tick).
+        template <bool SWZ, typename T>
+        __device__ __forceinline__ T LdIn(const T *p)
+        {
+            if constexpr (SWZ)
+            {
+                return __ldg(p);
+            }
+            else
+            {
+                return __ldcg(p);
+            }
+        }
+
         // One CTA's tile of a sweep: lines x0 .. x0+R-1 of the grid p.  tmap
         // is the grid's line tensor map (SWZ) or null.
         // Agent counts of write-out unit u: nc[e][i] = agents binned in cell
@@ -345,6 +362,7 @@ namespace halcuda
         // + e) * L + 4u + i (cells in layout A); 0 for the quad's lines at or
         // past quadLines (outside the grid).  With L % 4 == 0 each line's five
         // offsets are one 16-byte load and one 4-byte load.
+        template <bool SWZ>
         __device__ __forceinline__ void UnitCounts(const int32_t *__restrict__ off, int32_t line0, int32_t quadLines,
                                                    int32_t u, int32_t L, bool vecL, int32_t (&nc)[4][4])
         {
@@ -358,8 +376,8 @@ namespace halcuda
                 }
                 else if (vecL)
                 {
-                    const int4 a = __ldg(reinterpret_cast<const int4 *>(oc));
-                    const int32_t b = __ldg(oc + 4);
+                    const int4 a = LdIn<SWZ>(reinterpret_cast<const int4 *>(oc));
+                    const int32_t b = LdIn<SWZ>(oc + 4);
                     nc[e][0] = a.y - a.x;
                     nc[e][1] = a.z - a.y;
                     nc[e][2] = a.w - a.z;
@@ -370,10 +388,40 @@ namespace halcuda
 #pragma unroll
                     for (int i = 0; i < 4; i++)
                     {
-                        nc[e][i] = (4 * u + i < L) ? __ldg(oc + i + 1) - __ldg(oc + i) : 0;
+                        nc[e][i] = (4 * u + i < L) ? LdIn<SWZ>(oc + i + 1) - LdIn<SWZ>(oc + i) : 0;
                     }
                 }
             }
+        }
+
+        // The plan's coefficients and band (gCount entries; 0: not staged) into
+        // shared memory.  They do not come from the kernel before.
+        __device__ __forceinline__ void LoadPlan(const SweepParams &p, float *sCoef, float *sG, int gCount, int tid,
+                                                 int nthreads)
+        {
+            for (int q = tid; q < kCoefFloats / 4; q += nthreads)
+            {
+                const int t = q / (kCoefCount * M / 4);
+                St4(sCoef + t * kCoefTypeStride + 4 * (q - t * (kCoefCount * M / 4)),
+                    __ldg(reinterpret_cast<const float4 *>(p.plan.coef) + q));
+            }
+            for (int q = tid; q < gCount; q += nthreads)
+            {
+                sG[q] = __ldg(p.plan.gband + q);
+            }
+        }
+
+        // Chained launches: waits until the kernel before on the stream is
+        // complete, then lets the next one start its own preparation (us per
+        // tick without / with: 1500^2 25.1 / 23.8, 2047^2 25.9 / 24.8, 2049^2
+        // 43.0 / 39.8, 600 x 3000 23.5 / 21.8, 4000^2 141 / 135).  (The
+        // tensor-staged form is not chained: its CTAs hold an SM's registers,
+        // so the next one's could only wait, and its tensor copy would start
+        // after the plan's loads: 21.2 against 20.8 us per 2048^2 tick.)
+        __device__ __forceinline__ void ChainWait()
+        {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;");
         }
 
         // UPT: the y-sweep's commit has the agent uptake term (a separate
@@ -459,19 +507,7 @@ namespace halcuda
                         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(0), "r"(0), "r"(x0 - 1), "r"(bar)
                         : "memory");
                 }
-                for (int q = tid; q < kCoefFloats / 4; q += nthreads)
-                {
-                    const int t = q / (kCoefCount * M / 4);
-                    St4(sCoef + t * kCoefTypeStride + 4 * (q - t * (kCoefCount * M / 4)),
-                        __ldg(reinterpret_cast<const float4 *>(p.plan.coef) + q));
-                }
-                if (gInSmem)
-                {
-                    for (int q = tid; q < gCount; q += nthreads)
-                    {
-                        sG[q] = __ldg(p.plan.gband + q);
-                    }
-                }
+                LoadPlan(p, sCoef, sG, gInSmem ? gCount : 0, tid, nthreads);
                 __syncthreads();  // mbarrier initialised before anyone waits on it
             }
             else
@@ -480,6 +516,8 @@ namespace halcuda
                 {
                     s_fail = 0;
                 }
+                LoadPlan(p, sCoef, sG, gInSmem ? gCount : 0, tid, nthreads);
+                ChainWait();
                 // a warp copies whole lines, 16 bytes a lane, into the padded
                 // chunks; a line that its stride does not pad to 16-byte units
                 // (a ghost line) goes through registers
@@ -534,19 +572,6 @@ namespace halcuda
                         }
                     }
                 }
-                for (int q = tid; q < kCoefFloats / 4; q += nthreads)
-                {
-                    const int t = q / (kCoefCount * M / 4);
-                    St4(sCoef + t * kCoefTypeStride + 4 * (q - t * (kCoefCount * M / 4)),
-                        __ldg(reinterpret_cast<const float4 *>(p.plan.coef) + q));
-                }
-                if (gInSmem)
-                {
-                    for (int q = tid; q < gCount; q += nthreads)
-                    {
-                        sG[q] = __ldg(p.plan.gband + q);
-                    }
-                }
                 asm volatile("cp.async.wait_all;" ::: "memory");
             }
             if (tmaBytes > 0)
@@ -583,7 +608,7 @@ namespace halcuda
                     }
                     for (int32_t pos = tid; pos < L; pos += nthreads)
                     {
-                        sLines[SPos<SWZ>(rr, pos, P, p.LS)] = __ldg(src + pos);
+                        sLines[SPos<SWZ>(rr, pos, P, p.LS)] = LdIn<SWZ>(src + pos);
                     }
                 }
             }
@@ -694,11 +719,11 @@ namespace halcuda
                     const int32_t line = x0 + ll0 + j;
                     if (k == 0)
                     {
-                        z[j][0] = fmaf(p.r, __ldg(p.implLo + line), z[j][0]);
+                        z[j][0] = fmaf(p.r, LdIn<SWZ>(p.implLo + line), z[j][0]);
                     }
                     if (lastIdx >= 0 && lastIdx < M)
                     {
-                        const float add = p.r * __ldg(p.implHi + line);
+                        const float add = p.r * LdIn<SWZ>(p.implHi + line);
 #pragma unroll
                         for (int e = 0; e < M; e++)
                         {
@@ -817,9 +842,9 @@ namespace halcuda
 #pragma unroll
                     for (int i = 0; i < 4; i++)
                     {
-                        fv0[b][i] = ok ? __ldg(reinterpret_cast<const float4 *>(p.f + g0 + i * nl))
+                        fv0[b][i] = ok ? LdIn<SWZ>(reinterpret_cast<const float4 *>(p.f + g0 + i * nl))
                                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        sv0[b][i] = (ok && p.src != nullptr) ? __ldg(reinterpret_cast<const float4 *>(p.src + g0 + i * nl))
+                        sv0[b][i] = (ok && p.src != nullptr) ? LdIn<SWZ>(reinterpret_cast<const float4 *>(p.src + g0 + i * nl))
                                                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
                 }
@@ -953,10 +978,10 @@ namespace halcuda
                                             {
                                                 continue;  // past the line end: no output row
                                             }
-                                            fv[b][i] = __ldg(reinterpret_cast<const float4 *>(p.f + g0 + i * nl));
+                                            fv[b][i] = LdIn<SWZ>(reinterpret_cast<const float4 *>(p.f + g0 + i * nl));
                                             if (hasSrc)
                                             {
-                                                sv[b][i] = __ldg(reinterpret_cast<const float4 *>(p.src + g0 + i * nl));
+                                                sv[b][i] = LdIn<SWZ>(reinterpret_cast<const float4 *>(p.src + g0 + i * nl));
                                             }
                                         }
                                     }
@@ -976,7 +1001,7 @@ namespace halcuda
                                 (void)nc;  // read by the commit of MODE kSweepTick only
                                 if constexpr (UPT)
                                 {
-                                    UnitCounts(p.cellOffsets, line0, quadLines, u, L, vecL, nc);
+                                    UnitCounts<SWZ>(p.cellOffsets, line0, quadLines, u, L, vecL, nc);
                                 }
 #pragma unroll
                                 for (int i = 0; i < 4; i++)
@@ -1031,8 +1056,8 @@ namespace halcuda
 #pragma unroll
                                     for (int i = 0; i < 4; i++)
                                     {
-                                        fo[i] = __ldg(reinterpret_cast<const float4 *>(p.f + g0 + i * nl));
-                                        so[i] = hasSrc ? __ldg(reinterpret_cast<const float4 *>(p.src + g0 + i * nl))
+                                        fo[i] = LdIn<SWZ>(reinterpret_cast<const float4 *>(p.f + g0 + i * nl));
+                                        so[i] = hasSrc ? LdIn<SWZ>(reinterpret_cast<const float4 *>(p.src + g0 + i * nl))
                                                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                                     }
                                 };
@@ -1052,7 +1077,7 @@ namespace halcuda
                                     int32_t nc[4][4] = {};
                                     if constexpr (UPT)
                                     {
-                                        UnitCounts(p.cellOffsets, line0, quadLines, u, L, vecL, nc);
+                                        UnitCounts<SWZ>(p.cellOffsets, line0, quadLines, u, L, vecL, nc);
                                     }
 #pragma unroll
                                     for (int i = 0; i < 4; i++)
@@ -1125,10 +1150,10 @@ namespace halcuda
                                 const int64_t gi = static_cast<int64_t>(pos) * outRow + line0;
                                 if (vecOut)
                                 {
-                                    fv[b] = __ldg(reinterpret_cast<const float4 *>(p.f + gi));
+                                    fv[b] = LdIn<SWZ>(reinterpret_cast<const float4 *>(p.f + gi));
                                     if (p.src != nullptr)
                                     {
-                                        sv[b] = __ldg(reinterpret_cast<const float4 *>(p.src + gi));
+                                        sv[b] = LdIn<SWZ>(reinterpret_cast<const float4 *>(p.src + gi));
                                     }
                                 }
                                 else
@@ -1139,8 +1164,8 @@ namespace halcuda
                                     {
                                         if (line0 + e < p.Nlines)
                                         {
-                                            tf[e] = __ldg(p.f + gi + e);
-                                            ts[e] = (p.src != nullptr) ? __ldg(p.src + gi + e) : 0.0f;
+                                            tf[e] = LdIn<SWZ>(p.f + gi + e);
+                                            ts[e] = (p.src != nullptr) ? LdIn<SWZ>(p.src + gi + e) : 0.0f;
                                         }
                                     }
                                     fv[b] = make_float4(tf[0], tf[1], tf[2], tf[3]);
@@ -1154,7 +1179,7 @@ namespace halcuda
                                         if (line0 + e < p.Nlines)
                                         {
                                             const int64_t ci = static_cast<int64_t>(line0 + e) * L + pos;
-                                            nn[b][e] = __ldg(p.cellOffsets + ci + 1) - __ldg(p.cellOffsets + ci);
+                                            nn[b][e] = LdIn<SWZ>(p.cellOffsets + ci + 1) - LdIn<SWZ>(p.cellOffsets + ci);
                                         }
                                     }
                                 }
@@ -1444,12 +1469,12 @@ namespace halcuda
             {
                 if (k == 0)
                 {
-                    z[0] = fmaf(p.r, __ldg(p.implLo + line), z[0]);
+                    z[0] = fmaf(p.r, __ldcg(p.implLo + line), z[0]);
                 }
                 const int lastIdx = (L - 1) - k * M;
                 if (lastIdx >= 0 && lastIdx < M)
                 {
-                    const float add = p.r * __ldg(p.implHi + line);
+                    const float add = p.r * __ldcg(p.implHi + line);
 #pragma unroll
                     for (int e = 0; e < M; e++)
                     {
@@ -1663,6 +1688,25 @@ namespace halcuda
             }
         }
 
+        // A launch that may start while the kernel before it on the stream ends
+        // (the kernel waits, ChainWait).
+        template <class Kernel, class... Args>
+        int LaunchChainedSmem(Kernel kernel, unsigned blocks, unsigned threads, size_t smem, cudaStream_t s,
+                              const char *what, const Args &...args)
+        {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(blocks);
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            return CudaStatus(cudaLaunchKernelEx(&cfg, kernel, args...), what);
+        }
+
         // Lines up to kLineMaxP chunks go to AdiLines.
         bool UseLines(const SweepParams &p)
         {
@@ -1684,18 +1728,9 @@ namespace halcuda
             const int32_t lines = W * lpw;
             const size_t smem = sizeof(float) * static_cast<size_t>(lines + 2) * LineStride(P);
             HAL_TRY(s_limit.Ensure(AdiLines<MODE, UPT, W>, smem, "cudaFuncSetAttribute(AdiLines)"));
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(static_cast<unsigned>((p.Nlines + lines - 1) / lines));
-            cfg.blockDim = dim3(32 * W);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = s;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
             CountLaunch();
-            return CudaStatus(cudaLaunchKernelEx(&cfg, AdiLines<MODE, UPT, W>, p, lpw), "AdiLines launch");
+            return LaunchChainedSmem(AdiLines<MODE, UPT, W>, static_cast<unsigned>((p.Nlines + lines - 1) / lines),
+                                     32 * W, smem, s, "AdiLines launch", p, lpw);
         }
 
         template <int MODE, bool UPT>
@@ -1904,10 +1939,9 @@ namespace halcuda
         int LaunchTiles(const SweepParams *table, const int2 *tiles, int32_t nTiles, size_t smem, int32_t threads,
                         cudaStream_t s)
         {
-            AdiSweepTiles<MODE><<<static_cast<unsigned>(nTiles), static_cast<unsigned>(threads), smem, s>>>(table,
-                                                                                                       tiles);
             CountLaunch();
-            return LaunchStatus("AdiSweepTiles");
+            return LaunchChainedSmem(AdiSweepTiles<MODE>, static_cast<unsigned>(nTiles), static_cast<unsigned>(threads),
+                                     smem, s, "AdiSweepTiles", table, tiles);
         }
     }
 
@@ -2201,7 +2235,8 @@ namespace halcuda
                     CUtensorMap none;
                     std::memset(&none, 0, sizeof(none));
                     HAL_TRY((EnableSweepSmem<MODE, false, UPT>(sh.smem)));
-                    AdiSweep<MODE, false, UPT><<<blocks, sh.threads, sh.smem, s>>>(p, none);
+                    HAL_TRY(LaunchChainedSmem(AdiSweep<MODE, false, UPT>, blocks, static_cast<unsigned>(sh.threads),
+                                              sh.smem, s, "AdiSweep launch", p, none));
                 }
                 return HAL_CUDA_OK;
             };
