@@ -1343,6 +1343,260 @@ namespace halcuda
                                  deltas, pos, velocity, cellOf, arrival, counts);
         }
 
+        // ---- FP64 forces: a group of lanes per agent, only near pairs in FP64 --
+        // The FP64 pipe bounds the interface's FP64 sums (a warp's FP64
+        // instruction holds its pipe for 64 cycles, about 35 of them per pair
+        // with the square root and the divisions), and a thread per agent gives
+        // a dense cluster's long walks to a few warps.  Here eight lanes take an
+        // agent's candidates; each first compares an FP32 distance, made from
+        // the positions' bits without FP64 instructions and with its error
+        // bound on the safe side, and only the pairs that may be in range are
+        // queued.  Full queues of pairs then go through the FP64 operations, one
+        // pair per lane, and the terms are subtracted in the visiting order: the
+        // same operations on the same values as a thread's walk, bit for bit.
+        // A group takes up to four agents, one after another, once there are
+        // enough of them, so that a sparse grid's few pairs still fill the lanes.
+        // Measured on GB300, the interface's FP64 call, thread per agent / here
+        // (us): 50k agents in 256^2, 30% in a cluster, 380 / 159 (the kernel 298
+        // / 86); 5k in 100 x 77 207 / 66; 200k in 1024^2 453 / 287 with a cluster,
+        // 253 / 211 uniform; 20k in 256^2 at R = 2 632 / 220.  One agent a group
+        // throughout: 200k uniform 288; up to eight from 20k on: 50k 198, 200k with
+        // a cluster 359.
+        constexpr int kPairQueue = 32;  // pairs an agent's queue holds (a power of two)
+        constexpr int kPairDrain = 16;  // a queue this long is worked off
+        constexpr int32_t kPairGroups = 152 * 256;  // groups that fill the chip
+        constexpr int32_t kPairPerGroup = 4;        // agents a group takes, one after another, at most
+
+        // The FP32 value nearest towards zero of v, by its bits: zero below the
+        // normal range, NaN for what FP32 cannot hold (and for NaN itself).
+        __device__ __forceinline__ float Truncated(double v)
+        {
+            const int32_t hi = __double2hiint(v);
+            const uint32_t lo = static_cast<uint32_t>(__double2loint(v));
+            const uint32_t mag = static_cast<uint32_t>(hi) & 0x7fffffffu;
+            uint32_t f = __funnelshift_l(lo, mag - 0x38000000u, 3);
+            f = (mag < 0x38100000u) ? 0u : f;
+            f = (mag >= 0x47f00000u) ? 0x7fffffffu : f;
+            return __uint_as_float(f | (static_cast<uint32_t>(hi) & 0x80000000u));
+        }
+
+        template <bool WALLS>
+        __global__ void __launch_bounds__(128)
+            ForcesGroup64(const int32_t *__restrict__ bucket, const int32_t *__restrict__ offsets,
+                          const double2 *__restrict__ sPos, const double *__restrict__ sRad, int32_t n,
+                          int32_t perGroup, double interactionRad, LawParams<double> lp, int32_t xDim, int32_t yDim,
+                          int32_t wrapX, int32_t wrapY, double *vel, const double *velIn)
+        {
+            constexpr int G = kGroupLanes;
+            __shared__ int2 queue[128 / G][kPairQueue];  // (agent's slot, neighbour's slot)
+            __shared__ double2 terms[128 / G][G];
+            __shared__ int32_t owner[128 / G][G];
+            ChainEntry();
+            const int j = threadIdx.x & (G - 1);
+            const int group = threadIdx.x / G;
+            const int64_t first = (static_cast<int64_t>(blockIdx.x) * 128 + threadIdx.x) / G * perGroup;
+            const bool odd = (j & 1) != 0;
+            if (WALLS)
+            {
+                wrapX = wrapY = 0;
+            }
+            const float xDimF = static_cast<float>(xDim), yDimF = static_cast<float>(yDim);
+            const double xDimD = xDim, yDimD = yDim;
+            const float rF = __double2float_ru(interactionRad);
+            const uint64_t rBits = static_cast<uint64_t>(__double_as_longlong(interactionRad));
+            int32_t head = 0, tail = 0;  // the queue's pairs [head, tail), modulo its size
+            int32_t cur = -1;            // the agent whose sum v holds (its slot)
+            double v = 0.0;              // even lanes: the x sum, odd lanes: the y sum
+            auto start = [&](int32_t slot) {
+                return velIn == nullptr ? 0.0 : velIn[2 * static_cast<int64_t>(bucket[slot]) + (odd ? 1 : 0)];
+            };
+            auto store = [&](int32_t slot, double sum) {
+                if (j < 2)
+                {
+                    vel[2 * static_cast<int64_t>(bucket[slot]) + j] = sum;
+                }
+            };
+
+            // up to eight queued pairs, in order
+            auto drain = [&]() {
+                __syncwarp();
+                const bool valid = j < tail - head;
+                const int2 pair = valid ? queue[group][(head + j) & (kPairQueue - 1)] : make_int2(-1, -1);
+                head += min(tail - head, G);
+                double2 t = make_double2(0.0, 0.0);
+                if (valid)
+                {
+                    const double2 p = sPos[pair.x];
+                    const double2 pj = sPos[pair.y];
+                    const double radSum = Add(sRad[pair.x], sRad[pair.y]);
+                    const double x = Disp(p.x, pj.x, xDimD, wrapX != 0);
+                    const double y = Disp(p.y, pj.y, yDimD, wrapY != 0);
+                    const double dist = Sqrt(Add(Mul(x, x), Mul(y, y)));
+                    // 0 < dist < R by the bits of non-negative values (NaN's are larger)
+                    const uint64_t dBits = static_cast<uint64_t>(__double_as_longlong(dist));
+                    if (dBits != 0 && dBits < rBits)
+                    {
+                        const double force = OverlapForce<kLawLinear>(Sub(radSum, dist), lp);
+                        t.x = Mul(Div(x, dist), force);
+                        t.y = Mul(Div(y, dist), force);
+                    }
+                }
+                terms[group][j] = t;
+                owner[group][j] = pair.x;
+                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < G; u++)
+                {
+                    const int32_t o = owner[group][u];
+                    if (o >= 0 && o != cur)
+                    {
+                        if (cur >= 0)
+                        {
+                            store(cur, v);
+                        }
+                        cur = o;
+                        v = start(o);
+                    }
+                    // (subtracting the zero of a pair out of range changes nothing)
+                    v = Sub(v, reinterpret_cast<const double *>(&terms[group][u])[odd ? 1 : 0]);
+                }
+                __syncwarp();
+            };
+
+            for (int32_t a = 0; a < perGroup; a++)
+            {
+                const bool live = first + a < n;
+                const int32_t slot = live ? static_cast<int32_t>(first + a) : n - 1;
+                const double2 p = sPos[slot];
+                const int32_t before = tail;
+                // window bounds in FP64, as the CPU computes them, one per lane:
+                // floor(x - R), ceil(x + R), floor(y - R), ceil(y + R)
+                int32_t bound;
+                {
+                    const double c = (j & 2) ? p.y : p.x;
+                    const double b = __dadd_rn(c, odd ? interactionRad : -interactionRad);
+                    bound = static_cast<int32_t>(odd ? ceil(b) : floor(b));
+                }
+                int32_t xStart = __shfl_sync(0xffffffffu, bound, 0, G), xEnd = __shfl_sync(0xffffffffu, bound, 1, G);
+                int32_t yStart = __shfl_sync(0xffffffffu, bound, 2, G), yEnd = __shfl_sync(0xffffffffu, bound, 3, G);
+                if (!wrapX)
+                {
+                    xStart = max(xStart, 0);
+                    xEnd = min(xEnd, xDim);
+                }
+                if (!wrapY)
+                {
+                    yStart = max(yStart, 0);
+                    yEnd = min(yEnd, yDim);
+                }
+                const float pxF = Truncated(p.x), pyF = Truncated(p.y);
+                // |error| of an FP32 distance: per axis the coordinates'
+                // truncation (2^-23 of each), the difference's and the wrap's
+                // roundings (2^-24 of |a| + |b| and of |a| + |b| + dim), twice
+                // that where only one precision wraps: below
+                // 4.8e-7 (|a| + |b| + dim)
+                const float own = 6e-7f * (fabsf(pxF) + fabsf(pyF) + xDimF + yDimF) + 1e-30f;
+
+                // The window as runs of cells, in the visiting order: a round
+                // takes up to eight runs (one per row, two where a wrapped
+                // y-range crosses the edge; the y-range may wrap more than once).
+                const bool some = live && xEnd > xStart && yEnd > yStart;
+                int32_t row = xStart, yAt = yStart;  // the next run
+                while (__any_sync(0xffffffffu, some && row < xEnd))
+                {
+                    int32_t s0 = 0, len = 0;
+#pragma unroll 1
+                    for (int r = 0; r < G && some && row < xEnd; r++)
+                    {
+                        int32_t retX = row;
+                        if (retX < 0 || retX >= xDim)
+                        {
+                            retX %= xDim;  // only reached on a wrapped axis (clamped otherwise)
+                            retX = (retX < 0) ? retX + xDim : retX;
+                        }
+                        int32_t retY = yAt;
+                        if (retY < 0 || retY >= yDim)
+                        {
+                            retY %= yDim;
+                            retY = (retY < 0) ? retY + yDim : retY;
+                        }
+                        const int32_t run = min(yEnd - yAt, yDim - retY);
+                        if (r == j)
+                        {
+                            const int32_t cell = retX * yDim + retY;
+                            s0 = __ldg(offsets + cell);
+                            len = __ldg(offsets + cell + run) - s0;
+                        }
+                        yAt += run;
+                        if (yAt >= yEnd)
+                        {
+                            yAt = yStart;
+                            row++;
+                        }
+                    }
+                    __syncwarp();
+                    // candidate k is slot k + shift[r] of the first run r with k < end[r]
+                    int32_t end[G], shift[G];
+                    int32_t total = 0;
+#pragma unroll
+                    for (int r = 0; r < G; r++)
+                    {
+                        shift[r] = __shfl_sync(0xffffffffu, s0, r, G) - total;
+                        total += __shfl_sync(0xffffffffu, len, r, G);
+                        end[r] = total;
+                    }
+                    const int32_t most = __reduce_max_sync(0xffffffffu, total);
+                    for (int32_t k0 = 0; k0 < most; k0 += G)
+                    {
+                        const int32_t k = k0 + j;
+                        int32_t q = shift[G - 1];
+#pragma unroll
+                        for (int r = G - 2; r >= 0; r--)
+                        {
+                            q = (k < end[r]) ? shift[r] : q;
+                        }
+                        q += k;
+                        // the pairs that may be in range join the queue, in the lanes' order
+                        bool pass = false;
+                        if (k < total && q != slot)
+                        {
+                            const double2 pj = sPos[q];
+                            const float qx = Truncated(pj.x), qy = Truncated(pj.y);
+                            const float x = Disp(pxF, qx, xDimF, wrapX != 0);
+                            const float y = Disp(pyF, qy, yDimF, wrapY != 0);
+                            const float reach = rF + (own + 6e-7f * (fabsf(qx) + fabsf(qy)));
+                            // not greater: a NaN passes to the FP64 test
+                            pass = !(x * x + y * y > reach * reach * 1.00001f);
+                        }
+                        const uint32_t mine =
+                            (__ballot_sync(0xffffffffu, pass) >> (threadIdx.x & 24)) & ((1u << G) - 1u);
+                        if (pass)
+                        {
+                            queue[group][(tail + __popc(mine & ((1u << j) - 1u))) & (kPairQueue - 1)] =
+                                make_int2(slot, q);
+                        }
+                        tail += __popc(mine);
+                        while (__any_sync(0xffffffffu, tail - head >= kPairDrain))
+                        {
+                            drain();
+                        }
+                    }
+                }
+                if (live && tail == before)
+                {
+                    store(slot, start(slot));  // no neighbour near
+                }
+            }
+            while (__any_sync(0xffffffffu, tail > head))
+            {
+                drain();
+            }
+            if (cur >= 0)
+            {
+                store(cur, v);
+            }
+        }
+
         // ---- many independent wells in one pass ------------------------------
         // Agents of all wells are concatenated, and so are the cells of the
         // wells that have agents (well w's cells start at cellBase); the
@@ -1782,6 +2036,16 @@ namespace halcuda
                         go(Forces<T, TV, kLawLinear, false, false, true>);
                         break;
                     }
+                }
+                if constexpr (std::is_same<T, double>::value && std::is_same<TV, double>::value)
+                {
+                    const int32_t perGroup = std::min(std::max(n / kPairGroups, 1), kPairPerGroup);
+                    const int64_t groups = (static_cast<int64_t>(n) + perGroup - 1) / perGroup;
+                    LaunchChained(!wrapX && !wrapY ? ForcesGroup64<true> : ForcesGroup64<false>,
+                                  static_cast<unsigned>((groups * kGroupLanes + T_ - 1) / T_), T_, s, bucket.p,
+                                  offsets.p, SortedPosBuf(T()), sRad, n, perGroup, R + 0.0, lp, xDim, yDim,
+                                  static_cast<int32_t>(wrapX), static_cast<int32_t>(wrapY), vel, velIn);
+                    break;
                 }
                 go(Forces<T, TV, kLawLinear, false, false>);
                 break;
