@@ -125,6 +125,16 @@ namespace halcuda
             cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
         }
 
+        // The same kernels launched after their predecessor is complete, for
+        // work that differs much between CTAs: CTAs that start early fill the
+        // SMs that the ending kernel leaves, and a few SMs then hold the heavy
+        // ones (ForcesGroup64 with a pile of 2586 agents: 2.9 against 1.5 ms).
+        template <typename... KArgs, typename... Args>
+        void LaunchAfter(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args... args)
+        {
+            kernel<<<grid, block, 0, s>>>(static_cast<KArgs>(args)...);
+        }
+
         // Inclusive warp scan.
         __device__ __forceinline__ int32_t WarpScan(int32_t v, int lane)
         {
@@ -1356,14 +1366,18 @@ namespace halcuda
         // same operations on the same values as a thread's walk, bit for bit.
         // A group takes up to four agents, one after another, once there are
         // enough of them, so that a sparse grid's few pairs still fill the lanes.
+        // A CTA is one warp: the agents' walks differ much, and small CTAs spread
+        // them (20k in 256^2 at R = 2: CTAs of 128 threads 215, of 32 180 us).
         // Measured on GB300, the interface's FP64 call, thread per agent / here
-        // (us): 50k agents in 256^2, 30% in a cluster, 380 / 159 (the kernel 298
-        // / 86); 5k in 100 x 77 207 / 66; 200k in 1024^2 453 / 287 with a cluster,
-        // 253 / 211 uniform; 20k in 256^2 at R = 2 632 / 220.  One agent a group
-        // throughout: 200k uniform 288; up to eight from 20k on: 50k 198, 200k with
-        // a cluster 359.
+        // (us): 50k agents in 256^2, 30% in a cluster, 380 / 157 (the kernel 298
+        // / 86), the cluster clipped at a corner, with 2586 agents in one cell,
+        // 8360 / 1480; 5k in 100 x 77 207 / 67; 200k in 1024^2 453 / 283 with a
+        // cluster, 253 / 211 uniform; 20k in 256^2 at R = 2 632 / 180.  One agent
+        // a group throughout: 200k uniform 288; up to eight from 20k on: 50k 198,
+        // 200k with a cluster 359.
         constexpr int kPairQueue = 32;  // pairs an agent's queue holds (a power of two)
         constexpr int kPairDrain = 16;  // a queue this long is worked off
+        constexpr int kPairThreads = 32;
         constexpr int32_t kPairGroups = 152 * 256;  // groups that fill the chip
         constexpr int32_t kPairPerGroup = 4;        // agents a group takes, one after another, at most
 
@@ -1381,20 +1395,20 @@ namespace halcuda
         }
 
         template <bool WALLS>
-        __global__ void __launch_bounds__(128)
+        __global__ void __launch_bounds__(kPairThreads)
             ForcesGroup64(const int32_t *__restrict__ bucket, const int32_t *__restrict__ offsets,
                           const double2 *__restrict__ sPos, const double *__restrict__ sRad, int32_t n,
                           int32_t perGroup, double interactionRad, LawParams<double> lp, int32_t xDim, int32_t yDim,
                           int32_t wrapX, int32_t wrapY, double *vel, const double *velIn)
         {
             constexpr int G = kGroupLanes;
-            __shared__ int2 queue[128 / G][kPairQueue];  // (agent's slot, neighbour's slot)
-            __shared__ double2 terms[128 / G][G];
-            __shared__ int32_t owner[128 / G][G];
+            __shared__ int2 queue[kPairThreads / G][kPairQueue];  // (agent's slot, neighbour's slot)
+            __shared__ double2 terms[kPairThreads / G][G];
+            __shared__ int32_t owner[kPairThreads / G][G];
             ChainEntry();
             const int j = threadIdx.x & (G - 1);
             const int group = threadIdx.x / G;
-            const int64_t first = (static_cast<int64_t>(blockIdx.x) * 128 + threadIdx.x) / G * perGroup;
+            const int64_t first = (static_cast<int64_t>(blockIdx.x) * kPairThreads + threadIdx.x) / G * perGroup;
             const bool odd = (j & 1) != 0;
             if (WALLS)
             {
@@ -1565,8 +1579,11 @@ namespace halcuda
                             const float x = Disp(pxF, qx, xDimF, wrapX != 0);
                             const float y = Disp(pyF, qy, yDimF, wrapY != 0);
                             const float reach = rF + (own + 6e-7f * (fabsf(qx) + fabsf(qy)));
-                            // not greater: a NaN passes to the FP64 test
-                            pass = !(x * x + y * y > reach * reach * 1.00001f);
+                            // not greater: a NaN passes to the FP64 test; agents on
+                            // one spot (a pile at a clipped edge) are no pair
+                            const bool same = __double_as_longlong(pj.x) == __double_as_longlong(p.x) &&
+                                              __double_as_longlong(pj.y) == __double_as_longlong(p.y);
+                            pass = !same && !(x * x + y * y > reach * reach * 1.00001f);
                         }
                         const uint32_t mine =
                             (__ballot_sync(0xffffffffu, pass) >> (threadIdx.x & 24)) & ((1u << G) - 1u);
@@ -2041,9 +2058,9 @@ namespace halcuda
                 {
                     const int32_t perGroup = std::min(std::max(n / kPairGroups, 1), kPairPerGroup);
                     const int64_t groups = (static_cast<int64_t>(n) + perGroup - 1) / perGroup;
-                    LaunchChained(!wrapX && !wrapY ? ForcesGroup64<true> : ForcesGroup64<false>,
-                                  static_cast<unsigned>((groups * kGroupLanes + T_ - 1) / T_), T_, s, bucket.p,
-                                  offsets.p, SortedPosBuf(T()), sRad, n, perGroup, R + 0.0, lp, xDim, yDim,
+                    LaunchAfter(!wrapX && !wrapY ? ForcesGroup64<true> : ForcesGroup64<false>,
+                                  static_cast<unsigned>((groups * kGroupLanes + kPairThreads - 1) / kPairThreads), kPairThreads,
+                                  s, bucket.p, offsets.p, SortedPosBuf(T()), sRad, n, perGroup, R + 0.0, lp, xDim, yDim,
                                   static_cast<int32_t>(wrapX), static_cast<int32_t>(wrapY), vel, velIn);
                     break;
                 }
