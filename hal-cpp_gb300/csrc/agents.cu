@@ -5,7 +5,10 @@
 // scatter of agent indices, and a per-agent scan of the surrounding cells
 // summing a linear spring force.  Here each pass is data-parallel:
 //   BinCount     one thread per agent: clamped cell, atomic count, arrival rank
-//   scan         reduce-then-scan over the cells (three launches, no spin waits)
+//   scan         reduce-then-scan over the cells (at most three launches, no spin
+//                waits; in a resident run the move before adds up the tiles: 20k
+//                agents in 256^2 17.9 -> 16.5 us per tick, 200k in 1024^2 36.4 ->
+//                33.9, 400k in 2048^2 52.9 -> 49.5, 1M 90 either way)
 //   Scatter      agent -> offsets[cell] + arrival rank (order within a cell is
 //                the atomic arrival order, not yet the CPU's)
 //   Stabilize    one thread per arrival-order slot: its agent counts the
@@ -133,6 +136,18 @@ namespace halcuda
         void LaunchAfter(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args... args)
         {
             kernel<<<grid, block, 0, s>>>(static_cast<KArgs>(args)...);
+        }
+
+        // Adds the calling lanes' agents to the sums of their cells' scan tiles,
+        // one atomic per tile a warp meets (neighbouring slots share most).
+        __device__ __forceinline__ void AddToTiles(int32_t *__restrict__ tileSums, int32_t cell)
+        {
+            const int32_t tile = cell / kScanTile;
+            const uint32_t same = __match_any_sync(__activemask(), tile);
+            if (static_cast<int>(threadIdx.x & 31) == __ffs(same) - 1)
+            {
+                atomicAdd(tileSums + tile, __popc(same));
+            }
         }
 
         // Inclusive warp scan.
@@ -394,11 +409,21 @@ namespace halcuda
             }
         }
 
+        // With tileSums it also clears the nTiles tile sums, which the scan has
+        // used: the resident step's move adds to them.
         __global__ void Scatter(const int32_t *__restrict__ cellOf, const int32_t *__restrict__ arrival,
-                                const int32_t *__restrict__ offsets, int32_t n, int32_t *__restrict__ bucketTmp)
+                                const int32_t *__restrict__ offsets, int32_t n, int32_t *__restrict__ bucketTmp,
+                                int32_t *__restrict__ tileSums, int32_t nTiles)
         {
             ChainEntry();
             int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+            if (tileSums != nullptr)
+            {
+                for (int32_t t = i; t < nTiles; t += static_cast<int32_t>(gridDim.x * blockDim.x))
+                {
+                    tileSums[t] = 0;
+                }
+            }
             if (i >= n)
             {
                 return;
@@ -1085,7 +1110,7 @@ namespace halcuda
                                    MoveParams mp, float *__restrict__ deltas, float2 *__restrict__ pos,
                                    float2 *__restrict__ velocity, float *__restrict__ sums,
                                    int32_t *__restrict__ cellOf, int32_t *__restrict__ arrival,
-                                   int32_t *__restrict__ counts)
+                                   int32_t *__restrict__ counts, int32_t *__restrict__ tileSums)
         {
             ChainEntry();
             const int32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1115,6 +1140,7 @@ namespace halcuda
                 const int32_t c = CellCoord(p.x, xDim) * yDim + CellCoord(p.y, yDim);
                 cellOf[i] = c;
                 arrival[i] = atomicAdd(counts + c, 1);
+                AddToTiles(tileSums, c);
             }
         }
 
@@ -1312,7 +1338,8 @@ namespace halcuda
                                                       int32_t xDim, int32_t yDim, const MoveParams &mp,
                                                       float *__restrict__ deltas, float2 *__restrict__ pos,
                                                       float2 *__restrict__ velocity, int32_t *__restrict__ cellOf,
-                                                      int32_t *__restrict__ arrival, int32_t *__restrict__ counts)
+                                                      int32_t *__restrict__ arrival, int32_t *__restrict__ counts,
+                                                      int32_t *__restrict__ tileSums)
         {
             const bool lead = live && (threadIdx.x & (kGroupLanes - 1)) == 0;
             // the move's inputs, in flight during the sums
@@ -1334,6 +1361,7 @@ namespace halcuda
             const int32_t c = CellCoord(p.x, xDim) * yDim + CellCoord(p.y, yDim);
             cellOf[i] = c;
             arrival[i] = atomicAdd(counts + c, 1);
+            AddToTiles(tileSums, c);
         }
 
         template <bool WALLS>
@@ -1343,14 +1371,14 @@ namespace halcuda
                                         int32_t yDim, MoveParams mp, float *__restrict__ deltas,
                                         float2 *__restrict__ pos, float2 *__restrict__ velocity,
                                         int32_t *__restrict__ cellOf, int32_t *__restrict__ arrival,
-                                        int32_t *__restrict__ counts)
+                                        int32_t *__restrict__ counts, int32_t *__restrict__ tileSums)
         {
             ChainEntry();
             const int32_t at = (blockIdx.x * blockDim.x + threadIdx.x) / kGroupLanes;
             const bool live = at < n;
             const int32_t slot = live ? at : n - 1;
             MoveSlotGroup<WALLS>(slot, live, bucket, offsets, sPos, sRad, interactionRad, intR, R, lp, xDim, yDim, mp,
-                                 deltas, pos, velocity, cellOf, arrival, counts);
+                                 deltas, pos, velocity, cellOf, arrival, counts, tileSums);
         }
 
         // ---- FP64 forces: a group of lanes per agent, only near pairs in FP64 --
@@ -1886,9 +1914,10 @@ namespace halcuda
         bool sumsValid = false;  // sums32 holds the last dispatch's or step's sums
         int32_t nTiles = 0;
         bool countsDirty = true;  // counts not known to be zero (cleared by each scan)
-        // counts, cellOf and arrival hold the binning of the current pos32,
-        // counted by the last resident step's force kernel as it moved the
-        // agents: the next FP32 binning skips its count pass
+        // counts, cellOf, arrival and tileSums hold the binning of the current
+        // pos32, counted by the last resident step's force kernel as it moved
+        // the agents: the next FP32 binning skips its count pass and the
+        // scan's first
         bool binsPrecounted = false;
 
         // pos32 changed by other means than the resident step: the precounted
@@ -1968,17 +1997,22 @@ namespace halcuda
             {
                 cudaEventRecord(ev[0], s);
             }
-            LaunchChained(ScanReduce, nTiles, kScanThreads, s, counts.p, C, tileSums.p);
+            if (!pre)
+            {
+                // (the move that counted the agents has added up the tiles too)
+                LaunchChained(ScanReduce, nTiles, kScanThreads, s, counts.p, C, tileSums.p);
+                CountLaunch();
+            }
             if (nTiles <= kScanSumTiles)
             {
                 LaunchChained(ScanApplySum, nTiles, kScanThreads, s, counts.p, C, tileSums.p, offsets.p, n);
-                CountLaunch(2);
+                CountLaunch();
             }
             else
             {
                 LaunchChained(ScanTiles, 1u, kScanThreads, s, tileSums.p, nTiles);
                 LaunchChained(ScanApply<true>, nTiles, kScanThreads, s, counts.p, C, tileSums.p, offsets.p, n);
-                CountLaunch(3);
+                CountLaunch(2);
             }
             countsDirty = (cudaPeekAtLastError() != cudaSuccess);
             if (ev)
@@ -1987,7 +2021,7 @@ namespace halcuda
             }
             if (n > 0)
             {
-                LaunchChained(Scatter, ablocks, T, s, cellOf.p, arrival.p, offsets.p, n, bucketTmp.p);
+                LaunchChained(Scatter, ablocks, T, s, cellOf.p, arrival.p, offsets.p, n, bucketTmp.p, tileSums.p, nTiles);
                 CountLaunch();
             }
             if (ev)
@@ -2133,7 +2167,7 @@ namespace
             LaunchChained(kernel, blocks, T, s, a.bucket.p, a.offsets.p, a.sPos.p, a.sRad32.p, a.n, R,
                           static_cast<float>(R), lp, a.xDim, a.yDim, mp, a.vel32.p,
                           reinterpret_cast<float2 *>(a.pos32.p), a.velState.p, sums, a.cellOf.p, a.arrival.p,
-                          a.counts.p);
+                          a.counts.p, a.tileSums.p);
         };
         const bool walls = !mp.wrapX && !mp.wrapY;
         if (law.kind == kLawLinear && !law.sums && a.n <= kGroupAgents)
@@ -2142,7 +2176,7 @@ namespace
             LaunchChained(walls ? ForcesMoveGroup<true> : ForcesMoveGroup<false>, groups, T, s, a.bucket.p, a.offsets.p,
                           a.sPos.p, a.sRad32.p, a.n, R, IntegerRadius(R), static_cast<float>(R), lp, a.xDim, a.yDim, mp,
                           a.vel32.p, reinterpret_cast<float2 *>(a.pos32.p), a.velState.p, a.cellOf.p, a.arrival.p,
-                          a.counts.p);
+                          a.counts.p, a.tileSums.p);
         }
         else
         switch (law.kind * 2 + (law.sums ? 1 : 0))
@@ -2490,7 +2524,8 @@ namespace halcuda
             BinCount<float><<<static_cast<unsigned>((h->n + T - 1) / T), T, 0, s>>>(
                 h->pos32.p, h->n, h->xDim, h->yDim, static_cast<float2 *>(nullptr), h->cellOf.p, h->arrival.p,
                 h->counts.p);
-            CountLaunch();
+            ScanReduce<<<static_cast<unsigned>(h->nTiles), kScanThreads, 0, s>>>(h->counts.p, h->C, h->tileSums.p);
+            CountLaunch(2);
             HAL_TRY(LaunchStatus("agent binning"));
             h->binsPrecounted = true;
             h->countsDirty = false;
@@ -2945,7 +2980,7 @@ extern "C" int hal_cuda_agents_forces_noalloc(const float *positions, const floa
     ScanReduce<<<nTiles, kScanThreads, 0, s>>>(counts, C, tileSums);
     ScanTiles<<<1, kScanThreads, 0, s>>>(tileSums, static_cast<int32_t>(nTiles));
     ScanApply<false><<<nTiles, kScanThreads, 0, s>>>(counts, C, tileSums, offsets, n);
-    Scatter<<<ablocks, T, 0, s>>>(cellOf, arrival, offsets, n, bucketTmp);
+    Scatter<<<ablocks, T, 0, s>>>(cellOf, arrival, offsets, n, bucketTmp, nullptr, 0);
     Stabilize<float, float><<<ablocks, T, 0, s>>>(cellOf, offsets, bucketTmp, posF, radii, n, bucket, sPos, sRad);
     const int TF = 128;
     LawParams<float> lp;
@@ -2995,7 +3030,8 @@ namespace halcuda
         {
             LaunchChained(ScanApply<false>, nTiles, kScanThreads, s, a.counts, a.cells, a.tileSums, a.offsets, a.n);
         }
-        LaunchChained(Scatter, ablocks, T, s, a.cellOf, a.arrival, a.offsets, a.n, a.bucketTmp);
+        LaunchChained(Scatter, ablocks, T, s, a.cellOf, a.arrival, a.offsets, a.n, a.bucketTmp,
+                      static_cast<int32_t *>(nullptr), 0);
         LaunchChained(StabilizeWells, ablocks, T, s, a.cellOf, a.offsets, a.bucketTmp, a.posF, a.rad, a.wellOf,
                       a.wells, a.n, a.bucket, a.sPos, a.sRad, a.sCell);
         const int TF = (a.forceThreads == 64 || a.forceThreads == 256) ? a.forceThreads : 128;
