@@ -42,7 +42,7 @@ namespace halcuda
         constexpr int kScanItems = 4 * kScanGroups;
         constexpr int kScanTile = kScanThreads * kScanItems;
         // tiles whose prefix ScanApplySum forms itself (4.19M cells)
-        constexpr int kScanSumTiles = 1024;
+        constexpr int kScanSumTiles = kAgentScanSumTiles;
 
         // Position pairs in the precision of the path: float2 on the FP32
         // resident path, double2 on the FP64 interface path.
@@ -291,15 +291,13 @@ namespace halcuda
             }
         }
 
-        // Counts up to this many cells (in practice: all) are cleared by
-        // ScanApply as it reads them, writing only the 4-cell groups that
-        // hold a count; a memset before the binning clears counts not known
-        // to be zero.  With every group written, clearing in the scan had
-        // measured 3.5x slower than a memset at 109M cells; with only the
-        // occupied groups it is faster at both measured sizes (4.19M cells,
-        // 1M agents: 119.2 -> 115.0 us per dispatch; 109M cells, 5.2M
+        // The counts are cleared by the scan as it reads them, writing only the
+        // 4-cell groups that hold a count; a memset before the binning clears
+        // counts not known to be zero.  With every group written, clearing in
+        // the scan had measured 3.5x slower than a memset at 109M cells; with
+        // only the occupied groups it is faster at both measured sizes (4.19M
+        // cells, 1M agents: 119.2 -> 115.0 us per dispatch; 109M cells, 5.2M
         // agents: agent pass 0.818 -> 0.772 ms).
-        constexpr int64_t kClearInScanCells = int64_t(1) << 40;
 
         // The cells of a thread of passes 3: kScanItems consecutive cells
         // from tile + thread * kScanItems (in order, for the exclusive scan),
@@ -1646,10 +1644,19 @@ namespace halcuda
         // Agents of all wells are concatenated, and so are the cells of the
         // wells that have agents (well w's cells start at cellBase); the
         // count, scan, scatter and stable-rank passes then run unchanged over
-        // the concatenation, and each agent's window walks its own well.
+        // the concatenation, and each agent's window walks its own well.  With
+        // motion the move counts the agents for the next pass, as the resident
+        // step does, and the pass starts at the scan: 427k agents in 48 wells,
+        // 71.5 -> 65.0 us per pass.
+
+        __device__ __forceinline__ int32_t WellBin(const AgentWellDev &wd, float px, float py)
+        {
+            return static_cast<int32_t>(wd.binBase) + (CellCoord(px, wd.xDim) >> wd.binShift) * wd.binsY +
+                   (CellCoord(py, wd.yDim) >> wd.binShift);
+        }
 
         __global__ void BinCountWells(const float *__restrict__ pos, const int32_t *__restrict__ wellOf,
-                                      const AgentWellDev *__restrict__ wells, int32_t n, float2 *__restrict__ posF,
+                                      const AgentWellDev *__restrict__ wells, int32_t n,
                                       int32_t *__restrict__ binOf, int32_t *__restrict__ arrival,
                                       int32_t *__restrict__ counts)
         {
@@ -1662,9 +1669,7 @@ namespace halcuda
             const AgentWellDev wd = wells[wellOf[i]];
             const float px = pos[2 * static_cast<int64_t>(i)];
             const float py = pos[2 * static_cast<int64_t>(i) + 1];
-            posF[i] = make_float2(px, py);
-            const int32_t b = static_cast<int32_t>(wd.binBase) + (CellCoord(px, wd.xDim) >> wd.binShift) * wd.binsY +
-                              (CellCoord(py, wd.yDim) >> wd.binShift);
+            const int32_t b = WellBin(wd, px, py);
             binOf[i] = b;
             arrival[i] = atomicAdd(counts + b, 1);
         }
@@ -1672,11 +1677,10 @@ namespace halcuda
         // The order within a coarse bin: by cell, then by agent index (the
         // per-cell binning's order for each cell).  The agent at
         // arrival-order slot q counts the agents of its bin before it.
-        __global__ void StabilizeWells(const int32_t *__restrict__ binOf, const int32_t *__restrict__ offsets,
-                                       const int32_t *__restrict__ bucketTmp, const float2 *__restrict__ posF,
-                                       const float *__restrict__ rad, const int32_t *__restrict__ wellOf,
-                                       const AgentWellDev *__restrict__ wells, int32_t n,
-                                       int32_t *__restrict__ bucket, float2 *__restrict__ sPos,
+        __global__ void StabilizeWells(const int32_t *__restrict__ offsets, const int32_t *__restrict__ bucketTmp,
+                                       const float2 *__restrict__ posF, const float *__restrict__ rad,
+                                       const int32_t *__restrict__ wellOf, const AgentWellDev *__restrict__ wells,
+                                       int32_t n, int32_t *__restrict__ bucket, float2 *__restrict__ sPos,
                                        float *__restrict__ sRad, int32_t *__restrict__ sCell)
         {
             ChainEntry();
@@ -1686,24 +1690,29 @@ namespace halcuda
                 return;
             }
             const int32_t i = bucketTmp[q];
-            const AgentWellDev wd = wells[wellOf[q]];
+            const AgentWellDev wd = wells[wellOf[q]];  // the slots go well by well, as the agents do
             const float2 p = posF[i];
+            const float r = rad[i];
             const int32_t c = CellCoord(p.x, wd.xDim) * wd.yDim + CellCoord(p.y, wd.yDim);
-            const int32_t b = binOf[i];
+            const int32_t b = WellBin(wd, p.x, p.y);
             const int32_t s = offsets[b];
             const int32_t e = offsets[b + 1];
             int32_t rank = 0;
             for (int32_t t = s; t < e; t++)
             {
                 const int32_t j = bucketTmp[t];
-                const float2 pj = posF[j];
-                const int32_t cj = CellCoord(pj.x, wd.xDim) * wd.yDim + CellCoord(pj.y, wd.yDim);
+                int32_t cj = c;  // one cell per bin: the bin's agents share it
+                if (wd.binShift != 0)
+                {
+                    const float2 pj = posF[j];
+                    cj = CellCoord(pj.x, wd.xDim) * wd.yDim + CellCoord(pj.y, wd.yDim);
+                }
                 rank += (cj < c || (cj == c && j < i)) ? 1 : 0;
             }
             const int32_t slot = s + rank;
             bucket[slot] = i;
             sPos[slot] = p;
-            sRad[slot] = rad[i];
+            sRad[slot] = r;
             sCell[slot] = c;
         }
 
@@ -1843,7 +1852,9 @@ namespace halcuda
                                         const int32_t *__restrict__ sCell, const int32_t *__restrict__ wellOf,
                                         const AgentWellDev *__restrict__ wells, int32_t n, double interactionRad,
                                         bool intR, float R, float k, float friction, float maxVel, float *__restrict__ vel,
-                                        float2 *__restrict__ pos, float2 *__restrict__ velocity)
+                                        float2 *__restrict__ pos, float2 *__restrict__ velocity,
+                                        int32_t *__restrict__ binOf, int32_t *__restrict__ arrival,
+                                        int32_t *__restrict__ counts, int32_t *__restrict__ tileSums)
         {
             ChainEntry();
             const int32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1869,6 +1880,12 @@ namespace halcuda
             MoveAgent(mp, p, v);
             pos[i] = p;
             velocity[i] = v;
+            // BinCountWells' work for the next pass: this one's scan cleared the
+            // counts, its scatter the tile sums
+            const int32_t nb = WellBin(wd, p.x, p.y);
+            binOf[i] = nb;
+            arrival[i] = atomicAdd(counts + nb, 1);
+            AddToTiles(tileSums, nb);
         }
     }
 
@@ -3000,54 +3017,74 @@ namespace halcuda
         return static_cast<int32_t>((cells + kScanTile - 1) / kScanTile);
     }
 
-    int LaunchAgentWells(const AgentWellsArgs &a, cudaStream_t s)
+    int LaunchCountWells(const AgentWellsArgs &a, cudaStream_t s)
+    {
+        const int T = 256;
+        LaunchChained(BinCountWells, static_cast<unsigned>((a.n + T - 1) / T), T, s, a.pos, a.wellOf, a.wells, a.n,
+                      a.cellOf, a.arrival, a.counts);
+        LaunchChained(ScanReduce, static_cast<unsigned>(AgentScanTiles(a.cells)), kScanThreads, s, a.counts, a.cells,
+                      a.tileSums);
+        CountLaunch(2);
+        return LaunchStatus("agent wells count");
+    }
+
+    int LaunchBinWells(const AgentWellsArgs &a, cudaStream_t s)
     {
         if (a.n <= 0)
         {
             return HAL_CUDA_OK;
         }
-        // a.counts is zero here when small (allocated zeroed; every
-        // ScanApply<true> clears the counts it has read); large ones are
-        // cleared by a memset
-        const bool clearInScan = a.cells <= kClearInScanCells;
-        if (!clearInScan)
+        if (!a.counted)
         {
-            HAL_TRY(CudaStatus(cudaMemsetAsync(a.counts, 0, static_cast<size_t>(a.cells) * sizeof(int32_t), s),
-                               "cudaMemsetAsync(well counts)"));
+            HAL_TRY(LaunchCountWells(a, s));
         }
         const int T = 256;
         const unsigned ablocks = static_cast<unsigned>((a.n + T - 1) / T);
         const int32_t nTiles = AgentScanTiles(a.cells);
-        LaunchChained(BinCountWells, ablocks, T, s, a.pos, a.wellOf, a.wells, a.n, a.posF, a.cellOf, a.arrival,
-                      a.counts);
-        LaunchChained(ScanReduce, nTiles, kScanThreads, s, a.counts, a.cells, a.tileSums);
-        LaunchChained(ScanTiles, 1u, kScanThreads, s, a.tileSums, nTiles);
-        if (clearInScan)
+        // the scan clears the counts it has read
+        if (nTiles <= kScanSumTiles)
         {
-            LaunchChained(ScanApply<true>, nTiles, kScanThreads, s, a.counts, a.cells, a.tileSums, a.offsets, a.n);
+            LaunchChained(ScanApplySum, nTiles, kScanThreads, s, a.counts, a.cells, a.tileSums, a.offsets, a.n);
         }
         else
         {
-            LaunchChained(ScanApply<false>, nTiles, kScanThreads, s, a.counts, a.cells, a.tileSums, a.offsets, a.n);
+            LaunchChained(ScanTiles, 1u, kScanThreads, s, a.tileSums, nTiles);
+            LaunchChained(ScanApply<true>, nTiles, kScanThreads, s, a.counts, a.cells, a.tileSums, a.offsets, a.n);
+            CountLaunch();
         }
-        LaunchChained(Scatter, ablocks, T, s, a.cellOf, a.arrival, a.offsets, a.n, a.bucketTmp,
-                      static_cast<int32_t *>(nullptr), 0);
-        LaunchChained(StabilizeWells, ablocks, T, s, a.cellOf, a.offsets, a.bucketTmp, a.posF, a.rad, a.wellOf,
-                      a.wells, a.n, a.bucket, a.sPos, a.sRad, a.sCell);
+        LaunchChained(Scatter, ablocks, T, s, a.cellOf, a.arrival, a.offsets, a.n, a.bucketTmp, a.tileSums, nTiles);
+        LaunchChained(StabilizeWells, ablocks, T, s, a.offsets, a.bucketTmp, reinterpret_cast<const float2 *>(a.pos),
+                      a.rad, a.wellOf, a.wells, a.n, a.bucket, a.sPos, a.sRad, a.sCell);
+        CountLaunch(3);
+        return LaunchStatus("agent wells bins");
+    }
+
+    int LaunchForceWells(const AgentWellsArgs &a, cudaStream_t s)
+    {
+        if (a.n <= 0)
+        {
+            return HAL_CUDA_OK;
+        }
         const int TF = (a.forceThreads == 64 || a.forceThreads == 256) ? a.forceThreads : 128;
         const unsigned fblocks = static_cast<unsigned>((a.n + TF - 1) / TF);
         if (a.velState != nullptr)
         {
             LaunchChained(ForcesWellsMove, fblocks, TF, s, a.bucket, a.offsets, a.sPos, a.sRad, a.sCell, a.wellOf,
-                          a.wells, a.n, a.interactionRad, IntegerRadius(a.interactionRad), a.R, a.k, a.friction, a.maxVel, a.vel, a.posOut,
-                          a.velState);
+                          a.wells, a.n, a.interactionRad, IntegerRadius(a.interactionRad), a.R, a.k, a.friction,
+                          a.maxVel, a.vel, a.posOut, a.velState, a.cellOf, a.arrival, a.counts, a.tileSums);
         }
         else
         {
             LaunchChained(ForcesWells, fblocks, TF, s, a.bucket, a.offsets, a.sPos, a.sRad, a.sCell, a.wellOf,
                           a.wells, a.n, a.interactionRad, IntegerRadius(a.interactionRad), a.R, a.k, a.vel);
         }
-        CountLaunch(7);
+        CountLaunch();
         return LaunchStatus("agent wells");
+    }
+
+    int LaunchAgentWells(const AgentWellsArgs &a, cudaStream_t s)
+    {
+        HAL_TRY(LaunchBinWells(a, s));
+        return LaunchForceWells(a, s);
     }
 }

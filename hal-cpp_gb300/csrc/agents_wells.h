@@ -57,11 +57,11 @@ namespace halcuda
         const AgentWellDev *wells;
         int32_t n;
         int64_t cells;             // coarse bins of all wells (WellBins summed)
-        float2 *posF, *sPos;       // n each
+        float2 *sPos;              // n
         float *sRad;               // n
         int32_t *cellOf, *arrival, *bucketTmp, *bucket;  // n each (cellOf: the agent's bin)
         int32_t *sCell;            // n: each sorted slot's cell within its well
-        int32_t *counts;           // cells (bins), zero on entry (each binning's scan clears them again)
+        int32_t *counts;           // cells (bins): zero, or the agents counted (each binning's scan clears them)
         int32_t *offsets;          // cells (bins) + 1
         int32_t *tileSums;         // AgentScanTiles(cells)
         double interactionRad;
@@ -75,9 +75,15 @@ namespace halcuda
         float2 *velState = nullptr;  // n, or null: forces only
         float2 *posOut = nullptr;    // n: the positions, rewritten in place
         float friction = 1.0f, maxVel = -1.0f;
+        // cellOf, arrival, counts and tileSums hold the agents' count
+        // (LaunchCountWells, or the move of the pass before): the pass starts
+        // from it
+        bool counted = false;
     };
 
     int32_t AgentScanTiles(int64_t cells);
+    // up to this many scan tiles one launch sums up and applies them
+    constexpr int32_t kAgentScanSumTiles = 1024;
 
     // The bins of an agent handle's last binning, for other handles that act
     // per agent on a grid of the same size (hal_cuda_pdegrid_apply_agents).
@@ -91,8 +97,14 @@ namespace halcuda
         cudaStream_t stream;     // the handle's stream
     };
 
-    // Count, scan, scatter, stable rank and forces of every well's agents.
-    int LaunchAgentWells(const AgentWellsArgs &a, cudaStream_t s);
+    // Every well's agents: count (unless counted), scan, scatter, stable rank.
+    int LaunchBinWells(const AgentWellsArgs &a, cudaStream_t s);
+    // Their count alone (counts zero on entry).
+    int LaunchCountWells(const AgentWellsArgs &a, cudaStream_t s);
+    // The forces of binned agents; with velState the move too, which counts
+    // the moved agents for the next pass.
+    int LaunchForceWells(const AgentWellsArgs &a, cudaStream_t s);
+    int LaunchAgentWells(const AgentWellsArgs &a, cudaStream_t s);  // LaunchBinWells, then LaunchForceWells
 
     AgentBinsView AgentsBins(const hal_cuda_agents *a);
 }

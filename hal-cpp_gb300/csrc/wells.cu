@@ -112,8 +112,11 @@ namespace halcuda
         DevBuf<float> apos, arad, avel, sRad;
         DevBuf<float2> avelState;        // agents' own velocities, for motion
         bool motion = false;             // agents move after their forces each tick
+        // the bins' counts hold the agents where they are: each tick's move
+        // counts them for the next (motion only)
+        bool counted = false;
         float friction = 1.0f, maxVel = -1.0f;
-        DevBuf<float2> posF, sPos;
+        DevBuf<float2> sPos;
         DevBuf<int32_t> wellOf, cellOf, arrival, bucketTmp, bucket, sCell, binCounts, offsets, tileSums;
 
         GraphCache graph[2];             // one tick, by parity
@@ -326,7 +329,6 @@ namespace halcuda
             HAL_TRY(avelState.Alloc(m, "cudaMalloc(well agents)"));
             HAL_TRY(CudaStatus(cudaMemset(avelState.p, 0, m * sizeof(float2)), "cudaMemset"));
             HAL_TRY(sRad.Alloc(m, "cudaMalloc(well agents)"));
-            HAL_TRY(posF.Alloc(m, "cudaMalloc(well agents)"));
             HAL_TRY(sPos.Alloc(m, "cudaMalloc(well agents)"));
             HAL_TRY(wellOf.Alloc(m, "cudaMalloc(well agents)"));
             HAL_TRY(cellOf.Alloc(m, "cudaMalloc(well agents)"));
@@ -510,7 +512,6 @@ namespace halcuda
             a.wells = agentWells.p;
             a.n = nAgents;
             a.cells = agentCells;
-            a.posF = posF.p;
             a.sPos = sPos.p;
             a.sRad = sRad.p;
             a.cellOf = cellOf.p;
@@ -530,12 +531,44 @@ namespace halcuda
             a.posOut = reinterpret_cast<float2 *>(apos.p);
             a.friction = friction;
             a.maxVel = maxVel;
+            a.counted = motion;
             return a;
+        }
+
+        // Before ticks with motion: the agents counted into their bins.
+        int EnsureCounted(double R, double k)
+        {
+            if (!motion || counted || nAgents == 0)
+            {
+                return HAL_CUDA_OK;
+            }
+            HAL_TRY(LaunchCountWells(AgentArgs(R, k), stream.Get()));
+            counted = true;
+            return HAL_CUDA_OK;
+        }
+
+        // The agents or their motion change: no counts.
+        int DropCount()
+        {
+            if (!counted)
+            {
+                return HAL_CUDA_OK;
+            }
+            counted = false;
+            return CudaStatus(cudaMemsetAsync(binCounts.p, 0, static_cast<size_t>(agentCells) * sizeof(int32_t),
+                                              stream.Get()), "cudaMemsetAsync(well bins)");
+        }
+
+        // count and tile sums (without motion), scan, scatter, rank, forces
+        int AgentKernels() const
+        {
+            const int scan = AgentScanTiles(agentCells) <= kAgentScanSumTiles ? 1 : 2;
+            return nAgents > 0 ? (motion ? 0 : 2) + scan + 3 : 0;
         }
 
         int KernelsPerTick() const
         {
-            return (nTiles4 > 0) + (nTiles1 > 0) + (nTilesX > 0) + (nTilesY > 0) + (nAgents > 0 ? 7 : 0);
+            return (nTiles4 > 0) + (nTiles1 > 0) + (nTilesX > 0) + (nTilesY > 0) + AgentKernels();
         }
 
         // Mean device ms of one x-sweep plus one y-sweep launch over every
@@ -656,6 +689,7 @@ namespace halcuda
             {
                 return HAL_CUDA_OK;
             }
+            HAL_TRY(DropCount());
             cudaStream_t s = stream.Get();
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             HAL_TRY(CudaStatus(cudaEventCreate(&e0), "cudaEventCreate"));
@@ -667,13 +701,18 @@ namespace halcuda
                 forceThreads = t;
                 AgentWellsArgs a = AgentArgs(R, k);
                 a.velState = nullptr;  // timing runs compute forces only: the agents stay put
-                for (int it = 0; it < 5 && rc == HAL_CUDA_OK; it++)
+                a.counted = false;
+                if (t == 128 && rc == HAL_CUDA_OK)
                 {
-                    if (it == 2)
+                    rc = LaunchBinWells(a, s);
+                }
+                for (int it = 0; it < 4 && rc == HAL_CUDA_OK; it++)
+                {
+                    if (it == 1)
                     {
                         cudaEventRecord(e0, s);
                     }
-                    rc = LaunchAgentWells(a, s);
+                    rc = LaunchForceWells(a, s);
                 }
                 if (rc == HAL_CUDA_OK)
                 {
@@ -697,8 +736,7 @@ namespace halcuda
             {
                 cudaEventDestroy(e1);
             }
-            forceThreads = bestT;
-            ResetGraphs();
+            forceThreads = bestT;  // (part of the graphs' key)
             return rc;
         }
 
@@ -718,6 +756,7 @@ namespace halcuda
             {
                 HAL_TRY(TuneAgents(R, k));
             }
+            HAL_TRY(EnsureCounted(R, k));
             cudaStream_t s = stream.Get();
             char key[160];
             snprintf(key, sizeof(key), "%a|%a|%d|%d|%a|%a|%d|%p", R, k, nAgents, motion ? 1 : 0,
@@ -945,6 +984,7 @@ extern "C" int hal_cuda_wells_set_agents(hal_cuda_wells *h, const int32_t *count
     HAL_REQUIRE(n == 0 || (positions != nullptr && radii != nullptr), "hal_cuda_wells_set_agents: NULL array");
     using namespace halcuda;
     HAL_TRY(CudaStatus(cudaSetDevice(h->device), "cudaSetDevice"));
+    HAL_TRY(h->DropCount());
     cudaStream_t s = h->stream.Get();
     std::vector<int32_t> wellOf(static_cast<size_t>(n));
     int64_t at = 0;
@@ -975,6 +1015,8 @@ extern "C" int hal_cuda_wells_set_motion(hal_cuda_wells *h, int32_t enabled, dou
     HAL_REQUIRE(h != nullptr, "hal_cuda_wells_set_motion: handle is NULL");
     HAL_REQUIRE(std::isfinite(friction), "hal_cuda_wells_set_motion: friction must be finite");
     HAL_REQUIRE(!std::isnan(maxVel), "hal_cuda_wells_set_motion: maxVel is NaN");
+    HAL_TRY(halcuda::CudaStatus(cudaSetDevice(h->device), "cudaSetDevice"));
+    HAL_TRY(h->DropCount());
     h->motion = enabled != 0;
     h->friction = static_cast<float>(friction);
     h->maxVel = (maxVel < 0 || std::isinf(maxVel)) ? -1.0f : static_cast<float>(maxVel);
@@ -1072,6 +1114,7 @@ extern "C" int hal_cuda_wells_profile(hal_cuda_wells *h, int32_t iters, double i
     {
         HAL_TRY(h->TuneAgents(interactionRad, springConstant));
     }
+    HAL_TRY(h->EnsureCounted(interactionRad, springConstant));
     cudaStream_t s = h->stream.Get();
     cudaEvent_t ev[5];
     for (auto &e : ev)
