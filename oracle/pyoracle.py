@@ -40,6 +40,8 @@ def _reference_tree() -> str:
 
 
 REF_TREE = _reference_tree()
+if not os.path.isdir(os.path.join(REF_TREE, "src")):
+    REF_TREE = ""  # no tree there, or an empty mount point: nothing to compile
 
 _dp = ctypes.POINTER(ctypes.c_double)
 _ip = ctypes.POINTER(ctypes.c_int32)
