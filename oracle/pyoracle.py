@@ -41,7 +41,9 @@ def _reference_tree() -> str:
 
 REF_TREE = _reference_tree()
 if not os.path.isdir(os.path.join(REF_TREE, "src")):
-    REF_TREE = ""  # no tree there, or an empty mount point: nothing to compile
+    # no tree there, or an empty mount point: nothing to compile (a path that
+    # does not exist, since callers join names to it)
+    REF_TREE = os.path.join(HERE, "_no_reference_tree")
 
 _dp = ctypes.POINTER(ctypes.c_double)
 _ip = ctypes.POINTER(ctypes.c_int32)
