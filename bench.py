@@ -284,17 +284,21 @@ def secondary_explicit(hal, torch, stream, warm=5, iters=50):
                       ticks=10)
     cpu_s = time.perf_counter() - t0
     peak, _ = peaks()
-    # one kernel per tick: the graph's time per tick is the mean launch
-    # duration over back-to-back launches
-    ach = EXPLICIT_BYTES * CELLS / (ms_tick * 1e-3) / 1e9
+    # several ticks per launch, the field in registers between them: the FP32
+    # pipe bounds a tick (11 operations per cell: 4 differences, 3 additions of
+    # them, the rate, the decay, the source, the commit), not the passes over
+    # memory that one launch per tick made
+    sm_hz = 2.07e9
+    ops, fp32 = 11 * CELLS / (ms_tick * 1e-3) / 1e9, 152 * 128 * sm_hz / 1e9
+    equivalent = EXPLICIT_BYTES * CELLS / (ms_tick * 1e-3) / 1e9
     return {"workload": "explicit-2048x2048-r0.2-decay0.001-64sources-zeroflux",
             "value": CELLS / (ms_tick * 1e-3), "unit": "cell-updates/s",
             "ms_per_tick_graph": ms_tick,
-            "roofline": {"kernel": "TickKernel", "bound": "hbm", "achieved": ach, "peak": peak,
-                         "unit": "GB/s", "frac": ach / peak,
-                         "traffic": profile_traffic("TickKernel"),
-                         "launch_ms_basis": "graph replay of 100 ticks, one launch per tick",
-                         "isolated_launch_ms": ms_launch},
+            "roofline": {"kernel": "TickPatch", "bound": "fp32", "achieved": ops, "peak": fp32,
+                         "unit": "Gop/s", "frac": ops / fp32,
+                         "one_pass_per_tick_gbs": equivalent, "measured_copy_gbs": peak,
+                         "launch_ms_basis": "graph replay of 100 ticks, four ticks per launch",
+                         "single_tick_launch_ms": ms_launch},
             "accuracy": accuracy(got, ref, "FP64 oracle, 10 ticks from the same float32 field"),
             "cpu_baseline": {"value": 10 * CELLS / cpu_s, "unit": "cell-updates/s", "cores": 1, "kind": "port",
                              "sample": "10 FP64 ticks of the same 2048x2048 workload (oracle, 1 thread)"},
@@ -652,14 +656,17 @@ def secondary_pdegrid_adi(hal, torch, stream, warm=2, iters=10):
     pyoracle.Oracle.diffuse_adi(f0, np.zeros(CELLS), 5.0, N, N, False, False)
     cpu_ms = (time.perf_counter() - t0) * 1e3
     sm_hz = 2.07e9
-    chain_floor_ms = 2 * N * 7 * 64 / sm_hz * 1e3
+    # per cell and sweep: 4.25 FP64 operations of the right-hand side and 10 of
+    # the segments' elimination, back substitution and correction; a warp's FP64
+    # instruction holds its scheduler's pipe for 64 cycles (4 x 152 of them)
+    fp64_floor_ms = 2 * CELLS * 14.25 / 32 * 64 / (4 * 152 * sm_hz) * 1e3
     return {"workload": "pdegrid-fp64-adi-2048x2048-r5-zeroflux (DiffusionADI + MulAll + Update)",
             "ms_per_tick": ms, "value": CELLS / (ms * 1e-3), "unit": "cell-updates/s",
             "cpu_oracle_adi_ms": cpu_ms, "cpu_cores": 1,
             "speedup_vs_cpu_adi_step": cpu_ms / ms,
-            "chain_bound": {"bound": "fp64 issue of one warp (64 cycles per instruction)",
-                            "fp64_instructions_per_element": 7, "floor_ms_per_tick_at_2070_mhz": chain_floor_ms,
-                            "frac_of_tick": chain_floor_ms / ms},
+            "fp64_bound": {"bound": "fp64 issue (64 cycles per warp instruction and scheduler)",
+                           "fp64_instructions_per_cell_and_sweep": 14.25,
+                           "floor_ms_per_tick_at_2070_mhz": fp64_floor_ms, "frac_of_tick": fp64_floor_ms / ms},
             "note": "FP64, bit-identical to the reference's PDEGrid2D; the CPU figure is the oracle's "
                     "DiffusionADI step alone (1 thread)"}
 
