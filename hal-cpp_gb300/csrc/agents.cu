@@ -8,7 +8,7 @@
 //   scan         reduce-then-scan over the cells (at most three launches, no spin
 //                waits; in a resident run the move before adds up the tiles: 20k
 //                agents in 256^2 17.9 -> 16.5 us per tick, 200k in 1024^2 36.4 ->
-//                33.9, 400k in 2048^2 52.9 -> 49.5, 1M 90 either way)
+//                33.9, 400k in 2048^2 52.9 -> 49.5)
 //   Scatter      agent -> offsets[cell] + arrival rank (order within a cell is
 //                the atomic arrival order, not yet the CPU's)
 //   Stabilize    one thread per arrival-order slot: its agent counts the
@@ -1117,6 +1117,9 @@ namespace halcuda
                 return;
             }
             const int32_t i = bucket[slot];
+            // in flight during the sums (200k agents 34 -> 25 us per step, 400k 50 ->
+            // 45, 1M 91 -> 89)
+            float2 v = velocity[i];
             const ForceAcc<float> acc = ForceSlotLaw<float, LAW, SUM, false>(
                 slot, offsets, sPos, sRad, interactionRad, R, lp, xDim, yDim, WALLS ? 0 : mp.wrapX,
                 WALLS ? 0 : mp.wrapY, make_float2(0.f, 0.f));
@@ -1127,7 +1130,6 @@ namespace halcuda
                 sums[i] = acc.sum;
             }
             float2 p = sPos[slot];
-            float2 v = velocity[i];
             v.x = __fadd_rn(v.x, d.x);
             v.y = __fadd_rn(v.y, d.y);
             MoveAgent(mp, p, v);
@@ -1154,9 +1156,12 @@ namespace halcuda
         // so the sum is ForceSlotLaw's, bit for bit.  It issues more
         // instructions per pair than one thread per agent does, so the latter
         // stays beyond kGroupAgents agents.  Measured, us per resident step
-        // (benchmark distribution, thread / group per agent): 20k agents in
-        // 256^2 24.1 / 17.6, 50k in 512^2 133 / 62, 100k in 1024^2 36.6 / 36.0,
-        // 200k in 1024^2 36.5 / 52.4, 1M in 2048^2 90 / 214.  Leaving only the
+        // (30% in a cluster, thread / group per agent, over several clusters): 20k
+        // agents in 256^2 27 to 45 / 19 to 35, 50k in 512^2 19 to 126 / 23 to 66, 80k
+        // 44 to 199 / 31 to 117, 100k in 512^2 137 / 103 and in 1024^2 27 / 34, 200k
+        // in 512^2 35 / 57 and in 1024^2 25 / 52, 1M in 2048^2 89 / 214: up to 100k
+        // the group loses a little where the windows are short and wins much where
+        // the cluster is dense, beyond that it loses more.  Leaving only the
         // agents of long windows to groups, in a second launch, cost 3 us per
         // 1M-agent step and lost up to 2x where many agents had long windows.
         constexpr int kGroupLanes = 8;
@@ -1863,6 +1868,7 @@ namespace halcuda
                 return;
             }
             const int32_t i = bucket[slot];
+            float2 v = velocity[i];  // in flight during the sums (48 wells: 98 ticks 11.2 -> 9.7 ms)
             const AgentWellDev wd = wells[wellOf[slot]];  // the slots go well by well, as the agents do
             const V2<float> d = ForceSlotWell(slot, offsets, sPos, sRad, sCell, interactionRad, intR, R, k, wd);
             StoreDelta(vel, i, d);
@@ -1874,7 +1880,6 @@ namespace halcuda
             mp.wrapX = wd.wrapX;
             mp.wrapY = wd.wrapY;
             float2 p = sPos[slot];
-            float2 v = velocity[i];
             v.x = __fadd_rn(v.x, d.x);
             v.y = __fadd_rn(v.y, d.y);
             MoveAgent(mp, p, v);
