@@ -26,8 +26,8 @@
 //      memory through the same swizzle; otherwise a warp copies whole lines by
 //      16-byte asynchronous copies, each 32-element chunk into a 36-float
 //      slot.  (A bulk copy per chunk took longer: 128 bytes each, thousands a
-//      CTA; us per tick bulk / here: 2047 x 2049 40.8 / 37.0, 3179 x 2193
-//      80.4 / 71.6, 4000^2 192 / 141, 2040^2 29.0 / 26.4 against 20.7 for
+//      CTA; us per tick bulk / here: 2047 x 2049 40.8 / 33.0, 3179 x 2193
+//      80.4 / 67.2, 4000^2 192 / 141, 2040^2 29.0 / 26.4 against 20.7 for
 //      2048^2 through the tensor copy.)  Either way every later access is a
 //      conflict-free 128-bit LDS/STS;
 //   2. each thread solves one 32-row chunk of two lines (two interleaved
@@ -394,6 +394,39 @@ namespace halcuda
             }
         }
 
+        // A warp stages a line of L floats (null: zeros) into P padded chunks from
+        // row on.  vec: the line is 16-byte aligned and padded with zeros to whole
+        // units, copied by 16-byte asynchronous copies; lane's units are 32
+        // apart, so their addresses only step (with few warps on an SM the
+        // address arithmetic of a copy at a time had cost more than the copies).
+        __device__ __forceinline__ void StageLine(float *row, const float *__restrict__ src, int32_t L, int P, bool vec,
+                                                  int lane)
+        {
+            constexpr int kStep = 4 * kChunkStride;  // 32 units: four chunks
+            const int units = P * (M / 4);
+            float *dst = row + (lane >> 3) * kChunkStride + 4 * (lane & 7);
+            int u = lane;
+            if (src != nullptr && vec)
+            {
+                const int full = (L + 3) >> 2;
+                const float *from = src + 4 * lane;
+#pragma unroll 4
+                for (; u < full; u += 32, dst += kStep, from += 128)
+                {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(SmemAddr(dst)), "l"(from)
+                                 : "memory");
+                }
+            }
+            for (; u < units; u += 32, dst += kStep)
+            {
+                const int32_t pos = 4 * u;
+                const bool in = src != nullptr && pos < L;
+                St4(dst, make_float4(in ? src[pos] : 0.0f, in && pos + 1 < L ? src[pos + 1] : 0.0f,
+                                     in && pos + 2 < L ? src[pos + 2] : 0.0f,
+                                     in && pos + 3 < L ? src[pos + 3] : 0.0f));
+            }
+        }
+
         // The plan's coefficients and band (gCount entries; 0: not staged) into
         // shared memory.  They do not come from the kernel before.
         __device__ __forceinline__ void LoadPlan(const SweepParams &p, float *sCoef, float *sG, int gCount, int tid,
@@ -547,30 +580,7 @@ namespace halcuda
                         }
                     }
                     vec = vec && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-                    for (int u = lane; u < P * (M / 4); u += 32)
-                    {
-                        float *dst = sLines + SOff4<SWZ>(rr, u >> 3, u & 7, P, p.LS);
-                        const int32_t pos = 4 * u;
-                        if (src != nullptr && pos < L)
-                        {
-                            if (vec)
-                            {
-                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(SmemAddr(dst)),
-                                             "l"(src + pos)
-                                             : "memory");
-                            }
-                            else
-                            {
-                                St4(dst, make_float4(src[pos], pos + 1 < L ? src[pos + 1] : 0.0f,
-                                                     pos + 2 < L ? src[pos + 2] : 0.0f,
-                                                     pos + 3 < L ? src[pos + 3] : 0.0f));
-                            }
-                        }
-                        else
-                        {
-                            St4(dst, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-                        }
-                    }
+                    StageLine(sLines + SOff4<SWZ>(rr, 0, 0, P, p.LS), src, L, P, vec, lane);
                 }
                 asm volatile("cp.async.wait_all;" ::: "memory");
             }
@@ -1404,25 +1414,7 @@ namespace halcuda
                         vec = false;  // a ghost table's row: any alignment, no padding
                     }
                 }
-                for (int f = lane; f < P * (M / 4); f += 32)
-                {
-                    float *dst = rows + r * lineStride + (f >> 3) * kChunkStride + 4 * (f & 7);
-                    const int32_t pos = 4 * f;
-                    if (src != nullptr && vec && pos < L)
-                    {
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(SmemAddr(dst)), "l"(src + pos)
-                                     : "memory");
-                    }
-                    else if (src != nullptr && pos < L)
-                    {
-                        St4(dst, make_float4(src[pos], pos + 1 < L ? src[pos + 1] : 0.0f,
-                                             pos + 2 < L ? src[pos + 2] : 0.0f, pos + 3 < L ? src[pos + 3] : 0.0f));
-                    }
-                    else
-                    {
-                        St4(dst, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-                    }
-                }
+                StageLine(rows + r * lineStride, src, L, P, vec, lane);
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
@@ -1707,10 +1699,25 @@ namespace halcuda
             return CudaStatus(cudaLaunchKernelEx(&cfg, kernel, args...), what);
         }
 
-        // Lines up to kLineMaxP chunks go to AdiLines.
-        bool UseLines(const SweepParams &p)
+        // Lines up to kLineMaxP chunks go to AdiLines, as long as there are not
+        // many: from a wave of 1216 lines on (152 CTAs of eight) the tensor-staged
+        // sweep is the faster (us per tick, AdiLines / AdiSweep: 2048 x 1024 19.5 /
+        // 14.7, 4096 x 512 23.0 / 17.5, 1024 x 2000 25.7 / 19.9), and so is the
+        // chunked one for lines of more than 512 positions, which stand one to a
+        // warp, in CTAs that hold an SM each: always in the y-sweep (2000 x 900 25.4
+        // / 20.0), in the x-sweep where the last wave is less than half full (700 x
+        // 1250 23.2 / 16.4, 800 x 1300 18.1 / 16.3, 1000 x 4000 30.5 / 27.2; fuller:
+        // 900 x 2000 31.0 / 33.0; shorter lines: 300 x 4000 22.7 / 24.0).
+        template <int MODE>
+        bool UseLines(const SweepParams &p, bool swz)
         {
-            return p.plan.P <= kLineMaxP;
+            const int32_t wave = 2 * kLineFewLines;  // 152 CTAs of eight lines
+            if (p.plan.P > kLineMaxP || (swz && p.Nlines >= wave))
+            {
+                return false;
+            }
+            return p.plan.P <= 16 || p.Nlines < wave ||
+                   (MODE != kSweepTick && p.Nlines % wave >= wave / 2);
         }
 
         template <int MODE, bool UPT, int W>
@@ -2215,7 +2222,7 @@ namespace halcuda
             const bool swz = (tmap != nullptr);
             p.inStride = (p.L + 3) & ~3;
             p.outStride = (p.Nlines + 3) & ~3;
-            if (UseLines(p))
+            if (UseLines<MODE>(p, swz))
             {
                 return LaunchLines<MODE>(p, s);
             }
@@ -2235,8 +2242,23 @@ namespace halcuda
                     CUtensorMap none;
                     std::memset(&none, 0, sizeof(none));
                     HAL_TRY((EnableSweepSmem<MODE, false, UPT>(sh.smem)));
-                    HAL_TRY(LaunchChainedSmem(AdiSweep<MODE, false, UPT>, blocks, static_cast<unsigned>(sh.threads),
-                                              sh.smem, s, "AdiSweep launch", p, none));
+                    // Not chained where two CTAs fit an SM: started early they pair up
+                    // on the SMs that a sweep of few, large CTAs leaves idle (us per
+                    // tick chained / not: 900 x 2000 29.1 / 20.3, 1200 x 2000 28.8 /
+                    // 20.3, 600 x 2000 24.8 / 18.1; lost: 600 x 1820 16.7 / 17.5).  One
+                    // cannot, and smaller ones share the SMs with their predecessor's
+                    // (1100^2 14.7 / 16.2).
+                    constexpr int kHalfSm = 65536 / 128 / 2;  // threads of 128 registers
+                    if (sh.threads > kHalfSm / 3 * 2 && sh.threads <= kHalfSm)
+                    {
+                        AdiSweep<MODE, false, UPT><<<blocks, sh.threads, sh.smem, s>>>(p, none);
+                    }
+                    else
+                    {
+                        HAL_TRY(LaunchChainedSmem(AdiSweep<MODE, false, UPT>, blocks,
+                                                  static_cast<unsigned>(sh.threads), sh.smem, s, "AdiSweep launch", p,
+                                                  none));
+                    }
                 }
                 return HAL_CUDA_OK;
             };

@@ -19,7 +19,11 @@ pytestmark = pytest.mark.gpu
     [(1025, 40, False, False), (40, 1025, True, True), (1030, 1029, False, True), (1024, 1024, False, False)],
     # enough wells for several lines per warp
     [(63 + i, 130 - i, i % 2 == 0, i % 3 == 0) for i in range(60)],
-], ids=["one", "chunks", "long", "many"])
+    # around the numbers of lines at which a single grid leaves the warp per line
+    # (a wave of 1216) and comes back to it (half of the next)
+    [(520, 1215, False, True), (520, 1216, True, False), (1024, 1220, False, False), (1217, 993, True, True),
+     (544, 1823, False, False), (1824, 600, False, True), (512, 1300, False, False)],
+], ids=["one", "chunks", "long", "many", "many-lines"])
 def test_line_wells_equal_single_grids(hal, wells):
     rng = np.random.default_rng(len(wells))
     desc = [dict(xDim=x, yDim=y, kind="adi", diffRate=0.5 + i % 7, decay=0.01 * (i % 2), wrapX=wx, wrapY=wy,
