@@ -1389,6 +1389,7 @@ namespace halcuda
 
         constexpr int32_t kSegMaxWarps = 1216;  // 152 SMs x 4 FP64 pipes x 2
         constexpr int32_t kSegMinLen = 64;
+        constexpr int32_t kSegMinLine = 232;
 
         // Segments of a line's split solve, for `lines` lines.  As many as
         // give every FP64 pipe two warps, which cover each other's loads (the
@@ -1398,7 +1399,10 @@ namespace halcuda
         // more on their launches and meetings than the chain saves), and each
         // long enough that a trajectory's error falls below 2^-64 of itself
         // over it: otherwise, for large rates, segments would end before they
-        // meet the serial one.  One segment: the serial chain.
+        // meet the serial one.  One segment: the serial chain, also for lines
+        // below kSegMinLine, whose chain costs less than the segments' launches
+        // (four ticks, chain / segments: 200^2 574 / 696 us, 240^2 673 / 634, 320^2
+        // 868 / 639).
         void AddSegments(LinePlan64Host &p, int32_t lines)
         {
             const int32_t L = static_cast<int32_t>(p.bs.size());
@@ -1414,7 +1418,8 @@ namespace halcuda
             {
                 p.g[static_cast<size_t>(i)] = -p.off * p.bh[static_cast<size_t>(i)].y;
             }
-            for (int32_t segs = std::min(kSegMaxWarps / warps, L / kSegMinLen); segs >= 2; segs--)
+            const int32_t most = L < kSegMinLine ? 1 : std::min(kSegMaxWarps / warps, L / kSegMinLen);
+            for (int32_t segs = most; segs >= 2; segs--)
             {
                 const int32_t len = (L + segs - 1) / segs;
                 const int32_t n = (L + len - 1) / len;
