@@ -1,0 +1,80 @@
+// agent_window.h -- the cells of an agent's force window as runs of cells.
+//
+// The CPU backend visits the window's cells x-major then y, each index taken
+// modulo its side where that axis wraps (CpuAgentForceBackend2D.cpp:112-175).
+// Cells of one row are consecutive, and so are their agents' slots, so a row is
+// one run of cells, or two where its y-range passes the edge.  Host and device
+// code, so that the index arithmetic can be checked without a GPU.
+#pragma once
+
+#include <cstdint>
+
+#if defined(__CUDACC__)
+#define HAL_WINDOW_FN __host__ __device__ __forceinline__
+#else
+#define HAL_WINDOW_FN inline
+#endif
+
+namespace halcuda
+{
+    // i modulo dim, in [0, dim).
+    HAL_WINDOW_FN int32_t WrapIndex(int32_t i, int32_t dim)
+    {
+        if (i < 0 || i >= dim)
+        {
+            i %= dim;
+            i += (i < 0) ? dim : 0;
+        }
+        return i;
+    }
+
+    // The rows xStart .. xEnd - 1 of a window, each with the cells yStart ..
+    // yEnd - 1, as `runs` runs: run j is cells [cell, cell + count).
+    struct WindowRuns
+    {
+        int32_t runs;    // 0: no cells
+        int32_t perRow;  // 1, or 2 where the y-range passes the edge
+        int32_t y0, y1;  // the y-range reduced into the grid: y0 in [0, yDim), y1 - y0 cells
+        bool fits;       // the window is at most maxRuns runs
+
+        // On an axis that does not wrap the range lies within the grid.  An
+        // agent may lie anywhere (the binning clamps it), so that a window may
+        // lie wholly outside, by any number of sides: it is reduced first, and
+        // only then cut at the edge.
+        HAL_WINDOW_FN void Set(int32_t xStart, int32_t xEnd, int32_t yStart, int32_t yEnd, int32_t yDim, int32_t maxRuns)
+        {
+            const int64_t rows = static_cast<int64_t>(xEnd) - xStart;
+            const int64_t cells = static_cast<int64_t>(yEnd) - yStart;
+            runs = 0;
+            perRow = 1;
+            y0 = y1 = 0;
+            fits = true;
+            if (rows <= 0 || cells <= 0)
+            {
+                return;
+            }
+            if (cells > yDim || rows > maxRuns)
+            {
+                fits = false;
+                return;
+            }
+            y0 = WrapIndex(yStart, yDim);
+            y1 = y0 + static_cast<int32_t>(cells);
+            perRow = (y1 > yDim) ? 2 : 1;
+            runs = static_cast<int32_t>(rows) * perRow;
+            fits = runs <= maxRuns;
+        }
+
+        // Run j (0 <= j < runs), in the visiting order.
+        HAL_WINDOW_FN void Run(int32_t j, int32_t xStart, int32_t xDim, int32_t yDim, int32_t &cell,
+                               int32_t &count) const
+        {
+            const bool second = perRow == 2 && (j & 1) != 0;
+            const int32_t row = WrapIndex(xStart + (perRow == 2 ? j >> 1 : j), xDim);
+            const int32_t from = second ? 0 : y0;
+            const int32_t to = second ? y1 - yDim : (perRow == 2 ? yDim : y1);
+            cell = row * yDim + from;
+            count = to - from;
+        }
+    };
+}

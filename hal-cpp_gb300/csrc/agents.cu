@@ -26,6 +26,7 @@
 // contraction) on the FP64 interface path, where positions stay FP64 end to
 // end and the result matches the CPU backend bit for bit.
 #include "common.cuh"
+#include "agent_window.h"
 #include "agents_wells.h"
 
 #include <cmath>
@@ -1214,31 +1215,16 @@ namespace halcuda
                 yStart = max(yStart, 0);
                 yEnd = min(yEnd, yDim);
             }
-            // the window as runs of cells, in the visiting order: one per row,
-            // or two where a wrapped y-range crosses the edge
-            const int32_t nRows = max(xEnd - xStart, 0);
-            const bool below = yStart < 0, above = yEnd > yDim;
-            const int32_t perRow = (below || above) ? 2 : 1;
-            const bool empty = nRows == 0 || yEnd <= yStart;
-            const bool fits = empty || (nRows <= G / perRow && yEnd - yStart <= yDim && !(below && above));
+            // the window as runs of cells, in the visiting order, a lane's each
+            WindowRuns win;
+            win.Set(xStart, xEnd, yStart, yEnd, yDim, G);
             int32_t s0 = 0, len = 0;
-            if (live && fits && !empty && j < nRows * perRow)
+            if (live && win.fits && j < win.runs)
             {
-                int32_t row = xStart + ((perRow == 2) ? (j >> 1) : j);
-                if (row < 0 || row >= xDim)
-                {
-                    row %= xDim;  // only reached on a wrapped axis (clamped otherwise)
-                    row = (row < 0) ? row + xDim : row;
-                }
-                int32_t y0 = yStart, y1 = yEnd;
-                if (perRow == 2)
-                {
-                    const bool first = (j & 1) == 0;
-                    y0 = first ? (below ? yStart + yDim : yStart) : 0;
-                    y1 = first ? yDim : (below ? yEnd : yEnd - yDim);
-                }
-                s0 = __ldg(offsets + row * yDim + y0);
-                len = __ldg(offsets + row * yDim + y1) - s0;
+                int32_t cell, count;
+                win.Run(j, xStart, xDim, yDim, cell, count);
+                s0 = __ldg(offsets + cell);
+                len = __ldg(offsets + cell + count) - s0;
             }
             // candidate k is slot k + shift[r] of the first run r with k < end[r]
             int32_t end[G], shift[G];
@@ -1300,7 +1286,7 @@ namespace halcuda
                 pj = pn;
                 rj = rn;
             }
-            if (!fits && live)
+            if (!win.fits && live)
             {
                 // a window of more runs than lanes: one lane's walk for all
                 const ForceAcc<float> acc = ForceSlotLaw<float, kLawLinear, false, false>(
