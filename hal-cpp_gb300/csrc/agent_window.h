@@ -34,35 +34,38 @@ namespace halcuda
     {
         int32_t runs;    // 0: no cells
         int32_t perRow;  // 1, or 2 where the y-range passes the edge
-        int32_t y0, y1;  // the y-range reduced into the grid: y0 in [0, yDim), y1 - y0 cells
-        bool fits;       // the window is at most maxRuns runs
+        int32_t y0;      // the y-range reduced into the grid: `first` cells from y0 on,
+        int32_t first;   // and `over` cells from 0 on
+        int32_t over;
+        bool fits;       // the y-range is no longer than the side, so the runs are the whole window
 
         // On an axis that does not wrap the range lies within the grid.  An
         // agent may lie anywhere (the binning clamps it), so that a window may
         // lie wholly outside, by any number of sides: it is reduced first, and
         // only then cut at the edge.
-        HAL_WINDOW_FN void Set(int32_t xStart, int32_t xEnd, int32_t yStart, int32_t yEnd, int32_t yDim, int32_t maxRuns)
+        HAL_WINDOW_FN void Set(int32_t xStart, int32_t xEnd, int32_t yStart, int32_t yEnd, int32_t yDim)
         {
             const int64_t rows = static_cast<int64_t>(xEnd) - xStart;
             const int64_t cells = static_cast<int64_t>(yEnd) - yStart;
             runs = 0;
             perRow = 1;
-            y0 = y1 = 0;
+            y0 = first = over = 0;
             fits = true;
             if (rows <= 0 || cells <= 0)
             {
                 return;
             }
-            if (cells > yDim || rows > maxRuns)
+            if (cells > yDim || rows > (int64_t(1) << 29))
             {
                 fits = false;
                 return;
             }
             y0 = WrapIndex(yStart, yDim);
-            y1 = y0 + static_cast<int32_t>(cells);
-            perRow = (y1 > yDim) ? 2 : 1;
+            first = yDim - y0;
+            first = (cells < first) ? static_cast<int32_t>(cells) : first;
+            over = static_cast<int32_t>(cells) - first;
+            perRow = (over > 0) ? 2 : 1;
             runs = static_cast<int32_t>(rows) * perRow;
-            fits = runs <= maxRuns;
         }
 
         // Run j (0 <= j < runs), in the visiting order.
@@ -71,10 +74,8 @@ namespace halcuda
         {
             const bool second = perRow == 2 && (j & 1) != 0;
             const int32_t row = WrapIndex(xStart + (perRow == 2 ? j >> 1 : j), xDim);
-            const int32_t from = second ? 0 : y0;
-            const int32_t to = second ? y1 - yDim : (perRow == 2 ? yDim : y1);
-            cell = row * yDim + from;
-            count = to - from;
+            cell = row * yDim + (second ? 0 : y0);
+            count = second ? over : first;
         }
     };
 }

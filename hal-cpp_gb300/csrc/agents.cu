@@ -1154,7 +1154,12 @@ namespace halcuda
         // each lane finds one run of the window's cells, the lanes evaluate
         // that many candidates at a time, and the terms are then added in the
         // candidates' order by every lane (a candidate out of range adds -0),
-        // so the sum is ForceSlotLaw's, bit for bit.  It issues more
+        // so the sum is ForceSlotLaw's, bit for bit.  A window of more runs
+        // takes several rounds (a radius of 4 has nine rows, a radius of 2 at a
+        // wrapped edge five of two runs; us per step with such windows left to
+        // one lane's walk / in rounds: 20k agents in 256^2, radius 4, 161 / 48
+        // with a cluster, 37 / 19 uniform; 90k in 512^2, wrapped, 110 / 43).  It
+        // issues more
         // instructions per pair than one thread per agent does, so the latter
         // stays beyond kGroupAgents agents.  Measured, us per resident step
         // (30% in a cluster, thread / group per agent, over several clusters): 20k
@@ -1215,80 +1220,85 @@ namespace halcuda
                 yStart = max(yStart, 0);
                 yEnd = min(yEnd, yDim);
             }
-            // the window as runs of cells, in the visiting order, a lane's each
+            // the window as runs of cells, in the visiting order, eight a round, a
+            // lane's each
             WindowRuns win;
-            win.Set(xStart, xEnd, yStart, yEnd, yDim, G);
-            int32_t s0 = 0, len = 0;
-            if (live && win.fits && j < win.runs)
-            {
-                int32_t cell, count;
-                win.Run(j, xStart, xDim, yDim, cell, count);
-                s0 = __ldg(offsets + cell);
-                len = __ldg(offsets + cell + count) - s0;
-            }
-            // candidate k is slot k + shift[r] of the first run r with k < end[r]
-            int32_t end[G], shift[G];
-            int32_t total = 0;
-#pragma unroll
-            for (int r = 0; r < G; r++)
-            {
-                shift[r] = __shfl_sync(0xffffffffu, s0, r, G) - total;
-                total += __shfl_sync(0xffffffffu, len, r, G);
-                end[r] = total;
-            }
+            win.Set(xStart, xEnd, yStart, yEnd, yDim);
+            const int32_t runs = (live && win.fits) ? win.runs : 0;
             const float xDimF = static_cast<float>(xDim), yDimF = static_cast<float>(yDim);
             float vx = 0.0f, vy = 0.0f;
-            const int32_t most = __reduce_max_sync(0xffffffffu, total);
-            auto candidate = [&](int32_t k, int32_t &q, float2 &pj, float &rj)
+            for (int32_t r0 = 0; __any_sync(0xffffffffu, r0 < runs); r0 += G)
             {
-                q = -1;
-                if (k < total)
+                int32_t s0 = 0, len = 0;
+                if (r0 + j < runs)
                 {
-                    int32_t sh = shift[G - 1];
-#pragma unroll
-                    for (int r = G - 2; r >= 0; r--)
-                    {
-                        sh = (k < end[r]) ? shift[r] : sh;
-                    }
-                    q = k + sh;
-                    pj = sPos[q];
-                    rj = sRad[q];
+                    int32_t cell, count;
+                    win.Run(r0 + j, xStart, xDim, yDim, cell, count);
+                    s0 = __ldg(offsets + cell);
+                    len = __ldg(offsets + cell + count) - s0;
                 }
-            };
-            int32_t q;
-            float2 pj = make_float2(0.0f, 0.0f);
-            float rj = 0.0f;
-            candidate(j, q, pj, rj);
-            for (int32_t k0 = 0; k0 < most; k0 += G)
-            {
-                // the next round's loads, in flight during this one's sums
-                int32_t qn;
-                float2 pn = make_float2(0.0f, 0.0f);
-                float rn = 0.0f;
-                candidate(k0 + G + j, qn, pn, rn);
-                float x, y, scale;
-                const bool near = PairTerm32(
-                           q >= 0 && q != slot, Disp(pf.x, pj.x, xDimF, wrapX != 0), Disp(pf.y, pj.y, yDimF, wrapY != 0),
-                           __fadd_rn(rad, rj), R, lp.scale, x, y, scale);
-                // the terms, in the candidates' order, on every lane (walking
-                // only the ones in range took more instructions than it saved)
-                if (__any_sync(0xffffffffu, near))
+                // candidate k is slot k + shift[r] of the first run r with k < end[r]
+                int32_t end[G], shift[G];
+                int32_t total = 0;
+#pragma unroll
+                for (int r = 0; r < G; r++)
                 {
-#pragma unroll
-                    for (int t = 0; t < G; t++)
-                    {
-                        const float sc = __shfl_sync(0xffffffffu, scale, t, G);
-                        vx = fmaf(-__shfl_sync(0xffffffffu, x, t, G), sc, vx);
-                        vy = fmaf(-__shfl_sync(0xffffffffu, y, t, G), sc, vy);
-                    }
+                    shift[r] = __shfl_sync(0xffffffffu, s0, r, G) - total;
+                    total += __shfl_sync(0xffffffffu, len, r, G);
+                    end[r] = total;
                 }
-                q = qn;
-                pj = pn;
-                rj = rn;
+                const int32_t most = __reduce_max_sync(0xffffffffu, total);
+                auto candidate = [&](int32_t k, int32_t &q, float2 &pj, float &rj)
+                {
+                    q = -1;
+                    if (k < total)
+                    {
+                        int32_t sh = shift[G - 1];
+#pragma unroll
+                        for (int r = G - 2; r >= 0; r--)
+                        {
+                            sh = (k < end[r]) ? shift[r] : sh;
+                        }
+                        q = k + sh;
+                        pj = sPos[q];
+                        rj = sRad[q];
+                    }
+                };
+                int32_t q;
+                float2 pj = make_float2(0.0f, 0.0f);
+                float rj = 0.0f;
+                candidate(j, q, pj, rj);
+                for (int32_t k0 = 0; k0 < most; k0 += G)
+                {
+                    // the next round's loads, in flight during this one's sums
+                    int32_t qn;
+                    float2 pn = make_float2(0.0f, 0.0f);
+                    float rn = 0.0f;
+                    candidate(k0 + G + j, qn, pn, rn);
+                    float x, y, scale;
+                    const bool near = PairTerm32(
+                               q >= 0 && q != slot, Disp(pf.x, pj.x, xDimF, wrapX != 0),
+                               Disp(pf.y, pj.y, yDimF, wrapY != 0), __fadd_rn(rad, rj), R, lp.scale, x, y, scale);
+                    // the terms, in the candidates' order, on every lane (walking
+                    // only the ones in range took more instructions than it saved)
+                    if (__any_sync(0xffffffffu, near))
+                    {
+#pragma unroll
+                        for (int t = 0; t < G; t++)
+                        {
+                            const float sc = __shfl_sync(0xffffffffu, scale, t, G);
+                            vx = fmaf(-__shfl_sync(0xffffffffu, x, t, G), sc, vx);
+                            vy = fmaf(-__shfl_sync(0xffffffffu, y, t, G), sc, vy);
+                        }
+                    }
+                    q = qn;
+                    pj = pn;
+                    rj = rn;
+                }
             }
             if (!win.fits && live)
             {
-                // a window of more runs than lanes: one lane's walk for all
+                // a y-range longer than the side: one lane's walk for all
                 const ForceAcc<float> acc = ForceSlotLaw<float, kLawLinear, false, false>(
                     slot, offsets, sPos, sRad, interactionRad, R, lp, xDim, yDim, wrapX, wrapY,
                     make_float2(0.0f, 0.0f));

@@ -22,7 +22,6 @@ namespace
 int main()
 {
     using namespace halcuda;
-    constexpr int32_t kLanes = 8;
     const int32_t sides[] = {1, 2, 3, 5, 7, 8, 24, 64};
     const double radii[] = {1e-3, 0.75, 1.0, 1.5, 2.0, 3.5, 6.0};
     long windows = 0, runsSeen = 0;
@@ -73,13 +72,12 @@ int main()
                                 }
                             }
                             WindowRuns w;
-                            w.Set(x0, x1, y0, y1, yDim, kLanes);
+                            w.Set(x0, x1, y0, y1, yDim);
                             windows++;
                             if (!w.fits)
                             {
                                 // only what does not fit may be refused
-                                const int64_t rows = static_cast<int64_t>(x1) - x0, cells = static_cast<int64_t>(y1) - y0;
-                                if (2 * rows <= kLanes && cells <= yDim)
+                                if (static_cast<int64_t>(y1) - y0 <= yDim)
                                 {
                                     std::printf("refused: %d x %d, R %g, (%g, %g)\n", xDim, yDim, R, x, y);
                                     return 1;

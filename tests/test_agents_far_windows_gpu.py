@@ -1,7 +1,9 @@
 """Agents outside the grid by more than the interaction radius, up to several
 sides (uploads check no position; the binning clamps them, the windows wrap):
 a group of lanes per agent (few agents) against one thread per agent (many),
-forces and a step, bit for bit.  The many are a strip of agents beyond every
+forces and a step, bit for bit; also windows of more runs than a group has
+lanes (radii from 4 on, and 2 at a wrapped edge) and y-ranges longer than the
+side (9 cells, radius 6).  The many are a strip of agents beyond every
 window (tests/test_agents_group_gpu.py)."""
 import numpy as np
 import pytest
@@ -32,7 +34,7 @@ def _agents(dim, width, radius, rng):
 
 
 @pytest.mark.parametrize("wrap", [(False, False), (True, True), (True, False), (False, True)])
-@pytest.mark.parametrize("radius", [0.75, 1.0, 2.0])
+@pytest.mark.parametrize("radius", [0.75, 1.0, 2.0, 4.5, 6.0])
 @pytest.mark.parametrize("dim", [9, 64])
 def test_far_agents(hal, dim, radius, wrap):
     rng = np.random.default_rng(dim + int(8 * radius))
