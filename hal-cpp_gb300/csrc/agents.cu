@@ -1159,19 +1159,11 @@ namespace halcuda
         // wrapped edge five of two runs; us per step with such windows left to
         // one lane's walk / in rounds: 20k agents in 256^2, radius 4, 161 / 48
         // with a cluster, 37 / 19 uniform; 90k in 512^2, wrapped, 110 / 43).  It
-        // issues more
-        // instructions per pair than one thread per agent does, so the latter
-        // stays beyond kGroupAgents agents.  Measured, us per resident step
-        // (30% in a cluster, thread / group per agent, over several clusters): 20k
-        // agents in 256^2 27 to 45 / 19 to 35, 50k in 512^2 19 to 126 / 23 to 66, 80k
-        // 44 to 199 / 31 to 117, 100k in 512^2 137 / 103 and in 1024^2 27 / 34, 200k
-        // in 512^2 35 / 57 and in 1024^2 25 / 52, 1M in 2048^2 89 / 214: up to 100k
-        // the group loses a little where the windows are short and wins much where
-        // the cluster is dense, beyond that it loses more.  Leaving only the
-        // agents of long windows to groups, in a second launch, cost 3 us per
-        // 1M-agent step and lost up to 2x where many agents had long windows.
+        // issues more instructions per pair than one thread per agent does:
+        // GroupPerAgent says where it pays.  Leaving only the agents of long
+        // windows to groups, in a second launch, cost 3 us per 1M-agent step and
+        // lost up to 2x where many agents had long windows.
         constexpr int kGroupLanes = 8;
-        constexpr int32_t kGroupAgents = 100000;
 
         // floor(v - r) and ceil(v + r) as the CPU takes them, in FP64.  For an
         // integer r the FP32 floor and ceiling give the same (v is exact, and
@@ -1896,6 +1888,40 @@ namespace halcuda
         return r >= 0.0 && r <= 0x1p20 && r == std::floor(r);
     }
 
+    // Whether a force pass (step: with the move) takes a group of lanes per
+    // agent.  A thread per agent costs the longest window's chain, a group its
+    // instructions, n times: the group pays while the windows are long for the
+    // number of agents.  Their length is known as the candidates that a uniform
+    // population has in one, m = n / cells * (2 R + 1)^2; where the agents
+    // cluster, windows are longer and the group gains more.  Measured on GB300,
+    // us per step thread / group, uniform, and with 30% in a cluster:
+    //   R = 1    5k in 256^2 (m 0.7)  12.2 / 12.5   13.9 / 12.8
+    //           20k in 1024^2 (0.2)   15.5 / 18.0   16.0 / 18.0
+    //           20k in 256^2 (2.7)    14.4 / 16.8   19.9 / 17.0
+    //           50k in 512^2 (1.7)    16.6 / 23.4   19.1 / 24.1
+    //           50k in 256^2 (6.9)    17.0 / 23.6   27.4 / 25.4
+    //   R = 2   50k in 2048^2 (0.3)   23.6 / 26.6   24.2 / 25.3
+    //           50k in 512^2 (4.8)    19.6 / 24.4   31.1 / 25.9
+    //           90k in 512^2 (8.6)    24.1 / 32.5   46.4 / 37.3
+    //   R = 3.5 90k in 512^2 (22)     36.6 / 34.2   154 / 68
+    // The lines lie where a uniform population is no slower than it was with one
+    // thread per agent and branches per pair (us: step, 20k in 256^2 at R = 1 17.7,
+    // 50k 21.5, 90k in 512^2 at R = 2 30.5; a pass without the move gained less
+    // with a thread per agent: 20k in 256^2 18.3, thread 17.7, group 20.1).  On a
+    // wrapped axis a thread's test of the wrap per candidate costs more and they
+    // lie further out (step, R = 1, 50k in 256^2, uniform: 25.9 before, thread
+    // 22.0, group 23.4; with a cluster 43.8, 32.3 and 26.5).
+    inline bool GroupPerAgent(int32_t n, int64_t cells, double R, bool walls, bool step)
+    {
+        const double m = static_cast<double>(n) / static_cast<double>(cells) * (2.0 * R + 1.0) * (2.0 * R + 1.0);
+        if (R >= 2.0)
+        {
+            const int32_t most = (R >= 3.0 || !walls) ? 100000 : (step ? 70000 : 60000);
+            return n <= most && n <= m * (step ? 50000.0 : 25000.0);
+        }
+        return n <= (walls ? (step ? 30000 : 12000) : 55000) && n <= m * 8000.0;
+    }
+
     struct ForceLawSpec
     {
         int kind = kLawLinear;
@@ -2091,7 +2117,7 @@ namespace halcuda
                 // the interface's law on a grid with walls: the wrap tests compiled out
                 if constexpr (std::is_same<T, float>::value)
                 {
-                    if (n <= kGroupAgents && velIn == nullptr)
+                    if (GroupPerAgent(n, C, R, !wrapX && !wrapY, false) && velIn == nullptr)
                     {
                         const unsigned groups =
                             static_cast<unsigned>((static_cast<int64_t>(n) * kGroupLanes + T_ - 1) / T_);
@@ -2188,7 +2214,7 @@ namespace
                           a.counts.p, a.tileSums.p);
         };
         const bool walls = !mp.wrapX && !mp.wrapY;
-        if (law.kind == kLawLinear && !law.sums && a.n <= kGroupAgents)
+        if (law.kind == kLawLinear && !law.sums && GroupPerAgent(a.n, a.C, R, walls, true))
         {
             const unsigned groups = static_cast<unsigned>((static_cast<int64_t>(a.n) * kGroupLanes + T - 1) / T);
             LaunchChained(walls ? ForcesMoveGroup<true> : ForcesMoveGroup<false>, groups, T, s, a.bucket.p, a.offsets.p,
