@@ -336,7 +336,27 @@ namespace halcuda
             const double *g;
             const double *segP;
             const double *segQ;
+            int32_t *ctl;        // SegCtl, then each 32 lines' walks: elimination, back substitution
+            int32_t mendBudget;  // cycles of walks up to which segments are the faster
         };
+
+        // A split plan's record, in ctl: sweeps left to solve serially, how many
+        // the next time, and of the current sweep the most cycles that the walks
+        // of any 32 lines took (the longest of step 3 and 4, and all of step 5)
+        // and the CTAs that have reported.
+        enum SegCtl : int
+        {
+            kCtlSkip = 0,
+            kCtlPeriod = 1,
+            kCtlWorst = 2,
+            kCtlReported = 3,
+            kCtlCount = 4
+        };
+        __host__ __device__ __forceinline__ int32_t CtlLines(int32_t lines) { return (lines + 31) / 32; }
+        constexpr int32_t kSegMinPeriod = 4, kSegMaxPeriod = 32;
+        // cycles that mending an element takes (1820 of 2048 elements of a back
+        // substitution: 425 us)
+        constexpr int32_t kMendFwd = 160, kMendBwd = 480;
 
         // ImplicitBoundarySource (ADIequations.h:198-220) at position i of a
         // line of length L; 0 on a wrapped axis.
@@ -594,6 +614,7 @@ namespace halcuda
 
         constexpr int kChainFwd = 16;  // elements loaded ahead in the elimination
         constexpr int kChainBwd = 8;   // ... and in the back substitution
+        constexpr int kChainFix = 8;   // ... and where the elimination is checked
 
         // Thomas solve of one line per thread, TdmaSolver::TDMA
         // (TdmaSolver.h:26-66) in its operations and order, over the
@@ -609,15 +630,10 @@ namespace halcuda
         // line (TDMAperiodic, TdmaSolver.h:96-119) leaves its factor (y0 +
         // yL * vEnd) / (1 + vz) in factor[line].
         template <bool FAST>
-        __global__ void __launch_bounds__(32) AdiChain64(double *__restrict__ d, double *__restrict__ out,
-                                                          LinePlan64Dev pl, int32_t lines,
-                                                          double *__restrict__ factor)
+        __device__ __forceinline__ void ChainLine(double *__restrict__ d, double *__restrict__ out,
+                                                  const LinePlan64Dev &pl, int32_t lines, int32_t line,
+                                                  double *__restrict__ factor)
         {
-            const int32_t line = blockIdx.x * blockDim.x + threadIdx.x;
-            if (line >= lines)
-            {
-                return;
-            }
             const int32_t L = pl.L;
             auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
 
@@ -735,6 +751,18 @@ namespace halcuda
             }
         }
 
+        template <bool FAST>
+        __global__ void __launch_bounds__(32) AdiChain64(double *__restrict__ d, double *__restrict__ out,
+                                                          LinePlan64Dev pl, int32_t lines,
+                                                          double *__restrict__ factor)
+        {
+            const int32_t line = blockIdx.x * blockDim.x + threadIdx.x;
+            if (line < lines)
+            {
+                ChainLine<FAST>(d, out, pl, lines, line, factor);
+            }
+        }
+
         // ---- the same solve, each line split into segments ------------------
         // One thread per line is one dependent FP64 chain of 2 + 5
         // instructions per element, 64 cycles each: 580 us for 2048 lines of
@@ -758,40 +786,78 @@ namespace halcuda
         //      zero start, as in 1;
         //   4. AdiSegBack and AdiSegBackFix: the same for the back
         //      substitution;
-        //   5. AdiSegFinish: solves a marked line again serially.
+        //   5. of each 32 lines, the CTA that is the last to be done with step 3
+        //      (4) mends the marked lines, from segment to segment: a segment
+        //      that was entered with another value than the line now holds is
+        //      walked again, until it meets what is stored.
         // Every element is thus either checked against the serial recurrence
         // or follows from one that was: equality is bitwise, so zeros' signs,
         // infinities and NaN end in a marked line at worst.
         // 2048 lines of 2048: 122 us in all (19 segments a line; FP64 issue needs
         // 79 us for the ten operations per element), 580 us as one chain a line.
+        // Lines are marked where trajectories an ulp apart stay apart: on
+        // constant data, where each has its own rounded fixed point (a uniform
+        // field's back substitution), and where the right-hand side is zero, so
+        // that a relative difference neither grows nor shrinks (the tails of a
+        // point or a step in an empty field).
+
+        __device__ __forceinline__ bool SameBits(double a, double b)
+        {
+            return __double_as_longlong(a) == __double_as_longlong(b);
+        }
+
+        // A load that stays where it is written, ahead of its use (the compiler
+        // moves others down to it, past the walks' tests).
+        __device__ __forceinline__ double LdAhead(const double *p)
+        {
+            double v;
+            asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+            return v;
+        }
 
         // e[i] = d[i] - ws[i] * e[i - 1] over elements [a, b) of a line, from
-        // prev (unused at i = 0), in the reference's operations; returns the
-        // last value.  at(i): the element's offset.
-        template <typename At>
-        __device__ __forceinline__ double ElimRun(const double *__restrict__ d, double *__restrict__ e,
-                                                  const LinePlan64Dev &pl, int32_t a, int32_t b, double prev, At at)
+        // prev (unused at i = 0), in the reference's operations; prev becomes
+        // the last value.  at(i): the element's offset.  CHECK: the warp stops
+        // after a batch by which every lane had a batch whose last element came
+        // out bit-equal to the stored one, since the trajectories are one from
+        // where they meet; whether the lane's did.  (Nothing on the chain tests
+        // anything, and the lanes stay together: with a test per element, or
+        // lanes that stop by themselves, the walk took three times as long.)
+        template <bool CHECK, int B, typename At>
+        __device__ __forceinline__ bool ElimWalk(const double *__restrict__ d, double *__restrict__ e,
+                                                 const LinePlan64Dev &pl, int32_t a, int32_t b, double &prev, At at,
+                                                 int32_t *batches = nullptr)
         {
-            double rc[kChainFwd], wc[kChainFwd];
+            bool met = false;
+            double rc[B], wc[B], oc = 0.0;  // oc: the batch's last element as stored
 #pragma unroll
-            for (int k = 0; k < kChainFwd; k++)
+            for (int k = 0; k < B; k++)
             {
                 const int32_t i = min(a + k, b - 1);
-                rc[k] = __ldcg(d + at(i));
+                rc[k] = LdAhead(d + at(i));
                 wc[k] = __ldg(pl.ws + i);
             }
-            for (int32_t i0 = a; i0 < b; i0 += kChainFwd)
+            if (CHECK)
             {
-                double rn[kChainFwd], wn[kChainFwd];
+                oc = LdAhead(e + at(min(a + B - 1, b - 1)));
+                __syncwarp();  // (a line may be on two lanes)
+            }
+            for (int32_t i0 = a; i0 < b; i0 += B)
+            {
+                double rn[B], wn[B], on = 0.0;
 #pragma unroll
-                for (int k = 0; k < kChainFwd; k++)
+                for (int k = 0; k < B; k++)
                 {
-                    const int32_t i = min(i0 + kChainFwd + k, b - 1);
-                    rn[k] = __ldcg(d + at(i));
+                    const int32_t i = min(i0 + B + k, b - 1);
+                    rn[k] = LdAhead(d + at(i));
                     wn[k] = __ldg(pl.ws + i);
                 }
+                if (CHECK)
+                {
+                    on = LdAhead(e + at(min(i0 + 2 * B - 1, b - 1)));
+                }
 #pragma unroll
-                for (int k = 0; k < kChainFwd; k++)
+                for (int k = 0; k < B; k++)
                 {
                     const int32_t i = i0 + k;
                     if (i < b)
@@ -800,14 +866,27 @@ namespace halcuda
                         e[at(i)] = prev;
                     }
                 }
+                if (batches != nullptr)
+                {
+                    (*batches)++;
+                }
+                if (CHECK)
+                {
+                    met = met || SameBits(prev, oc);
+                    if (__all_sync(0xffffffffu, met))
+                    {
+                        break;
+                    }
+                }
+                oc = on;
 #pragma unroll
-                for (int k = 0; k < kChainFwd; k++)
+                for (int k = 0; k < B; k++)
                 {
                     rc[k] = rn[k];
                     wc[k] = wn[k];
                 }
             }
-            return prev;
+            return met;
         }
 
         // The exact quotient num / bs[i] for any numerator.
@@ -816,89 +895,184 @@ namespace halcuda
             return PlanDivisionOutOfRange(num) ? __ddiv_rn(num, bh.x) : DivByPlan(num, bh, lo);
         }
 
-        // x[i] = (e[i] - off * x[i + 1]) / bs[i] over [a, b) downwards, from x
-        // (unused at i = L - 1), in the reference's operations; returns x[a].
-        // FAST: a numerator outside DivByPlan's range has the segment run
-        // again with the division chosen per element (a branch on the chain).
-        template <bool FAST, typename At>
-        __device__ __forceinline__ double BackRun(const double *__restrict__ e, double *__restrict__ out,
-                                                  const LinePlan64Dev &pl, int32_t a, int32_t b, double x, At at)
+        // Elements i1, i1 - 1, .. i0 of the back substitution from x, with
+        // numerators that DivByPlan does not take; *again: there was one.  Not
+        // inlined (HalfStepExact).
+        __device__ __noinline__ double BackSlow(const double *e, double *out, const double2 *bh, const int2 *lo,
+                                                double off, int32_t L, int32_t i1, int32_t i0, double x,
+                                                int32_t lines, int32_t line, bool *again)
         {
-            const double x0 = x;
-            uint32_t redo = 0;
-            double dc[kChainBwd];
-            double2 bc[kChainBwd];
-            int2 lc[kChainBwd];
+            constexpr int B = 8;
+            double ev[B];
+            double2 bv[B];
+            int2 lv[B];
 #pragma unroll
-            for (int k = 0; k < kChainBwd; k++)
+            for (int k = 0; k < B; k++)
+            {
+                const int32_t i = max(i1 - k, i0);
+                ev[k] = __ldcg(e + static_cast<int64_t>(i) * lines + line);
+                bv[k] = __ldg(bh + i);
+                lv[k] = __ldg(lo + i);
+            }
+            uint32_t rare = 0;
+#pragma unroll
+            for (int k = 0; k < B; k++)
+            {
+                const int32_t i = i1 - k;
+                if (i >= i0)
+                {
+                    const double num = (i == L - 1) ? ev[k] : __dsub_rn(ev[k], __dmul_rn(off, x));
+                    rare |= PlanDivisionOutOfRange(num);
+                    x = DivExact(num, bv[k], lv[k]);
+                    out[static_cast<int64_t>(i) * lines + line] = x;
+                }
+            }
+            *again = rare != 0;
+            return x;
+        }
+
+        // x[i] = (e[i] - off * x[i + 1]) / bs[i] over [a, b) downwards, from x
+        // (unused at i = L - 1), in the reference's operations; x becomes x[a].
+        // A batch that has a numerator outside DivByPlan's range is computed
+        // again with the division chosen per element (a branch on the chain),
+        // and so are the next ones until a batch has none.  CHECK as in
+        // ElimWalk.
+        template <bool CHECK>
+        __device__ __forceinline__ bool BackWalk(const double *__restrict__ e, double *__restrict__ out,
+                                                 const LinePlan64Dev &pl, int32_t lines, int32_t line, int32_t a,
+                                                 int32_t b, double &x, int32_t *batches = nullptr)
+        {
+            constexpr int B = kChainBwd;
+            static_assert(B == 8, "BackSlow's batch");
+            auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
+            bool slow = false, met = false;
+            double dc[B], oc = 0.0;
+            double2 bc[B];
+            int2 lc[B];
+#pragma unroll
+            for (int k = 0; k < B; k++)
             {
                 const int32_t i = max(b - 1 - k, a);
                 dc[k] = __ldcg(e + at(i));
                 bc[k] = __ldg(pl.bh + i);
                 lc[k] = __ldg(pl.lo + i);
             }
-            for (int32_t i0 = b - 1; i0 >= a; i0 -= kChainBwd)
+            if (CHECK)
             {
-                double dn[kChainBwd];
-                double2 bn[kChainBwd];
-                int2 ln[kChainBwd];
+                oc = LdAhead(out + at(max(b - B, a)));
+                __syncwarp();
+            }
+            for (int32_t i0 = b - 1; i0 >= a; i0 -= B)
+            {
+                double dn[B], on = 0.0;
+                double2 bn[B];
+                int2 ln[B];
 #pragma unroll
-                for (int k = 0; k < kChainBwd; k++)
+                for (int k = 0; k < B; k++)
                 {
-                    const int32_t i = max(i0 - kChainBwd - k, a);
+                    const int32_t i = max(i0 - B - k, a);
                     dn[k] = __ldcg(e + at(i));
                     bn[k] = __ldg(pl.bh + i);
                     ln[k] = __ldg(pl.lo + i);
                 }
-#pragma unroll
-                for (int k = 0; k < kChainBwd; k++)
+                if (CHECK)
                 {
-                    const int32_t i = i0 - k;
-                    if (i >= a)
+                    on = LdAhead(out + at(max(i0 - 2 * B + 1, a)));
+                }
+                const double x0 = x;
+                uint32_t rare = slow ? 1u : 0u;
+                if (!slow)
+                {
+#pragma unroll
+                    for (int k = 0; k < B; k++)
                     {
-                        const double num = (i == pl.L - 1) ? dc[k] : __dsub_rn(dc[k], __dmul_rn(pl.off, x));
-                        if constexpr (FAST)
+                        const int32_t i = i0 - k;
+                        if (i >= a)
                         {
+                            const double num = (i == pl.L - 1) ? dc[k] : __dsub_rn(dc[k], __dmul_rn(pl.off, x));
                             x = DivByPlan(num, bc[k], lc[k]);
-                            redo |= PlanDivisionOutOfRange(num);
+                            rare |= PlanDivisionOutOfRange(num);
+                            out[at(i)] = x;
                         }
-                        else
-                        {
-                            x = DivExact(num, bc[k], lc[k]);
-                        }
-                        out[at(i)] = x;
                     }
                 }
+                if (rare != 0)
+                {
+                    x = BackSlow(e, out, pl.bh, pl.lo, pl.off, pl.L, i0, max(i0 - B + 1, a), x0, lines, line, &slow);
+                }
+                if (batches != nullptr)
+                {
+                    (*batches)++;
+                }
+                if (CHECK)
+                {
+                    met = met || SameBits(x, oc);
+                    if (__all_sync(0xffffffffu, met))
+                    {
+                        break;
+                    }
+                }
+                oc = on;
 #pragma unroll
-                for (int k = 0; k < kChainBwd; k++)
+                for (int k = 0; k < B; k++)
                 {
                     dc[k] = dn[k];
                     bc[k] = bn[k];
                     lc[k] = ln[k];
                 }
             }
-            if constexpr (FAST)
+            return met;
+        }
+
+        // Whether the CTA (one warp: 32 lines of one segment) is the last of its
+        // lines' CTAs to come here, and may read what the others wrote.  No CTA
+        // waits for another.  arrived: one count per 32 lines, zero between
+        // kernels.
+        __device__ __forceinline__ bool LastOfLines(int32_t *__restrict__ arrived)
+        {
+            __threadfence();
+            __syncwarp();
+            int32_t before = 0;
+            if (threadIdx.x == 0)
             {
-                if (redo != 0)
-                {
-                    x = BackRun<false>(e, out, pl, a, b, x0, at);
-                }
+                before = atomicAdd(arrived + blockIdx.x, 1);
             }
-            return x;
+            before = __shfl_sync(0xffffffffu, before, 0);
+            if (before != static_cast<int32_t>(gridDim.y) - 1)
+            {
+                return false;
+            }
+            if (threadIdx.x == 0)
+            {
+                arrived[blockIdx.x] = 0;
+            }
+            __threadfence();
+            return true;
         }
 
-        __device__ __forceinline__ bool SameBits(double a, double b)
+        __device__ __forceinline__ bool Serial(const LinePlan64Dev &pl)
         {
-            return __double_as_longlong(a) == __double_as_longlong(b);
+            return __ldcg(pl.ctl + kCtlSkip) > 0;
         }
 
-        // Step 1 (segments 0 .. segs - 2): y[seg * lines + line].
-        __global__ void __launch_bounds__(32) AdiSegEnds(const double *__restrict__ d, LinePlan64Dev pl, int32_t lines,
-                                                          double *__restrict__ y)
+        // Step 1 (segments 0 .. segs - 2): y[seg * lines + line].  In a serial
+        // sweep the first segment's CTAs solve their lines whole.
+        __global__ void __launch_bounds__(32) AdiSegEnds(double *__restrict__ d, LinePlan64Dev pl, int32_t lines,
+                                                          double *__restrict__ y, double *__restrict__ out,
+                                                          double *__restrict__ factor)
         {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y;
             if (line >= lines)
             {
+                return;
+            }
+            if (Serial(pl))
+            {
+                if (seg == 0)
+                {
+                    ChainLine<true>(d, out, pl, lines, line, factor);
+                }
                 return;
             }
             const int32_t a = seg * pl.segLen, b = a + pl.segLen;
@@ -945,64 +1119,49 @@ namespace halcuda
                                                           LinePlan64Dev pl, int32_t lines,
                                                           const double *__restrict__ y, double *__restrict__ ends)
         {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y;
             if (line >= lines)
             {
                 return;
             }
+            const bool serial = Serial(pl);
             const int32_t a = seg * pl.segLen, b = min(a + pl.segLen, pl.L);
             double prev = 0.0;
             for (int32_t q = 0; q < seg; q++)
             {
                 prev = __fma_rn(__ldg(pl.segP + q), prev, __ldcg(y + static_cast<int64_t>(q) * lines + line));
             }
-            prev = ElimRun(d, e, pl, a, b, prev, [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; });
+            if (serial)
+            {
+                return;
+            }
+            ElimWalk<false, kChainFwd>(d, e, pl, a, b, prev,
+                                       [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; });
             ends[static_cast<int64_t>(seg) * lines + line] = prev;
         }
 
         // Step 3; z[seg * lines + line]: segments 1 .. segs - 1 of the back
-        // substitution from a zero start.
+        // substitution from a zero start (of a marked line from values that may
+        // be an ulp off: they only estimate).
         __global__ void __launch_bounds__(32) AdiSegFix(const double *__restrict__ d, double *__restrict__ e,
                                                          LinePlan64Dev pl, int32_t lines,
                                                          const double *__restrict__ ends, double *__restrict__ z,
-                                                         int32_t *__restrict__ marks)
+                                                         int32_t *__restrict__ marks, int32_t *__restrict__ arrived)
         {
-            constexpr int B = 8;
-            const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y + 1;
-            if (line >= lines)
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (Serial(pl))
             {
                 return;
             }
+            // (lanes past the last line repeat it: the walks take the whole warp)
+            const int32_t line = min(static_cast<int32_t>(blockIdx.x * 32 + threadIdx.x), lines - 1);
+            const int32_t seg = blockIdx.y + 1;
             const int32_t a = seg * pl.segLen, b = min(a + pl.segLen, pl.L);
             auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
+            int32_t batches = 0;
             double prev = __ldcg(ends + static_cast<int64_t>(seg - 1) * lines + line);
-            bool met = false;
-            for (int32_t i0 = a; i0 < b && !met; i0 += B)
-            {
-                double dv[B], ev[B], wv[B];
-#pragma unroll
-                for (int k = 0; k < B; k++)
-                {
-                    const int32_t i = min(i0 + k, b - 1);
-                    dv[k] = __ldcg(d + at(i));
-                    ev[k] = __ldcg(e + at(i));
-                    wv[k] = __ldg(pl.ws + i);
-                }
-#pragma unroll
-                for (int k = 0; k < B; k++)
-                {
-                    if (i0 + k < b && !met)
-                    {
-                        prev = __dsub_rn(dv[k], __dmul_rn(wv[k], prev));
-                        met = SameBits(prev, ev[k]);
-                        if (!met)
-                        {
-                            e[at(i0 + k)] = prev;
-                        }
-                    }
-                }
-            }
-            if (!met && seg < pl.segs - 1)
+            if (!ElimWalk<true, kChainFix>(d, e, pl, a, b, prev, at, &batches) && seg < pl.segs - 1)
             {
                 marks[line] = 1;
             }
@@ -1027,6 +1186,33 @@ namespace halcuda
                 }
             }
             z[static_cast<int64_t>(seg) * lines + line] = v;
+            int32_t *walked = pl.ctl + kCtlCount + blockIdx.x;
+            if (threadIdx.x == 0)
+            {
+                atomicMax(walked, batches);
+            }
+            if (!LastOfLines(arrived))
+            {
+                return;
+            }
+            // step 5 of the elimination
+            const bool marked = __any_sync(0xffffffffu, __ldcg(marks + line) != 0);
+            marks[line] = 0;
+            batches = 0;
+            for (int32_t q = 1; marked && q < pl.segs; q++)
+            {
+                const int32_t qa = q * pl.segLen;
+                prev = __ldcg(e + at(qa - 1));
+                if (__any_sync(0xffffffffu,
+                               !SameBits(prev, __ldcg(ends + static_cast<int64_t>(q - 1) * lines + line))))
+                {
+                    ElimWalk<true, kChainFix>(d, e, pl, qa, min(qa + pl.segLen, pl.L), prev, at, &batches);
+                }
+            }
+            if (threadIdx.x == 0)
+            {
+                *walked = kMendFwd * kChainFix * (__ldcg(walked) + batches);
+            }
         }
 
         // Step 4: the back substitution; starts[seg * lines + line] = its x[a].
@@ -1034,92 +1220,94 @@ namespace halcuda
                                                           LinePlan64Dev pl, int32_t lines,
                                                           const double *__restrict__ z, double *__restrict__ starts)
         {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y;
             if (line >= lines)
             {
                 return;
             }
+            const bool serial = Serial(pl);
             const int32_t a = seg * pl.segLen, b = min(a + pl.segLen, pl.L);
             double x = 0.0;
             for (int32_t q = pl.segs - 1; q > seg; q--)
             {
                 x = __fma_rn(__ldg(pl.segQ + q), x, __ldcg(z + static_cast<int64_t>(q) * lines + line));
             }
-            x = BackRun<true>(e, out, pl, a, b, x, [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; });
+            if (serial)
+            {
+                return;
+            }
+            BackWalk<false>(e, out, pl, lines, line, a, b, x);
             starts[static_cast<int64_t>(seg) * lines + line] = x;
         }
 
+        // With a periodic line's factor (see AdiChain64).
         __global__ void __launch_bounds__(32) AdiSegBackFix(const double *__restrict__ e, double *__restrict__ out,
                                                              LinePlan64Dev pl, int32_t lines,
                                                              const double *__restrict__ starts,
-                                                             int32_t *__restrict__ marks)
+                                                             int32_t *__restrict__ marks,
+                                                             int32_t *__restrict__ arrived, double *__restrict__ factor)
         {
-            constexpr int B = 8;
-            const int32_t line = blockIdx.x * 32 + threadIdx.x, seg = blockIdx.y;
-            if (line >= lines)
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (Serial(pl))
             {
                 return;
             }
+            const int32_t line = min(static_cast<int32_t>(blockIdx.x * 32 + threadIdx.x), lines - 1);
+            const int32_t seg = blockIdx.y;
             const int32_t a = seg * pl.segLen, b = a + pl.segLen;
-            auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
+            int32_t batches = 0;
             double x = __ldcg(starts + static_cast<int64_t>(seg + 1) * lines + line);
-            bool met = false;
-            for (int32_t i0 = b - 1; i0 >= a && !met; i0 -= B)
-            {
-                double ev[B], xv[B];
-                double2 bv[B];
-                int2 lv[B];
-#pragma unroll
-                for (int k = 0; k < B; k++)
-                {
-                    const int32_t i = max(i0 - k, a);
-                    ev[k] = __ldcg(e + at(i));
-                    xv[k] = __ldcg(out + at(i));
-                    bv[k] = __ldg(pl.bh + i);
-                    lv[k] = __ldg(pl.lo + i);
-                }
-#pragma unroll
-                for (int k = 0; k < B; k++)
-                {
-                    if (i0 - k >= a && !met)
-                    {
-                        x = DivExact(__dsub_rn(ev[k], __dmul_rn(pl.off, x)), bv[k], lv[k]);
-                        met = SameBits(x, xv[k]);
-                        if (!met)
-                        {
-                            out[at(i0 - k)] = x;
-                        }
-                    }
-                }
-            }
-            if (!met && seg > 0)
+            if (!BackWalk<true>(e, out, pl, lines, line, a, b, x, &batches) && seg > 0)
             {
                 marks[line] = 1;
             }
-        }
-
-        // Step 5, and a periodic line's factor (see AdiChain64).  Clears the
-        // marks.
-        __global__ void __launch_bounds__(32) AdiSegFinish(const double *__restrict__ d, double *__restrict__ e,
-                                                            double *__restrict__ out, LinePlan64Dev pl, int32_t lines,
-                                                            int32_t *__restrict__ marks, double *__restrict__ factor)
-        {
-            const int32_t line = blockIdx.x * 32 + threadIdx.x;
-            if (line >= lines)
+            int32_t *walked = pl.ctl + kCtlCount + blockIdx.x;
+            batches = __reduce_max_sync(0xffffffffu, batches);
+            if (threadIdx.x == 0)
+            {
+                atomicMax(walked + CtlLines(lines), batches);
+            }
+            if (!LastOfLines(arrived))
             {
                 return;
             }
+            // step 5 of the back substitution
             auto at = [&](int32_t i) { return static_cast<int64_t>(i) * lines + line; };
-            if (marks[line] != 0)
+            const bool marked = __any_sync(0xffffffffu, __ldcg(marks + line) != 0);
+            marks[line] = 0;
+            batches = 0;
+            for (int32_t q = pl.segs - 2; marked && q >= 0; q--)
             {
-                marks[line] = 0;
-                ElimRun(d, e, pl, 0, pl.L, 0.0, at);
-                BackRun<false>(e, out, pl, 0, pl.L, 0.0, at);
+                const int32_t qb = (q + 1) * pl.segLen;
+                x = __ldcg(out + at(qb));
+                if (__any_sync(0xffffffffu,
+                               !SameBits(x, __ldcg(starts + static_cast<int64_t>(q + 1) * lines + line))))
+                {
+                    BackWalk<true>(e, out, pl, lines, line, q * pl.segLen, qb, x, &batches);
+                }
             }
             if (pl.periodic)
             {
-                const double vy = __dadd_rn(out[at(0)], __dmul_rn(out[at(pl.L - 1)], pl.vEnd));
+                const double vy = __dadd_rn(__ldcg(out + at(0)), __dmul_rn(__ldcg(out + at(pl.L - 1)), pl.vEnd));
                 factor[line] = __ddiv_rn(vy, pl.onePlusVz);
+            }
+            // the record
+            if (threadIdx.x == 0)
+            {
+                int32_t *ctl = pl.ctl;
+                int32_t *back = walked + CtlLines(lines);
+                atomicMax(ctl + kCtlWorst, __ldcg(walked) + kMendBwd * kChainBwd * (__ldcg(back) + batches));
+                *walked = *back = 0;
+                __threadfence();
+                if (atomicAdd(ctl + kCtlReported, 1) == static_cast<int32_t>(gridDim.x) - 1)
+                {
+                    const bool late = atomicExch(ctl + kCtlWorst, 0) > pl.mendBudget;
+                    const int32_t period = late ? ctl[kCtlPeriod] : 0;
+                    ctl[kCtlReported] = 0;
+                    ctl[kCtlPeriod] = late ? min(2 * period, kSegMaxPeriod) : kSegMinPeriod;
+                    ctl[kCtlSkip] = late ? period + 1 : 0;  // (the transpose of this sweep counts one)
+                }
             }
         }
 
@@ -1157,9 +1345,13 @@ namespace halcuda
         template <bool COMMIT>
         __global__ void Transpose64(const double *__restrict__ in, double *__restrict__ out, int32_t rows,
                                     int32_t cols, const double *__restrict__ f, const double *__restrict__ fac,
-                                    const double *__restrict__ zs)
+                                    const double *__restrict__ zs, int32_t *__restrict__ ctl)
         {
             __shared__ double tile[32][33];
+            if (ctl != nullptr && blockIdx.x + blockIdx.y + threadIdx.x + threadIdx.y == 0 && ctl[kCtlSkip] > 0)
+            {
+                ctl[kCtlSkip]--;
+            }
             const int32_t c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
             for (int j = threadIdx.y; j < 32; j += blockDim.y)
             {
@@ -1221,7 +1413,7 @@ namespace halcuda
             double off = 0, vEnd = 0, onePlusVz = 0;
             bool periodic = false;
             bool fastDiv = false;
-            int32_t segs = 1, segLen = 0;
+            int32_t segs = 1, segLen = 0, mendBudget = 0;
             std::vector<double> g, segP, segQ;
         };
 
@@ -1390,6 +1582,7 @@ namespace halcuda
         constexpr int32_t kSegMaxWarps = 1216;  // 152 SMs x 4 FP64 pipes x 2
         constexpr int32_t kSegMinLen = 64;
         constexpr int32_t kSegMinLine = 232;
+        constexpr int32_t kSegMinCount = 3;
 
         // Segments of a line's split solve, for `lines` lines.  As many as
         // give every FP64 pipe two warps, which cover each other's loads (the
@@ -1399,7 +1592,9 @@ namespace halcuda
         // more on their launches and meetings than the chain saves), and each
         // long enough that a trajectory's error falls below 2^-64 of itself
         // over it: otherwise, for large rates, segments would end before they
-        // meet the serial one.  One segment: the serial chain, also for lines
+        // meet the serial one.  One segment: the serial chain, also where only
+        // two segments would do (they cost more than the chain where they meet
+        // late: 2048^2 at r = 500 1010 against 660 us per sweep) and for lines
         // below kSegMinLine, whose chain costs less than the segments' launches
         // (four ticks, chain / segments: 200^2 574 / 696 us, 240^2 673 / 634, 320^2
         // 868 / 639).
@@ -1419,7 +1614,7 @@ namespace halcuda
                 p.g[static_cast<size_t>(i)] = -p.off * p.bh[static_cast<size_t>(i)].y;
             }
             const int32_t most = L < kSegMinLine ? 1 : std::min(kSegMaxWarps / warps, L / kSegMinLen);
-            for (int32_t segs = most; segs >= 2; segs--)
+            for (int32_t segs = most; segs >= kSegMinCount; segs--)
             {
                 const int32_t len = (L + segs - 1) / segs;
                 const int32_t n = (L + len - 1) / len;
@@ -1435,10 +1630,18 @@ namespace halcuda
                     ok = ok && (q == n - 1 || (std::fabs(P[static_cast<size_t>(q)]) <= 0x1p-64 &&
                                                std::fabs(Q[static_cast<size_t>(q)]) <= 0x1p-64));
                 }
-                if (ok && n >= 2)
+                if (ok && n >= kSegMinCount)
                 {
                     p.segs = n;
                     p.segLen = len;
+                    // what the chain takes less the segments' kernels, as
+                    // measured (cycles): 586 per element (2048: 580 us), and 831
+                    // per segment's element and warp that shares a pipe, and
+                    // 72000 (2048^2 122 us, 512^2 65 us; at least the walks of
+                    // ordinary fields)
+                    const double perPipe = std::max(1.0, static_cast<double>(n) * warps / 608.0);
+                    p.mendBudget =
+                        static_cast<int32_t>(std::max(20000.0, 586.0 * L - 831.0 * len * perPipe - 72000.0));
                     p.segP = P;
                     p.segQ = Q;
                     return;
@@ -1446,9 +1649,26 @@ namespace halcuda
             }
         }
 
+        // Launches a kernel of the split solve, which waits for the one before.
+        template <typename... KArgs, typename... Args>
+        void ChainedSeg(void (*kernel)(KArgs...), dim3 grid, cudaStream_t s, Args... args)
+        {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = grid;
+            cfg.blockDim = dim3(32);
+            cfg.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+        }
+
         struct PlanBuf64
         {
             DevBuf<double> buf;  // the plan's arrays
+            DevBuf<int32_t> ctl; // of a split plan
             LinePlan64Dev dev;
         };
     }
@@ -1573,7 +1793,7 @@ namespace halcuda
         DevBuf<double> wA, wB, vB, dS;  // scratch (grown on first use)
         DevBuf<double> fac;             // periodic factors of the current sweep's lines
         DevBuf<double> segA, segB;      // split solve: values at the segments' ends
-        DevBuf<int32_t> marks;          // split solve: lines to solve again (zero between sweeps)
+        DevBuf<int32_t> marks;          // split solve: lines to mend, CTAs arrived (zero between kernels)
         std::map<std::string, std::unique_ptr<PlanBuf64>> plans;
 
         int Ensure(DevBuf<double> &b, size_t n, cudaStream_t s, const char *what)
@@ -1586,10 +1806,12 @@ namespace halcuda
             return HAL_CUDA_OK;
         }
 
-        int Plan(int32_t L, int32_t lines, double r, bool wrap, bool dirichlet, LinePlan64Dev *out)
+        // (each axis has its own, with its own record)
+        int Plan(char axis, int32_t L, int32_t lines, double r, bool wrap, bool dirichlet, LinePlan64Dev *out)
         {
             char key[96];
-            snprintf(key, sizeof(key), "%d|%d|%a|%d|%d", L, lines, r, wrap ? 1 : 0, (dirichlet && !wrap) ? 1 : 0);
+            snprintf(key, sizeof(key), "%c%d|%d|%a|%d|%d", axis, L, lines, r, wrap ? 1 : 0,
+                     (dirichlet && !wrap) ? 1 : 0);
             auto it = plans.find(key);
             if (it == plans.end())
             {
@@ -1632,6 +1854,17 @@ namespace halcuda
                 pb->dev.g = pb->buf.p + 6 * Ls;
                 pb->dev.segP = pb->buf.p + 7 * Ls;
                 pb->dev.segQ = pb->buf.p + 7 * Ls + h.segs;
+                pb->dev.ctl = nullptr;
+                pb->dev.mendBudget = h.mendBudget;
+                if (h.segs > 1)
+                {
+                    std::vector<int32_t> ctl(kCtlCount + 2 * static_cast<size_t>(CtlLines(lines)), 0);
+                    ctl[kCtlPeriod] = kSegMinPeriod;
+                    HAL_TRY(pb->ctl.Alloc(ctl.size(), "cudaMalloc(ADI plan)"));
+                    HAL_TRY(CudaStatus(cudaMemcpy(pb->ctl.p, ctl.data(), ctl.size() * sizeof(int32_t),
+                                                  cudaMemcpyHostToDevice), "cudaMemcpy(ADI plan)"));
+                    pb->dev.ctl = pb->ctl.p;
+                }
                 it = plans.emplace(key, std::move(pb)).first;
             }
             *out = it->second->dev;
@@ -1655,8 +1888,8 @@ namespace halcuda
         HAL_TRY(m.Ensure(m.vB, n, s, "cudaMalloc(ADI scratch)"));
         HAL_TRY(m.Ensure(m.dS, n, s, "cudaMalloc(ADI scratch)"));
         LinePlan64Dev px, py;
-        HAL_TRY(m.Plan(xDim, yDim, r, wrapX != 0, g != nullptr, &px));
-        HAL_TRY(m.Plan(yDim, xDim, r, wrapY != 0, g != nullptr, &py));
+        HAL_TRY(m.Plan('x', xDim, yDim, r, wrapX != 0, g != nullptr, &px));
+        HAL_TRY(m.Plan('y', yDim, xDim, r, wrapY != 0, g != nullptr, &py));
         // per sweep: the right-hand sides on every SM, the chains one line
         // per thread and one warp per block (the lines spread over the most
         // SMs), then the transpose that applies the periodic correction
@@ -1678,11 +1911,12 @@ namespace halcuda
         {
             HAL_TRY(m.Ensure(m.segA, nSeg, s, "cudaMalloc(ADI scratch)"));
             HAL_TRY(m.Ensure(m.segB, nSeg, s, "cudaMalloc(ADI scratch)"));
-            if (m.marks.n < nFac || m.marks.p == nullptr)
+            const size_t nMarks = nFac + Blocks(static_cast<int64_t>(nFac), T);  // and the counts of arrived CTAs
+            if (m.marks.n != nMarks || m.marks.p == nullptr)
             {
                 HAL_TRY(CudaStatus(cudaStreamSynchronize(s), "cudaMalloc(ADI scratch)"));
-                HAL_TRY(m.marks.Alloc(nFac, "cudaMalloc(ADI scratch)"));
-                HAL_TRY(CudaStatus(cudaMemsetAsync(m.marks.p, 0, nFac * sizeof(int32_t), s), "ADI scratch"));
+                HAL_TRY(m.marks.Alloc(nMarks, "cudaMalloc(ADI scratch)"));
+                HAL_TRY(CudaStatus(cudaMemsetAsync(m.marks.p, 0, nMarks * sizeof(int32_t), s), "ADI scratch"));
             }
         }
         // e: a scratch array that the sweep does not use otherwise (the split
@@ -1691,13 +1925,14 @@ namespace halcuda
             if (pl.segs > 1)
             {
                 const unsigned b = Blocks(lines, T), segs = static_cast<unsigned>(pl.segs);
-                AdiSegEnds<<<dim3(b, segs - 1), T, 0, s>>>(m.dS.p, pl, lines, m.segA.p);
-                AdiSegElim<<<dim3(b, segs), T, 0, s>>>(m.dS.p, e, pl, lines, m.segA.p, m.segB.p);
-                AdiSegFix<<<dim3(b, segs - 1), T, 0, s>>>(m.dS.p, e, pl, lines, m.segB.p, m.segA.p, m.marks.p);
-                AdiSegBack<<<dim3(b, segs), T, 0, s>>>(e, out, pl, lines, m.segA.p, m.segB.p);
-                AdiSegBackFix<<<dim3(b, segs - 1), T, 0, s>>>(e, out, pl, lines, m.segB.p, m.marks.p);
-                AdiSegFinish<<<b, T, 0, s>>>(m.dS.p, e, out, pl, lines, m.marks.p, m.fac.p);
-                CountLaunch(5);
+                ChainedSeg(AdiSegEnds, dim3(b, segs - 1), s, m.dS.p, pl, lines, m.segA.p, out, m.fac.p);
+                ChainedSeg(AdiSegElim, dim3(b, segs), s, m.dS.p, e, pl, lines, m.segA.p, m.segB.p);
+                ChainedSeg(AdiSegFix, dim3(b, segs - 1), s, m.dS.p, e, pl, lines, m.segB.p, m.segA.p, m.marks.p,
+                           m.marks.p + nFac);
+                ChainedSeg(AdiSegBack, dim3(b, segs), s, e, out, pl, lines, m.segA.p, m.segB.p);
+                ChainedSeg(AdiSegBackFix, dim3(b, segs - 1), s, e, out, pl, lines, m.segB.p, m.marks.p,
+                           m.marks.p + nFac, m.fac.p);
+                CountLaunch(4);
             }
             else if (pl.fastDiv)
             {
@@ -1712,12 +1947,12 @@ namespace halcuda
                                                         g ? g + 2 * static_cast<size_t>(yDim) : nullptr, g, r);
         chain(px, yDim, m.wA.p, m.vB.p);
         Transpose64<false><<<dim3((yDim + 31) / 32, (xDim + 31) / 32), tb, 0, s>>>(
-            m.wA.p, m.wB.p, xDim, yDim, nullptr, px.periodic ? m.fac.p : nullptr, px.zs);
+            m.wA.p, m.wB.p, xDim, yDim, nullptr, px.periodic ? m.fac.p : nullptr, px.zs, px.ctl);
         AdiRhs64<<<rhsGrid(xDim, yDim), rhsThreads(xDim), 0, s>>>(m.wB.p, m.dS.p, yDim, xDim, wrapX, wrapY, g,
                                                         g ? g + 2 * static_cast<size_t>(yDim) : nullptr, r);
         chain(py, xDim, m.vB.p, m.wA.p);
         Transpose64<true><<<dim3((xDim + 31) / 32, (yDim + 31) / 32), tb, 0, s>>>(
-            m.vB.p, deltas, yDim, xDim, f, py.periodic ? m.fac.p : nullptr, py.zs);
+            m.vB.p, deltas, yDim, xDim, f, py.periodic ? m.fac.p : nullptr, py.zs, py.ctl);
         CountLaunch(6);
         return LaunchStatus("DiffusionADI (FP64)");
     }
