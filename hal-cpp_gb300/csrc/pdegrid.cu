@@ -793,13 +793,20 @@ namespace halcuda
         // Every element is thus either checked against the serial recurrence
         // or follows from one that was: equality is bitwise, so zeros' signs,
         // infinities and NaN end in a marked line at worst.
-        // 2048 lines of 2048: 122 us in all (19 segments a line; FP64 issue needs
-        // 79 us for the ten operations per element), 580 us as one chain a line.
         // Lines are marked where trajectories an ulp apart stay apart: on
         // constant data, where each has its own rounded fixed point (a uniform
         // field's back substitution), and where the right-hand side is zero, so
         // that a relative difference neither grows nor shrinks (the tails of a
-        // point or a step in an empty field).
+        // point or a step in an empty field).  Where mending them costs more than
+        // the segments save, the sweep is slower than one chain a line, so the
+        // device keeps a record per plan (SegCtl) and solves the next sweeps
+        // serially, in AdiSegEnds: 4, then 8, 16, 32 between attempts.  The bits
+        // are the same either way.
+        // us per sweep at r = 5, the right-hand sides and the transpose included,
+        // one chain a line / here: random values in 2048^2 659 / 177 (19 segments
+        // a line; FP64 issue needs 79 for the ten operations per element), in
+        // 512^2 161 / 72, in 256^2 87 / 72; a uniform field, over forty sweeps, in
+        // 2048^2 659 / 663, in 512^2 161 / 165, in 256^2 87 / 92.
 
         __device__ __forceinline__ bool SameBits(double a, double b)
         {
@@ -1649,7 +1656,10 @@ namespace halcuda
             }
         }
 
-        // Launches a kernel of the split solve, which waits for the one before.
+        // Launches a kernel of the split solve, which waits for the one before
+        // at its start; none triggers its successor early, so that its CTAs come
+        // to SMs that have been left (us per sweep without / with: random 512^2
+        // 82 / 72, 2048^2 193 / 182).
         template <typename... KArgs, typename... Args>
         void ChainedSeg(void (*kernel)(KArgs...), dim3 grid, cudaStream_t s, Args... args)
         {
