@@ -488,16 +488,35 @@ namespace halcuda
 
     namespace
     {
-        // A[cell] = value for every point source (no cell twice).
-        __global__ void ScatterPoints(float *__restrict__ A, const int32_t *__restrict__ row,
-                                      const int32_t *__restrict__ col, const float *__restrict__ val, int32_t n,
-                                      int32_t yDim)
+        // A[cell] = 0 for the cells of the point sources before.
+        __global__ void ClearPoints(float *__restrict__ A, const int32_t *__restrict__ cells, int32_t n)
         {
             const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
             if (k < n)
             {
-                A[static_cast<int64_t>(row[k]) * yDim + col[k]] = val[k];
+                A[cells[k]] = 0.0f;
             }
+        }
+
+        // A[cell] = value for every point source (no cell twice), noted in
+        // cells, and a flag for each patch that reads it.
+        __global__ void ScatterPoints(float *__restrict__ A, int32_t *__restrict__ cells, uint8_t *__restrict__ flags,
+                                      TickPatchShape sh, const int32_t *__restrict__ row,
+                                      const int32_t *__restrict__ col, const float *__restrict__ val, int32_t n,
+                                      int32_t xDim, int32_t yDim)
+        {
+            const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+            if (k >= n)
+            {
+                return;
+            }
+            const int32_t x = row[k], y = col[k];
+            A[static_cast<int64_t>(x) * yDim + y] = val[k];
+            cells[k] = x * yDim + y;
+            TickPatchReaders(x, sh.strips, sh.rows, sh.halo, xDim, [&](int32_t st) {
+                TickPatchReaders(y, sh.windows, sh.cols, sh.haloCols, yDim,
+                                 [&](int32_t w) { flags[static_cast<int64_t>(st) * sh.windows + w] = 1; });
+            });
         }
     }
 
@@ -544,9 +563,13 @@ namespace halcuda
         // array of the grid and the patches that hold one (when no cell is
         // listed twice; otherwise one tick runs per launch).
         TickPatchShape patch;
+        // Built by the first run that uses them (PatchPoints).
         DevBuf<float> patchPts;
         DevBuf<uint8_t> patchFlags;
-        bool patchPtsOk = false;
+        DevBuf<int32_t> patchCells;        // the cells that patchPts holds
+        int32_t patchCount = 0;
+        std::vector<int32_t> pointCells;   // the last set_point_sources'
+        bool patchPtsDirty = false, patchPtsOk = false;
         // Temporal blocking through shared memory: ticks per launch 1 or 2 (0
         // = automatic, which never takes it).  The two-tick kernel stages
         // tiles with a tensor map per field buffer and reads the dense source
@@ -613,71 +636,73 @@ namespace halcuda
 
         // Several ticks per launch wherever the patch kernel takes the run: it
         // has no uptake term, and its point sources no repeated cells.
-        bool UsePatch(int32_t ticks, bool useExtras) const
+        int UsePatch(int32_t ticks, bool useExtras, cudaStream_t s, bool *use)
         {
-            return patch.windows > 0 && ticks >= 2 && blockMode == 0 && agents == nullptr &&
-                   !(useExtras && hasPoints && !patchPtsOk);
+            *use = patch.windows > 0 && ticks >= 2 && blockMode == 0 && agents == nullptr;
+            if (*use && useExtras && hasPoints)
+            {
+                HAL_TRY(PatchPoints(s));
+                *use = patchPtsOk;
+            }
+            return HAL_CUDA_OK;
         }
 
-        // Point sources of the patch kernel: scatters them into an array of
-        // the grid and flags the patches that read each one (the wrapped
-        // columns and rows of the edge patches included).
-        int SetPatchPoints(int32_t n, const int32_t *cells)
+        // The patch kernel's form of the point sources: an array of the grid and
+        // flags for the patches that read one.  Only the cells of the sources
+        // before are cleared, so that a caller who sets sources between short
+        // runs pays for its sources, and one who runs single ticks for none of
+        // this (five times set and run 10 ticks on 2048^2: 0.74 ms with one tick
+        // per launch, 1.6 with the whole array cleared and the readers listed on
+        // the host, 0.63 here).  Without memory for the array runs go one tick
+        // per launch.
+        int PatchPoints(cudaStream_t s)
         {
-            patchPtsOk = false;
-            if (patch.windows == 0)
+            if (!patchPtsDirty)
             {
                 return HAL_CUDA_OK;
             }
-            std::vector<int32_t> sorted(cells, cells + n);
+            patchPtsOk = false;
+            std::vector<int32_t> sorted(pointCells);
             std::sort(sorted.begin(), sorted.end());
             if (std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end())
             {
+                patchPtsDirty = false;
                 return HAL_CUDA_OK;
             }
-            const auto cover = [](int32_t count, int32_t len, int32_t halo, int32_t dim)
-            {
-                std::vector<std::vector<int32_t>> by(static_cast<size_t>(dim));
-                for (int32_t i = 0; i < count; i++)
-                {
-                    const int32_t at = TickPatchStart(i, count, len, halo, dim) - halo;
-                    for (int32_t c = at; c < at + len + 2 * halo; c++)
-                    {
-                        by[static_cast<size_t>(c < 0 ? c + dim : (c >= dim ? c - dim : c))].push_back(i);
-                    }
-                }
-                return by;
-            };
-            const auto cols = cover(patch.windows, patch.cols, patch.haloCols, yDim);
-            const auto rows = cover(patch.strips, patch.rows, patch.halo, xDim);
-            std::vector<uint8_t> flags(static_cast<size_t>(patch.windows) * patch.strips, 0);
-            for (const int32_t c : sorted)
-            {
-                for (const int32_t st : rows[static_cast<size_t>(c / yDim)])
-                {
-                    for (const int32_t w : cols[static_cast<size_t>(c % yDim)])
-                    {
-                        flags[static_cast<size_t>(st) * patch.windows + w] = 1;
-                    }
-                }
-            }
-            cudaStream_t s = stream.Get();
-            HAL_TRY(CudaStatus(cudaStreamSynchronize(s), "point sources"));
+            const size_t nFlags = static_cast<size_t>(patch.windows) * patch.strips;
             if (patchPts.p == nullptr)
             {
-                HAL_TRY(patchPts.Alloc(Length(), "cudaMalloc(points)"));
-                HAL_TRY(patchFlags.Alloc(flags.size(), "cudaMalloc(points)"));
+                if (patchPts.Alloc(Length(), "cudaMalloc(points)") != HAL_CUDA_OK ||
+                    patchFlags.Alloc(nFlags, "cudaMalloc(points)") != HAL_CUDA_OK)
+                {
+                    cudaGetLastError();
+                    patchPts.Free();
+                    patchPtsDirty = false;
+                    return HAL_CUDA_OK;
+                }
+                HAL_TRY(CudaStatus(cudaMemsetAsync(patchPts.p, 0, Length() * sizeof(float), s), "point sources"));
             }
-            HAL_TRY(CudaStatus(cudaMemsetAsync(patchPts.p, 0, Length() * sizeof(float), s), "point sources"));
-            ScatterPoints<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(patchPts.p, ptRow.p, ptCol.p, ptVal.p, n,
-                                                                                yDim);
+            const unsigned T = 256;
+            if (patchCount > 0)
+            {
+                ClearPoints<<<(static_cast<unsigned>(patchCount) + T - 1) / T, T, 0, s>>>(patchPts.p, patchCells.p,
+                                                                                         patchCount);
+                CountLaunch();
+                patchCount = 0;
+            }
+            const size_t n = static_cast<size_t>(nPoints);
+            if (patchCells.n < n || patchCells.p == nullptr)
+            {
+                HAL_TRY(CudaStatus(cudaStreamSynchronize(s), "point sources"));
+                HAL_TRY(patchCells.Alloc(n, "cudaMalloc(points)"));
+            }
+            HAL_TRY(CudaStatus(cudaMemsetAsync(patchFlags.p, 0, nFlags, s), "point sources"));
+            ScatterPoints<<<(static_cast<unsigned>(n) + T - 1) / T, T, 0, s>>>(
+                patchPts.p, patchCells.p, patchFlags.p, patch, ptRow.p, ptCol.p, ptVal.p, nPoints, xDim, yDim);
             CountLaunch();
             HAL_TRY(LaunchStatus("point sources"));
-            HAL_TRY(CudaStatus(cudaMemcpyAsync(patchFlags.p, flags.data(), flags.size(), cudaMemcpyHostToDevice, s),
-                               "point sources"));
-            // the array is complete before the call returns, whichever stream
-            // the ticks are put on later
-            HAL_TRY(CudaStatus(cudaStreamSynchronize(s), "point sources"));
+            patchCount = nPoints;
+            patchPtsDirty = false;
             patchPtsOk = true;
             return HAL_CUDA_OK;
         }
@@ -875,7 +900,11 @@ namespace halcuda
             {
                 HAL_TRY(CombinedSource(extras, &S, s));
             }
-            const bool patched = !blocked && UsePatch(ticks, extras);
+            bool patched = false;
+            if (!blocked)
+            {
+                HAL_TRY(UsePatch(ticks, extras, s, &patched));
+            }
             // launches: two ticks each when blocked (plus one single tick
             // for an odd count), up to the shape's halo when patched; each
             // launch flips the buffers
@@ -1362,7 +1391,9 @@ extern "C" int hal_cuda_diffusion_set_point_sources(hal_cuda_diffusion *h, int32
                                 "cudaMemcpy(points)"));
     h->hasPoints = true;
     h->nPoints = nPoints;
-    return h->SetPatchPoints(nPoints, cells);
+    h->pointCells.assign(cells, cells + nPoints);
+    h->patchPtsDirty = true;
+    return HAL_CUDA_OK;
 }
 
 extern "C" int hal_cuda_diffusion_set_uptake(hal_cuda_diffusion *h, hal_cuda_agents *agents, double uptake)

@@ -119,6 +119,31 @@ namespace halcuda
         return at < most ? at : most;
     }
 
+    // Calls fn(i) for every window (strip) i of n whose patch reads column (row)
+    // c, across a wrapped edge included.  Only the last two are shifted and only
+    // the first and the last read across an edge; the others lie at i * len.
+    template <typename Fn>
+    __host__ __device__ inline void TickPatchReaders(int32_t c, int32_t n, int32_t len, int32_t halo, int32_t dim, Fn fn)
+    {
+        const int32_t lo = (c - halo) / len - 1, hi = (c + halo) / len;
+        for (int32_t k = -3; k <= hi - lo; k++)
+        {
+            // the first, the last two, then the ones about c
+            const int32_t i = k == -3 ? 0 : (k == -2 ? n - 1 : (k == -1 ? n - 2 : lo + k));
+            const bool special = i == 0 || i >= n - 2;
+            if (i < 0 || i >= n || (k >= 0 && special) || (k == -1 && i == 0) || (k == -2 && i == 0))
+            {
+                continue;
+            }
+            const int32_t at = c - (TickPatchStart(i, n, len, halo, dim) - halo);
+            const int32_t span = len + 2 * halo;
+            if ((at >= 0 && at < span) || (at + dim >= 0 && at + dim < span) || (at - dim >= 0 && at - dim < span))
+            {
+                fn(i);
+            }
+        }
+    }
+
     TickPatchShape TickPatchShapeFor(int32_t xDim, int32_t yDim);
     int LaunchTickPatch(const TickPatchShape &shape, TickPatchParams &p, bool adv, cudaStream_t s);
 }
