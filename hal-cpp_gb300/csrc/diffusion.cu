@@ -570,6 +570,9 @@ namespace halcuda
         int32_t patchCount = 0;
         std::vector<int32_t> pointCells;   // the last set_point_sources'
         bool patchPtsDirty = false, patchPtsOk = false;
+        // whether the sources are finite in the columns that the patches beside a
+        // closed y edge read across it
+        bool srcFinite = true, pointsFinite = true;
         // Temporal blocking through shared memory: ticks per launch 1 or 2 (0
         // = automatic, which never takes it).  The two-tick kernel stages
         // tiles with a tensor map per field buffer and reads the dense source
@@ -634,11 +637,32 @@ namespace halcuda
             return tmapOk && ticks >= 2 && blockMode == 2 && agents == nullptr;
         }
 
-        // Several ticks per launch wherever the patch kernel takes the run: it
-        // has no uptake term, and its point sources no repeated cells.
-        int UsePatch(int32_t ticks, bool useExtras, cudaStream_t s, bool *use)
+        // Whether a dense source (host) is finite in the outer columns.
+        bool FiniteAtEdges(const float *dense) const
         {
-            *use = patch.windows > 0 && ticks >= 2 && blockMode == 0 && agents == nullptr;
+            const int32_t halo = std::min(patch.haloCols, yDim);
+            bool finite = true;
+            for (int32_t x = 0; x < xDim; x++)
+            {
+                const float *row = dense + static_cast<int64_t>(x) * yDim;
+                for (int32_t y = 0; y < halo; y++)
+                {
+                    finite = finite && std::isfinite(row[y]) && std::isfinite(row[yDim - 1 - y]);
+                }
+            }
+            return finite;
+        }
+
+        // Several ticks per launch wherever the patch kernel takes the run: it
+        // has no uptake term, and its point sources no repeated cells.  Beside a
+        // closed y edge its patches hold cells that read the opposite edge's
+        // source and multiply it by 0, so that source has to be finite (a choice
+        // in the kernel instead cost registers: 1024^2 with a dense source 1.21
+        // us per tick, with a choice 1.45 to 1.6).
+        int UsePatch(int32_t ticks, bool wrapY, bool useExtras, cudaStream_t s, bool *use)
+        {
+            *use = patch.windows > 0 && ticks >= 2 && blockMode == 0 && agents == nullptr &&
+                   (wrapY || !useExtras || ((!hasSrc || srcFinite) && (!hasPoints || pointsFinite)));
             if (*use && useExtras && hasPoints)
             {
                 HAL_TRY(PatchPoints(s));
@@ -903,7 +927,7 @@ namespace halcuda
             bool patched = false;
             if (!blocked)
             {
-                HAL_TRY(UsePatch(ticks, extras, s, &patched));
+                HAL_TRY(UsePatch(ticks, wrapY, extras, s, &patched));
             }
             // launches: two ticks each when blocked (plus one single tick
             // for an odd count), up to the shape's halo when patched; each
@@ -1327,6 +1351,7 @@ extern "C" int hal_cuda_diffusion_set_source(hal_cuda_diffusion *h, const float 
     HAL_TRY(halcuda::CudaStatus(cudaMemcpy(h->src.p, dense, h->Length() * sizeof(float), cudaMemcpyHostToDevice),
                                 "cudaMemcpy(src)"));
     h->hasSrc = true;
+    h->srcFinite = h->FiniteAtEdges(dense);
     h->combDirty = true;
     h->ResetGraphs();
     return HAL_CUDA_OK;
@@ -1391,6 +1416,7 @@ extern "C" int hal_cuda_diffusion_set_point_sources(hal_cuda_diffusion *h, int32
                                 "cudaMemcpy(points)"));
     h->hasPoints = true;
     h->nPoints = nPoints;
+    h->pointsFinite = std::all_of(values, values + nPoints, [](float v) { return std::isfinite(v); });
     h->pointCells.assign(cells, cells + nPoints);
     h->patchPtsDirty = true;
     return HAL_CUDA_OK;
