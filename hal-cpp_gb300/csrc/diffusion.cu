@@ -571,8 +571,9 @@ namespace halcuda
         std::vector<int32_t> pointCells;   // the last set_point_sources'
         bool patchPtsDirty = false, patchPtsOk = false;
         // whether the sources are finite in the columns that the patches beside a
-        // closed y edge read across it
-        bool srcFinite = true, pointsFinite = true;
+        // closed y edge read across it, and the boundary values of the y edges
+        // (differences of theirs included)
+        bool srcFinite = true, pointsFinite = true, ghostFinite = true;
         // Temporal blocking through shared memory: ticks per launch 1 or 2 (0
         // = automatic, which never takes it).  The two-tick kernel stages
         // tiles with a tensor map per field buffer and reads the dense source
@@ -658,11 +659,13 @@ namespace halcuda
         // closed y edge its patches hold cells that read the opposite edge's
         // source and multiply it by 0, so that source has to be finite (a choice
         // in the kernel instead cost registers: 1024^2 with a dense source 1.21
-        // us per tick, with a choice 1.45 to 1.6).
+        // us per tick, with a choice 1.45 to 1.6).  The cells that hold boundary
+        // values have differences with one another, also multiplied by 0.
         int UsePatch(int32_t ticks, bool wrapY, bool useExtras, cudaStream_t s, bool *use)
         {
             *use = patch.windows > 0 && ticks >= 2 && blockMode == 0 && agents == nullptr &&
-                   (wrapY || !useExtras || ((!hasSrc || srcFinite) && (!hasPoints || pointsFinite)));
+                   (wrapY || !useExtras ||
+                    ((!hasSrc || srcFinite) && (!hasPoints || pointsFinite) && (!hasGhost || ghostFinite)));
             if (*use && useExtras && hasPoints)
             {
                 HAL_TRY(PatchPoints(s));
@@ -1499,6 +1502,8 @@ extern "C" int hal_cuda_diffusion_set_dirichlet(hal_cuda_diffusion *h, const flo
     HAL_TRY(halcuda::CudaStatus(cudaMemcpy(h->ghost.p, ghost, ng * sizeof(float), cudaMemcpyHostToDevice),
                                 "cudaMemcpy(ghost)"));
     h->hasGhost = true;
+    h->ghostFinite = std::all_of(ghost + 2 * static_cast<size_t>(h->yDim), ghost + ng,
+                                 [](float v) { return std::fabs(v) <= 0x1p120f; });
     return HAL_CUDA_OK;
 }
 
