@@ -89,29 +89,24 @@ namespace halcuda
 
         // V values of a lane at q (consecutive columns, 4 * V-byte aligned
         // when VEC), or one by one at q[col[k]].
-        template <int V, bool VEC>
+        // FIELD: what the launch before may have written, through the L2 (the
+        // read-only path is for data that no kernel in flight writes).
+        template <int V, bool VEC, bool FIELD>
         __device__ __forceinline__ void LoadCells(const float *__restrict__ q, const int32_t (&col)[V], float (&v)[V])
         {
             if constexpr (VEC && V == 2)
             {
-                const float2 t = __ldg(reinterpret_cast<const float2 *>(q + col[0]));
+                const float2 *at = reinterpret_cast<const float2 *>(q + col[0]);
+                const float2 t = FIELD ? __ldcg(at) : __ldg(at);
                 v[0] = t.x;
                 v[1] = t.y;
-            }
-            else if constexpr (VEC && V == 4)
-            {
-                const float4 t = __ldg(reinterpret_cast<const float4 *>(q + col[0]));
-                v[0] = t.x;
-                v[1] = t.y;
-                v[2] = t.z;
-                v[3] = t.w;
             }
             else
             {
 #pragma unroll
                 for (int k = 0; k < V; k++)
                 {
-                    v[k] = __ldg(q + col[k]);
+                    v[k] = FIELD ? __ldcg(q + col[k]) : __ldg(q + col[k]);
                 }
             }
         }
@@ -163,8 +158,8 @@ namespace halcuda
 #pragma unroll
                 for (int i = 0; i < N; i++)
                 {
-                    LoadCells<V, VEC>(rowOf(p.f, i), col, lo[i]);
-                    LoadCells<V, VEC>(rowOf(p.f, i + N), col, hi[i]);
+                    LoadCells<V, VEC, true>(rowOf(p.f, i), col, lo[i]);
+                    LoadCells<V, VEC, true>(rowOf(p.f, i + N), col, hi[i]);
                 }
 #pragma unroll
                 for (int i = 0; i < N; i++)
@@ -186,8 +181,8 @@ namespace halcuda
                 for (int i = 0; i < N; i++)
                 {
                     float lo[V], hi[V];
-                    LoadCells<V, VEC>(rowOf(sA, i), col, lo);
-                    LoadCells<V, VEC>(rowOf(sA, i + N), col, hi);
+                    LoadCells<V, VEC, false>(rowOf(sA, i), col, lo);
+                    LoadCells<V, VEC, false>(rowOf(sA, i + N), col, hi);
 #pragma unroll
                     for (int k = 0; k < V; k++)
                     {
@@ -320,8 +315,8 @@ namespace halcuda
                     float bLo[V], bHi[V];
                     if constexpr (SRC > 1)
                     {
-                        LoadCells<V, VEC>(rowOf(sB, i), col, bLo);
-                        LoadCells<V, VEC>(rowOf(sB, i + N), col, bHi);
+                        LoadCells<V, VEC, false>(rowOf(sB, i), col, bLo);
+                        LoadCells<V, VEC, false>(rowOf(sB, i + N), col, bHi);
                     }
 #pragma unroll
                     for (int k = 0; k < V; k++)
@@ -375,10 +370,6 @@ namespace halcuda
                 if constexpr (VEC && V == 2)
                 {
                     *reinterpret_cast<float2 *>(q) = make_float2(v[0], v[1]);
-                }
-                else if constexpr (VEC && V == 4)
-                {
-                    *reinterpret_cast<float4 *>(q) = make_float4(v[0], v[1], v[2], v[3]);
                 }
                 else
                 {
