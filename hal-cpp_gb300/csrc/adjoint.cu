@@ -476,13 +476,75 @@ namespace halcuda
             }
         }
 
-        // Sums of two floats (or a product) and their rounding errors.
-        __device__ __forceinline__ void AddTwo(float &hi, float &lo, float x)
+        // s + x and its rounding error (Knuth's two-sum).
+        __device__ __forceinline__ float TwoSum(float &s, float x)
         {
-            const float s = __fadd_rn(hi, x);
-            const float b = __fsub_rn(s, hi);
-            lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
-            hi = s;
+            const float t = __fadd_rn(s, x);
+            const float b = __fsub_rn(t, s);
+            const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b));
+            s = t;
+            return e;
+        }
+
+        // The power of two, as its exponent, that brings the largest of |v| into
+        // [1, 2) (or next to it at the ends of the range).
+        template <int M>
+        __device__ __forceinline__ int Exponent(const float (&v)[M], bool &finite)
+        {
+            float m = 0.0f;
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                m = fmaxf(m, fabsf(v[i]));
+                finite = finite && v[i] == v[i];  // (fmaxf leaves NaN out)
+            }
+            const int e = static_cast<int>(__float_as_uint(m) >> 23);
+            finite = finite && e < 255;
+            return min(max(e, 1), 253) - 127;
+        }
+
+        // sum - <g, f> over a lane's positions.  An FP64 instruction holds its
+        // pipe for 64 cycles, conversions included: M products summed in FP64 made
+        // a step of a 300 x 700 gradient 2.5 us longer.  Here the operands are
+        // scaled by powers of two so that no product leaves FP32's range, each
+        // product is a pair of floats and the sum three, all without error but
+        // the third's (2^-72 of the largest term), and only their total is added
+        // in FP64: fewer roundings than a sum in FP64 throughout.
+        template <int M>
+        __device__ __forceinline__ double SubDot(double sum, const float (&g)[M], const float (&f)[M])
+        {
+            bool finite = true;
+            const int eg = Exponent<M>(g, finite), ef = Exponent<M>(f, finite);
+            if (!finite)
+            {
+#pragma unroll 1
+                for (int i = 0; i < M; i++)
+                {
+                    float a = 0.0f, b = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < M; k++)
+                    {
+                        a = (k == i) ? g[k] : a;
+                        b = (k == i) ? f[k] : b;
+                    }
+                    sum = fma(-static_cast<double>(a), static_cast<double>(b), sum);
+                }
+                return sum;
+            }
+            const float kg = __uint_as_float(static_cast<uint32_t>(127 - eg) << 23);
+            const float kf = __uint_as_float(static_cast<uint32_t>(127 - ef) << 23);
+            float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
+#pragma unroll
+            for (int i = 0; i < M; i++)
+            {
+                const float a = __fmul_rn(g[i], kg), b = __fmul_rn(f[i], kf);
+                const float p = __fmul_rn(a, b);
+                const float e = TwoSum(s0, p);
+                s2 = __fadd_rn(s2, TwoSum(s1, __fmaf_rn(a, b, -p)));
+                s2 = __fadd_rn(s2, TwoSum(s1, e));
+            }
+            const double t = (static_cast<double>(s2) + static_cast<double>(s1)) + static_cast<double>(s0);
+            return fma(-t, __hiloint2double((1023 + eg + ef) << 20, 0), sum);
         }
 
         enum BwdYMode : int
@@ -493,21 +555,21 @@ namespace halcuda
         };
 
         // Backward along y for step t: [gbar from step t+1] then the y-solve.
-        // All arrays by y, but b2bar, which leaves by x.  ddecay's sum goes to
-        // one float pair (sum, its rounding) per lane and line: FP32 pairs
-        // hold the exact products and the sum to 2^-48, without the FP64
-        // instructions that would stand on the step's critical path.
+        // All arrays by y, but b2bar, which leaves by x.  ddecay's sum is FP64,
+        // one per lane and line.  A step's term, -<gbar of t, f_t>, is added by
+        // the launch of step t-1 (the tail for step 0), whose gPrev and fNext are
+        // its factors and are loaded before the wait: the sum may run while the
+        // kernel before does, off the step's critical path.
         template <int M>
         __global__ void __launch_bounds__(32 * kAdjLines)
             BwdY(Axis ax, int mode, const float *__restrict__ par,
                  const float *__restrict__ b1bar,  // step t+1's x-solve adjoint (kBwdNext/Tail)
                  const float *__restrict__ gPrev,  // adjoint of f_t+2 (kBwdNext/Tail), or gbar (kBwdFirst)
                  const float *__restrict__ fNext,  // f_t+1 (kBwdNext/Tail)
-                 const float *__restrict__ fT,     // f_t (input of step t)
                  const float *__restrict__ vT,     // v_t
                  float *__restrict__ gOut,         // adjoint of f_t+1 (gbar of step t)
                  float *__restrict__ b2bar, float *__restrict__ dD, float *__restrict__ dS,
-                 float2 *__restrict__ dDecay)
+                 double *__restrict__ dDecay)
         {
             __shared__ __align__(16) float tile[kAdjLines][32 * (M + 4)];
             const int lane = threadIdx.x & 31;
@@ -529,6 +591,11 @@ namespace halcuda
             for (int i = 0; i < M; i++)
             {
                 acc[i] = 0.0f;
+            }
+            if (mode != kBwdFirst && live)
+            {
+                double *at = dDecay + static_cast<int64_t>(line) * 32 + lane;
+                *at = SubDot<M>(__ldcg(at), g, q);
             }
             WaitForPredecessor();
             if (mode != kBwdFirst)
@@ -562,12 +629,10 @@ namespace halcuda
             Solve<M>(ax, k, line, lane, d);
             // the accumulators' rows, in flight during the write-out (the
             // factors' registers are free now)
-            float sD[M], sS[M], ft[M];
+            float sD[M], sS[M];
             LoadRow<M>(vT + row, ax.ld, lane, q);
             LoadRow<M>(dD + row, ax.ld, lane, sD);
             LoadRow<M>(dS + row, ax.ld, lane, sS);
-            LoadRow<M>(fT + row, ax.ld, lane, ft);
-            float2 sum = __ldcg(dDecay + static_cast<int64_t>(line) * 32 + lane);
 #pragma unroll
             for (int i = 0; i < M; i++)
             {
@@ -585,17 +650,9 @@ namespace halcuda
             {
                 sD[i] += acc[i];
                 sS[i] += g[i];
-                const float p = __fmul_rn(-g[i], ft[i]);
-                const float pe = __fmaf_rn(-g[i], ft[i], -p);
-                AddTwo(sum.x, sum.y, p);
-                sum.y = __fadd_rn(sum.y, pe);
             }
             StoreRow<M>(dD + row, ax.ld, lane, sD);
             StoreRow<M>(dS + row, ax.ld, lane, sS);
-            const float s = __fadd_rn(sum.x, sum.y);
-            sum.y = __fsub_rn(sum.y, __fsub_rn(s, sum.x));
-            sum.x = s;
-            dDecay[static_cast<int64_t>(line) * 32 + lane] = sum;
         }
 
         // Backward along x for step t: wbar = (I + Lx/2) b2bar, b1bar = (I - Lx/2)^-1 wbar.
@@ -903,10 +960,9 @@ namespace halcuda
             }
         }
 
-        // acc[0] = sum of part; acc[1] = sum of the pairs (one CTA, a fixed
-        // order).
+        // acc[0] = sum of part; acc[1] = sum of dDecay (one CTA, a fixed order).
         __global__ void __launch_bounds__(1024)
-            Totals(const double *__restrict__ part, int32_t nPart, const float2 *__restrict__ pairs, int64_t nPairs,
+            Totals(const double *__restrict__ part, int32_t nPart, const double *__restrict__ dDecay, int64_t nDecay,
                    double *__restrict__ acc)
         {
             __shared__ double sred[32];
@@ -915,9 +971,9 @@ namespace halcuda
             {
                 a += part[i];
             }
-            for (int64_t i = threadIdx.x; i < nPairs; i += blockDim.x)
+            for (int64_t i = threadIdx.x; i < nDecay; i += blockDim.x)
             {
-                b += static_cast<double>(pairs[i].x) + static_cast<double>(pairs[i].y);
+                b += dDecay[i];
             }
             a = BlockSum(a, sred);
             b = BlockSum(b, sred);
@@ -1027,7 +1083,7 @@ namespace halcuda
         StreamSlot recomputeStream;         // recomputes segment s-1 while segment s is differentiated
         DevBuf<float> coefX, extX, coefY, extY;
         DevBuf<float> par;                  // decay, -decay
-        DevBuf<float2> dDecay;              // BwdY's sums
+        DevBuf<double> dDecay;              // BwdY's sums
         DevBuf<double> part, acc;           // the loss's partial sums; [0] loss, [1] d loss / d decay
         float msForward = 0.0f, msGradient = 0.0f;
         // runs of steps as graphs (the pointers are the problem's): see Replay
@@ -1141,12 +1197,12 @@ namespace halcuda
             return HAL_CUDA_OK;
         }
 
-        int LaunchBwdY(int mode, const float *gPrev, const float *fNext, const float *fT, const float *vT, float *gOut,
-                       bool chained, cudaStream_t s)
+        int LaunchBwdY(int mode, const float *gPrev, const float *fNext, const float *vT, float *gOut, bool chained,
+                       cudaStream_t s)
         {
             CountLaunch();
             return WithLaneLen(LaneLen(yDim), [&](auto m) {
-                return LaunchChained(BwdY<m()>, xDim, chained, s, axY, mode, par.p, b1.p, gPrev, fNext, fT, vT, gOut,
+                return LaunchChained(BwdY<m()>, xDim, chained, s, axY, mode, par.p, b1.p, gPrev, fNext, vT, gOut,
                                      b2.p, dD.p, dS.p, dDecay.p);
             });
         }
@@ -1245,7 +1301,7 @@ namespace halcuda
                     float *gn = cur == 0 ? gB.p : gA.p;
                     const bool lead = i == count - 1;
                     HAL_TRY(LaunchBwdY(first && lead ? kBwdFirst : kBwdNext, gc, segF[b].p + (k + 1) * nA,
-                                       segF[b].p + k * nA, segV[b].p + k * nA, gn, !lead, t));
+                                       segV[b].p + k * nA, gn, !lead, t));
                     HAL_TRY(LaunchBwdX(segW[b].p + k * nB, t));
                     cur ^= 1;
                 }
@@ -1475,7 +1531,7 @@ namespace halcuda
             HAL_TRY(CudaStatus(cudaMemsetAsync(dD.p, 0, nA * sizeof(float), s), "cudaMemset(dD)"));
             HAL_TRY(CudaStatus(cudaMemsetAsync(dDT.p, 0, nB * sizeof(float), s), "cudaMemset(dD)"));
             HAL_TRY(CudaStatus(cudaMemsetAsync(dS.p, 0, nA * sizeof(float), s), "cudaMemset(dS)"));
-            HAL_TRY(CudaStatus(cudaMemsetAsync(dDecay.p, 0, static_cast<size_t>(xDim) * 32 * sizeof(float2), s),
+            HAL_TRY(CudaStatus(cudaMemsetAsync(dDecay.p, 0, static_cast<size_t>(xDim) * 32 * sizeof(double), s),
                                "cudaMemset(dDecay)"));
             const float *srcp = useSrc ? src.p : nullptr;
             int g = 0;
@@ -1491,8 +1547,8 @@ namespace halcuda
             {
                 // the y-stencil part of step 0's (I + Ly/2) b1bar: its D terms
                 // (buffer 0 holds segment 0's states)
-                HAL_TRY(LaunchBwdY(kBwdTail, g == 0 ? gA.p : gB.p, segF[0].p, segF[0].p, segV[0].p,
-                                   g == 0 ? gB.p : gA.p, false, s));
+                HAL_TRY(LaunchBwdY(kBwdTail, g == 0 ? gA.p : gB.p, segF[0].p, segV[0].p, g == 0 ? gB.p : gA.p, false,
+                                   s));
             }
             // the x-faces' part of dL/dD
             TransposeRows<true><<<dim3((yDim + 31) / 32, (xDim + 31) / 32), dim3(32, 8), 0, s>>>(dDT.p, ldX, dD.p, ldY,
