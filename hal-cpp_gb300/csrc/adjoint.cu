@@ -1087,7 +1087,7 @@ namespace halcuda
         DevBuf<double> part, acc;           // the loss's partial sums; [0] loss, [1] d loss / d decay
         float msForward = 0.0f, msGradient = 0.0f;
         // runs of steps as graphs (the pointers are the problem's): see Replay
-        std::map<std::string, std::pair<cudaGraphExec_t, int64_t>> graphs;
+        std::map<std::string, cudaGraphExec_t> graphs;
 
         ~Adjoint() { DropGraphs(); }
 
@@ -1095,7 +1095,7 @@ namespace halcuda
         {
             for (auto &g : graphs)
             {
-                cudaGraphExecDestroy(g.second.first);
+                cudaGraphExecDestroy(g.second);
             }
             graphs.clear();
         }
@@ -1215,22 +1215,23 @@ namespace halcuda
             });
         }
 
-        // Enqueues on s what `body(s)` enqueues, replayed from a graph of that
-        // key: a launch of a run of steps instead of one per kernel.
+        // Enqueues on s what `body(s)` enqueues (`kernels` of them), replayed from
+        // a graph of that key: a launch of a run of steps instead of one per
+        // kernel.
         template <typename Body>
-        int Replay(const std::string &key, cudaStream_t s, Body body)
+        int Replay(const std::string &key, int64_t kernels, cudaStream_t s, Body body)
         {
             auto it = graphs.find(key);
             if (it == graphs.end())
             {
-                const int64_t before = g_launches.load();
                 HAL_TRY(CudaStatus(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture"));
                 const int rc = body(s);
                 cudaGraph_t g = nullptr;
                 const cudaError_t e = cudaStreamEndCapture(s, &g);
-                // counted again by each replay
-                const int64_t count = g_launches.load() - before;
-                CountLaunch(-count);
+                if (rc == HAL_CUDA_OK)
+                {
+                    CountLaunch(-kernels);  // counted by each replay
+                }
                 if (rc != HAL_CUDA_OK || e != cudaSuccess)
                 {
                     if (g != nullptr)
@@ -1243,10 +1244,10 @@ namespace halcuda
                 const cudaError_t ei = cudaGraphInstantiate(&x, g, 0);
                 cudaGraphDestroy(g);
                 HAL_TRY(CudaStatus(ei, "cudaGraphInstantiate"));
-                it = graphs.emplace(key, std::make_pair(x, count)).first;
+                it = graphs.emplace(key, x).first;
             }
-            CountLaunch(it->second.second);
-            return CudaStatus(cudaGraphLaunch(it->second.first, s), "cudaGraphLaunch");
+            CountLaunch(kernels);
+            return CudaStatus(cudaGraphLaunch(it->second, s), "cudaGraphLaunch");
         }
 
         // `count` steps between the work fields, from work[c]; returns the
@@ -1265,7 +1266,7 @@ namespace halcuda
                 }
                 return static_cast<int>(HAL_CUDA_OK);
             };
-            return Run("F" + std::to_string(c0) + "." + std::to_string(count) + (srcp ? "s" : ""), count, s, body);
+            return Run("F" + std::to_string(c0) + "." + std::to_string(count) + (srcp ? "s" : ""), count, count, s, body);
         }
 
         // The states of `count` steps in buffer b, from its first field (fB
@@ -1282,7 +1283,7 @@ namespace halcuda
                 }
                 return static_cast<int>(HAL_CUDA_OK);
             };
-            return Run("S" + std::to_string(b) + "." + std::to_string(count) + (srcp ? "s" : ""), count, s, body);
+            return Run("S" + std::to_string(b) + "." + std::to_string(count) + (srcp ? "s" : ""), count, count, s, body);
         }
 
         // Reverse steps over the `count` states in buffer b; g: the index of
@@ -1309,20 +1310,21 @@ namespace halcuda
             };
             return Run("B" + std::to_string(b) + "." + std::to_string(g0) + "." + std::to_string(count) +
                            (first ? "f" : ""),
-                       first ? steps : count, s, body);
+                       first ? steps : count, count, s, body);
         }
 
-        // A run of steps: whole segments from a graph; runs that occur once in
+        // A run of steps of two kernels each: whole segments (`repeated` as long
+        // as a run that the call repeats) from a graph; runs that occur once in
         // a call (every state kept, the last segment) launch by launch, which
         // takes the host less than capturing them.
         template <typename Body>
-        int Run(const std::string &key, int32_t count, cudaStream_t s, Body body)
+        int Run(const std::string &key, int32_t repeated, int32_t count, cudaStream_t s, Body body)
         {
-            if (count != Chunk())
+            if (repeated != Chunk())
             {
                 return body(s);
             }
-            return Replay(key, s, body);
+            return Replay(key, 2 * static_cast<int64_t>(count), s, body);
         }
 
         // Steps of a run that a call repeats.
