@@ -715,8 +715,25 @@ namespace halcuda
 
         // ---- the factors -----------------------------------------------------
 
+        // 1 / b by Newton's iteration from the hardware's approximation (20
+        // bits, then 40, then all but the last rounding), for finite b >= 1 and
+        // thereabouts.  An IEEE division is three times as long a chain of FP64
+        // instructions, and the factors leave in FP32.
+        __device__ __forceinline__ double Reciprocal(double b)
+        {
+            double y;
+            asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+            y = fma(fma(-b, y, 1.0), y, y);
+            return fma(fma(-b, y, 1.0), y, y);
+        }
+
         // Factors every line of an axis (one warp a line, FP64): see the top of
-        // this file.  Positions beyond the line are rows of the identity.
+        // this file.  Positions beyond the line are rows of the identity.  Bound
+        // by its chains of FP64 instructions, 64 cycles and more each: us per
+        // axis of 64^2 / 512^2 / 1024^2 with IEEE divisions 19 / 29 / 80, so 11 /
+        // 23 / 63, and the axes run side by side.  (A call of one step still pays
+        // more for its factors than it gains: forward 64^2 77 us against 54 with
+        // the reductions, even from some 8 steps on; gradients from 2 or 3.)
         template <int M>
         __global__ void __launch_bounds__(32 * kAdjLines) Factor(Axis ax, float *__restrict__ coef, float *__restrict__ ext)
         {
@@ -733,48 +750,49 @@ namespace halcuda
             // split as T + u v^T
             const bool split = ax.wrap && n >= 3;
             const double eW = split ? static_cast<double>(D[n - 1]) : 0.0;
-            auto face = [&](int32_t j)  // face (j, j+1) within the line
+            // a face's coefficient -D/2 is exact in FP32 (but for the sum of a
+            // wrapped pair's two faces)
+            auto half = [&](int32_t j)  // -1/2 of face (j, j+1) within the line
             {
                 if (j < 0 || j >= n - 1)
                 {
                     return 0.0;
                 }
-                return static_cast<double>(D[j]) + ((ax.wrap && n == 2) ? static_cast<double>(D[1]) : 0.0);
+                const double h = static_cast<double>(-0.5f * D[j]);
+                return (ax.wrap && n == 2) ? h - 0.5 * static_cast<double>(D[1]) : h;
             };
             const double a0 = -0.5 * eW;  // row 0's coefficient of x_n-1, and row n-1's of x_0
-            const double gamma = -(1.0 + 0.5 * (eW + face(0)));
+            const double gamma = -(1.0 - a0 - half(0));
             double a[M], b[M], c[M];
+            double before = half(lane * M - 1);
 #pragma unroll
             for (int i = 0; i < M; i++)
             {
                 const int32_t j = lane * M + i;
-                const double lo = face(j - 1), hi = face(j);
-                a[i] = (j < n) ? -0.5 * lo : 0.0;
-                c[i] = (j < n) ? -0.5 * hi : 0.0;
-                b[i] = 1.0;
-                if (j < n)
+                const double here = half(j);
+                a[i] = (j < n) ? before : 0.0;
+                c[i] = here;
+                b[i] = 1.0 - (a[i] + c[i]);
+                if (split && j == 0)
                 {
-                    b[i] = 1.0 + 0.5 * (lo + hi + ((j == 0 || j == n - 1) ? eW : 0.0));
-                    if (split && j == 0)
-                    {
-                        b[i] -= gamma;
-                    }
-                    if (split && j == n - 1)
-                    {
-                        b[i] -= a0 * a0 / gamma;
-                    }
+                    b[i] = b[i] - a0 - gamma;
                 }
+                if (split && j == n - 1)
+                {
+                    b[i] = b[i] - a0 - a0 * a0 / gamma;
+                }
+                before = here;
             }
             double fw[M], ib[M], cb[M], p[M], q[M];
             double bp = b[0];
             fw[0] = 0.0;
-            ib[0] = 1.0 / bp;
+            ib[0] = Reciprocal(bp);
 #pragma unroll
             for (int i = 1; i < M - 1; i++)
             {
                 fw[i] = a[i] * ib[i - 1];
                 bp = b[i] - fw[i] * c[i - 1];
-                ib[i] = 1.0 / bp;
+                ib[i] = Reciprocal(bp);
             }
 #pragma unroll
             for (int i = 0; i < M - 1; i++)
@@ -810,13 +828,13 @@ namespace halcuda
                              cl = __shfl_up_sync(kAll, C, s);
                 const double ar = __shfl_down_sync(kAll, A, s), br = __shfl_down_sync(kAll, B, s),
                              cr = __shfl_down_sync(kAll, C, s);
-                lo[t] = lane >= s ? -A / bl : 0.0;
-                hi[t] = lane + s < 32 ? -C / br : 0.0;
+                lo[t] = lane >= s ? -A * Reciprocal(bl) : 0.0;
+                hi[t] = lane + s < 32 ? -C * Reciprocal(br) : 0.0;
                 B += (lane >= s ? lo[t] * cl : 0.0) + (lane + s < 32 ? hi[t] * ar : 0.0);
                 A = lane >= s ? lo[t] * al : 0.0;
                 C = lane + s < 32 ? hi[t] * cr : 0.0;
             }
-            const double binv = 1.0 / B;
+            const double binv = Reciprocal(B);
             const int nc = ax.wrap ? 6 : 5;
             float *o = coef + static_cast<int64_t>(line) * nc * M * 32 + 4 * lane;
             auto put = [&](int k, const double (&v)[M])
@@ -885,11 +903,11 @@ namespace halcuda
                         zn = (lane * M + i == n - 1) ? z[i] : zn;
                     }
                     zn = __shfl_sync(kAll, zn, (n - 1) / M);
-                    const double den = 1.0 + __shfl_sync(kAll, z[0], 0) + bog * zn;
+                    const double inv = 1.0 / (1.0 + __shfl_sync(kAll, z[0], 0) + bog * zn);
 #pragma unroll
                     for (int i = 0; i < M; i++)
                     {
-                        z[i] /= den;
+                        z[i] *= inv;
                     }
                 }
                 put(kCoefZ, z);
@@ -961,7 +979,9 @@ namespace halcuda
         }
 
         // acc[0] = sum of part; acc[1] = sum of dDecay (one CTA, a fixed order).
-        __global__ void __launch_bounds__(1024)
+        constexpr int kTotalThreads = 256;
+
+        __global__ void __launch_bounds__(kTotalThreads)
             Totals(const double *__restrict__ part, int32_t nPart, const double *__restrict__ dDecay, int64_t nDecay,
                    double *__restrict__ acc)
         {
@@ -976,7 +996,7 @@ namespace halcuda
                 b += dDecay[i];
             }
             a = BlockSum(a, sred);
-            b = BlockSum(b, sred);
+            b = nDecay > 0 ? BlockSum(b, sred) : 0.0;
             if (threadIdx.x == 0)
             {
                 acc[0] = a;
@@ -1089,7 +1109,16 @@ namespace halcuda
         // runs of steps as graphs (the pointers are the problem's): see Replay
         std::map<std::string, cudaGraphExec_t> graphs;
 
-        ~Adjoint() { DropGraphs(); }
+        cudaEvent_t factored = nullptr;     // the y-lines' factors, made on recomputeStream
+
+        ~Adjoint()
+        {
+            DropGraphs();
+            if (factored != nullptr)
+            {
+                cudaEventDestroy(factored);
+            }
+        }
 
         void DropGraphs()
         {
@@ -1116,6 +1145,7 @@ namespace halcuda
             HAL_TRY(CudaStatus(cudaDeviceGetStreamPriorityRange(&least, &greatest), "cudaDeviceGetStreamPriorityRange"));
             HAL_TRY(stream.Create("cudaStreamCreate", greatest));
             HAL_TRY(recomputeStream.Create("cudaStreamCreate", least));
+            HAL_TRY(CudaStatus(cudaEventCreateWithFlags(&factored, cudaEventDisableTiming), "cudaEventCreate"));
             xDim = xd;
             yDim = yd;
             ldX = (xDim + 3) & ~3;
@@ -1153,14 +1183,23 @@ namespace halcuda
         }
 
         // Host arrays (xDim x yDim) to and from the padded "by y" layout.
+        // (as one run of bytes where nothing is padded)
         int ToDevice(float *d, const float *h, cudaStream_t s, const char *what) const
         {
+            if (ldY == yDim)
+            {
+                return CudaStatus(cudaMemcpyAsync(d, h, nA * sizeof(float), cudaMemcpyHostToDevice, s), what);
+            }
             return CudaStatus(cudaMemcpy2DAsync(d, ldY * sizeof(float), h, yDim * sizeof(float), yDim * sizeof(float),
                                                 static_cast<size_t>(xDim), cudaMemcpyHostToDevice, s), what);
         }
 
         int ToHost(float *h, const float *d, cudaStream_t s, const char *what) const
         {
+            if (ldY == yDim)
+            {
+                return CudaStatus(cudaMemcpyAsync(h, d, nA * sizeof(float), cudaMemcpyDeviceToHost, s), what);
+            }
             return CudaStatus(cudaMemcpy2DAsync(h, yDim * sizeof(float), d, ldY * sizeof(float), yDim * sizeof(float),
                                                 static_cast<size_t>(xDim), cudaMemcpyDeviceToHost, s), what);
         }
@@ -1347,12 +1386,21 @@ namespace halcuda
             const float hp[2] = {static_cast<float>(decay), static_cast<float>(-decay)};
             HAL_TRY(CudaStatus(cudaMemcpyAsync(par.p, hp, sizeof(hp), cudaMemcpyHostToDevice, s), "cudaMemcpy(decay)"));
             HAL_TRY(CudaStatus(cudaEventRecord(begin, s), "cudaEventRecord"));
+            if (steps == 0)
+            {
+                return HAL_CUDA_OK;
+            }
+            // the axes side by side
+            cudaStream_t rs = recomputeStream.Get();
+            HAL_TRY(CudaStatus(cudaStreamWaitEvent(rs, begin, 0), "cudaStreamWaitEvent"));
+            HAL_TRY(WithLaneLen(LaneLen(yDim), [&](auto m) {
+                return LaunchChained(Factor<m()>, xDim, false, rs, axY, coefY.p, extY.p);
+            }));
+            HAL_TRY(CudaStatus(cudaEventRecord(factored, rs), "cudaEventRecord"));
             HAL_TRY(WithLaneLen(LaneLen(xDim), [&](auto m) {
                 return LaunchChained(Factor<m()>, yDim, false, s, axX, coefX.p, extX.p);
             }));
-            HAL_TRY(WithLaneLen(LaneLen(yDim), [&](auto m) {
-                return LaunchChained(Factor<m()>, xDim, false, s, axY, coefY.p, extY.p);
-            }));
+            HAL_TRY(CudaStatus(cudaStreamWaitEvent(s, factored, 0), "cudaStreamWaitEvent"));
             CountLaunch(2);
             return HAL_CUDA_OK;
         }
@@ -1373,7 +1421,7 @@ namespace halcuda
 
         int LaunchTotals(bool decayToo, cudaStream_t s)
         {
-            Totals<<<1, 1024, 0, s>>>(part.p, LossParts(), dDecay.p, decayToo ? static_cast<int64_t>(xDim) * 32 : 0,
+            Totals<<<1, kTotalThreads, 0, s>>>(part.p, LossParts(), dDecay.p, decayToo ? static_cast<int64_t>(xDim) * 32 : 0,
                                       acc.p);
             CountLaunch();
             return LaunchStatus("adjoint totals");
