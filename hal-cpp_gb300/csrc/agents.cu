@@ -1393,12 +1393,16 @@ namespace halcuda
         // 8360 / 1480; 5k in 100 x 77 207 / 67; 200k in 1024^2 453 / 283 with a
         // cluster, 253 / 211 uniform; 20k in 256^2 at R = 2 632 / 180.  One agent
         // a group throughout: 200k uniform 288; up to eight from 20k on: 50k 198,
-        // 200k with a cluster 359.
+        // 200k with a cluster 359.  Two agents a group already from kPairSparse on
+        // where a window holds fewer than two of a uniform population: 50k uniform
+        // in 512^2, wrapped, 111 with a thread per agent, 120 with one agent a
+        // group, 106 with two (a cluster clipped at a corner 348 / 161 / 169).
         constexpr int kPairQueue = 32;  // pairs an agent's queue holds (a power of two)
         constexpr int kPairDrain = 16;  // a queue this long is worked off
         constexpr int kPairThreads = 32;
         constexpr int32_t kPairGroups = 152 * 256;  // groups that fill the chip
         constexpr int32_t kPairPerGroup = 4;        // agents a group takes, one after another, at most
+        constexpr int32_t kPairSparse = 40000;
 
         // The FP32 value nearest towards zero of v, by its bits: zero below the
         // normal range, NaN for what FP32 cannot hold (and for NaN itself).
@@ -1888,6 +1892,12 @@ namespace halcuda
         return r >= 0.0 && r <= 0x1p20 && r == std::floor(r);
     }
 
+    // The agents of a uniform population that a window holds.
+    inline double WindowAgents(int32_t n, int64_t cells, double R)
+    {
+        return static_cast<double>(n) / static_cast<double>(cells) * (2.0 * R + 1.0) * (2.0 * R + 1.0);
+    }
+
     // Whether a force pass (step: with the move) takes a group of lanes per
     // agent.  A thread per agent costs the longest window's chain, a group its
     // instructions, n times: the group pays while the windows are long for the
@@ -1913,7 +1923,7 @@ namespace halcuda
     // 22.0, group 23.4; with a cluster 43.8, 32.3 and 26.5).
     inline bool GroupPerAgent(int32_t n, int64_t cells, double R, bool walls, bool step)
     {
-        const double m = static_cast<double>(n) / static_cast<double>(cells) * (2.0 * R + 1.0) * (2.0 * R + 1.0);
+        const double m = WindowAgents(n, cells, R);
         if (R >= 2.0)
         {
             const int32_t most = (R >= 3.0 || !walls) ? 100000 : (step ? 70000 : 60000);
@@ -2134,12 +2144,26 @@ namespace halcuda
                 }
                 if constexpr (std::is_same<T, double>::value && std::is_same<TV, double>::value)
                 {
-                    const int32_t perGroup = std::min(std::max(n / kPairGroups, 1), kPairPerGroup);
+                    // (few agents a window: kPairSparse; and chained, 2 to 9 us of
+                    // 100, since no CTA's work is long enough to gather on an SM)
+                    const bool sparse = WindowAgents(n, C, R) < 2.0;
+                    const int32_t least = sparse && n >= kPairSparse ? 2 : 1;
+                    const int32_t perGroup = std::min(std::max(n / kPairGroups, least), kPairPerGroup);
                     const int64_t groups = (static_cast<int64_t>(n) + perGroup - 1) / perGroup;
-                    LaunchAfter(!wrapX && !wrapY ? ForcesGroup64<true> : ForcesGroup64<false>,
-                                  static_cast<unsigned>((groups * kGroupLanes + kPairThreads - 1) / kPairThreads), kPairThreads,
-                                  s, bucket.p, offsets.p, SortedPosBuf(T()), sRad, n, perGroup, R + 0.0, lp, xDim, yDim,
-                                  static_cast<int32_t>(wrapX), static_cast<int32_t>(wrapY), vel, velIn);
+                    const auto launch = [&](auto start) {
+                        start(!wrapX && !wrapY ? ForcesGroup64<true> : ForcesGroup64<false>,
+                              static_cast<unsigned>((groups * kGroupLanes + kPairThreads - 1) / kPairThreads),
+                              kPairThreads, s, bucket.p, offsets.p, SortedPosBuf(T()), sRad, n, perGroup, R + 0.0, lp,
+                              xDim, yDim, static_cast<int32_t>(wrapX), static_cast<int32_t>(wrapY), vel, velIn);
+                    };
+                    if (sparse)
+                    {
+                        launch([](auto... args) { LaunchChained(args...); });
+                    }
+                    else
+                    {
+                        launch([](auto... args) { LaunchAfter(args...); });
+                    }
                     break;
                 }
                 go(Forces<T, TV, kLawLinear, false, false>);
