@@ -45,25 +45,26 @@ namespace halcuda
         // only then cut at the edge.
         HAL_WINDOW_FN void Set(int32_t xStart, int32_t xEnd, int32_t yStart, int32_t yEnd, int32_t yDim)
         {
-            const int64_t rows = static_cast<int64_t>(xEnd) - xStart;
-            const int64_t cells = static_cast<int64_t>(yEnd) - yStart;
+            // (unsigned: the bounds may be the ends of int32's range)
+            const uint32_t rows = static_cast<uint32_t>(xEnd) - static_cast<uint32_t>(xStart);
+            const uint32_t cells = static_cast<uint32_t>(yEnd) - static_cast<uint32_t>(yStart);
             runs = 0;
             perRow = 1;
             y0 = first = over = 0;
             fits = true;
-            if (rows <= 0 || cells <= 0)
+            if (xEnd <= xStart || yEnd <= yStart)
             {
                 return;
             }
-            if (cells > yDim || rows > (int64_t(1) << 29))
+            if (cells > static_cast<uint32_t>(yDim) || rows > (uint32_t(1) << 29))
             {
                 fits = false;
                 return;
             }
             y0 = WrapIndex(yStart, yDim);
-            first = yDim - y0;
-            first = (cells < first) ? static_cast<int32_t>(cells) : first;
-            over = static_cast<int32_t>(cells) - first;
+            const int32_t n = static_cast<int32_t>(cells), left = yDim - y0;
+            first = (n < left) ? n : left;
+            over = n - first;
             perRow = (over > 0) ? 2 : 1;
             runs = static_cast<int32_t>(rows) * perRow;
         }
