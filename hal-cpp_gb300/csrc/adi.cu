@@ -1707,12 +1707,15 @@ namespace halcuda
         // warp, in CTAs that hold an SM each: always in the y-sweep (2000 x 900 25.4
         // / 20.0), in the x-sweep where the last wave is less than half full (700 x
         // 1250 23.2 / 16.4, 800 x 1300 18.1 / 16.3, 1000 x 4000 30.5 / 27.2; fuller:
-        // 900 x 2000 31.0 / 33.0; shorter lines: 300 x 4000 22.7 / 24.0).
+        // 900 x 2000 31.0 / 33.0; shorter lines: 300 x 4000 22.7 / 24.0).  Wrapped
+        // lines near 1024 go to the tensor-staged sweep already from three quarters
+        // of a wave on, since the correction reads its vector in both (1024^2,
+        // wrapped, 15.2 / 14.3; 768 x 1024 14.2 / 14.3, 640 x 1024 12.1 / 14.3).
         template <int MODE>
         bool UseLines(const SweepParams &p, bool swz)
         {
             const int32_t wave = 2 * kLineFewLines;  // 152 CTAs of eight lines
-            if (p.plan.P > kLineMaxP || (swz && p.Nlines >= wave))
+            if (p.plan.P > kLineMaxP || (swz && (p.Nlines >= wave || (p.plan.periodic && p.plan.P > 24 && 4 * p.Nlines >= 3 * wave))))
             {
                 return false;
             }
