@@ -39,3 +39,15 @@ def test_decay_gradient_many_steps(hal, oracle):
         a.set_problem(f0, target, steps, 10)
         got = a.gradient(D, 0.005, src)[2]
     assert abs(got - ref) <= 1e-6 * abs(ref)
+
+
+def test_forward_and_gradient_sum_the_loss_alike(hal):
+    """The loss of a forward call and of a gradient call are the same bits, also
+    with as many partial sums as there are."""
+    n = 512 * 512
+    rng = np.random.default_rng(7)
+    f0, target = rng.random(n, dtype=np.float32), rng.random(n, dtype=np.float32)
+    D = (0.5 + 4.5 * rng.random(n)).astype(np.float32)
+    with hal.Adjoint(512, 512) as a:
+        a.set_problem(f0, target, 3, 0)
+        assert a.forward(D, 0.005) == a.gradient(D, 0.005)[0]
