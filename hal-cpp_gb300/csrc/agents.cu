@@ -692,10 +692,10 @@ namespace halcuda
         // edge) is bound by its one thread's instructions and goes run by run,
         // without the choice of the run per candidate; a short one keeps the
         // runs joined, where groups cut short at each run's end would cost more.
-        // Measured on GB300, 1M agents in 2048^2, 30% in a cluster, forces and
-        // move, branches per pair / here: cluster inside 38 / 37 us, half
-        // clipped at an edge 93 / 74 us, at a corner 387 / 285 us (groups of
-        // eight in the long walk: 298 us).
+        // Measured on GB300, 1M agents in 2048^2, 30% in a cluster, the force
+        // pass, branches per pair / here: cluster inside 38 / 37 us, clipped at
+        // an edge 66 / 51 us, at a corner 394 / 294 us (groups of eight in the
+        // long walk were 5% slower there).
         __device__ __forceinline__ void WalkRuns32(const int32_t (&rs)[4], const int32_t (&re)[4], int32_t slot,
                                                    float2 pf, float rad, const float2 *__restrict__ sPos,
                                                    const float *__restrict__ sRad, float R, float k, float xDimF,

@@ -160,8 +160,9 @@ int hal_cuda_diffusion_set_uptake(hal_cuda_diffusion *h, hal_cuda_agents *agents
  * library choose: up to 8 ticks of a patch in registers per launch, bit for
  * bit the one-tick results (measured 7.4x faster at 256^2 and 1.9x to 2.4x at
  * 2048^2), and one tick per launch where a run has agent uptake, a point
- * source listed twice in a cell, or a grid smaller than a patch.  1: always
- * one tick per launch.  2: a CTA stages its tile with a 2-cell halo by TMA
+ * source listed twice in a cell, a grid smaller than a patch, or, with y not
+ * wrapped, a boundary value or a source in the outer columns that is not
+ * finite.  1: always one tick per launch.  2: a CTA stages its tile with a 2-cell halo by TMA
  * and computes two ticks in shared memory (slower than both; needs yDim % 4
  * == 0, ENOTSUP otherwise; the dense source and the point sources are added
  * as one pre-summed array, so results match the others to FP32 rounding, not
