@@ -46,7 +46,7 @@
 // (factors, rates, kept states, accumulators) is loaded before the wait for it.
 // A run of steps between checkpoints is replayed from a small CUDA graph.
 // Measured at 512^2, 500 steps, zero-flux: forward 3.2 ms (12.3 ms with the
-// reductions), gradient with checkpoints every 22 steps 8.8 ms (28.8 ms); its
+// reductions), gradient with checkpoints every 22 steps 8.5 ms (28.8 ms); its
 // error against 64 bits is unchanged (1.5e-6 for dL/dD).  What is left per
 // kernel is latency: 1.7 us of it is there on a 64^2 field too.
 //
